@@ -13,11 +13,16 @@ with the reference's message text when the input contract is violated.
 
 All arithmetic happens in ``librwkv7_b200.so`` (hand-written sm_100a CUDA, see
 ``csrc/``); torch only owns device memory and streams here.  There is no CPU
-fallback: importing works without a GPU, calling an operator does not.
+fallback: importing works without a GPU, calling an operator does not.  The operators reach
+the library through ``rwkv7_b200_torch.so`` (``csrc/torch/binding.cpp``), which builds the descriptors and
+allocates the outputs in native code; :func:`lib` and :func:`describe` are the same boundary by ctypes, for
+callers that hold their own descriptors.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 from dataclasses import dataclass
 from typing import Optional, Sequence
@@ -92,6 +97,27 @@ def lib() -> ctypes.CDLL:
         L.rwkv7_wkv7_backward_workspace_bytes.argtypes = [ctypes.c_int64] * 4
         _lib = L
     return _lib
+
+
+BINDING_PATH = os.path.join(_HERE, "rwkv7_b200_torch.so")
+_native = None
+
+
+def native():
+    """The torch binding, opened on :data:`LIB_PATH`; fails loudly when it has not been built."""
+    global _native
+    if _native is None:
+        lib()
+        if not os.path.exists(BINDING_PATH):
+            raise RuntimeError(
+                f"{BINDING_PATH} is missing: build it with `python {os.path.join(_HERE, 'build.py')}`. "
+                "There is no fallback path.")
+        loader = importlib.machinery.ExtensionFileLoader("rwkv7_b200_torch", BINDING_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("rwkv7_b200_torch", loader))
+        loader.exec_module(mod)
+        mod.open(LIB_PATH, KernelInputsError)
+        _native = mod
+    return _native
 
 
 def describe(t: Optional[torch.Tensor], device: Optional[int] = None) -> Optional[Tensor]:
@@ -202,48 +228,12 @@ class Wkv7StatepassForwardOutput:
     next_state: torch.Tensor
 
 
-def _wkv7_workspace(r: torch.Tensor) -> tuple[Optional[torch.Tensor], int]:
-    if r.dim() != 4:
-        return None, 0
-    B, T, H, N = r.shape
-    n = int(lib().rwkv7_wkv7_workspace_bytes(B, T, H, N, _DTYPES.get(r.dtype, 0)))
-    if n == 0:
-        return None, 0
-    return torch.empty(n, dtype=torch.uint8, device=r.device), n
-
-
 def _wkv7_call(inputs: Wkv7PretrainForwardInputs, initial_state, want_state: bool,
                next_state: Optional[torch.Tensor] = None, output: Optional[torch.Tensor] = None,
                workspace: Optional[torch.Tensor] = None):
-    r = inputs.receptance
-    six = [describe(t) for t in inputs.six()]
-    y = torch.empty_like(r) if output is None else output
-    yd = describe(y)
-    if workspace is None:
-        workspace, ws_bytes = _wkv7_workspace(r)
-    else:
-        ws_bytes = workspace.numel() * workspace.element_size()
-    ws_ptr = ctypes.c_void_p(workspace.data_ptr() if workspace is not None else 0)
-    stream = _stream(r)
-    L = lib()
-    cl = ctypes.c_int64(inputs.chunk_len)
-    if initial_state is None:
-        st = L.rwkv7_fused_wkv7_pretrain(*[_ref(d) for d in six], cl, _ref(yd), ws_ptr,
-                                         ctypes.c_size_t(ws_bytes), stream)
-        _check(st)
-        return y, None
-    s0d = describe(initial_state)
-    if not want_state:
-        st = L.rwkv7_fused_wkv7_statetune(_ref(s0d), *[_ref(d) for d in six], cl, _ref(yd), ws_ptr,
-                                          ctypes.c_size_t(ws_bytes), stream)
-        _check(st)
-        return y, None
-    s_out = torch.empty_like(initial_state) if next_state is None else next_state
-    sod = describe(s_out)
-    st = L.rwkv7_fused_wkv7_statepass(_ref(s0d), *[_ref(d) for d in six], cl, _ref(yd), _ref(sod),
-                                      ws_ptr, ctypes.c_size_t(ws_bytes), stream)
-    _check(st)
-    return y, s_out
+    return (_native or native()).wkv7(
+        initial_state, inputs.receptance, inputs.weight_decay, inputs.replacement_key, inputs.value,
+        inputs.removal_key_normalized, inputs.replacement, inputs.chunk_len, want_state, next_state, output, workspace)
 
 
 def wkv7_pretrain_custom(inputs: Wkv7PretrainForwardInputs, *, reference_contract: bool = True,
@@ -311,18 +301,7 @@ def wkv7_forward_saved(inputs: Wkv7PretrainForwardInputs, initial_state: Optiona
                        want_state: bool = False) -> Wkv7SavedForward:
     """``rwkv7_fused_wkv7_forward_saved``: the recurrence plus the tensors the backward pass needs."""
     inputs.check(True)
-    r = inputs.receptance
-    B, T, H, N = r.shape
-    y = torch.empty_like(r)
-    sa = torch.empty_like(r)
-    snaps = torch.empty((B, H, T // inputs.chunk_len, N, N), dtype=torch.float32, device=r.device)
-    s_out = torch.empty((B, H, N, N), dtype=torch.float32, device=r.device) if want_state else None
-    descs = [describe(initial_state)] + [describe(t) for t in inputs.six()]
-    outs = [describe(y), describe(s_out), describe(snaps), describe(sa)]
-    workspace, ws_bytes = _wkv7_workspace(r)
-    ws_ptr = ctypes.c_void_p(workspace.data_ptr() if workspace is not None else 0)
-    _check(lib().rwkv7_fused_wkv7_forward_saved(*[_ref(d) for d in descs], ctypes.c_int64(inputs.chunk_len),
-                                                *[_ref(d) for d in outs], ws_ptr, ctypes.c_size_t(ws_bytes), _stream(r)))
+    y, s_out, snaps, sa = native().wkv7_saved(initial_state, *inputs.six(), inputs.chunk_len, want_state)
     return Wkv7SavedForward(output=y, next_state=s_out, snapshots=snaps, state_replacement=sa)
 
 
@@ -342,26 +321,8 @@ def wkv7_backward(inputs: Wkv7PretrainForwardInputs, saved: Wkv7SavedForward, ou
     gradients in input order, initial_state_grad or None)`` (``Wkv7BackwardPrimitiveOutputs``,
     ``wkv7/backward.rs:567-575``).  ``workspace``: a uint8 tensor of ``wkv7_backward_workspace_bytes``;
     allocated here when omitted."""
-    r = inputs.receptance
-    B, T, H, N = r.shape
-    grads = [torch.empty_like(r) for _ in range(6)]
-    ds0 = torch.empty((B, H, N, N), dtype=torch.float32, device=r.device) if want_state_grad else None
-    gd = [describe(t) for t in grads]
-    arr = (ctypes.POINTER(Tensor) * 6)(*[ctypes.pointer(d) for d in gd])
-    descs = [describe(initial_state)] + [describe(t) for t in inputs.six()] + [describe(saved.snapshots),
-                                                                            describe(saved.state_replacement)]
-    dyd, dsd, ds0d = describe(output_grad.contiguous()), describe(next_state_grad), describe(ds0)
-    if parallel and r.dtype == torch.bfloat16:
-        need = wkv7_backward_workspace_bytes(B, T, H, N)
-        if workspace is None:
-            workspace = torch.empty(max(need, 1), dtype=torch.uint8, device=r.device)
-        _check(lib().rwkv7_fused_wkv7_backward_parallel(
-            *[_ref(d) for d in descs], ctypes.c_int64(inputs.chunk_len), _ref(dyd), _ref(dsd), arr, _ref(ds0d),
-            ctypes.c_void_p(workspace.data_ptr()), ctypes.c_size_t(workspace.numel()), _stream(r)))
-        return grads, ds0
-    _check(lib().rwkv7_fused_wkv7_backward(*[_ref(d) for d in descs], ctypes.c_int64(inputs.chunk_len), _ref(dyd),
-                                           _ref(dsd), arr, _ref(ds0d), _stream(r)))
-    return grads, ds0
+    return native().wkv7_backward(initial_state, *inputs.six(), saved.snapshots, saved.state_replacement,
+                                  inputs.chunk_len, output_grad, next_state_grad, want_state_grad, parallel, workspace)
 
 
 class _Wkv7Function(torch.autograd.Function):
@@ -484,12 +445,8 @@ def wkv7_statepass_noalloc(initial_state: torch.Tensor, sequence: Wkv7PretrainFo
     workspace: the library's own fixed 256 KiB flag array is used instead, which
     limits ``B*H`` to 65536 chains.  Calls on one device must not overlap on the
     GPU, since they share that array.  Nothing is allocated here either: the
-    descriptors are plain ctypes structures on the host."""
-    desc = [describe(initial_state)] + [describe(t) for t in sequence.six()]
-    yd, sd = describe(output), describe(next_state)
-    st = lib().rwkv7_fused_wkv7_statepass_noalloc(*[_ref(d) for d in desc], ctypes.c_int64(sequence.chunk_len),
-                                                  _ref(yd), _ref(sd), _stream(sequence.receptance))
-    _check(st)
+    descriptors live on the host's stack."""
+    native().wkv7_noalloc(initial_state, *sequence.six(), sequence.chunk_len, output, next_state)
     return Wkv7StatepassForwardOutput(output=output, next_state=next_state)
 
 
@@ -503,31 +460,14 @@ MIX6_BRANCHES = ("receptance_input", "weight_decay_input", "key_input", "value_i
                  "learning_rate_input", "gate_input")
 
 
-def _ptr_array(descs: Sequence[Optional[Tensor]]):
-    arr = (ctypes.POINTER(Tensor) * len(descs))()
-    for i, d in enumerate(descs):
-        arr[i] = ctypes.pointer(d) if d is not None else None
-    return arr
-
-
 def mix6_custom(embedded_context: torch.Tensor, receptance_scale, weight_decay_scale, key_scale,
                 value_scale, learning_rate_scale, gate_scale, *, stacked: bool = False):
     """``mix6_custom`` (``mix6/mod.rs:76-108``).  Returns a dict of the six
     ``[B,T,C]`` outputs, or one ``[6,B,T,C]`` tensor when ``stacked``."""
-    x = embedded_context
-    scales = [receptance_scale, weight_decay_scale, key_scale, value_scale, learning_rate_scale, gate_scale]
-    xd = describe(x)
-    sd = [describe(s) for s in scales]
-    L = lib()
+    scales = (receptance_scale, weight_decay_scale, key_scale, value_scale, learning_rate_scale, gate_scale)
     if stacked:
-        out = torch.empty((6,) + tuple(x.shape), dtype=x.dtype, device=x.device)
-        od = describe(out)
-        _check(L.rwkv7_fused_mix6_stacked(_ref(xd), _ptr_array(sd), _ref(od), _stream(x)))
-        return out
-    outs = [torch.empty_like(x) for _ in range(6)]
-    od = [describe(o) for o in outs]
-    _check(L.rwkv7_fused_mix6(_ref(xd), _ptr_array(sd), _ptr_array(od), _stream(x)))
-    return dict(zip(MIX6_BRANCHES, outs))
+        return native().mix6_stacked(embedded_context, *scales)
+    return dict(zip(MIX6_BRANCHES, (_native or native()).mix6(embedded_context, *scales)))
 
 
 mix6 = mix6_custom
@@ -539,22 +479,14 @@ def addcmul_custom(base: torch.Tensor, diff: torch.Tensor, scale: torch.Tensor, 
                    inplace: bool = False) -> torch.Tensor:
     """``addcmul_custom`` (``addcmul/mod.rs:100-105``): ``base + diff * scale``.
     ``inplace`` writes over ``base`` like the reference does for a uniquely owned buffer."""
-    out = base if inplace else torch.empty_like(base)
-    bd, dd, sd, od = describe(base), describe(diff), describe(scale), describe(out)
-    _check(lib().rwkv7_fused_addcmul(_ref(bd), _ref(dd), _ref(sd), _ref(od), _stream(base)))
-    return out
+    return (_native or native()).addcmul(base, diff, scale, inplace)
 
 
 def addcmul5_custom(base: torch.Tensor, diff: torch.Tensor, receptance_scale, weight_decay_scale,
                     key_scale, value_scale, learning_rate_scale):
     """``addcmul5_custom`` (``addcmul/mod.rs:138-157``): five outputs sharing base and diff."""
-    scales = [receptance_scale, weight_decay_scale, key_scale, value_scale, learning_rate_scale]
-    outs = [torch.empty_like(base) for _ in range(5)]
-    bd, dd = describe(base), describe(diff)
-    sd = [describe(s) for s in scales]
-    od = [describe(o) for o in outs]
-    _check(lib().rwkv7_fused_addcmul5(_ref(bd), _ref(dd), _ptr_array(sd), _ptr_array(od), _stream(base)))
-    return dict(zip(MIX6_BRANCHES[:5], outs))
+    return dict(zip(MIX6_BRANCHES, (_native or native()).addcmul5(
+        base, diff, receptance_scale, weight_decay_scale, key_scale, value_scale, learning_rate_scale)))
 
 
 addcmul = addcmul_custom
@@ -577,11 +509,7 @@ def token_shift_diff_custom(embedded_context: torch.Tensor, embedded_token_shift
     """``token_shift_diff_custom`` (``token_shift_diff/mod.rs:82-111``).  The state
     buffer is updated in place by the kernel; unless ``inplace_state`` the caller's
     tensor is cloned first so that the call is functional like the reference's."""
-    state = embedded_token_shift if inplace_state else embedded_token_shift.clone()
-    diff = torch.empty_like(embedded_context)
-    xd, sd, idd, dd = describe(embedded_context), describe(state), describe(batch_ids), describe(diff)
-    _check(lib().rwkv7_fused_token_shift_diff(_ref(xd), _ref(sd), _ref(idd), _ref(dd),
-                                              _stream(embedded_context)))
+    diff, state = (_native or native()).token_shift_diff(embedded_context, embedded_token_shift, batch_ids, inplace_state)
     return TokenShiftDiffForwardOutput(token_shifted_diff=diff, next_token_shift=state)
 
 
@@ -612,18 +540,11 @@ def weight_prepare_epilogue(key_precursor: torch.Tensor, learning_rate_lora: tor
     ``learning_rate_lora``, ``weight_decay_lora`` and ``value_residual_lora`` are the LoRA
     modules' outputs, before the sigmoid / softplus that ``forward`` applies to them; the three value tensors are given for every
     cell but the first (there ``value`` is ``value_precursor`` and is returned as is)."""
-    outs = [torch.empty_like(key_precursor) for _ in range(4)]
-    with_value = value_precursor is not None
-    value = torch.empty_like(key_precursor) if with_value else None
-    descs = [describe(t) for t in (key_precursor, learning_rate_lora, weight_decay_lora, key_removal,
-                                   key_replacement, value_precursor, value_from_first_cell,
-                                   value_residual_lora)]
-    od = [describe(t) for t in outs] + [describe(value)]
-    _check(lib().rwkv7_fused_weight_prepare(*[_ref(d) for d in descs], ctypes.c_int64(num_heads),
-                                            *[_ref(d) for d in od], _stream(key_precursor)))
-    return WeightPrepareEpilogueOutput(weight_decay=outs[0], replacement_key=outs[1],
-                                       value=value if with_value else None,
-                                       removal_key_normalized=outs[2], replacement=outs[3])
+    w, kt, a, b, value = (_native or native()).weight_prepare(
+        key_precursor, learning_rate_lora, weight_decay_lora, key_removal, key_replacement, value_precursor,
+        value_from_first_cell, value_residual_lora, num_heads)
+    return WeightPrepareEpilogueOutput(weight_decay=w, replacement_key=kt, value=value, removal_key_normalized=a,
+                                       replacement=b)
 
 
 def gated_readout_epilogue(wkv7_output: torch.Tensor, receptance: torch.Tensor, replacement_key: torch.Tensor,
@@ -634,33 +555,15 @@ def gated_readout_epilogue(wkv7_output: torch.Tensor, receptance: torch.Tensor, 
     (``gated_readout.rs:123-141``): per-head GroupNorm of the WKV7 output, the
     receptance-key bonus and the gate, in one kernel.  Returns ``[B,T,C]``-shaped
     like ``wkv7_output``; ``gate`` is the gate LoRA's output as it is (``gated_readout.rs:121``)."""
-    out = torch.empty_like(wkv7_output)
-    descs = [describe(t) for t in (wkv7_output, receptance, replacement_key, value, gate, group_norm_gamma,
-                                   group_norm_beta, receptance_key_bonus)]
-    od = describe(out)
-    _check(lib().rwkv7_fused_gated_readout(*[_ref(d) for d in descs], ctypes.c_double(epsilon),
-                                           ctypes.c_int64(num_heads), _ref(od), _stream(wkv7_output)))
-    return out
+    return (_native or native()).gated_readout(wkv7_output, receptance, replacement_key, value, gate, group_norm_gamma,
+                                               group_norm_beta, receptance_key_bonus, num_heads, epsilon)
 
 
 def channel_mixer_custom(embedded_context: torch.Tensor, key_scale: torch.Tensor, key_weight: torch.Tensor,
                          value_weight: torch.Tensor, *, workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``channel_mixer`` (``kernels/train/channel_mixer/mod.rs:130-144``): token-shift mix, key
     projection with relu^2 in its epilogue, value projection; bf16 tensors."""
-    out = torch.empty_like(embedded_context)
-    ws_ptr, ws_bytes = ctypes.c_void_p(0), 0
-    if embedded_context.dim() == 3 and key_weight.dim() == 2:
-        B, T, C = embedded_context.shape
-        ws_bytes = int(lib().rwkv7_channel_mixer_workspace_bytes(B, T, C, key_weight.shape[0]))
-        if workspace is None and ws_bytes:
-            workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=embedded_context.device)
-        if workspace is not None:
-            ws_ptr, ws_bytes = ctypes.c_void_p(workspace.data_ptr()), workspace.numel() * workspace.element_size()
-    descs = [describe(t) for t in (embedded_context, key_scale, key_weight, value_weight)]
-    od = describe(out)
-    _check(lib().rwkv7_fused_channel_mixer(*[_ref(d) for d in descs], _ref(od), ws_ptr, ctypes.c_size_t(ws_bytes),
-                                           _stream(embedded_context)))
-    return out
+    return (_native or native()).channel_mixer(embedded_context, key_scale, key_weight, value_weight, workspace)
 
 
 channel_mixer = channel_mixer_custom
@@ -670,28 +573,14 @@ def lm_head_ce_partial(x: torch.Tensor, weight_shard: torch.Tensor, targets: tor
                        vocab_offset: int = 0) -> torch.Tensor:
     """Per-row ``(max, sumexp, target logit)`` of ``x @ weight_shard.T`` over one
     vocabulary shard, ``[R,3]`` fp32; logits are never materialised."""
-    R = x.shape[0]
-    partials = torch.empty((R, 3), dtype=torch.float32, device=x.device)
-    n = int(lib().rwkv7_lm_head_ce_workspace_bytes(R, x.shape[1], weight_shard.shape[0]))
-    ws = torch.empty(max(n, 1), dtype=torch.uint8, device=x.device)
-    xd, wd, td, pd = describe(x), describe(weight_shard), describe(targets), describe(partials)
-    _check(lib().rwkv7_fused_lm_head_ce_partial(_ref(xd), _ref(wd), _ref(td), ctypes.c_int64(vocab_offset),
-                                                _ref(pd), ctypes.c_void_p(ws.data_ptr()),
-                                                ctypes.c_size_t(n), _stream(x)))
-    return partials
+    return native().lm_head_ce_partial(x, weight_shard, targets, vocab_offset)
 
 
 def lm_head_ce_finalize(partials_all: torch.Tensor, targets: torch.Tensor):
     """Combines ``[num_shards,R,3]`` partials into per-row ``(lse, loss)``."""
-    R = partials_all.shape[1]
-    lse = torch.empty(R, dtype=torch.float32, device=partials_all.device)
-    loss = torch.empty(R, dtype=torch.float32, device=partials_all.device)
-    pd, td, ld, sd = describe(partials_all), describe(targets), describe(lse), describe(loss)
-    _check(lib().rwkv7_lm_head_ce_finalize(_ref(pd), _ref(td), _ref(ld), _ref(sd), _stream(partials_all)))
-    return lse, loss
+    return native().lm_head_ce_finalize(partials_all, targets)
 
 
 def lm_head_ce(x: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor):
     """Single-GPU fused LM-head cross entropy: per-row ``(lse, loss)``."""
-    p = lm_head_ce_partial(x, weight, targets, 0)
-    return lm_head_ce_finalize(p.unsqueeze(0), targets)
+    return (_native or native()).lm_head_ce(x, weight, targets)

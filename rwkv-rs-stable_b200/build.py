@@ -1,8 +1,9 @@
-"""Builds ``librwkv7_b200.so`` (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds ``librwkv7_b200.so`` (the C-ABI library) in-tree with nvcc for sm_100a, and
+``rwkv7_b200_torch.so`` (its binding to torch tensors, a CPython module) with g++.
 
-Run as ``python build.py`` from this directory or call :func:`build_library`.
-Objects go to ``build/`` next to this file; the shared library is written beside
-this file so that it is found by :mod:`ctypes` without installation.
+Run as ``python build.py`` from this directory or call :func:`build_library` and
+:func:`build_binding`.  Objects go to ``build/`` next to this file; the shared objects are written
+beside this file so that they are found without installation.
 """
 from __future__ import annotations
 
@@ -11,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -99,5 +101,42 @@ def build_library(force: bool = False, verbose: bool = False, extra_flags: list[
     return LIB
 
 
+def build_binding(force: bool = False) -> str:
+    """The torch binding; it opens the library when the package does, and links none of it."""
+    src = os.path.join(CSRC, "torch", "binding.cpp")
+    out = os.path.join(HERE, "rwkv7_b200_torch.so")
+    headers = [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
+    if not force and not _newer(out, [src] + headers):
+        return out
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    lib = os.path.join(root, "lib")
+    cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+    includes = [INCLUDE, os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = [cxx, "-std=c++17", "-O2", "-fPIC", "-shared", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[a for i in includes for a in ("-isystem" if i != INCLUDE else "-I", i)], src, "-o", out,
+           "-L", lib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10", "-ldl"]
+    # (the CUDA runtime torch itself has loaded: a second one would not know its streams' device state)
+    cudart = _torch_cudart(root)
+    cmd += [cudart] if cudart else ["-L", os.path.join(cuda, "lib64"), "-lcudart"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + res.stdout + res.stderr)
+        raise RuntimeError("building the torch binding failed")
+    return out
+
+
+def _torch_cudart(root: str) -> str | None:
+    for base in (os.path.join(root, "lib"), os.path.join(os.path.dirname(root), "nvidia", "cuda_runtime", "lib")):
+        if os.path.isdir(base):
+            for f in sorted(os.listdir(base)):
+                if f.startswith("libcudart") and ".so" in f:
+                    return os.path.join(base, f)
+    return None
+
+
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_binding(force="--force" in sys.argv))

@@ -5,8 +5,6 @@
 
 #include <atomic>
 #include <cstdint>
-#include <mutex>
-#include <vector>
 
 #include "check.h"
 #include "kernels.h"
@@ -20,8 +18,7 @@ namespace {
 std::atomic<int> g_wkv7_path{RWKV7_WKV7_AUTO};
 
 constexpr int kMaxDevices = 64;
-std::mutex g_props_mu;
-int g_num_sms[kMaxDevices] = {};
+std::atomic<int> g_num_sms[kMaxDevices] = {};
 
 // Makes `device` current for the duration of a call and restores the caller's.
 class DeviceGuard {
@@ -51,14 +48,13 @@ int cuda_fail(const char *what, int err) {
 int num_sms(int device, int *out) {
     if (device < 0 || device >= kMaxDevices)
         return fail(RWKV7_ERR_BAD_ARGUMENT, "BadArgument: device ordinal %d out of range", device);
-    std::lock_guard<std::mutex> lock(g_props_mu);
-    if (g_num_sms[device] == 0) {
-        int v = 0;
+    int v = g_num_sms[device].load(std::memory_order_relaxed);
+    if (v == 0) {
         cudaError_t e = cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device);
         if (e != cudaSuccess) return cuda_fail("cudaDeviceGetAttribute", (int)e);
-        g_num_sms[device] = v;
+        g_num_sms[device].store(v, std::memory_order_relaxed);
     }
-    *out = g_num_sms[device];
+    *out = v;
     return RWKV7_OK;
 }
 
@@ -84,10 +80,9 @@ int check_wkv7_sequence(const TensorInfo six[6], int64_t chunk_len) {
     RWKV7_TRY(check_axis_non_empty(r, 1));
     RWKV7_TRY(check_axis_non_empty(r, 3));
     RWKV7_TRY(check_axes_equal({{six[0], 0}, {six[1], 0}, {six[2], 0}, {six[3], 0}, {six[4], 0}, {six[5], 0}}));
-    const std::vector<int64_t> expected(r.t->shape, r.t->shape + 4);
-    for (int i = 1; i < 6; ++i) RWKV7_TRY(check_shape(six[i], expected));
-    RWKV7_TRY(check_same_dtype({six[0], six[1], six[2], six[3], six[4], six[5]}));
-    RWKV7_TRY(check_same_device({six[0], six[1], six[2], six[3], six[4], six[5]}));
+    for (int i = 1; i < 6; ++i) RWKV7_TRY(check_shape(six[i], r.t->shape, 4));
+    RWKV7_TRY(check_same_dtype(six, 6));
+    RWKV7_TRY(check_same_device(six, 6));
     for (int i = 0; i < 6; ++i) RWKV7_TRY(check_contiguous(six[i]));
     if (!float_dtype_supported(r.t->dtype))
         return fail(RWKV7_ERR_UNSUPPORTED, "Unsupported: wkv7 computes F32 or BF16 inputs, got %s",
@@ -123,7 +118,7 @@ int wkv7_validate(const rwkv7_tensor *s0, const rwkv7_tensor *const six_t[6], in
     if (has_s0) RWKV7_TRY(check_wkv7_state(TensorInfo{"initial_state", s0}, r));
     const TensorInfo out{"output", y};
     RWKV7_TRY(check_present(out, 4));
-    RWKV7_TRY(check_shape(out, std::vector<int64_t>(r.t->shape, r.t->shape + 4)));
+    RWKV7_TRY(check_shape(out, r.t->shape, 4));
     RWKV7_TRY(check_same_dtype({r, out}));
     RWKV7_TRY(check_same_device({r, out}));
     RWKV7_TRY(check_contiguous(out));
@@ -207,22 +202,22 @@ int wkv7_run(const rwkv7_tensor *s0, const rwkv7_tensor *const six_t[6], int64_t
 // Shared contract of the [1,1,C] scale tensors (mix6/io.rs:48-86, addcmul/io.rs:42-54).
 int check_scales(const TensorInfo &x, const rwkv7_tensor *const *scales, const char *const *names, int n) {
     const int64_t C = x.dim(2);
-    std::vector<TensorInfo> all{x};
+    TensorInfo all[7] = {x};
     for (int s = 0; s < n; ++s) {
-        TensorInfo info{names[s], scales[s]};
+        const TensorInfo info{names[s], scales[s]};
         RWKV7_TRY(check_present(info, 3));
         RWKV7_TRY(check_shape(info, {1, 1, C}));
-        all.push_back(info);
+        all[1 + s] = info;
     }
-    RWKV7_TRY(check_same_dtype(all));
-    RWKV7_TRY(check_same_device(all));
-    for (auto &t : all) RWKV7_TRY(check_contiguous(t));
+    RWKV7_TRY(check_same_dtype(all, 1 + n));
+    RWKV7_TRY(check_same_device(all, 1 + n));
+    for (int s = 0; s < 1 + n; ++s) RWKV7_TRY(check_contiguous(all[s]));
     return RWKV7_OK;
 }
 
 int check_output_like(const TensorInfo &x, const TensorInfo &out) {
     RWKV7_TRY(check_present(out, x.t->ndim));
-    RWKV7_TRY(check_shape(out, std::vector<int64_t>(x.t->shape, x.t->shape + x.t->ndim)));
+    RWKV7_TRY(check_shape(out, x.t->shape, x.t->ndim));
     RWKV7_TRY(check_same_dtype({x, out}));
     RWKV7_TRY(check_same_device({x, out}));
     RWKV7_TRY(check_contiguous(out));
@@ -762,16 +757,16 @@ static int addcmul_run(const rwkv7_tensor *base_t, const rwkv7_tensor *diff_t,
     RWKV7_TRY(check_axis_non_empty(base, 2));
     RWKV7_TRY(check_same_shape({base, diff}));
     const int64_t C = base.dim(2);
-    std::vector<TensorInfo> all{base, diff};
+    TensorInfo all[7] = {base, diff};
     for (int s = 0; s < n; ++s) {
-        TensorInfo info{scale_names[s], scales[s]};
+        const TensorInfo info{scale_names[s], scales[s]};
         RWKV7_TRY(check_present(info, 3));
         RWKV7_TRY(check_shape(info, {1, 1, C}));
-        all.push_back(info);
+        all[2 + s] = info;
     }
-    RWKV7_TRY(check_same_dtype(all));
-    RWKV7_TRY(check_same_device(all));
-    for (auto &t : all) RWKV7_TRY(check_contiguous(t));
+    RWKV7_TRY(check_same_dtype(all, 2 + n));
+    RWKV7_TRY(check_same_device(all, 2 + n));
+    for (int s = 0; s < 2 + n; ++s) RWKV7_TRY(check_contiguous(all[s]));
     if (!float_dtype_supported(base_t->dtype))
         return fail(RWKV7_ERR_UNSUPPORTED, "Unsupported: addcmul computes F32 or BF16, got %s", dtype_name(base_t->dtype));
     AddcmulArgs p{};

@@ -81,42 +81,40 @@ int check_axis_non_empty(const TensorInfo &x, int axis) {
     return RWKV7_OK;
 }
 
-int check_axes_equal(const std::vector<std::pair<TensorInfo, int>> &axes) {
-    if (axes.empty()) return RWKV7_OK;
-    const auto &ref = axes[0];
+int check_axes_equal(std::initializer_list<std::pair<TensorInfo, int>> axes) {
+    if (axes.size() == 0) return RWKV7_OK;
+    const auto &ref = *axes.begin();
     const int64_t ref_dim = ref.first.dim(ref.second);
-    for (size_t i = 1; i < axes.size(); ++i) {
-        const int64_t d = axes[i].first.dim(axes[i].second);
+    for (const auto &x : axes) {
+        const int64_t d = x.first.dim(x.second);
         if (d != ref_dim)
             return fail(RWKV7_ERR_AXIS_MISMATCH,
                         "AxisMismatch: kernel input axis mismatch: %s[%d]=%lld != %s[%d]=%lld",
-                        ref.first.name, ref.second, (long long)ref_dim, axes[i].first.name,
-                        axes[i].second, (long long)d);
+                        ref.first.name, ref.second, (long long)ref_dim, x.first.name,
+                        x.second, (long long)d);
     }
     return RWKV7_OK;
 }
 
-int check_shape(const TensorInfo &x, const std::vector<int64_t> &expected) {
-    bool same = (int)expected.size() == x.t->ndim;
+int check_shape(const TensorInfo &x, const int64_t *expected, int ndim) {
+    bool same = ndim == x.t->ndim;
     for (int i = 0; same && i < x.t->ndim; ++i) same = x.t->shape[i] == expected[i];
     if (!same)
         return fail(RWKV7_ERR_SHAPE_MISMATCH,
                     "ShapeMismatch: kernel input shape mismatch for %s: expected=%s, actual=%s", x.name,
-                    shape_string(expected.data(), (int)expected.size()).c_str(),
+                    shape_string(expected, ndim).c_str(),
                     shape_string(x.t->shape, x.t->ndim).c_str());
     return RWKV7_OK;
 }
 
-int check_same_shape(const std::vector<TensorInfo> &xs) {
-    if (xs.empty()) return RWKV7_OK;
-    std::vector<int64_t> expected(xs[0].t->shape, xs[0].t->shape + xs[0].t->ndim);
-    for (size_t i = 1; i < xs.size(); ++i)
-        if (int st = check_shape(xs[i], expected)) return st;
+int check_same_shape(std::initializer_list<TensorInfo> xs) {
+    for (const TensorInfo &x : xs)
+        if (int st = check_shape(x, xs.begin()->t->shape, xs.begin()->t->ndim)) return st;
     return RWKV7_OK;
 }
 
-int check_same_dtype(const std::vector<TensorInfo> &xs) {
-    for (size_t i = 1; i < xs.size(); ++i)
+int check_same_dtype(const TensorInfo *xs, size_t n) {
+    for (size_t i = 1; i < n; ++i)
         if (xs[i].t->dtype != xs[0].t->dtype)
             return fail(RWKV7_ERR_DTYPE_MISMATCH,
                         "DTypeMismatch: kernel input dtype mismatch: %s=%s, %s=%s", xs[0].name,
@@ -124,8 +122,8 @@ int check_same_dtype(const std::vector<TensorInfo> &xs) {
     return RWKV7_OK;
 }
 
-int check_same_device(const std::vector<TensorInfo> &xs) {
-    for (size_t i = 1; i < xs.size(); ++i)
+int check_same_device(const TensorInfo *xs, size_t n) {
+    for (size_t i = 1; i < n; ++i)
         if (xs[i].t->device != xs[0].t->device)
             return fail(RWKV7_ERR_DEVICE_MISMATCH,
                         "DeviceMismatch: kernel input device mismatch: %s=Cuda(%d), %s=Cuda(%d)",

@@ -5,8 +5,9 @@
 
 #include <cstdarg>
 #include <cstdint>
+#include <initializer_list>
 #include <string>
-#include <vector>
+#include <utility>
 
 #include "rwkv7_b200.h"
 
@@ -33,15 +34,22 @@ int check_present(const TensorInfo &x, int ndim);
 // check.rs:166-178
 int check_axis_non_empty(const TensorInfo &x, int axis);
 // check.rs:115-138: every listed (tensor, axis) must equal the first.
-int check_axes_equal(const std::vector<std::pair<TensorInfo, int>> &axes);
+// (Lists and plain ranges: a call that passes its checks touches no heap.  The vectors these took cost a decode-sized
+// call about a microsecond.)
+int check_axes_equal(std::initializer_list<std::pair<TensorInfo, int>> axes);
 // check.rs:140-164
-int check_shape(const TensorInfo &x, const std::vector<int64_t> &expected);
+int check_shape(const TensorInfo &x, const int64_t *expected, int ndim);
+inline int check_shape(const TensorInfo &x, std::initializer_list<int64_t> expected) {
+    return check_shape(x, expected.begin(), (int)expected.size());
+}
 // check.rs:180-200 (expected = the first tensor's shape)
-int check_same_shape(const std::vector<TensorInfo> &xs);
+int check_same_shape(std::initializer_list<TensorInfo> xs);
 // check.rs:202-222
-int check_same_dtype(const std::vector<TensorInfo> &xs);
+int check_same_dtype(const TensorInfo *xs, size_t n);
+inline int check_same_dtype(std::initializer_list<TensorInfo> xs) { return check_same_dtype(xs.begin(), xs.size()); }
 // check.rs:224-244
-int check_same_device(const std::vector<TensorInfo> &xs);
+int check_same_device(const TensorInfo *xs, size_t n);
+inline int check_same_device(std::initializer_list<TensorInfo> xs) { return check_same_device(xs.begin(), xs.size()); }
 // The CubeBackend impls assert is_contiguous() (wkv7/mod.rs:56-76).
 int check_contiguous(const TensorInfo &x);
 
