@@ -92,11 +92,12 @@ typedef struct rwkv7_tensor {
 
 /* Which kernel the WKV7 entry points dispatch to.  AUTO picks the decode sweep for T <= 4; for N == 64 and
  * BF16 or F32 tensors the two-kernel tensor-core prefill (SPLIT: per-chunk operators in fp16, then one scan per
- * chain) from 512 tokens on when the workspace holds at least one chunk of operators per chain; for BF16 tensors
- * otherwise the fused tf32 chunked kernel (CHUNKED) from 64 tokens on; the sequential kernel for everything else
+ * chain) from 64 tokens (BF16) or 512 (F32) on when the workspace holds at least one chunk of operators per chain;
+ * for BF16 tensors otherwise the fused tf32 chunked kernel (CHUNKED) from 64 tokens on; the sequential kernel for everything else
  * (F32 tensors under 512 tokens, other head sizes).  Chains that the fp16 operators of SPLIT cannot resolve (a
- * chunk's log-decay beyond 18 in some channel, or a non-finite operator) are recomputed by CHUNKED (BF16 tensors),
- * and chains beyond its range (80), or flagged chains of F32 tensors, by SEQUENTIAL, inside the same call; a final
+ * log-decay beyond 12 in 16 tokens in some channel; beyond 18 in 64 tokens when the path is selected explicitly) are
+ * recomputed by CHUNKED (BF16 tensors), and chains beyond its range (80), or flagged chains of F32 tensors, by
+ * SEQUENTIAL, inside the same call; under 512 tokens, and where a value overflows fp16, token by token by the scan; a final
  * state that aliases the initial state is only written once a chain's result is final. */
 typedef enum rwkv7_wkv7_path {
     RWKV7_WKV7_AUTO = 0,
@@ -177,7 +178,7 @@ int rwkv7_selftest_bounded_wait(int device, int64_t max_polls, rwkv7_stream stre
  */
 
 /* Scratch bytes the WKV7 entry points prefer for this shape (0 for the sequential and decode kernels; B*H*4
- * for the tf32 chunked kernel; for the two-kernel prefill the flags, 1024 work counters, a carried state per
+ * for the tf32 chunked kernel; for the two-kernel prefill the flags, a carried state per
  * chain and 32.5 KB per 64-token chunk of a segment of the call, at most 768 MB of operators).  A smaller
  * workspace is accepted: the call is cut into more segments, and below one chunk per chain the tf32 kernel
  * (BF16 tensors) or the sequential scan runs instead.  The size depends on the SM count of the calling thread's

@@ -60,8 +60,14 @@ int num_sms(int device, int *out) {
 
 bool float_dtype_supported(int32_t dt) { return dt == RWKV7_F32 || dt == RWKV7_BF16; }
 
-// Shortest sequence the automatic choice gives to the two-kernel prefill.
-constexpr int64_t kSplitMinTokens = 512;
+// Shortest sequences the automatic choice gives to the two-kernel prefill.  bf16: one chunk; up to kSplitTiersTokens the scan
+// recomputes a flagged chain itself (token by token), so that a short call is two launches, beyond that the chain goes
+// through the tf32 chunked kernel, which is faster from about there.  fp32: the scan's fp16 operands are less precise
+// than the sequential kernel, which short sequences therefore keep.
+constexpr int64_t kSplitMinTokens = 64;
+constexpr int64_t kSplitTiersTokens = 512;
+constexpr int64_t kSplitMinTokensF32 = 512;
+int64_t split_min_tokens(bool bf16) { return bf16 ? kSplitMinTokens : kSplitMinTokensF32; }
 
 #define RWKV7_TRY(expr)                 \
     do {                                \
@@ -158,9 +164,11 @@ int wkv7_dispatch(Wkv7Args &p, void *workspace, size_t workspace_bytes, rwkv7_st
         return fail(RWKV7_ERR_WORKSPACE_TOO_SMALL, "WorkspaceTooSmall: wkv7 needs %zu workspace bytes, got %zu",
                     wkv7_split_min_workspace_bytes(p.B, p.T, p.H, p.N), workspace == nullptr ? (size_t)0 : workspace_bytes);
     }
-    if (path == RWKV7_WKV7_SPLIT || (path == RWKV7_WKV7_AUTO && split_fits && p.T >= kSplitMinTokens)) {
-        if (int e = launch_wkv7_split(p, workspace, workspace_bytes, (cudaStream_t)stream))
+    if (path == RWKV7_WKV7_SPLIT || (path == RWKV7_WKV7_AUTO && split_fits && p.T >= split_min_tokens(p.bf16))) {
+        const bool own_tier = path == RWKV7_WKV7_AUTO && p.T < kSplitTiersTokens;
+        if (int e = launch_wkv7_split(p, workspace, workspace_bytes, path == RWKV7_WKV7_AUTO, own_tier, (cudaStream_t)stream))
             return cuda_fail("wkv7 split launch", e);
+        if (own_tier) return RWKV7_OK;
         // (the tf32 chunked kernel reads bf16 tiles: flagged chains of fp32 tensors go straight to the sequential scan)
         if (int e = p.bf16 ? launch_wkv7_chunked_flagged(p, workspace, (cudaStream_t)stream)
                            : launch_wkv7_sequential_flagged(p, static_cast<const int *>(workspace), (cudaStream_t)stream))
@@ -330,7 +338,7 @@ int rwkv7_selftest_bounded_wait(int device, int64_t max_polls, rwkv7_stream stre
 size_t rwkv7_wkv7_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int32_t dtype) {
     const int path = g_wkv7_path.load();
     if (path == RWKV7_WKV7_SEQUENTIAL) return 0;
-    if ((path == RWKV7_WKV7_SPLIT || (path == RWKV7_WKV7_AUTO && T >= kSplitMinTokens)) &&
+    if ((path == RWKV7_WKV7_SPLIT || (path == RWKV7_WKV7_AUTO && T >= split_min_tokens(dtype == RWKV7_BF16))) &&
         (dtype == RWKV7_BF16 || dtype == RWKV7_F32) && N == 64)
     {
         // (the size depends on whether the scan will overlap the operator kernel, i.e. on the SM count of

@@ -84,7 +84,10 @@ int wkv7_split_overlap();
 void wkv7_set_split_overlap(int on);
 size_t wkv7_split_min_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t N);
 bool wkv7_split_supported(const Wkv7Args &p);
-int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes, cudaStream_t stream);
+// `wide_range`: decays up to e^-12 per 16 tokens instead of e^-18 per 64.  `resolve_flagged`: the scan itself
+// recomputes flagged chains token by token (short sequences); no flag is left for the caller then.
+int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes, bool wide_range, bool resolve_flagged,
+                      cudaStream_t stream);
 // The flagged chains only, by the tf32 chunked kernel (one CTA per chain), then by the sequential scan
 // for those that are still flagged afterwards.
 int launch_wkv7_chunked_flagged(const Wkv7Args &p, void *workspace, cudaStream_t stream);

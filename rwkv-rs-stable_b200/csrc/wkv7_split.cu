@@ -1,36 +1,38 @@
 // Two-kernel WKV7 prefill for sm_100a (N == 64, bf16 or fp32 tensors, 64-token chunks, fp16 tensor-core
 // operands): everything that does not depend on the running state is computed for all chunks in
 // parallel by `wkv7_chunk_operator_kernel`, which folds a chunk into one linear operator, and
-// `wkv7_state_scan_kernel` then walks each (b,h) chain with one dependent tensor-core product per
-// chunk.
+// `wkv7_state_scan_kernel` then walks each (b,h) chain chunk by chunk.
 //
 // Reference semantics: crates/rwkv-nn/src/kernels/train/time_mixer/wkv7/mod.rs:179-242 (token
 // recurrence; the reference kernel, kernel.rs:82-195, scans token by token).
 //
-// Per chain and chunk, with the in-chunk inclusive prefix c_t of the log-decay l_t = -exp(w_t),
-// c_L its value at the chunk's end and the reference point m = c_L / 2 (per channel):
-//     At = a_t e^{c_{t-1} - m}   Rt = r_t e^{c_t - m}   Bh = b_t e^{m - c_t}   Kh = k_t e^{m - c_t}
-//     G  = [At;Rt] [Bh;Kh]^T  ->  A_ab, A_ak (strictly lower), A_rb, A_rk (lower)
-//     T  = (I - A_ab)^-1                                   (fp32, CUDA cores, blocked)
-//     [A~ | A~k] = T [At e^{m} | A_ak]                     (u_t = S_{t-1} a_t = A~ S^T + A~k V)
-//     P  = A~^T Bh     Kt = Kh + A~k^T Bh     W = R + A_rb A~     Ark = A_rk + A_rb A~k
+// Per chain and chunk, with the in-chunk inclusive prefix c_t of the log-decay l_t = -exp(w_t) and its value c_L at
+// the chunk's end:
+//     A_ab[t][s] = sum_n a_t[n] b_s[n] e^{c_{t-1}[n] - c_s[n]}  (s < t), A_ak likewise with k_s,
+//     A_rb[t][s] = sum_n r_t[n] b_s[n] e^{c_t[n] - c_s[n]}      (s <= t), A_rk likewise with k_s
+//     [A~ | A~k] = (I - A_ab)^-1 [a_t e^{c_{t-1}} | A_ak]       (u_t = S_{t-1} a_t = A~ S^T + A~k V)
+//     Be_s = b_s e^{c_L - c_s}, Ke_s = k_s e^{c_L - c_s}
+//     P  = A~^T Be     Kt = Ke + A~k^T Be     W = r_t e^{c_t} + A_rb A~     Ark = A_rk + A_rb A~k
 // so that, for the state S[i][j] entering the chunk and V[s][i]:
-//     S'[i][j'] = e^{c_L} S[i][j'] + e^{c_L - m} ( sum_j S[i][j] P[j][j'] + sum_s V[s][i] Kt[s][j'] )
+//     S'[i][j'] = e^{c_L} S[i][j'] + sum_j S[i][j] P[j][j'] + sum_s V[s][i] Kt[s][j']
 //     y[t][i]   = sum_j W[t][j] S[i][j] + sum_s Ark[t][s] V[s][i].
-// The operator of a chunk is the 128 x 128 fp16 matrix O[k][n], k = (j | s), n = (j' | t):
-//     O = [[P, W^T], [Kt, Ark^T]],
-// stored in global memory exactly as its shared-memory image (two 128-row panels of 128 bytes,
-// 128-byte swizzle), together with the two fp32 vectors e^{c_L} and e^{c_L - m}.
 //
-// Every tensor-core operand is fp16 (the same 11-bit significand as tf32).  fp16 has a narrow
-// exponent range, which is why the decay factors are taken relative to the middle of the chunk;
-// a chunk whose total log-decay exceeds kMaxLogDecay in any channel, or whose operator holds a
-// non-finite value, flags its chain, and flagged chains are recomputed by the next kernel in line
-// (the launcher passes them to the tf32 chunked kernel or the sequential scan).
+// Every tensor-core operand is fp16 (the same 11-bit significand as tf32) and every product runs on warp-level
+// matrix instructions (see sm100_mma.cuh for why not tcgen05).  fp16 has a narrow exponent range, and the factors of the
+// four A matrices, e^{c_t} and e^{-c_s}, do not.  A chunk whose decay exceeds what the references below resolve is marked
+// and its chain flagged; non-finite values (keys or values beyond fp16) are detected in the scan.
 //
-// Shared-memory operand tiles are [rows][64] 16-bit panels with 128-byte rows, 16-byte chunks
-// XOR-ed with (row & 7).  The same tile serves as a K-major operand (rows = M/N index) and as an
-// MN-major operand (rows = K index): no transposed copies exist anywhere.
+// References.  The factor e^{c_t - c_s} of an A matrix is split between its two operands at a reference point, per
+// channel, chosen as e^{c_L} times a power of two.  Then
+//   - b and k operands differ from Be and Ke by powers of two only, so one tile serves the A matrices and P, Kt;
+//   - the a and r operands carry the factor 1/fx, fx[j] = e^{c_L} 2^..., which is the same for everything in column j of
+//     A~ and R: the operator's rows P[j][.] and W[.][j] are stored divided by fx[j], and the scan multiplies the state
+//     by fx[j] in fp32 before it rounds it to fp16.
+// Where the decay of both halves of the chunk is mild (kMildDecay) one point near the middle serves all blocks and every
+// power of two is the same per channel (it is applied in the scan too).  Otherwise each 16-token block has points of its
+// own at its two ends, so that no factor exceeds 2, and the power of two of a pair of blocks is multiplied into one of the
+// fp16 operands on its way into the matrix instruction, which is exact.  That resolves decays of e^-12 per block
+// (kBlockDecay); the model's range (w < -0.5, weight_prepare.rs:272-274) ends at e^-9.7.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -43,6 +45,7 @@
 #include <type_traits>
 
 #include "kernels.h"
+#include "sm100_mma.cuh"
 #include "sm100_umma.cuh"
 #include "trace.h"
 
@@ -56,562 +59,654 @@ using namespace sm100;
 
 constexpr int kN = 64;
 constexpr int kL = 64;
-// |c_L| per chunk and channel up to which fp16 operands keep their precision (the small factor
-// e^{-|c_L|/2} times a typical vector entry stays a normal fp16 number).  Whether the large factor
-// e^{+|c_L|/2} overflows depends on the data (keys and receptances of magnitude 5 overflow from about
-// |c_L| = 17); overflow is not predicted but detected: it turns the chunk's operator non-finite, the
-// scan sees that in its outputs and flags the chain.
-constexpr float kMaxLogDecay = 18.f;
-constexpr float kOpScale = 4.f;          // decay-scaled operands are stored times 4: centres fp16's range
-constexpr float kInvOpScale = 1.f / kOpScale;
-constexpr uint32_t kPanel = 8192;        // one [64][64] 16-bit tile
-constexpr uint32_t kOperatorBytes = 4 * kPanel;   // O: 128 x 128 fp16
-constexpr uint32_t kVecFloats = 128;              // e^{c_L}[64], e^{c_L - m}[64]
+constexpr float kMildDecay = 9.118820e-4f;    // e^-7: both halves of the chunk at or above it take one reference point
+                                              // (factors up to 2200: room for entries of 29 and, below, down to 6e-2)
+constexpr float kBlockDecay = 6.144212e-6f;   // e^-12: a block below it (or a NaN) marks the chunk
+constexpr float kNarrowDecay = 1.522998e-8f;  // e^-18: least decay over a chunk when the wide range is switched off
+constexpr int kWideShift = 6;                 // block-wise references: operands are stored times 2^6, because there the
+constexpr float kWideScale = 64.f;            // factors reach down to e^-12 and a typical entry has to stay a normal number
+constexpr uint32_t kPanel = 8192;             // one [64][64] 16-bit tile, 128-byte rows, 16-byte pieces XOR-ed with (row & 7)
+constexpr uint32_t kBlk = 512;                // one 16 x 16 fp16 block: two halves of 8 columns, each [16 rows][16 bytes]
 
-// Byte offset of element (row, col) in a [rows][64] 16-bit panel.
+// What the builder leaves of a chunk in global memory: the 128 x 128 fp16 operator O[n][k], n = (j' | t), as the core
+// matrices (eight rows n, eight k, 128 bytes) of a K-major tcgen05 operand without swizzle, 16 of them along k and 16 along n.
+// The contraction index (64 j, then 64 s) is ordered so that a lane of the builder holds four neighbouring k of a row in its
+// accumulators: the eight of core 4 c + q are {2q, 2q+1, 2q+8, 2q+9} of the 16-block 2 c, then the same of 2 c + 1.  Behind
+// the operator e^{c_L}[64] in fp32, two signed exponents per channel (fx = e^{c_L} 2^ef; P and Kt are stored times 2^eg), and
+// the mark.
+constexpr uint32_t kOperatorBytes = 4 * kPanel;
+constexpr uint32_t kDecayAt = kOperatorBytes, kExpAt = kDecayAt + 256;
+constexpr uint32_t kVectorBytes = 256 + 128;
+constexpr uint32_t kMarkAt = kDecayAt + kVectorBytes;   // int: the chunk is beyond what fp16 operands resolve
+constexpr size_t kRecord = 33280;                        // bytes per chunk in the workspace
+__host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
+
 __device__ __forceinline__ uint32_t off16(int row, int col) {
     return (uint32_t)row * 128u + ((((uint32_t)col >> 3) ^ ((uint32_t)row & 7u)) << 4) + ((uint32_t)col & 7u) * 2u;
-}
-// Descriptors.  K-major: rows = M/N index, one K-step (16 elements) is 32 bytes along the row.
-// MN-major: rows = K index, one K-step is 16 rows (2048 bytes); `lbo` is the distance between
-// consecutive 64-element blocks of the M/N index.
-__device__ __forceinline__ uint64_t dK(uint32_t addr, int ks) { return make_smem_desc(addr + (uint32_t)ks * 32u, 16u, 1024u); }
-__device__ __forceinline__ uint64_t dMN(uint32_t addr, uint32_t lbo, int ks) {
-    return make_smem_desc(addr + (uint32_t)ks * 2048u, lbo, 1024u);
-}
-__host__ __device__ constexpr uint32_t idesc16(int M, int N, bool a_mn, bool b_mn) {
-    return make_idesc(kFmtF16, M, N, a_mn, b_mn);
-}
-
-__device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t *>(&h);
-}
-__device__ __forceinline__ float2 unpack_h2(uint32_t u) {
-    return __half22float2(*reinterpret_cast<const __half2 *>(&u));
 }
 __device__ __forceinline__ float2 unpack_bf2(uint32_t u) {
     return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
 }
 
+// Lane addresses of ldmatrix.x4 for a 16 x 16 block, as byte offsets.  In a swizzled tile the block starts at (row0,
+// column 16 c); in a compact block the rows are 16 bytes and the halves 256.  "plain" gives A order; "cols" swaps the
+// two middle matrices: B order for a block stored [column][k], and, with .trans, A order of the transposed block.
+__device__ __forceinline__ uint32_t tile_plain(int lane, int row0, int c) {
+    const int r = row0 + (lane & 15), ch = 2 * c + (lane >> 4);
+    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
+}
+__device__ __forceinline__ uint32_t tile_cols(int lane, int row0, int c) {
+    const int r = row0 + (lane & 7) + ((lane >> 4) << 3), ch = 2 * c + ((lane >> 3) & 1);
+    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
+}
+__device__ __forceinline__ uint32_t blk_plain(int lane) { return (uint32_t)lane * 16u; }
+__device__ __forceinline__ uint32_t blk_cols(int lane) {
+    return (uint32_t)((lane >> 3) & 1) * 256u + (uint32_t)((lane & 7) + ((lane >> 4) << 3)) * 16u;
+}
+
+// Bounded wait for a whole warp without compiler-made divergence handling around the loop.
+__device__ __forceinline__ bool mbar_wait_tight(uint64_t *bar, uint32_t parity, uint32_t limit) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, r;\n\t.reg .u32 n;\n\t"
+        "mov.u32 n, %3;\n"
+        "POLL_%=:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE_%=;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 r, n, 0;\n\t"
+        "@r bra POLL_%=;\n"
+        "DONE_%=:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(limit)
+        : "memory");
+    return ok != 0;
+}
+
 // ------------------------------------------------------------------------------------------
-// Kernel 1: the operator of every chunk.  One CTA of 256 threads works through chunks
-// blockIdx.x, blockIdx.x + gridDim.x, ...; two CTAs share an SM.
+// Kernel 1: the operator of every chunk.  One CTA of four warps per chunk at a time, four CTAs per SM.
+//
+// Bound by shared-memory bandwidth (2.8 k cycles per chunk at one 128-byte access a cycle) and by the latency of a chunk's
+// phases, which the CTAs of an SM cover for one another; hence few warps per chunk, each with the largest tile its
+// registers hold (eight warps per chunk read a quarter more and were slower).  Per chunk:
+//   1. decays: warp = 16-token block, lane = channel pair; prefix and suffix products within the block
+//   2. scaled fp16 operands, in place over the bf16 tiles that TMA delivered
+//   3. the A matrices: one 128 x 128 tcgen05 product [a; r] [b; k]^T, read back a row per thread, lower triangle only; with
+//      block-wise references on warp-level instructions, warp = one of A_ab, A_ak, A_rb, A_rk
+//   4. two warps: inverses of the four diagonal blocks I - A_bb in fp32 (forward substitution, a column per lane)
+//   5. warp = 16 columns j and 16 columns s of [A~ | A~k]: block forward substitution on the transposed system, where
+//      these columns are independent of all others, then every operator row from the same registers, and out.
+// The next chunk's tiles are brought into L2 meanwhile and requested behind phase 5, w first.
 // ------------------------------------------------------------------------------------------
-constexpr int kThreads1 = 256;
-// shared-memory map (bytes from a 1024-aligned base)
-constexpr uint32_t kRaw = 0;                       // five bf16 tiles r, w, k, a, b (40 KB); later scratch
-constexpr uint32_t kRawBytes = 5 * kPanel;
-constexpr int kPitchF = 36;                        // floats per row of the fp32 scratch matrices (a row's own 32-block)
-constexpr uint32_t kAm = kRaw;                     // fp32 diagonal 32 x 32 blocks of A_ab [64][36]
-constexpr uint32_t kTm = kAm + 64 * kPitchF * 4;   // fp32 their inverses           [64][36]
-constexpr uint32_t kWm = kTm + 64 * kPitchF * 4;   // fp32 join scratch [32][20]
-constexpr uint32_t kT16 = kRaw + 24 * 1024;        // fp16 T [t][u]
-constexpr uint32_t kW2 = kT16 + kPanel;            // fp16 A10 T00 [s][c], 32 rows
-constexpr uint32_t kRtrue = kRaw + kRawBytes;      // fp16 r_t e^{c_t} [t][j]
-constexpr uint32_t kAR = kRtrue + kPanel;          // fp16 [At; Rt] (Rt's half later holds A_ak)
-constexpr uint32_t kAf = kAR;                      // fp16 [A~ e^m | A~k]^T [c][t], 128 rows: replaces [At | A_ak] once it has been read
-constexpr uint32_t kArb = kAR + 2 * kPanel;        // fp16 A_rb [t][s]
-constexpr uint32_t kArk = kArb + kPanel;           // fp16 A_rk [t][s]
-constexpr uint32_t kStage = kAR;                   // the finished operator (32 KB) over AR, A_rb, A_rk
-constexpr uint32_t kBK = kArk + kPanel;            // fp16 [Bh; Kh]
-constexpr uint32_t kI64 = kBK + 2 * kPanel;        // fp16 identity [64][64]
-constexpr uint32_t kMisc1 = kI64 + kPanel;         // barriers, group sums, e^m
-constexpr uint32_t kSmem1 = kMisc1 + 3072 + 1024;  // + alignment slack
-static_assert(kWm + 32 * 20 * 4 <= kT16, "inverse scratch runs into the fp16 tile of T");
-static_assert(kW2 + kPanel / 2 <= kRaw + kRawBytes, "scratch exceeds the raw-tile region");
-static_assert(kStage + kOperatorBytes == kBK, "operator staging must cover AR, A_rb, A_rk exactly");
-static_assert(2 * (kSmem1 + 1024) <= 232448, "two CTAs per SM");
-constexpr uint32_t kSmem1F32 = kSmem1 + kRawBytes;   // fp32 tensors: raw tiles of 16 KB, one CTA per SM
-static_assert(kSmem1F32 + 1024 <= 232448, "the fp32 variant must fit an SM");
+constexpr int kOpThreads = 128;
+enum { XA = 0, XR = 1, XB = 2, XK = 3, XW = 4 };
+constexpr uint32_t kTiles = 0;                        // a, r, b, k, w; w's place is part of the next region
+// Compact lower triangles.  A_ab: six blocks below the diagonal, then the diagonal in fp32 (4 x [16][16]), each block
+// replaced by its fp16 inverse; A_ak, A_rb, A_rk: ten blocks each.
+constexpr uint32_t kAab = kTiles + 4 * kPanel;
+constexpr uint32_t kDiag = kAab + 6 * kBlk;
+constexpr uint32_t kAak = kDiag + 4 * 1024;
+constexpr uint32_t kArb = kAak + 10 * kBlk;
+constexpr uint32_t kArk = kArb + 10 * kBlk;
+constexpr uint32_t kE = kArk;                         // block decays [4][64] (dead before A_rk is written; beyond w's tile)
+constexpr uint32_t kPow = kArk + 10 * kBlk;           // exponents of powers of two (block-wise references): 19 x [64] bytes
+constexpr uint32_t kBar1 = kPow + 19 * 64;
+constexpr uint32_t kSmem1 = kBar1 + 64;
+static_assert(kE >= kTiles + 5 * kPanel, "the decays must not lie under w's tile");
+static_assert(4 * (kSmem1 + 1024) <= 233472, "four CTAs per SM");
+__host__ __device__ constexpr int below(int t) { return t * (t - 1) / 2; }   // first block of row t of A_ab
+// kPow rows: the a/r side and the b/k side of a diagonal block, block pairs (2,0) (3,0) (3,1), then per block what takes
+// an a/r operand to the scale of its column of A~ (PX) and a b/k operand to Be, Ke (PE).
+enum { PA = 0, PB = 4, PF = 8, PX = 11, PE = 15 };
 
 struct OperatorMaps {
-    CUtensorMap m[5];   // r, w, k, a, b as [B*T, H*N] (bf16 or fp32), box 64 x 64, no swizzle
+    CUtensorMap m[5];   // a, r, b, k, w as [B*T, H*N] bf16, box 64 x 64, 128-byte swizzle (bf16 tensors only)
 };
-enum { XR = 0, XW = 1, XK = 2, XA = 3, XB = 4 };
+struct OperatorPtrs {
+    const void *p[5];   // the same tensors
+};
+
+// d = exp(-exp(w)) of a channel pair
+// (subnormal results flushed: without that every exponential costs a compare and two more multiplications)
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float2 decay2(float2 w) {
+    constexpr float kLog2e = 1.4426950408889634f;
+    const float2 x = mul2(w, make_float2(kLog2e, kLog2e));
+    const float2 z = mul2(make_float2(ex2(x.x), ex2(x.y)), make_float2(-kLog2e, -kLog2e));
+    return make_float2(ex2(z.x), ex2(z.y));
+}
+__device__ __forceinline__ uint32_t pack2(float2 v) { return pack_half2(v.x, v.y); }
+__device__ __forceinline__ int exponent_of(float v) { return (int)(__float_as_uint(v) >> 23); }   // biased; v > 0
+__device__ __forceinline__ float exp2_of(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }   // -126 <= e <= 127
+__device__ __forceinline__ int lds_s8(uint32_t addr) {
+    int v;
+    asm volatile("ld.shared.s8 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t power_pair(uint32_t addr) {   // 2^e of two neighbouring exponents
+    return pack_half2(exp2_of(lds_s8(addr)), exp2_of(lds_s8(addr + 1)));
+}
+__device__ __forceinline__ uint32_t power_twice(uint32_t addr) {
+    const float f = exp2_of(lds_s8(addr));
+    return pack_half2(f, f);
+}
 
 template <typename TIn>
-__global__ void __launch_bounds__(kThreads1, 2)
-wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, unsigned char *__restrict__ operators,
-                           float *__restrict__ vectors, int *__restrict__ flags, int Tlen, int H, int chunk0,
-                           int seg_chunks, int nchains, int *work_counter, int *status) {
+__global__ void __launch_bounds__(kOpThreads, 4)
+wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPtrs ptrs, unsigned char *__restrict__ records,
+                           int Tlen, int H, int chunk0, int seg_chunks, int nchains, int wide_range, int *status) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    // fp32 tensors: the five raw tiles are twice as large, everything behind them moves up by X
-    constexpr uint32_t kRawTile = kL * kN * sizeof(TIn), kRawBytesT = 5 * kRawTile, X = kRawBytesT - kRawBytes;
+    constexpr bool kTma = sizeof(TIn) == 2;
     if (smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0) atomicExch(status, (int)kDevInternal);
         return;
     }
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int quarter = warp & 3, hf = warp >> 2;
-    const int row = quarter * 32 + lane;          // TMEM lane of this thread
-    unsigned char *raw = smem + kRaw;
-    float *Am = reinterpret_cast<float *>(smem + kAm);
-    float *Tm = reinterpret_cast<float *>(smem + kTm);
-    float *Wm = reinterpret_cast<float *>(smem + kWm);
-    uint64_t *bar_tma = reinterpret_cast<uint64_t *>(smem + (kMisc1 + X));
-    uint64_t *bar_mma = bar_tma + 1;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + (kMisc1 + X) + 32);
-    int *abort_flag = reinterpret_cast<int *>(smem + (kMisc1 + X) + 48);
-    int *next_slot = abort_flag + 1;   // the chunk this CTA works on next (thread 0 draws it, all read it)
-    float *grp = reinterpret_cast<float *>(smem + (kMisc1 + X) + 256);     // [8][64]
-    float *emv = reinterpret_cast<float *>(smem + (kMisc1 + X) + 256 + 2048);   // e^{m_j} / kOpScale [64]
-
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (uniform: no divergence handling around what depends on it)
+    const int g = lane >> 2, q = lane & 3;
+    const uint32_t sb = smem_u32(smem);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + kBar1);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + kBar1 + 32);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + kBar1 + 40);
+    if (warp == 0) tmem_alloc(tmem_slot, 128);
     if (tid == 0) {
-        mbar_init(bar_tma, 1);
-        mbar_init(bar_mma, 1);
+        mbar_init(bar, 1);       // w
+        mbar_init(bar + 1, 1);   // a, r, b, k
+        mbar_init(bar + 2, 1);   // the tcgen05 product
         mbar_fence_init();
         *abort_flag = 0;
-        // Chunks are drawn from a counter (zeroed by the host), so that CTAs which start late - the scan of
-        // the previous segment may still hold their place on the SM - simply take fewer of them.
-        *next_slot = work_counter ? atomicAdd(work_counter, 1) : (int)blockIdx.x;
+    }
+    const long long units = (long long)nchains * seg_chunks;
+    auto tile = [&](int x, long long unit, uint64_t *b) {
+        const int chain = (int)(unit / seg_chunks), chunk = chunk0 + (int)(unit % seg_chunks);
+        tma_load_2d(smem + kTiles + x * kPanel, &maps.m[x], (chain % H) * kN, (chain / H) * Tlen + chunk * kL, b);
+    };
+    auto request = [&](long long unit) {
+        mbar_expect_tx(bar, kPanel);
+        tile(XW, unit, bar);
+        mbar_expect_tx(bar + 1, 4 * kPanel);
 #pragma unroll
-        for (int i = 0; i < 5; ++i) tma_prefetch_desc(&maps.m[i]);
-    }
-    // identity tile (constant for the whole kernel)
-    for (int idx = tid; idx < kL * 8; idx += kThreads1) {
-        const int r = idx >> 3, ch = idx & 7;
-        uint4 z = make_uint4(0, 0, 0, 0);
-        if ((r >> 3) == ch) {
-            const uint32_t one = 0x3c00u << ((r & 1) * 16);
-            uint32_t *w = &z.x;
-            w[(r & 7) >> 1] = one;
-        }
-        *reinterpret_cast<uint4 *>(smem + (kI64 + X) + r * 128 + ((ch ^ (r & 7)) << 4)) = z;
-    }
-    if (warp == 0) tmem_alloc(tmem_slot, 128);
+        for (int x = 0; x < 4; ++x) tile(x, unit, bar + 1);
+    };
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    const uint32_t sb = smem_u32(smem);
-    const long long units = (long long)nchains * seg_chunks;
-
-    auto issue_tma = [&](long long unit) {
-        const int chain = (int)(unit / seg_chunks), chunk = chunk0 + (int)(unit % seg_chunks);
-        const int bi = chain / H, h = chain % H;
-        if (!RWKV7_IN_RANGE(chain < nchains && chunk * kL < Tlen, status)) return;   // (the wait then expires)
-        mbar_expect_tx(bar_tma, kRawBytesT);
-        const int trow = bi * Tlen + chunk * kL;
+    if (kTma && tid == 0 && blockIdx.x < units) request(blockIdx.x);
+    uint32_t mma_phase = 0;
+    uint32_t phase = 0;
+    int seq = 0;                               // chunks this CTA has begun
+    const int tb = warp;                       // token block of phases 1 and 2
+    const int ch = 2 * lane;                   // channel pair
+    uint32_t po[8];                            // this thread's place in row u (mod 8) of its block of a tile
 #pragma unroll
-        for (int i = 0; i < 5; ++i) tma_load_2d(raw + i * kRawTile, &maps.m[i], h * kN, trow, bar_tma);
-    };
-    long long unit = *next_slot;
-    if (tid == 0 && unit < units) issue_tma(unit);
-    uint32_t tma_phase = 0, mma_phase = 0;
-    bool tma_pending = unit < units;   // a tile batch is in flight (thread 0's view is what matters)
-    bool failed = false;
+    for (int u = 0; u < 8; ++u) po[u] = sb + kTiles + off16(16 * tb + u, ch);
+    auto at = [&](int x, int u) -> uint32_t { return po[u & 7] + (uint32_t)x * kPanel + (uint32_t)(u >> 3) * 1024u; };
 
-    for (; unit < units; unit = *next_slot) {
+    for (long long unit = blockIdx.x; unit < units; unit += gridDim.x, ++seq, phase ^= 1u) {
+        const bool more = unit + gridDim.x < units;
         const int chain = (int)(unit / seg_chunks), chunk = chunk0 + (int)(unit % seg_chunks);
         const int valid = min(kL, Tlen - chunk * kL);
-        if (!mbar_wait(bar_tma, tma_phase)) atomicOr(abort_flag, 1);
-        tma_phase ^= 1;
-        tma_pending = false;
-        if (valid < kL) {
-            // partial last chunk: rows past the end become no-op tokens (w = -inf: log-decay -0)
-            for (int idx = tid; idx < (kL - valid) * kN; idx += kThreads1) {
-                const int t = valid + idx / kN, jj = idx % kN;
+        const int nv = min(16, max(0, valid - 16 * tb));   // tokens of this block that exist
+        const size_t gbase = (((size_t)(chain / H) * Tlen + chunk * kL + 16 * tb) * H + chain % H) * kN + ch;
+        const size_t gstep = (size_t)H * kN;
+        // (token u of this warp's block, channel pair) of a tensor; tokens past the end are no-ops: w = -inf, the rest zero
+        using Raw = std::conditional_t<kTma, uint32_t, float2>;
+        auto load16 = [&](int x, Raw (&v)[16]) {   // (all loads first: what follows stores to the same memory)
 #pragma unroll
-                for (int x = 0; x < 5; ++x) {
-                    if constexpr (sizeof(TIn) == 2)
-                        *reinterpret_cast<unsigned short *>(raw + x * kRawTile + (t * kN + jj) * 2) =
-                            (x == XW) ? (unsigned short)0xFF80 : (unsigned short)0;
-                    else
-                        *reinterpret_cast<uint32_t *>(raw + x * kRawTile + (t * kN + jj) * 4) = (x == XW) ? 0xFF800000u : 0u;
+            for (int u = 0; u < 16; ++u) {
+                if constexpr (kTma) v[u] = lds32(at(x, u));
+                else {
+                    const float none = x == XW ? -INFINITY : 0.f;
+                    v[u] = make_float2(none, none);
+                    if (u < nv && RWKV7_IN_RANGE(chain < nchains && chunk * kL + 16 * tb + u < Tlen, status))
+                        v[u] = *reinterpret_cast<const float2 *>(static_cast<const float *>(ptrs.p[x]) + gbase + u * gstep);
                 }
             }
-            __syncthreads();
-        }
-        // ---------------- phase A: decay prefix sums, scaled fp16 operands
-        const int j2 = lane, tg = warp;            // channel pair (2 j2, 2 j2 + 1), tokens 8 tg .. 8 tg + 7
-        const unsigned char *rp = raw + (tg * 8 * kN + 2 * j2) * sizeof(TIn);
-        auto ld2 = [&](int tensor, int u) {
-            if constexpr (sizeof(TIn) == 2)
-                return unpack_bf2(*reinterpret_cast<const uint32_t *>(rp + tensor * kRawTile + u * (kN * 2)));
-            else
-                return *reinterpret_cast<const float2 *>(rp + tensor * kRawTile + u * (kN * 4));
         };
-        float c0[8], c1[8];
-        {
-            float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const float2 w2 = ld2(XW, u);
-                s0 -= __expf(w2.x);
-                s1 -= __expf(w2.y);
-                c0[u] = s0;
-                c1[u] = s1;
-            }
-            *reinterpret_cast<float2 *>(grp + tg * 64 + 2 * j2) = make_float2(s0, s1);
+        auto value = [&](Raw v) -> float2 {
+            if constexpr (kTma) return unpack_bf2(v);
+            else return v;
+        };
+        if constexpr (kTma) {
+            if (!mbar_wait(bar, phase)) *abort_flag = 1;
+            __syncwarp();
+            if (valid < kL)   // (each thread rewrites only what it reads itself)
+                for (int u = nv; u < 16; ++u) sts32(sb + kTiles + XW * kPanel + off16(16 * tb + u, ch), 0xff80ff80u);
         }
-        // the previous operator must have left its staging area before AR / A_rb / A_rk are rewritten
-        if (tid == 0) bulk_wait_group_read<0>();
+        // ---------------- 1. decays
+        float2 d[16];
+        float2 e = make_float2(1.f, 1.f);
+        {
+            Raw w[16];
+            load16(XW, w);
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                d[u] = decay2(value(w[u]));
+                e = mul2(e, d[u]);
+            }
+        }
+        sts_f2(sb + kE + (tb * 64 + ch) * 4, e.x, e.y);
         __syncthreads();
-        if (*abort_flag) { failed = true; break; }
-        {
-            float base0 = 0.f, base1 = 0.f, tot0 = 0.f, tot1 = 0.f;
+        if (*abort_flag) break;
+        if (kTma && tid == 0 && more) {   // the next chunk's tiles: into L2 now, here when there is room
+            const long long u = unit + gridDim.x;
+            const int cn = (int)(u / seg_chunks), x0 = (cn % H) * kN, y0 = (cn / H) * Tlen + (chunk0 + (int)(u % seg_chunks)) * kL;
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-                const float2 x = *reinterpret_cast<const float2 *>(grp + g * 64 + 2 * j2);
-                tot0 += x.x;
-                tot1 += x.y;
-                if (g < tg) { base0 += x.x; base1 += x.y; }
-            }
-            const float m0 = 0.5f * tot0, m1 = 0.5f * tot1;
-            const float em0 = __expf(m0), em1 = __expf(m1);
-            if (tg == 7) {
-                if (tot0 < -kMaxLogDecay || tot1 < -kMaxLogDecay || !(tot0 <= 0.f) || !(tot1 <= 0.f))
-                    atomicOr(&flags[chain], 1);
-                float *vec = vectors + (size_t)unit * kVecFloats;
-                if (RWKV7_IN_RANGE(unit < units && 2 * j2 + 1 < kN, status)) {
-                    *reinterpret_cast<float2 *>(vec + 2 * j2) = make_float2(__expf(tot0), __expf(tot1));
-                    *reinterpret_cast<float2 *>(vec + 64 + 2 * j2) = make_float2(__expf(tot0 - m0), __expf(tot1 - m1));
-                }
-                *reinterpret_cast<float2 *>(emv + 2 * j2) = make_float2(em0 * kInvOpScale, em1 * kInvOpScale);
-            }
-            float ep0 = __expf(base0 - m0) * kOpScale, ep1 = __expf(base1 - m1) * kOpScale;   // e^{c_{t-1} - m} * scale
-            const float rs0 = em0 * kInvOpScale, rs1 = em1 * kInvOpScale;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int t = tg * 8 + u;
-                const float e0 = __expf(base0 + c0[u] - m0) * kOpScale, e1 = __expf(base1 + c1[u] - m1) * kOpScale;
-                // e^{m - c_t} * scale
-                const float i0 = __fdividef(kOpScale * kOpScale, e0), i1 = __fdividef(kOpScale * kOpScale, e1);
-                const float2 a2 = ld2(XA, u), r2 = ld2(XR, u), b2 = ld2(XB, u), k2 = ld2(XK, u);
-                const uint32_t o = off16(t, 2 * j2);
-                if (!RWKV7_IN_RANGE(o + 4 <= kPanel, status)) continue;
-                *reinterpret_cast<uint32_t *>(smem + (kAR + X) + o) = pack_h2(a2.x * ep0, a2.y * ep1);
-                *reinterpret_cast<uint32_t *>(smem + (kAR + X) + kPanel + o) = pack_h2(r2.x * e0, r2.y * e1);
-                *reinterpret_cast<uint32_t *>(smem + (kBK + X) + o) = pack_h2(b2.x * i0, b2.y * i1);
-                *reinterpret_cast<uint32_t *>(smem + (kBK + X) + kPanel + o) = pack_h2(k2.x * i0, k2.y * i1);
-                *reinterpret_cast<uint32_t *>(smem + (kRtrue + X) + o) = pack_h2(r2.x * e0 * rs0, r2.y * e1 * rs1);
-                ep0 = e0;
-                ep1 = e1;
-            }
+            for (int x = 0; x < 5; ++x)
+                asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(&maps.m[x]), "r"(x0), "r"(y0) : "memory");
         }
-        fence_proxy_async();
-        // A chain that is flagged (by this chunk's decay just now, or by an earlier chunk) is recomputed by
-        // the next kernel in line whatever happens here: skip the rest of its chunks.  (Another CTA may set
-        // the flag at any moment: the barrier makes one decision of what the threads read.)
-        if (__syncthreads_or(*reinterpret_cast<volatile int *>(&flags[chain]) != 0)) {
-            if (tid == 0) {
-                const long long next = work_counter ? (long long)atomicAdd(work_counter, 1) : unit + gridDim.x;
-                *next_slot = next < units ? (int)next : 0x7fffffff;
-                if (next < units && !*abort_flag) {
-                    issue_tma(next);
-                    tma_pending = true;
-                }
-            }
-            __syncthreads();
+        // Every warp sees the whole chunk's decays (its 32 lanes hold all channels): no further agreement is needed.
+        float E[2][4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const float2 v = lds_f2(sb + kE + (b * 64 + ch) * 4);
+            E[0][b] = v.x;
+            E[1][b] = v.y;
+        }
+        bool over = false, strong = false;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) over |= !(E[x][b] >= kBlockDecay);
+            const float h0 = E[x][0] * E[x][1], h1 = E[x][2] * E[x][3];
+            strong |= !(h0 >= kMildDecay && h1 >= kMildDecay);
+            if (!wide_range) over |= !(h0 * h1 >= kNarrowDecay);
+        }
+        over = __any_sync(0xffffffffu, over);
+        const bool wide = __any_sync(0xffffffffu, strong);
+        unsigned char *record = records + (size_t)unit * kRecord;
+        if (tid == 0 && RWKV7_IN_RANGE(unit >= 0 && unit < units, status)) *reinterpret_cast<int *>(record + kMarkAt) = over;
+        if constexpr (kTma) {
+            if (!mbar_wait(bar + 1, phase)) *abort_flag = 1;
+            __syncwarp();
+            if (valid < kL)
+                for (int u = nv; u < 16; ++u)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) sts32(sb + kTiles + x * kPanel + off16(16 * tb + u, ch), 0u);
+        }
+        if (over) {   // the chain is recomputed elsewhere: nothing more to do for this chunk
+            if (kTma) fence_proxy_async();
+            __syncthreads();   // (everyone has read the decays)
+            if (kTma && tid == 0 && more) request(unit + gridDim.x);
             continue;
         }
-        // ---------------- G = [At;Rt] [Bh;Kh]^T   (128 x 128, contraction over the 64 channels)
-        if (tid == 0) {
-            tc_fence_after();
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-                umma_f16(tmem, dK(sb + (kAR + X), ks), dK(sb + (kBK + X), ks), idesc16(128, 128, false, false), ks > 0);
-            umma_commit(bar_mma);
-        }
-        if (!mbar_wait(bar_mma, mma_phase)) atomicOr(abort_flag, 1);
-        mma_phase ^= 1;
-        tc_fence_after();
-        // ---------------- G -> A_ab, A_ak, A_rb, A_rk, masked to the lower triangle.  A_ab's two diagonal
-        // 32 x 32 blocks go to the fp32 scratch of the inverse, its lower-left block straight into the
-        // fp16 tile of T (where the second level of the inverse replaces it); the others are fp16 tiles.
+        // ---------------- 2. scaled operands
         {
-            const bool rt_rows = quarter >= 2;        // Rt rows keep the diagonal
-            const int t = row & 63;
-            const bool low_rows = t < 32;             // (warp-uniform: one quarter is 32 consecutive rows)
-            const int lim = rt_rows ? t : t - 1;      // keep s <= lim
-            constexpr float sc = kInvOpScale * kInvOpScale;
+            float mA[2], mB[2], dec[2];
+            int ef[2], eg[2];
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const bool zero_half = low_rows && half == 1;   // columns 32..63 of rows 0..31: above the diagonal
-                if (!rt_rows && hf == 0) {
-                    if (zero_half) continue;
-                    uint32_t v[32];
-                    tmem_ld32(tmem + lane_base + half * 32, v);
-                    tmem_ld_wait();
-                    if (low_rows == (half == 0)) {   // diagonal block of this row: fp32, strictly lower
-                        float *dst = Am + t * kPitchF;
+            for (int x = 0; x < 2; ++x) {
+                const float p1 = E[x][0], p2 = p1 * E[x][1], p3 = p2 * E[x][2], p4 = p3 * E[x][3];
+                const float pre = tb == 0 ? 1.f : tb == 1 ? p1 : tb == 2 ? p2 : p3;    // decay up to this block's start,
+                const float post = tb == 0 ? p1 : tb == 1 ? p2 : tb == 2 ? p3 : p4;    // to its end,
+                const float tail = tb == 3 ? 1.f : tb == 2 ? E[x][3] : tb == 1 ? E[x][2] * E[x][3] : E[x][1] * E[x][2] * E[x][3];   // and from there to the chunk's
+                const int x4 = exponent_of(p4);
+                dec[x] = p4;
+                if (!wide) {
+                    ef[x] = eg[x] = exponent_of(p2) - x4;
+                    const float up = exp2_of(ef[x]);
+                    mA[x] = pre * rcp(p4 * up);
+                    mB[x] = tail * up;
+                } else {
+                    const int xs = exponent_of(pre), xe = exponent_of(post);
+                    mA[x] = pre * exp2_of(kWideShift) * rcp(p4 * exp2_of(xs - x4));
+                    mB[x] = tail * exp2_of(xe - x4 + kWideShift);
+                    ef[x] = 127 - x4;
+                    eg[x] = 0;
+                    signed char *pw = reinterpret_cast<signed char *>(smem + kPow) + ch + x;
+                    auto power = [&](int row, int e) { pw[row * 64] = (signed char)max(e, -100); };   // (fp16 ends at 2^-24)
+                    const int ha = (xs - xe) >> 1;
+                    power(PA + tb, ha - kWideShift);
+                    power(PB + tb, xs - xe - ha - kWideShift);
+                    if (tb < 3)   // (2,0), (3,0), (3,1): start of the row block over the end of the column block
+                        power(PF + tb, exponent_of(tb == 0 ? p2 : p3) - exponent_of(tb == 2 ? p2 : p1));
+                    power(PX + tb, xs - 127 - kWideShift);
+                    power(PE + tb, x4 - xe - kWideShift);
+                }
+            }
+            if (tb == 3 && RWKV7_IN_RANGE(unit >= 0 && unit < units, status)) {
+                *reinterpret_cast<float2 *>(record + kDecayAt + ch * 4) = make_float2(dec[0], dec[1]);
+                *reinterpret_cast<char2 *>(record + kExpAt + ch) = make_char2((signed char)ef[0], (signed char)ef[1]);
+                *reinterpret_cast<char2 *>(record + kExpAt + 64 + ch) = make_char2((signed char)eg[0], (signed char)eg[1]);
+            }
+            Raw v0[16], v1[16];
+            load16(XA, v0);
+            load16(XR, v1);
+            float2 f = make_float2(mA[0], mA[1]);
 #pragma unroll
-                        for (int e4 = 0; e4 < 8; ++e4) {
-                            float4 o;
-                            float *of = &o.x;
+            for (int u = 0; u < 16; ++u) {
+                sts32(at(XA, u), pack2(mul2(value(v0[u]), f)));
+                f = mul2(f, d[u]);
+                sts32(at(XR, u), pack2(mul2(value(v1[u]), f)));
+            }
+            load16(XB, v0);
+            load16(XK, v1);
+            f = make_float2(mB[0], mB[1]);
+#pragma unroll
+            for (int u = 15; u >= 0; --u) {
+                sts32(at(XB, u), pack2(mul2(value(v0[u]), f)));
+                sts32(at(XK, u), pack2(mul2(value(v1[u]), f)));
+                f = mul2(f, d[u]);
+            }
+        }
+        fence_proxy_async();
+        __syncthreads();
+        // ---------------- 3. the A matrices, lower triangles
+        if (!wide) {
+            if (warp == 0 && elect_one()) {
+                tc_fence_after();
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+                    umma_f16(tmem, make_smem_desc(sb + kTiles + XA * kPanel + ks * 32u, 16u, 1024u), make_smem_desc(sb + kTiles + XB * kPanel + ks * 32u, 16u, 1024u),
+                             make_idesc(kFmtF16, 128, 128, false, false), ks > 0);
+                umma_commit(bar + 2);
+            }
+            __syncwarp();
+            if (!mbar_wait_tight(bar + 2, mma_phase, 4000000u)) *abort_flag = 1;
+            __syncwarp();
+            mma_phase ^= 1u;
+            tc_fence_after();
+            // This thread's row t of [A_ab | A_ak] (warps 0, 1) or [A_rb | A_rk]; block row bt, the other half-warp's is bt0 or bt0 + 1.
+            const int bt0 = 2 * (warp & 1), bt = bt0 + (lane >> 4), r = lane & 15;
+            const bool top = warp < 2;                 // strictly lower
+            const uint32_t col0 = tmem + ((uint32_t)(warp * 32) << 16);
+            uint32_t keep[8];                          // column pairs of a diagonal block that this row keeps
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int n = r + (top ? 0 : 1) - 2 * e;   // of these two columns, how many
+                keep[e] = n <= 0 ? 0u : n == 1 ? 0xffffu : ~0u;
+            }
+            const uint32_t sub = r * 16, row = sub + tri(bt) * kBlk;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int m = i >> 1, sp = i & 1;
+                if (sp == 1 && bt0 == 0) continue;     // (uniform) above the diagonal for the whole warp
+                const bool ab = m == 0 && top;
+                const uint32_t out = m == 0 ? (top ? sb + kAab + sub + below(bt) * kBlk : sb + kArb + row) : (top ? sb + kAak : sb + kArk) + row;
+                uint32_t d[32];
+                tmem_ld32(col0 + i * 32, d);
+                tmem_ld_wait();
+#pragma unroll
+                for (int s1 = 0; s1 < 2; ++s1) {
+                    const int sc = 2 * sp + s1;
+                    if (sc == bt && ab) {          // fp32 for the inverse (which reads below the diagonal only)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const uint32_t x[4] = {d[16 * s1 + 4 * e], d[16 * s1 + 4 * e + 1], d[16 * s1 + 4 * e + 2], d[16 * s1 + 4 * e + 3]};
+                            sts128(sb + kDiag + bt * 1024 + r * 64 + ((e ^ ((r >> 1) & 3)) << 4), x);
+                        }
+                    } else if (sc <= bt) {
+                        const uint32_t all = sc == bt ? 0u : ~0u;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t x[4];
 #pragma unroll
                             for (int e = 0; e < 4; ++e)
-                                of[e] = (half * 32 + e4 * 4 + e <= lim) ? __uint_as_float(v[e4 * 4 + e]) * sc : 0.f;
-                            *reinterpret_cast<float4 *>(dst + e4 * 4) = o;
-                        }
-                    } else {                          // rows 32..63, columns 0..31: A_10 of the second level
-#pragma unroll
-                        for (int e8 = 0; e8 < 4; ++e8) {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int e2 = 0; e2 < 4; ++e2)
-                                w[e2] = pack_h2(__uint_as_float(v[e8 * 8 + e2 * 2]) * sc, __uint_as_float(v[e8 * 8 + e2 * 2 + 1]) * sc);
-                            *reinterpret_cast<uint4 *>(smem + kT16 + off16(t, e8 * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
+                                x[e] = pack_half2(__uint_as_float(d[16 * s1 + 8 * h + 2 * e]), __uint_as_float(d[16 * s1 + 8 * h + 2 * e + 1])) & (keep[4 * h + e] | all);
+                            sts128(out + sc * kBlk + h * 256, x);
                         }
                     }
-                } else {
-                    const uint32_t tile = !rt_rows ? ((kAR + X) + kPanel) : (hf == 0 ? (kArb + X) : (kArk + X));   // A_ak takes Rt's place
-                    uint32_t v[32];
-                    if (!zero_half) {
-                        tmem_ld32(tmem + lane_base + hf * 64 + half * 32, v);
-                        tmem_ld_wait();
+                }
+            }
+            tc_fence_before();
+        } else {
+            const uint32_t rows = sb + kTiles + (warp < 2 ? XA : XR) * kPanel, cols = sb + kTiles + (warp & 1 ? XK : XB) * kPanel;
+            const uint32_t mat = sb + (warp == 0 ? kAab : warp == 1 ? kAak : warp == 2 ? kArb : kArk) + lane * 4;
+            const int keep = warp >= 2 ? 0 : -1;    // r rows keep the diagonal
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                float c[4][2][4] = {};
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    uint32_t A[4];
+                    ldsm4(A, rows + tile_plain(lane, 16 * t, kk));
+#pragma unroll
+                    for (int s = 0; s <= t; ++s) {
+                        uint32_t As[4] = {A[0], A[1], A[2], A[3]}, Bs[4];
+                        ldsm4(Bs, cols + tile_cols(lane, 16 * s, kk));
+                        const uint32_t f = sb + kPow + kk * 16 + 2 * q;
+                        if (t != s + 1) {
+                            const int pa = (s == t ? PA + t : PF + (t == 2 ? 0 : 1 + s)) * 64;
+                            const uint32_t lo = power_pair(f + pa), hi = power_pair(f + pa + 8);
+                            As[0] = mul_half2(As[0], lo);
+                            As[1] = mul_half2(As[1], lo);
+                            As[2] = mul_half2(As[2], hi);
+                            As[3] = mul_half2(As[3], hi);
+                        }
+                        if (t == s) {
+                            const uint32_t lo = power_pair(f + (PB + t) * 64), hi = power_pair(f + (PB + t) * 64 + 8);
+                            Bs[0] = mul_half2(Bs[0], lo);
+                            Bs[1] = mul_half2(Bs[1], hi);
+                            Bs[2] = mul_half2(Bs[2], lo);
+                            Bs[3] = mul_half2(Bs[3], hi);
+                        }
+                        mma16816(c[s][0], As, Bs[0], Bs[1]);
+                        mma16816(c[s][1], As, Bs[2], Bs[3]);
                     }
+                }
 #pragma unroll
-                    for (int e8 = 0; e8 < 4; ++e8) {
-                        uint32_t w[4] = {0u, 0u, 0u, 0u};
-                        if (!zero_half) {
+                for (int h = 0; h < 2; ++h)
 #pragma unroll
-                            for (int e2 = 0; e2 < 4; ++e2) {
-                                const int sidx = half * 32 + e8 * 8 + e2 * 2;
-                                const float x0 = (sidx <= lim) ? __uint_as_float(v[e8 * 8 + e2 * 2]) * sc : 0.f;
-                                const float x1 = (sidx + 1 <= lim) ? __uint_as_float(v[e8 * 8 + e2 * 2 + 1]) * sc : 0.f;
-                                w[e2] = pack_h2(x0, x1);
+                    for (int e = 0; e < 4; ++e)
+                        if (8 * h + 2 * q + (e & 1) > g + (e >> 1) * 8 + keep) c[t][h][e] = 0.f;
+                // (the diagonal blocks' powers have taken the operands' common scale out already)
+#pragma unroll
+                for (int s = 0; s < t; ++s)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) c[s][h][e] *= 1.f / (kWideScale * kWideScale);
+#pragma unroll
+                for (int s = 0; s <= t; ++s) {
+                    if (s == t && warp == 0) {   // fp32 for the inverse
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int r = 0; r < 2; ++r) {
+                                const int row = g + 8 * r, piece = 2 * h + (q >> 1);
+                                sts_f2(sb + kDiag + t * 1024 + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4) + (q & 1) * 8, c[s][h][2 * r], c[s][h][2 * r + 1]);
                             }
-                        }
-                        *reinterpret_cast<uint4 *>(smem + tile + off16(t, half * 32 + e8 * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                }
-            }
-        }
-        tc_fence_before();
-        // ---------------- T = (I - A_ab)^-1.  The two 32 x 32 diagonal blocks in fp32 on the CUDA cores:
-        // 16 x 16 blocks by forward substitution (the 64 threads that wrote the scratch go on as soon as they
-        // are done, the others are still writing their tiles), then [[T00, 0], [T11 A10 T00, T11]].
-        if (tid < 64) {
-            asm volatile("bar.sync 1, 64;" ::: "memory");
-            const int b = tid >> 4, cc = tid & 15;
-            const float *Ab = Am + (16 * b) * kPitchF + 16 * (b & 1);
-            float x[16];
+                    } else {
+                        const uint32_t o = mat + ((warp == 0 ? below(t) : tri(t)) + s) * kBlk;
 #pragma unroll
-            for (int t = 0; t < 16; ++t) {
-                float acc0 = 0.f, acc1 = 0.f;
-#pragma unroll
-                for (int s4 = 0; s4 < (t + 3) / 4; ++s4) {
-                    const float4 a4 = *reinterpret_cast<const float4 *>(Ab + t * kPitchF + 4 * s4);
-                    if (4 * s4 + 0 < t) acc0 = fmaf(a4.x, x[4 * s4 + 0], acc0);
-                    if (4 * s4 + 1 < t) acc1 = fmaf(a4.y, x[4 * s4 + 1], acc1);
-                    if (4 * s4 + 2 < t) acc0 = fmaf(a4.z, x[4 * s4 + 2], acc0);
-                    if (4 * s4 + 3 < t) acc1 = fmaf(a4.w, x[4 * s4 + 3], acc1);
-                }
-                x[t] = (t == cc) ? 1.f : ((t > cc) ? acc0 + acc1 : 0.f);
-                Tm[(16 * b + t) * kPitchF + 16 * (b & 1) + cc] = x[t];
-            }
-        }
-        __syncthreads();
-        if (*abort_flag) { failed = true; break; }
-        {   // the two pairs of 16-blocks; 512 outputs per product, two per thread
-            const int pr = tid >> 7, t = (tid >> 3) & 15, cb = (tid & 7) * 2;
-            const float *arow = Am + (32 * pr + 16 + t) * kPitchF;       // A10[t][.]  (row-local columns 0..15)
-            const float *tcol = Tm + (32 * pr) * kPitchF + cb;           // T00[.][cb..]
-            float w0 = 0.f, w1 = 0.f;
-#pragma unroll
-            for (int s = 0; s < 16; ++s) {
-                const float a = arow[s];
-                const float2 tt = *reinterpret_cast<const float2 *>(tcol + s * kPitchF);
-                w0 = fmaf(a, tt.x, w0);   // (T00 is complete: zeros above its diagonal were written)
-                w1 = fmaf(a, tt.y, w1);
-            }
-            *reinterpret_cast<float2 *>(Wm + (16 * pr + t) * 20 + cb) = make_float2(w0, w1);
-            __syncthreads();
-            const float *trow = Tm + (32 * pr + 16 + t) * kPitchF + 16;   // T11[t][.]
-            const float *wcol = Wm + (16 * pr) * 20 + cb;
-            float z0 = 0.f, z1 = 0.f;
-#pragma unroll
-            for (int s = 0; s < 16; ++s) {
-                const float a = trow[s];
-                const float2 ww = *reinterpret_cast<const float2 *>(wcol + s * 20);
-                z0 = fmaf(a, ww.x, z0);
-                z1 = fmaf(a, ww.y, z1);
-            }
-            *reinterpret_cast<float2 *>(Tm + (32 * pr + 16 + t) * kPitchF + cb) = make_float2(z0, z1);
-        }
-        __syncthreads();
-        {   // diagonal 32-blocks -> fp16 tile T[t][u] (zero above the diagonal), and zeros in the block above them
-            const int t = tid >> 2, c0 = (tid & 3) * 8, tl = t & 31;
-            const float *src = Tm + t * kPitchF + c0;
-            const float4 x0 = *reinterpret_cast<const float4 *>(src), x1 = *reinterpret_cast<const float4 *>(src + 4);
-            const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-            uint32_t w[4];
-#pragma unroll
-            for (int e2 = 0; e2 < 4; ++e2)
-                w[e2] = pack_h2(c0 + 2 * e2 <= tl ? xs[2 * e2] : 0.f, c0 + 2 * e2 + 1 <= tl ? xs[2 * e2 + 1] : 0.f);
-            *reinterpret_cast<uint4 *>(smem + kT16 + off16(t, 32 * (t >> 5) + c0)) = make_uint4(w[0], w[1], w[2], w[3]);
-            if (tid < 128)   // rows 0..31, columns 32..63
-                *reinterpret_cast<uint4 *>(smem + kT16 + off16(tid >> 2, 32 + (tid & 3) * 8)) = make_uint4(0, 0, 0, 0);
-        }
-        fence_proxy_async();
-        __syncthreads();
-        // second level on the tensor core: T10 = T11 (A10 T00), fp16 operands, two dependent products
-        // (N = 64: the upper 32 columns of both results are never read)
-        if (tid == 0) {
-            tc_fence_after();
-#pragma unroll
-            for (int ks = 0; ks < 2; ++ks)   // rows 32.. of the tile (A10) against T00[u][c] (rows u of the same tile, MN-major)
-                umma_f16(tmem, dK(sb + kT16 + 32 * 128, ks), dMN(sb + kT16, kPanel, ks), idesc16(128, 64, false, true), ks > 0);
-            umma_commit(bar_mma);
-        }
-        if (!mbar_wait(bar_mma, mma_phase)) atomicOr(abort_flag, 1);
-        mma_phase ^= 1;
-        tc_fence_after();
-        if (quarter == 0) {   // lanes 0..31 hold the 32 rows; 16 columns per warp
-            uint32_t v[16];
-            tmem_ld16(tmem + hf * 16, v);
-            tmem_ld_wait();
-            uint32_t w[8];
-#pragma unroll
-            for (int e2 = 0; e2 < 8; ++e2) w[e2] = pack_h2(__uint_as_float(v[2 * e2]), __uint_as_float(v[2 * e2 + 1]));
-            *reinterpret_cast<uint4 *>(smem + kW2 + off16(lane, hf * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
-            *reinterpret_cast<uint4 *>(smem + kW2 + off16(lane, hf * 16 + 8)) = make_uint4(w[4], w[5], w[6], w[7]);
-        }
-        tc_fence_before();
-        fence_proxy_async();
-        __syncthreads();
-        if (*abort_flag) { failed = true; break; }
-        if (tid == 0) {
-            tc_fence_after();
-#pragma unroll
-            for (int ks = 0; ks < 2; ++ks)   // T11 (rows 32.., columns 32..63) against W[s][c] (MN-major)
-                umma_f16(tmem, dK(sb + kT16 + 32 * 128, 2 + ks), dMN(sb + kW2, kPanel, ks), idesc16(128, 64, false, true), ks > 0);
-            umma_commit(bar_mma);
-        }
-        if (!mbar_wait(bar_mma, mma_phase)) atomicOr(abort_flag, 1);
-        mma_phase ^= 1;
-        tc_fence_after();
-        if (quarter == 0) {
-            uint32_t v[16];
-            tmem_ld16(tmem + hf * 16, v);
-            tmem_ld_wait();
-            uint32_t w[8];
-#pragma unroll
-            for (int e2 = 0; e2 < 8; ++e2) w[e2] = pack_h2(__uint_as_float(v[2 * e2]), __uint_as_float(v[2 * e2 + 1]));
-            *reinterpret_cast<uint4 *>(smem + kT16 + off16(32 + lane, hf * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
-            *reinterpret_cast<uint4 *>(smem + kT16 + off16(32 + lane, hf * 16 + 8)) = make_uint4(w[4], w[5], w[6], w[7]);
-        }
-        tc_fence_before();
-        fence_proxy_async();
-        __syncthreads();
-        // ---------------- [A~ | A~k]^T = [At | A_ak]^T T^T   (rows c = (j | s), columns t)
-        if (tid == 0) {
-            tc_fence_after();
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-                umma_f16(tmem, dMN(sb + (kAR + X), kPanel, ks), dK(sb + kT16, ks), idesc16(128, 64, true, false), ks > 0);
-            umma_commit(bar_mma);
-        }
-        if (!mbar_wait(bar_mma, mma_phase)) atomicOr(abort_flag, 1);
-        mma_phase ^= 1;
-        tc_fence_after();
-        // T has been read: the raw-tile region (scratch of the inverse, T, W) is dead, request the next chunk's tiles
-        if (tid == 0) {
-            const long long next = work_counter ? (long long)atomicAdd(work_counter, 1) : unit + gridDim.x;
-            *next_slot = next < units ? (int)next : 0x7fffffff;
-            if (next < units && !*abort_flag) {
-                issue_tma(next);
-                tma_pending = true;
-            } else {
-                // this CTA is on its last chunk: the kernel launched behind this one may be set up now
-                asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-            }
-        }
-        {
-            uint32_t v[32];
-            tmem_ld32(tmem + lane_base + hf * 32, v);
-            tmem_ld_wait();
-            const float scale = row < 64 ? emv[row] : 1.f;   // A~ rows: back to the true scale
-#pragma unroll
-            for (int e8 = 0; e8 < 4; ++e8) {
-                uint32_t w[4];
-#pragma unroll
-                for (int e2 = 0; e2 < 4; ++e2)
-                    w[e2] = pack_h2(__uint_as_float(v[e8 * 8 + 2 * e2]) * scale, __uint_as_float(v[e8 * 8 + 2 * e2 + 1]) * scale);
-                *reinterpret_cast<uint4 *>(smem + (kAf + X) + off16(row, hf * 32 + e8 * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-        }
-        tc_fence_before();
-        fence_proxy_async();
-        __syncthreads();
-        if (*abort_flag) { failed = true; break; }
-        // ---------------- O = [A~|A~k]^T [Bh | A_rb^T]  +  [R|A_rk]^T [0 | I]
-        if (tid == 0) {
-            tc_fence_after();
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)   // columns j': contraction over t with Bh[t][j'] (MN-major B)
-                umma_f16(tmem, dK(sb + (kAf + X), ks), dMN(sb + (kBK + X), kPanel, ks), idesc16(128, 64, false, true), ks > 0);
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)   // columns t': contraction over t with A_rb[t'][t]
-                umma_f16(tmem + 64, dK(sb + (kAf + X), ks), dK(sb + (kArb + X), ks), idesc16(128, 64, false, false), ks > 0);
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)   // + R[t'][j] and A_rk[t'][s], through the identity
-                umma_f16(tmem + 64, dMN(sb + (kRtrue + X), (kArk + X) - (kRtrue + X), ks), dK(sb + (kI64 + X), ks), idesc16(128, 64, true, false), true);
-            umma_commit(bar_mma);
-        }
-        if (!mbar_wait(bar_mma, mma_phase)) atomicOr(abort_flag, 1);
-        mma_phase ^= 1;
-        tc_fence_after();
-        {
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t v[32];
-                tmem_ld32(tmem + lane_base + hf * 64 + half * 32, v);
-                tmem_ld_wait();
-                float add[32];
-                const bool kt_rows = hf == 0 && row >= 64;      // Kt = Kh + A~k^T Bh
-                const float sc = hf == 0 ? kInvOpScale : 1.f;   // Bh and Kh carry the operand scale
-                if (kt_rows) {
-#pragma unroll
-                    for (int e8 = 0; e8 < 4; ++e8) {
-                        const uint4 q = *reinterpret_cast<const uint4 *>(smem + (kBK + X) + kPanel + off16(row - 64, half * 32 + e8 * 8));
-                        const uint32_t qs[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                        for (int e2 = 0; e2 < 4; ++e2) {
-                            const float2 f = unpack_h2(qs[e2]);
-                            add[e8 * 8 + 2 * e2] = f.x;
-                            add[e8 * 8 + 2 * e2 + 1] = f.y;
+                        for (int h = 0; h < 2; ++h) {
+                            sts32(o + h * 256, pack_half2(c[s][h][0], c[s][h][1]));
+                            sts32(o + h * 256 + 128, pack_half2(c[s][h][2], c[s][h][3]));
                         }
                     }
                 }
-#pragma unroll
-                for (int e8 = 0; e8 < 4; ++e8) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int e2 = 0; e2 < 4; ++e2) {
-                        float x0 = __uint_as_float(v[e8 * 8 + 2 * e2]), x1 = __uint_as_float(v[e8 * 8 + 2 * e2 + 1]);
-                        if (kt_rows) { x0 += add[e8 * 8 + 2 * e2]; x1 += add[e8 * 8 + 2 * e2 + 1]; }
-                        w[e2] = pack_h2(x0 * sc, x1 * sc);
-                    }
-                    // panel hf, row k = this thread's lane, 16-byte chunk of columns n
-                    const uint32_t so = hf * (2 * kPanel) + off16(row, half * 32 + e8 * 8);
-                    if (RWKV7_IN_RANGE(so + 16 <= kOperatorBytes, status))
-                        *reinterpret_cast<uint4 *>(smem + (kStage + X) + so) = make_uint4(w[0], w[1], w[2], w[3]);
-                }
             }
         }
-        tc_fence_before();
-        fence_proxy_async();
         __syncthreads();
-        if (tid == 0 && RWKV7_IN_RANGE(unit >= 0 && unit < units, status)) {
-            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(operators + (size_t)unit * kOperatorBytes),
-                         "r"(sb + (kStage + X)), "r"(kOperatorBytes)
-                         : "memory");
-            bulk_commit_group();
+        // ---------------- 4. T_bb = (I - A_bb)^-1: two warps, a half-warp per diagonal block, a column per lane
+        {
+            const int pair = (warp + seq) & 3;   // (which two warps changes from chunk to chunk: each sits on its own scheduler)
+            if (pair < 2) {
+                const int cc = lane & 15, b = 2 * pair + (lane >> 4);
+                const uint32_t src = sb + kDiag + b * 1024;
+                float x[16];
+#pragma unroll
+                for (int t = 0; t < 16; ++t) {
+                    float acc0 = 0.f, acc1 = 0.f;
+#pragma unroll
+                    for (int s4 = 0; s4 < (t + 3) / 4; ++s4) {
+                        const float4 a4 = lds_f4(src + t * 64 + ((s4 ^ ((t >> 1) & 3)) << 4));
+                        if (4 * s4 + 0 < t) acc0 = fmaf(a4.x, x[4 * s4 + 0], acc0);
+                        if (4 * s4 + 1 < t) acc1 = fmaf(a4.y, x[4 * s4 + 1], acc1);
+                        if (4 * s4 + 2 < t) acc0 = fmaf(a4.z, x[4 * s4 + 2], acc0);
+                        if (4 * s4 + 3 < t) acc1 = fmaf(a4.w, x[4 * s4 + 3], acc1);
+                    }
+                    x[t] = (t == cc) ? 1.f : acc0 + acc1;   // (zero above: every term up to there is)
+                }
+                unsigned char *dst = smem + kDiag + b * 1024 + (cc >> 3) * 256 + (cc & 7) * 2;   // (every lane has read the block)
+#pragma unroll
+                for (int t = 0; t < 16; ++t) *reinterpret_cast<__half *>(dst + t * 16) = __float2half_rn(x[t]);
+            }
         }
+        __syncthreads();
+        // ---------------- 5. [A~ | A~k]^T for columns j = 16 ct.. and s = 16 ct.., then the operator's rows they are
+        auto finish = [&](auto block_wise) {
+            constexpr bool kWide = decltype(block_wise)::value;
+            const int ct = (warp + seq) & 3;   // (block ct of s has 4 - ct row blocks to do: the share goes round)
+            uint32_t U[2][4][4];   // A order, rows = own columns (0: j, 1: s), columns = tokens of block b
+            auto unpack8 = [&](const uint32_t (&X)[4], float (&c)[2][4]) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const float2 v = unpack_half2(X[2 * h + r]);
+                        c[h][2 * r] = v.x;
+                        c[h][2 * r + 1] = v.y;
+                    }
+            };
+            // a/r or b/k operand block, rows = channels 16 c.., times its row's power of two (block-wise references)
+            auto row_power = [&](int table, int c, uint32_t (&X)[4]) {
+                const uint32_t f0 = power_twice(sb + kPow + table * 64 + 16 * c + g), f1 = power_twice(sb + kPow + table * 64 + 16 * c + g + 8);
+                X[0] = mul_half2(X[0], f0);
+                X[1] = mul_half2(X[1], f1);
+                X[2] = mul_half2(X[2], f0);
+                X[3] = mul_half2(X[3], f1);
+            };
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                uint32_t X[2][4];
+                float c[2][2][4];
+                ldsm4_t(X[0], sb + kTiles + XA * kPanel + tile_cols(lane, 16 * b, ct));
+                if constexpr (kWide) row_power(PX + b, ct, X[0]);
+                const bool live = b >= ct;   // A~k[t][s] is zero above the diagonal
+                if (live) ldsm4_t(X[1], sb + kAak + (tri(b) + ct) * kBlk + blk_cols(lane));
+                else X[1][0] = X[1][1] = X[1][2] = X[1][3] = 0;
+                if (b > 0) {
+                    unpack8(X[0], c[0]);
+                    unpack8(X[1], c[1]);
+#pragma unroll
+                    for (int p = 0; p < b; ++p) {
+                        uint32_t M[4];
+                        ldsm4(M, sb + kAab + (below(b) + p) * kBlk + blk_cols(lane));
+                        mma16816(c[0][0], U[0][p], M[0], M[1]);
+                        mma16816(c[0][1], U[0][p], M[2], M[3]);
+                        mma16816(c[1][0], U[1][p], M[0], M[1]);   // (zero for p < ct: cheaper than a branch)
+                        mma16816(c[1][1], U[1][p], M[2], M[3]);
+                    }
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        X[x][0] = pack_half2(c[x][0][0], c[x][0][1]);
+                        X[x][1] = pack_half2(c[x][0][2], c[x][0][3]);
+                        X[x][2] = pack_half2(c[x][1][0], c[x][1][1]);
+                        X[x][3] = pack_half2(c[x][1][2], c[x][1][3]);
+                    }
+                }
+                uint32_t Tb[4];
+                ldsm4(Tb, sb + kDiag + b * 1024 + blk_cols(lane));
+                float o[2][2][4];
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    mma16816_first(o[x][0], X[x], Tb[0], Tb[1]);
+                    mma16816_first(o[x][1], X[x], Tb[2], Tb[3]);
+                }
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    U[x][b][0] = pack_half2(o[x][0][0], o[x][0][1]);
+                    U[x][b][1] = pack_half2(o[x][0][2], o[x][0][3]);
+                    U[x][b][2] = pack_half2(o[x][1][0], o[x][1][1]);
+                    U[x][b][3] = pack_half2(o[x][1][2], o[x][1][3]);
+                }
+            }
+            // Sixteen rows n of the operator, columns k of this warp's two blocks: four k of a row per lane (see kRecord)
+            unsigned char *dst = record + (ct >> 1) * 512 + (ct & 1) * 8 + q * 128 + g * 16;
+            auto put = [&](int n16, const float (&c)[2][2][4]) {
+                if (RWKV7_IN_RANGE(unit >= 0 && unit < units && n16 < 8, status)) {
+#pragma unroll
+                    for (int r = 0; r < 2; ++r)
+#pragma unroll
+                        for (int x = 0; x < 2; ++x)
+                            *reinterpret_cast<uint2 *>(dst + (2 * n16 + r) * 2048 + x * 1024) =
+                                make_uint2(pack_half2(c[x][0][2 * r], c[x][0][2 * r + 1]), pack_half2(c[x][1][2 * r], c[x][1][2 * r + 1]));
+                }
+            };
+            // (This loop, like the one over the quarters of the product above, is kept as a loop: a chunk's straight-line code is
+            // larger than the SM's instruction cache, and sixteen warps in different phases of it waited for instructions.)
+            // rows j' of the next state: P^T = Be^T A~, Kt^T = Ke^T + Be^T A~k
+#pragma unroll 1
+            for (int n = 0; n < 4; ++n) {
+                float c[2][2][4];
+                uint32_t X[4];
+                ldsm4_t(X, sb + kTiles + XK * kPanel + tile_cols(lane, 16 * ct, n));
+                if constexpr (kWide) row_power(PE + ct, n, X);
+                unpack8(X, c[1]);
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    uint32_t A[4];
+                    ldsm4_t(A, sb + kTiles + XB * kPanel + tile_cols(lane, 16 * b, n));
+                    if constexpr (kWide) row_power(PE + b, n, A);
+                    if (b == 0) {
+                        mma16816_first(c[0][0], A, U[0][b][0], U[0][b][2]);
+                        mma16816_first(c[0][1], A, U[0][b][1], U[0][b][3]);
+                    } else {
+                        mma16816(c[0][0], A, U[0][b][0], U[0][b][2]);
+                        mma16816(c[0][1], A, U[0][b][1], U[0][b][3]);
+                    }
+                    mma16816(c[1][0], A, U[1][b][0], U[1][b][2]);
+                    mma16816(c[1][1], A, U[1][b][1], U[1][b][3]);
+                }
+                put(n, c);
+            }
+            // rows t of the output: W = r e^{c} + A_rb A~, Ark = A_rk + A_rb A~k
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                float c[2][2][4];
+                uint32_t X[4];
+                ldsm4(X, sb + kTiles + XR * kPanel + tile_plain(lane, 16 * n, ct));
+                if constexpr (kWide) {
+                    const uint32_t fa = sb + kPow + (PX + n) * 64 + 16 * ct + 2 * q;
+                    const uint32_t f0 = power_pair(fa), f1 = power_pair(fa + 8);
+                    X[0] = mul_half2(X[0], f0);
+                    X[1] = mul_half2(X[1], f0);
+                    X[2] = mul_half2(X[2], f1);
+                    X[3] = mul_half2(X[3], f1);
+                }
+                unpack8(X, c[0]);
+                if (n >= ct) ldsm4(X, sb + kArk + (tri(n) + ct) * kBlk + blk_plain(lane));
+                else X[0] = X[1] = X[2] = X[3] = 0;
+                unpack8(X, c[1]);
+#pragma unroll
+                for (int b = 0; b <= n; ++b) {
+                    uint32_t A[4];
+                    ldsm4(A, sb + kArb + (tri(n) + b) * kBlk + blk_plain(lane));
+                    mma16816(c[0][0], A, U[0][b][0], U[0][b][2]);
+                    mma16816(c[0][1], A, U[0][b][1], U[0][b][3]);
+                    mma16816(c[1][0], A, U[1][b][0], U[1][b][2]);
+                    mma16816(c[1][1], A, U[1][b][1], U[1][b][3]);
+                }
+                put(4 + n, c);
+            }
+        };
+        if (wide) finish(std::true_type{});   // (two copies: merging them costs the common one a move per operand register)
+        else finish(std::false_type{});
+        if (kTma) fence_proxy_async();   // the tiles are handed back to TMA
+        __syncthreads();
+        if (kTma && tid == 0 && more) request(unit + gridDim.x);
+        // (the last chunk of this CTA: the scan may be set up)
+        if (!more) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
-    // ---------------- epilogue
-    __syncthreads();
-    if (*abort_flag) failed = true;
-    if (tid == 0) {
-        bulk_wait_group<0>();
-        if (failed) {
-            if (tma_pending) mbar_wait(bar_tma, tma_phase);   // tiles in flight must land before the CTA leaves
-            atomicExch(status, (int)kDevTimeout);
+    if (tid == 0 && *abort_flag) {
+        if (kTma) {   // what is in flight lands before the CTA leaves
+            mbar_wait(bar, phase, 100000u);
+            mbar_wait(bar + 1, phase, 100000u);
         }
+        atomicExch(status, (int)kDevTimeout);
     }
     tc_fence_before();
     __syncthreads();
@@ -619,437 +714,403 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, unsigned c
 }
 
 // ------------------------------------------------------------------------------------------
-// Kernel 2: the scan.  One CTA per chain.  Warps 0-7 own the 128 TMEM lanes twice over (two
-// column halves): lanes 0-63 are the state rows j' (fp32 state Z[j'][i] = S[i][j'] in registers),
-// lanes 64-127 the output tokens t.  Warp 8 streams operators, V tiles and the decay vectors into a
-// ring of stages, warp 9 issues the MMAs, warp 10 (four-stage variant) turns each V tile into fp16 as it
-// lands.  Per chunk
-// D[(j' | t)][i] = sum_k O[k][(j' | t)] [Z ; V][k][i]: the V half is issued as soon as a stage is
-// ready, only the Z half waits for the previous chunk.
+// Kernel 2: the scan, one CTA per chain.  D[n][i] = sum_k O[n][k] [Z; V][k][i] per chunk, four tcgen05 products of M = 128,
+// N = 64, K = 16 over V, issued a chunk ahead, and four over Z: TMEM lanes 0-63 are the rows j' of the next state (fp32 state Z[j'][i] = S[i][j'] in registers, two
+// warps per column half), lanes 64-127 the output tokens.  Warps 0-7 own the lanes twice over (two column halves), warp 8
+// streams records and V tiles into a ring, warp 9 issues, warps 10 and 11 turn V tiles into fp16 rows of [Z; V] ahead of time.
+//
+// Bound by the serial step of a chain: TMEM read, multiply-add with the decays, fp16 rows of Z, hand-over to the issuing
+// warp, the products over Z, their completion.  Hand-overs are hardware barriers (16 cycles; a satisfied mbarrier wait
+// written as a C loop costs a warp 127, with its loop in one asm statement 53): one that the state warps arrive on when
+// Z is written, one for the V products (tile converted, accumulator read back).  Only the completion of products and the
+// arrival of a stage go through an mbarrier.  (A version on warp-level matrix instructions, the state in their
+// accumulators, was bound by shared-memory bandwidth: each warp reads its operator columns and all of Z and V, 1.8 k
+// cycles a chunk.)
 // ------------------------------------------------------------------------------------------
-constexpr int kComputeWarps = 8;
-// The four-stage variant (one CTA per SM) has warps of its own for the V conversion and one for issuing the V half
-// of the products; in the two-stage variant
-// (two CTAs per SM, or beside an operator CTA) the compute warps do it between their other work, which measured
-// faster there (32 chains x 1024 chunks overlapped with the operator kernel: 1.41 against 1.53 ms).
-template <int NS> struct ScanWarps {
-    static constexpr bool kConvWarp = NS > 2;
-    static constexpr int kConv = 4;   // converter warps (one alone needs about 770 cycles per tile: as long as the whole serial step)
-    // warps 8 loader, 9 MMA issuer; then 10 converter, 11 issuer of the V half, 12.. the other converters
-    static constexpr int kThreads = (kComputeWarps + 2 + (kConvWarp ? 1 + kConv : 0)) * 32;
-};
-constexpr uint32_t kVecBytes = kVecFloats * 4;              // the chunk's two decay vectors
-
-// A stage: the operator, the fp16 V tile the tensor core reads and, for fp32 tensors, the fp32 tile as
-// it lands (bf16 tiles are converted in place).
-template <int NS, typename TIO>
-struct ScanSmem {
+template <typename TIO>
+struct Scan {
     static constexpr bool kF32 = sizeof(TIO) == 4;
-    static constexpr uint32_t kVLand = kOperatorBytes + (kF32 ? kPanel : 0u);      // where the V tile lands in a stage
+    static constexpr int kThreads = 12 * 32;
+    static constexpr int kStages = kF32 ? 3 : 4;
     static constexpr uint32_t kVBytes = kL * kN * sizeof(TIO);
-    static constexpr uint32_t kStage = kOperatorBytes + kPanel + (kF32 ? kVBytes : 0u);
-    static constexpr uint32_t kStages = 0;
-    static constexpr uint32_t kZ = NS * kStage;            // fp16 state tile Z[j][i]
-    static constexpr uint32_t kY = kZ + kPanel;            // two output tiles [t][i] on their way out (128-byte swizzle; fp32: two panels of 32 channels each)
+    static constexpr uint32_t kV = kOperatorBytes;                // stage: operator, V tile, vectors
+    static constexpr uint32_t kVec = kV + kVBytes;
+    static constexpr uint32_t kStage = kVec + 1024;
+    static constexpr uint32_t kZV = kStages * kStage;             // two tiles each of Z and V, 64 rows k of 64 channels, 128-byte swizzle
     static constexpr uint32_t kYTile = kL * kN * sizeof(TIO);
-    static constexpr uint32_t kVecs = kY + 2 * kYTile;     // per stage: e^{c_L}[64], e^{c_L - m}[64]
-    static constexpr uint32_t kBars = kVecs + NS * kVecBytes;
-    static constexpr uint32_t kBytes = kBars + 512 + 1024;   // + alignment slack
+    static constexpr uint32_t kY = kZV + 2 * 2 * kPanel;          // two output tiles (fp32: each two panels of 32 channels)
+    static constexpr uint32_t kBars = kY + 2 * kYTile;
+    static constexpr uint32_t kBytes = kBars + 128;
+    static_assert(kBytes <= 232448, "the scan exceeds an SM");
 };
-static_assert(ScanSmem<4, __nv_bfloat16>::kBytes <= 232448 && ScanSmem<3, float>::kBytes <= 232448, "scan stages exceed an SM");
 
 struct ScanMaps {
-    CUtensorMap v;   // [B*T, H*N]: bf16, box 64 x 64, 128-byte swizzle; fp32, box 64 x 64, no swizzle
-    CUtensorMap y;   // the output, same view: bf16, box 64 x 64; fp32, box 32 channels x 64 tokens; 128-byte swizzle
+    CUtensorMap v;   // [B*T, H*N], 128-byte swizzle: bf16, box 64 x 64; fp32, box 32 channels x 64 tokens (two per tile)
+    CUtensorMap y;   // the output, the same
 };
 
-template <int NS, typename TIO>
-__global__ void __launch_bounds__(ScanWarps<NS>::kThreads, NS <= 2 ? 2 : 1)
-wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, const unsigned char *__restrict__ operators,
-                       const float *__restrict__ vectors, const float *state_in, float *state_out,
-                       TIO *__restrict__ y, int *flags, int Tlen, int H, int chunk0,
-                       int seg_chunks, int nseg, int check_flags, int *status) {
-    using SM = ScanSmem<NS, TIO>;
-    constexpr bool kF32 = SM::kF32;
-    constexpr uint32_t kStageBytes = SM::kStage;
-    static_assert(!kF32 || ScanWarps<NS>::kConvWarp, "fp32 tiles need the converter warp");
+// Row of the Z tile (and position of the contraction index in the operator) of state column j, or of the V tile of token s.
+__device__ __forceinline__ int k_position(int j) {
+    return ((j >> 5) * 4 + ((j & 7) >> 1)) * 8 + ((j >> 4) & 1) * 4 + (j & 1) + (((j & 15) >> 3) << 1);
+}
+
+// Descriptor of the operator as K-major A operand without swizzle: 8 x 16-byte core matrices, 128 bytes apart along k, 2048
+// along n; one K-step is two of them.
+__device__ __forceinline__ uint64_t desc_operator(uint32_t addr, int ks) {
+    return (uint64_t)(((addr + (uint32_t)ks * 256u) >> 4) & 0x3fffu) | (uint64_t)(128u >> 4) << 16 | (uint64_t)(2048u >> 4) << 32 | (uint64_t)1 << 46;
+}
+
+// Token-by-token recomputation of one chain over tokens t0 .. t1 - 1, fp32 throughout: what a
+// CTA does when a value overflowed fp16 on the way, or the chain is flagged and no later kernel is there to take it.  Four
+// lanes per row; columns and sums in the order of the sequential scan (wkv7_seq.cu), whose bits it reproduces.
+template <typename TIO>
+__device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TIO *v, TIO *y, const float *s_in, float *s_out,
+                                                int bi, int h, int H, int Tlen, int t0, int t1) {
+    const int row = (int)threadIdx.x >> 2, c0 = ((int)threadIdx.x & 3) * 4;   // columns c0 + 16 kk + e
+    float S[4][4];
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[kk][e] = s_in ? s_in[row * kN + c0 + 16 * kk + e] : 0.f;
+    for (int t = t0; t < t1; ++t) {
+        const size_t o = (((size_t)bi * Tlen + t) * H + h) * kN;
+        auto f = [&](int x, int kk, int e) -> float { return static_cast<float>(static_cast<const TIO *>(in.p[x])[o + c0 + 16 * kk + e]); };
+        float p[4] = {}, yy[4] = {};
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) p[e] = fmaf(S[kk][e], f(XA, kk, e), p[e]);
+        float sa = (p[0] + p[1]) + (p[2] + p[3]);
+        sa += __shfl_xor_sync(0xffffffffu, sa, 1);
+        sa += __shfl_xor_sync(0xffffffffu, sa, 2);
+        const float vi = static_cast<float>(v[o + row]);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                S[kk][e] = fmaf(S[kk][e], expf(-expf(f(XW, kk, e))), fmaf(sa, f(XB, kk, e), vi * f(XK, kk, e)));
+                yy[e] = fmaf(S[kk][e], f(XR, kk, e), yy[e]);
+            }
+        float out = (yy[0] + yy[1]) + (yy[2] + yy[3]);
+        out += __shfl_xor_sync(0xffffffffu, out, 1);
+        out += __shfl_xor_sync(0xffffffffu, out, 2);
+        if (c0 == 0) {
+            if constexpr (sizeof(TIO) == 4) y[o + row] = out;
+            else y[o + row] = __float2bfloat16_rn(out);
+        }
+    }
+    if (s_out != nullptr) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s_out[row * kN + c0 + 16 * kk + e] = S[kk][e];
+    }
+}
+
+template <typename TIO>
+__global__ void __launch_bounds__(Scan<TIO>::kThreads, 1)
+wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs, const TIO *__restrict__ v,
+                       const unsigned char *__restrict__ records, const float *state_in, float *state_out,
+                       TIO *__restrict__ y, int *flags, int Tlen, int H, int chunk0, int n, int resolve_flagged, int *status) {
+    using SM = Scan<TIO>;
+    constexpr int NS = SM::kStages;
     extern __shared__ __align__(1024) unsigned char smem[];
     if (smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0) atomicExch(status, (int)kDevInternal);
         return;
     }
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // (launched behind the operator kernel with programmatic stream serialization: this kernel may start while
-    // that one is still finishing; everything below reads what it wrote)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    uint64_t *bar_full = reinterpret_cast<uint64_t *>(smem + SM::kBars);   // [NS] stage landed (bytes)
-    constexpr bool kConvWarp = ScanWarps<NS>::kConvWarp;
-    uint64_t *bar_vready = bar_full + NS;      // [NS] V tile converted to fp16 (one arrival per converting warp)
-    uint64_t *bar_empty = bar_vready + NS;     // [NS] the stage's MMAs are done
-    uint64_t *bar_accfull = bar_empty + NS;    // [2] accumulator complete
-    uint64_t *bar_accfree = bar_accfull + 2;   // [2] accumulator read back (8 arrivals)
-    uint64_t *bar_zready = bar_accfree + 2;    // state tile written (4 arrivals)
-    uint64_t *bar_vdone = bar_zready + 1;      // [2] (four-stage variant) the V half of the accumulator is complete
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_vdone + 2);
-    int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
-    int *chain_bad = abort_flag + 1;
-
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const uint32_t sb = smem_u32(smem);
+    uint64_t *bar_full = reinterpret_cast<uint64_t *>(smem + SM::kBars);   // [NS] a stage has landed
+    uint64_t *bar_empty = bar_full + NS;                                   // [NS] its products are done
+    uint64_t *bar_acc = bar_empty + NS;                                    // [2] an accumulator is complete
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_acc + 2);
+    volatile int *bad = reinterpret_cast<volatile int *>(tmem_slot + 1);   // bit 0: a wait expired, bit 1: a value is not finite
     const int chain = blockIdx.x;
     const int bi = chain / H, h = chain % H;
-    const int n = nseg;   // chunks this launch covers: chunk0 .. chunk0 + n - 1
-
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
             mbar_init(bar_full + s, 1);
-            mbar_init(bar_vready + s, kConvWarp ? ScanWarps<NS>::kConv : 8);      // one arrival per converting warp
             mbar_init(bar_empty + s, 1);
         }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(bar_accfull + a, 1);
-            mbar_init(bar_accfree + a, 8);                     // one arrival per compute warp
-        }
-        mbar_init(bar_zready, 4);                              // one arrival per state warp
-        mbar_init(bar_vdone + 0, 1);
-        mbar_init(bar_vdone + 1, 1);
+        mbar_init(bar_acc, 1);
+        mbar_init(bar_acc + 1, 1);
         mbar_fence_init();
-        *abort_flag = 0;
-        *chain_bad = 0;
+        *bad = 0;
         tma_prefetch_desc(&maps.v);
         tma_prefetch_desc(&maps.y);
     }
     if (warp == 0) tmem_alloc(tmem_slot, 128);
     tc_fence_before();
-    // A chain that is already flagged (by the operator kernel, or by the scan of an earlier segment) is
-    // recomputed by the next kernel in line: nothing to do here.
-    const bool skip_chain = __syncthreads_or(*reinterpret_cast<volatile int *>(&flags[chain]) != 0) != 0;
+    __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    if (skip_chain) {
-        tc_fence_before();
-        __syncthreads();
-        if (warp == 0) tmem_dealloc(tmem, 128);
-        return;
-    }
-    // A warp's threads meet, then its first lane arrives for all of them: an mbarrier takes one arrival at a time,
-    // and 128 or 256 of them in a row were a visible part of the chain's serial step.
-    auto warp_arrive = [&](uint64_t *bar) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar);
-    };
-    // A wait of a whole warp: every lane polls (one polling lane and a broadcast measured far slower: 264 against
-    // 231 us at 96 chains x 64 chunks), then a vote makes the outcome the same in all lanes, so that every lane takes
-    // the same way out of a loop whose lanes meet at warp barriers.
-    auto warp_wait = [&](uint64_t *bar, uint32_t parity, bool spin) -> bool {
-        const bool ok = spin ? mbar_wait_spin(bar, parity) : mbar_wait(bar, parity);
-        return __all_sync(0xffffffffu, ok) != 0;
-    };
-    const uint32_t sb = smem_u32(smem);
-    const unsigned char *ops = operators + ((size_t)chain * seg_chunks) * kOperatorBytes;
-    const float *vecs = vectors + ((size_t)chain * seg_chunks) * kVecFloats;
-
-    if (warp == kComputeWarps) {
-        // ---------------- loader: operator (bulk copy) + V tile (TMA) per stage
+    // (launched behind the operator kernel with programmatic stream serialization: everything below reads what it wrote)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const float *s_in = state_in ? state_in + (size_t)chain * kN * kN : nullptr;
+    float *s_out = state_out ? state_out + (size_t)chain * kN * kN : nullptr;
+    const unsigned char *rec = records + (size_t)chain * n * kRecord;
+    // A chain is flagged by any of its chunks, in this segment or (as the scan of that segment left it) an earlier one.
+    int mark = chunk0 > 0 && tid == 0 ? *reinterpret_cast<volatile int *>(&flags[chain]) : 0;
+    for (int c = tid; c < n; c += SM::kThreads) mark |= *reinterpret_cast<const int *>(rec + (size_t)c * kRecord + kMarkAt);
+    const bool flagged = __syncthreads_or(mark) != 0;
+    if (tid == 0) flags[chain] = flagged && !resolve_flagged;
+    const int t_end = min(Tlen, (chunk0 + n) * kL);
+    // Z of a chunk is written: four state warps arrive, the issuing warp waits.  V of chunk c is converted and the chunk's
+    // accumulator, the one of two chunks before, read back: two converters and four output warps arrive.
+    auto z_arrive = [] { asm volatile("bar.arrive 3, 160;" ::: "memory"); };
+    auto v_arrive = [](int c) { asm volatile("bar.arrive %0, 224;" ::"r"(4 + (c & 1)) : "memory"); };
+    uint32_t limit = 4000000u;   // polls a wait may take; after the first that expires this thread stops waiting, and the call reports it
+    auto wait = [&](uint64_t *b, uint32_t parity) { limit = mbar_wait_tight(b, parity, limit) ? limit : 1u; };
+    if (flagged) {
+        // (recomputed below, or by the next kernel in line)
+    } else if (warp == 8) {
+        // ---------------- loader
         if (lane == 0) {
-            int issued = 0, landed_needed = 0;
-            for (int c = 0; c < n; ++c) {
+            int issued = 0;
+            for (int c = 0; c < n; ++c, ++issued) {
                 const int s = c % NS;
-                if (c >= NS && !mbar_wait(bar_empty + s, (uint32_t)((c / NS - 1) & 1))) { atomicOr(abort_flag, 1); break; }
-                if (*reinterpret_cast<volatile int *>(abort_flag)) break;
-                if (!RWKV7_IN_RANGE(c < seg_chunks && (chunk0 + c) * kL < Tlen, status)) break;
-                mbar_expect_tx(bar_full + s, kOperatorBytes + SM::kVBytes + kVecBytes);
+                if (c >= NS) wait(bar_empty + s, (uint32_t)((c / NS - 1) & 1));
+                if (limit == 1u) break;
+                const uint32_t st = sb + s * SM::kStage;
+                mbar_expect_tx(bar_full + s, kOperatorBytes + kVectorBytes + SM::kVBytes);
+                const unsigned char *src = rec + (size_t)c * kRecord;
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(sb + SM::kStages + s * kStageBytes), "l"(ops + (size_t)c * kOperatorBytes),
-                               "r"(kOperatorBytes), "r"(smem_u32(bar_full + s))
+                             ::"r"(st), "l"(src), "r"(kOperatorBytes), "r"(smem_u32(bar_full + s))
                              : "memory");
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(sb + SM::kVecs + s * kVecBytes), "l"(vecs + (size_t)c * kVecFloats),
-                               "r"(kVecBytes), "r"(smem_u32(bar_full + s))
+                             ::"r"(st + SM::kVec), "l"(src + kDecayAt), "r"(kVectorBytes), "r"(smem_u32(bar_full + s))
                              : "memory");
-                tma_load_2d(smem + SM::kStages + s * kStageBytes + SM::kVLand, &maps.v, h * kN,
-                            bi * Tlen + (chunk0 + c) * kL, bar_full + s);
-                ++issued;
+                const int trow = bi * Tlen + (chunk0 + c) * kL;
+                tma_load_2d(smem + s * SM::kStage + SM::kV, &maps.v, h * kN, trow, bar_full + s);
+                if (SM::kF32) tma_load_2d(smem + s * SM::kStage + SM::kV + SM::kVBytes / 2, &maps.v, h * kN + 32, trow, bar_full + s);
             }
-            // On an abort the copies already requested must land before the CTA gives up its shared memory.
-            if (*reinterpret_cast<volatile int *>(abort_flag)) {
-                (void)landed_needed;
-                for (int c = max(0, issued - NS); c < issued; ++c) mbar_wait(bar_full + c % NS, (uint32_t)((c / NS) & 1));
-            }
+            // what has been requested lands before the CTA leaves, whatever became of the warps that read it
+            for (int c = max(0, issued - NS); c < issued; ++c) mbar_wait(bar_full + c % NS, (uint32_t)((c / NS) & 1));
         }
-    } else if (warp == kComputeWarps + 1) {
-        // ---------------- MMA issuer.  Two-stage variant: both halves of the chunk's product.  Four-stage variant:
-        // the Z half only (k = j: rows 0..63 of the operator against Z[j][i]); the V half is issued ahead of time by
-        // another thread into the same accumulator, and since products issued by different threads are ordered
-        // only through a barrier, this thread waits until that half is complete before it adds to it.
-        if (lane == 0) {
-            constexpr uint32_t id = idesc16(128, 64, true, true);
-            for (int c = 0; c < n; ++c) {
-                const int s = c % NS, a = c & 1;
-                const uint32_t op = sb + SM::kStages + s * kStageBytes, vt = op + kOperatorBytes;
-                if constexpr (kConvWarp) {
-                    if (!mbar_wait(bar_vdone + a, (uint32_t)((c >> 1) & 1))) { atomicOr(abort_flag, 1); break; }
-                } else {
-                    if (!mbar_wait(bar_vready + s, (uint32_t)((c / NS) & 1))) { atomicOr(abort_flag, 1); break; }
-                    if (!mbar_wait(bar_accfree + a, (uint32_t)(((c >> 1) & 1) ^ 1))) { atomicOr(abort_flag, 1); break; }
-                    tc_fence_after();
-#pragma unroll
-                    for (int ks = 0; ks < 4; ++ks)   // k = 64 + s: rows 64.. of both operator panels against V[s][i]
-                        umma_f16(tmem + a * 64, dMN(op, 2 * kPanel, 4 + ks), dMN(vt, kPanel, ks), id, ks > 0);
-                }
-                if (!mbar_wait_spin(bar_zready, (uint32_t)(c & 1))) { atomicOr(abort_flag, 1); break; }
+        __syncwarp();
+    } else if (warp == 9) {
+        // ---------------- issuing warp
+        constexpr uint32_t id = make_idesc(kFmtF16, 128, 64, false, true);
+        auto v_products = [&](int c) {
+            const int s = c % NS, a = c & 1;
+            wait(bar_full + s, (uint32_t)((c / NS) & 1));
+            asm volatile("bar.sync %0, 224;" ::"r"(4 + a) : "memory");
+            if (elect_one()) {
                 tc_fence_after();
-#pragma unroll
-                for (int ks = 0; ks < 4; ++ks)   // k = j: rows 0..63 against Z[j][i]
-                    umma_f16(tmem + a * 64, dMN(op, 2 * kPanel, ks), dMN(sb + SM::kZ, kPanel, ks), id, true);
-                umma_commit(bar_accfull + a);
-                umma_commit(bar_empty + s);
-            }
-        }
-    } else if (kConvWarp && warp == kComputeWarps + 3) {
-        // ---------------- issuer of the V half (four-stage variant): O[64 + s][(j' | t)] against V[s][i], as soon as
-        // the tile is converted and the accumulator has been read back, one chunk ahead of the chain.
-        if (lane == 0) {
-            constexpr uint32_t id = idesc16(128, 64, true, true);
-            for (int c = 0; c < n; ++c) {
-                const int s = c % NS, a = c & 1;
-                const uint32_t op = sb + SM::kStages + s * kStageBytes, vt = op + kOperatorBytes;
-                if (!mbar_wait(bar_vready + s, (uint32_t)((c / NS) & 1))) { atomicOr(abort_flag, 1); break; }
-                if (!mbar_wait(bar_accfree + a, (uint32_t)(((c >> 1) & 1) ^ 1))) { atomicOr(abort_flag, 1); break; }
-                tc_fence_after();
+                const uint32_t op = sb + s * SM::kStage, vt = sb + SM::kZV + a * 2 * kPanel + kPanel;
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                    umma_f16(tmem + a * 64, dMN(op, 2 * kPanel, 4 + ks), dMN(vt, kPanel, ks), id, ks > 0);
-                umma_commit(bar_vdone + a);
+                    umma_f16(tmem + a * 64, desc_operator(op, 4 + ks), make_smem_desc(vt + ks * 2048u, kPanel, 1024u), id, ks > 0);
             }
-        }
-    } else if (kConvWarp && (warp == kComputeWarps + 2 || warp >= kComputeWarps + 4)) {
-        // ---------------- V converters.  The V tile arrives as bf16 and the tensor core wants both operands
-        // of a product in one format: these warps turn it into fp16 in place (element by element, the layout
-        // is untouched; each a quarter of the tile) as soon as the stage has landed, well ahead of the product
-        // that reads it.  (Done by the compute warps between their other work, the conversion sat on the chain's
-        // serial path.)
-        constexpr int kConv = ScanWarps<NS>::kConv;
-        const int ci = warp == kComputeWarps + 2 ? 0 : warp - (kComputeWarps + 3);   // 0 .. kConv - 1
+            __syncwarp();
+        };
+        if (n > 0) v_products(0);
         for (int c = 0; c < n; ++c) {
-            const int s = c % NS;
-            if (!warp_wait(bar_full + s, (uint32_t)((c / NS) & 1), false)) { atomicOr(abort_flag, 1); break; }
-            unsigned char *vt = smem + SM::kStages + s * kStageBytes + kOperatorBytes;
-            if constexpr (!kF32) {
-                uint4 *p = reinterpret_cast<uint4 *>(vt);
-                constexpr int kShare = (int)(kPanel / 16 / 32) / kConv;
-                uint4 x[kShare];
+            const int s = c % NS, a = c & 1;
+            asm volatile("bar.sync 3, 160;" ::: "memory");
+            if (elect_one()) {
+                tc_fence_after();
+                const uint32_t op = sb + s * SM::kStage, zt = sb + SM::kZV + a * 2 * kPanel;
 #pragma unroll
-                for (int q = 0; q < kShare; ++q) x[q] = p[(ci * kShare + q) * 32 + lane];
+                for (int ks = 0; ks < 4; ++ks)
+                    umma_f16(tmem + a * 64, desc_operator(op, ks), make_smem_desc(zt + ks * 2048u, kPanel, 1024u), id, true);
+                umma_commit(bar_acc + a);
+                umma_commit(bar_empty + s);
+            }
+            __syncwarp();
+            if (c + 1 < n) v_products(c + 1);
+        }
+    } else if (warp >= 10) {
+        // ---------------- V converters: tile -> fp16 rows in the order of the contraction index, 16-byte pieces; rows past the sequence's end belong to
+        // another one, whatever they hold stays out of the sums
+        constexpr int kShare = kL * kN / 8 / 32 / 2;
+        for (int c = 0; c < n; ++c) {
+            const int s = c % NS, a = c & 1;
+            wait(bar_full + s, (uint32_t)((c / NS) & 1));
+            if (c >= 2) wait(bar_acc + a, (uint32_t)(((c >> 1) - 1) & 1));   // the products that last read this tile
+            const uint32_t vt = sb + s * SM::kStage + SM::kV, out = sb + SM::kZV + a * 2 * kPanel + kPanel;
+            const int valid = Tlen - (chunk0 + c) * kL;
 #pragma unroll
-                for (int q = 0; q < kShare; ++q) {
-                    uint32_t *xs = &x[q].x;
+            for (int k0 = 0; k0 < kShare; k0 += 4) {
+                uint32_t x[4][4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float2 f = unpack_bf2(xs[e]);
-                        xs[e] = pack_h2(f.x, f.y);
+                for (int k = 0; k < 4; ++k) {
+                    const int p = ((warp - 10) * kShare + k0 + k) * 32 + lane, t = p >> 3, cg = p & 7;
+                    if constexpr (!SM::kF32) {
+                        lds128(x[k], vt + off16(t, cg * 8));
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) x[k][e] = bf2_to_half2(x[k][e]);
+                    } else {                                // two pieces of a panel of 32 channels
+                        const uint32_t row = vt + (cg >> 2) * (SM::kVBytes / 2) + t * 128;
+                        const float4 lo = lds_f4(row + (((2 * cg & 7) ^ (t & 7)) << 4)), hi = lds_f4(row + (((2 * cg & 7) + 1) ^ (t & 7)) * 16);
+                        x[k][0] = pack_half2(lo.x, lo.y);
+                        x[k][1] = pack_half2(lo.z, lo.w);
+                        x[k][2] = pack_half2(hi.x, hi.y);
+                        x[k][3] = pack_half2(hi.z, hi.w);
                     }
-                    p[(ci * kShare + q) * 32 + lane] = x[q];
+                    if (t >= valid) x[k][0] = x[k][1] = x[k][2] = x[k][3] = 0;
                 }
-            } else {
-                // fp32 tile [t][i] (rows of 256 bytes) -> fp16 panel: eight channels of one token per step
-                const unsigned char *land = smem + SM::kStages + s * kStageBytes + SM::kVLand;
-                constexpr int kShare = kL * kN / 8 / 32 / kConv;
 #pragma unroll
-                for (int q = 0; q < kShare; ++q) {
-                    const int idx = (ci * kShare + q) * 32 + lane, t = idx >> 3, cg = idx & 7;
-                    const float4 x0 = *reinterpret_cast<const float4 *>(land + t * (kN * 4) + cg * 32);
-                    const float4 x1 = *reinterpret_cast<const float4 *>(land + t * (kN * 4) + cg * 32 + 16);
-                    *reinterpret_cast<uint4 *>(vt + off16(t, cg * 8)) =
-                        make_uint4(pack_h2(x0.x, x0.y), pack_h2(x0.z, x0.w), pack_h2(x1.x, x1.y), pack_h2(x1.z, x1.w));
+                for (int k = 0; k < 4; ++k) {
+                    const int p = ((warp - 10) * kShare + k0 + k) * 32 + lane;
+                    sts128(out + off16(k_position(p >> 3), (p & 7) * 8), x[k]);
                 }
             }
             fence_proxy_async();
-            warp_arrive(bar_vready + s);
+            v_arrive(c);
         }
     } else {
         const int quarter = warp & 3, hf = warp >> 2;
-        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + hf * 32;
         const int i0 = hf * 32;                       // this thread's 32 value channels
-        // Two-stage variant: the 256 compute threads turn the V tile into fp16 in place, 32 bytes each, one
-        // chunk ahead of the product that reads it.
-        auto convert_v = [&](int c) -> bool {
-            if constexpr (kConvWarp) return true;
-            const int s = c % NS;
-            if (!warp_wait(bar_full + s, (uint32_t)((c / NS) & 1), false)) return false;
-            uint4 *p = reinterpret_cast<uint4 *>(smem + SM::kStages + s * kStageBytes + kOperatorBytes + tid * 32);
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                uint4 x = p[q];
-                uint32_t *xs = &x.x;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 f = unpack_bf2(xs[e]);
-                    xs[e] = pack_h2(f.x, f.y);
-                }
-                p[q] = x;
-            }
-            fence_proxy_async();
-            warp_arrive(bar_vready + s);
-            return true;
-        };
         if (quarter < 2) {
             // ---------------- state rows j'
             const int jp = quarter * 32 + lane;
-            float Z[32];
+            const uint32_t zrow = sb + SM::kZV + off16(k_position(jp), 0);
+            const uint32_t sw = ((uint32_t)k_position(jp) & 7u) << 4;
+            float2 Z[16];
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
-                Z[e] = state_in ? state_in[((size_t)chain * kN + i0 + e) * kN + jp] : 0.f;
-            auto put_tile = [&]() {
+            for (int e = 0; e < 16; ++e)
+                Z[e] = s_in ? make_float2(s_in[(i0 + 2 * e) * kN + jp], s_in[(i0 + 2 * e + 1) * kN + jp]) : make_float2(0.f, 0.f);
+            // this row's scalars of a chunk: e^{c_L}, fx, factor of P and Kt
+            auto load_vec = [&](int c, float &gx, float &fx, float &g2) {
+                const int s = c % NS;
+                wait(bar_full + s, (uint32_t)((c / NS) & 1));
+                const unsigned char *vec = smem + s * SM::kStage + SM::kVec;
+                gx = *reinterpret_cast<const float *>(vec + jp * 4);
+                const int ef = *reinterpret_cast<const signed char *>(vec + 256 + jp), eg = *reinterpret_cast<const signed char *>(vec + 320 + jp);
+                fx = gx * exp2_of(ef);
+                g2 = exp2_of(-eg);
+            };
+            // the state a chunk starts with, as operand: times fx, fp16
+            auto put_z = [&](int c, float fx) {
+                const float2 f = make_float2(fx, fx);
 #pragma unroll
-                for (int e8 = 0; e8 < 4; ++e8) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int e2 = 0; e2 < 4; ++e2) w[e2] = pack_h2(Z[e8 * 8 + 2 * e2], Z[e8 * 8 + 2 * e2 + 1]);
-                    if (RWKV7_IN_RANGE(off16(jp, i0 + e8 * 8) + 16 <= kPanel, status))
-                        *reinterpret_cast<uint4 *>(smem + SM::kZ + off16(jp, i0 + e8 * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
+                for (int e = 0; e < 4; ++e) {
+                    const uint32_t x[4] = {pack2(mul2(Z[4 * e], f)), pack2(mul2(Z[4 * e + 1], f)), pack2(mul2(Z[4 * e + 2], f)), pack2(mul2(Z[4 * e + 3], f))};
+                    // (16-byte pieces XOR-ed with the row: zrow is piece 0's place)
+                    sts128((zrow ^ sw) + (c & 1) * 2 * kPanel + ((uint32_t)((i0 / 8 + e) << 4) ^ sw), x);
                 }
                 fence_proxy_async();
-                warp_arrive(bar_zready);
+                tc_fence_before();
+                z_arrive();
             };
-            put_tile();
-            // this row's two decay factors per chunk come with the stage; they are read one chunk ahead (the
-            // stage of chunk c + 1 cannot be refilled before this thread has handed over that chunk's state)
-            const float *ring = reinterpret_cast<const float *>(smem + SM::kVecs);
-            auto load_gg = [&](int c, float2 &out) -> bool {
-                if (c >= n) { out = make_float2(1.f, 0.f); return true; }
-                const int s = c % NS;
-                // (in the two-stage variant this thread has just waited for the stage in convert_v)
-                if (kConvWarp && !warp_wait(bar_full + s, (uint32_t)((c / NS) & 1), false)) return false;
-                out = make_float2(ring[s * kVecFloats + jp], ring[s * kVecFloats + 64 + jp]);
-                return true;
-            };
-            float2 gg, gg_next = make_float2(1.f, 0.f);
-            if (n > 0 && !convert_v(0)) atomicOr(abort_flag, 1);
-            if (!load_gg(0, gg)) atomicOr(abort_flag, 1);
+            float gx, fx, g2, gxn = 1.f, fxn = 1.f, g2n = 0.f;
+            load_vec(0, gx, fx, g2);
+            put_z(0, fx);
             for (int c = 0; c < n; ++c) {
                 const int a = c & 1;
-                // (the tensor core is busy with this chunk's state product: time for the next chunk's vectors and tile)
-                if (c + 1 < n && !convert_v(c + 1)) { atomicOr(abort_flag, 1); break; }
-                if (!load_gg(c + 1, gg_next)) { atomicOr(abort_flag, 1); break; }
-                // (polled without suspending: this wait is on the serial path of the chain)
-                if (!warp_wait(bar_accfull + a, (uint32_t)((c >> 1) & 1), true)) { atomicOr(abort_flag, 1); break; }
+                if (c + 1 < n) load_vec(c + 1, gxn, fxn, g2n);   // (while the products run)
+                wait(bar_acc + a, (uint32_t)((c >> 1) & 1));
                 tc_fence_after();
-                uint32_t v[32];
-                tmem_ld32(tmem + lane_base + a * 64 + i0, v);
+                uint32_t d[32];
+                tmem_ld32(acc + a * 64, d);
                 tmem_ld_wait();
-                tc_fence_before();
-                warp_arrive(bar_accfree + a);
+                const float2 gx2 = make_float2(gx, gx), gg = make_float2(g2, g2);
 #pragma unroll
-                for (int e = 0; e < 32; ++e) Z[e] = fmaf(gg.y, __uint_as_float(v[e]), gg.x * Z[e]);
-                if (c + 1 < n) put_tile();
-                gg = gg_next;
+                for (int e = 0; e < 16; ++e)
+                    Z[e] = __ffma2_rn(gx2, Z[e], mul2(gg, make_float2(__uint_as_float(d[2 * e]), __uint_as_float(d[2 * e + 1]))));
+                if (c + 1 < n) put_z(c + 1, fxn);
+                gx = gxn;
+                g2 = g2n;
             }
-            // A non-finite operator (fp16 overflow upstream) shows in the state for good: flag the chain.
-            bool bad = false;
+            bool off = false;   // a non-finite operand upstream stays in the state for good
 #pragma unroll
-            for (int e = 0; e < 32; ++e) bad |= !(fabsf(Z[e]) <= 3.0e38f);
-            if (bad) atomicOr(chain_bad, 1);
-            asm volatile("bar.sync 1, 256;" ::: "memory");   // the eight compute warps: every flag of this chain is in
-            const bool skip = *chain_bad != 0 || (check_flags && flags[chain] != 0);   // flagged chains are recomputed from state_in
-            if (state_out != nullptr && !skip && !*reinterpret_cast<volatile int *>(abort_flag)) {
+            for (int e = 0; e < 16; ++e) off |= !(fabsf(Z[e].x) <= 3.0e38f) | !(fabsf(Z[e].y) <= 3.0e38f);
+            if (off) atomicOr(const_cast<int *>(bad), 2);
+            if (limit == 1u) atomicOr(const_cast<int *>(bad), 1);
+            // the eight compute warps have all reported before the state is written: it may alias what a recomputation
+            // starts from
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (*bad == 0 && s_out != nullptr) {
 #pragma unroll
-                for (int e = 0; e < 32; ++e)
-                    if (RWKV7_IN_RANGE(i0 + e < kN && jp < kN, status)) state_out[((size_t)chain * kN + i0 + e) * kN + jp] = Z[e];
+                for (int e = 0; e < 16; ++e)
+                    if (RWKV7_IN_RANGE(i0 + 2 * e + 1 < kN && jp < kN, status)) {
+                        s_out[(i0 + 2 * e) * kN + jp] = Z[e].x;
+                        s_out[(i0 + 2 * e + 1) * kN + jp] = Z[e].y;
+                    }
             }
         } else {
-            // ---------------- output tokens t.  A chunk's y tile is staged in shared memory (one of two
-            // buffers, 128-byte swizzle) and leaves by one bulk tensor store; a partial last chunk is stored
-            // by the threads themselves.
+            // ---------------- output tokens t.  A chunk's y tile is staged in shared memory (one of two buffers) and leaves
+            // by a bulk tensor store; a partial last chunk is stored by the threads themselves.
             const int tq = (quarter - 2) * 32 + lane;     // token within the chunk
             const bool elected = warp == 2 && lane == 0;
-            float ysum = 0.f;    // a non-finite output (or one too large for bf16) flags the chain for recomputation
-            // After an expired wait this thread stops waiting but still walks the loop, so that the four
-            // warps keep meeting at the named barrier below (the call then reports a time-out).
-            bool dead = n > 0 && !convert_v(0);
+            float ysum = 0.f;    // a non-finite output makes the sum non-finite for good
+            v_arrive(0);
+            if (n > 1) v_arrive(1);
             for (int c = 0; c < n; ++c) {
                 const int a = c & 1;
-                if (!dead && c + 1 < n && !convert_v(c + 1)) dead = true;
-                if (!dead && !warp_wait(bar_accfull + a, (uint32_t)((c >> 1) & 1), false)) dead = true;
+                wait(bar_acc + a, (uint32_t)((c >> 1) & 1));
                 tc_fence_after();
-                uint32_t v[32];
-                tmem_ld32(tmem + lane_base + a * 64 + i0, v);
+                uint32_t d[32];
+                tmem_ld32(acc + a * 64, d);
                 tmem_ld_wait();
                 tc_fence_before();
-                warp_arrive(bar_accfree + a);
+                if (c + 2 < n) v_arrive(c + 2);
                 const int t0 = (chunk0 + c) * kL;
-                if constexpr (!kF32) {
-                    uint32_t w[16];
+                float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int e = 0; e < 32; ++e) sum[e & 3] += fabsf(__uint_as_float(d[e]));
+                ysum += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+                constexpr int kPieces = SM::kF32 ? 8 : 4;   // 16-byte pieces of this thread's channels
+                uint32_t w[4 * kPieces];
+                if constexpr (!SM::kF32) {
 #pragma unroll
                     for (int e2 = 0; e2 < 16; ++e2) {
-                        const float x0 = __uint_as_float(v[2 * e2]), x1 = __uint_as_float(v[2 * e2 + 1]);
-                        ysum += fabsf(x0) + fabsf(x1);   // (a non-finite output makes the sum non-finite for good)
-                        const __nv_bfloat162 b2 = __floats2bfloat162_rn(x0, x1);
+                        const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(d[2 * e2]), __uint_as_float(d[2 * e2 + 1]));
                         w[e2] = *reinterpret_cast<const uint32_t *>(&b2);
                     }
-                    if (t0 + kL <= Tlen) {
-                        unsigned char *stage = smem + SM::kY + a * SM::kYTile;
-                        // the store that last read this buffer (two chunks ago) must be done with it
-                        if (elected) bulk_wait_group_read<1>();
-                        asm volatile("bar.sync 2, 128;" ::: "memory");
-#pragma unroll
-                        for (int e8 = 0; e8 < 4; ++e8)
-                            if (RWKV7_IN_RANGE(off16(tq, i0 + e8 * 8) + 16 <= kPanel, status))
-                                *reinterpret_cast<uint4 *>(stage + off16(tq, i0 + e8 * 8)) = make_uint4(w[4 * e8], w[4 * e8 + 1], w[4 * e8 + 2], w[4 * e8 + 3]);
-                        fence_proxy_async();
-                        asm volatile("bar.sync 2, 128;" ::: "memory");
-                        if (elected) {
-                            tma_store_2d(&maps.y, h * kN, bi * Tlen + t0, stage);
-                            bulk_commit_group();
-                        }
-                    } else if (t0 + tq < Tlen) {
-                        TIO *dst = y + (((size_t)bi * Tlen + t0 + tq) * H + h) * kN + i0;
-#pragma unroll
-                        for (int e8 = 0; e8 < 4; ++e8)
-                            *reinterpret_cast<uint4 *>(dst + e8 * 8) = make_uint4(w[4 * e8], w[4 * e8 + 1], w[4 * e8 + 2], w[4 * e8 + 3]);
-                    }
                 } else {
-                    // fp32 output: this thread's 32 channels are one 128-byte row of panel `hf` of the staged tile
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) ysum += fabsf(__uint_as_float(v[e]));
-                    if (t0 + kL <= Tlen) {
-                        unsigned char *stage = smem + SM::kY + a * SM::kYTile + hf * (SM::kYTile / 2);
-                        if (elected) bulk_wait_group_read<1>();   // (a chunk's two stores form one group)
-                        asm volatile("bar.sync 2, 128;" ::: "memory");
+                    for (int e = 0; e < 32; ++e) w[e] = d[e];
+                }
+                if (t0 + kL <= Tlen) {
+                    // (bf16: 128-byte rows of 64 channels; fp32: two panels of 32 channels)
+                    const uint32_t stage = sb + SM::kY + a * SM::kYTile + (SM::kF32 ? hf * (SM::kYTile / 2) : 0u) + (uint32_t)tq * 128u;
+                    if (elected) bulk_wait_group_read<1>();   // the store that last read this buffer (two chunks ago) is done with it
+                    asm volatile("bar.sync 2, 128;" ::: "memory");
 #pragma unroll
-                        for (int e4 = 0; e4 < 8; ++e4) {
-                            const uint32_t o = (uint32_t)tq * 128u + (((uint32_t)e4 ^ ((uint32_t)tq & 7u)) << 4);
-                            if (RWKV7_IN_RANGE(o + 16 <= SM::kYTile / 2, status))
-                                *reinterpret_cast<uint4 *>(stage + o) = make_uint4(v[4 * e4], v[4 * e4 + 1], v[4 * e4 + 2], v[4 * e4 + 3]);
-                        }
-                        fence_proxy_async();
-                        asm volatile("bar.sync 2, 128;" ::: "memory");
-                        if (elected) {
-                            unsigned char *tile = smem + SM::kY + a * SM::kYTile;
-                            tma_store_2d(&maps.y, h * kN, bi * Tlen + t0, tile);
-                            tma_store_2d(&maps.y, h * kN + 32, bi * Tlen + t0, tile + SM::kYTile / 2);
-                            bulk_commit_group();
-                        }
-                    } else if (t0 + tq < Tlen) {
-                        TIO *dst = y + (((size_t)bi * Tlen + t0 + tq) * H + h) * kN + i0;
-#pragma unroll
-                        for (int e4 = 0; e4 < 8; ++e4)
-                            *reinterpret_cast<uint4 *>(dst + e4 * 4) = make_uint4(v[4 * e4], v[4 * e4 + 1], v[4 * e4 + 2], v[4 * e4 + 3]);
+                    for (int e = 0; e < kPieces; ++e) {
+                        const uint32_t x[4] = {w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]};
+                        const uint32_t o = (uint32_t)(((SM::kF32 ? 0 : i0 / 8) + e) ^ (tq & 7)) << 4;
+                        if (RWKV7_IN_RANGE(o + 16 <= 128u, status)) sts128(stage + o, x);
                     }
+                    fence_proxy_async();
+                    asm volatile("bar.sync 2, 128;" ::: "memory");
+                    if (elected) {
+                        unsigned char *tile = smem + SM::kY + a * SM::kYTile;
+                        tma_store_2d(&maps.y, h * kN, bi * Tlen + t0, tile);
+                        if (SM::kF32) tma_store_2d(&maps.y, h * kN + 32, bi * Tlen + t0, tile + SM::kYTile / 2);
+                        bulk_commit_group();
+                    }
+                } else if (t0 + tq < Tlen) {
+                    TIO *dst = y + (((size_t)bi * Tlen + t0 + tq) * H + h) * kN + i0;
+#pragma unroll
+                    for (int e = 0; e < kPieces; ++e)
+                        *reinterpret_cast<uint4 *>(dst + e * (16 / sizeof(TIO))) = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
                 }
             }
-            if (elected) bulk_wait_group<0>();   // the stores read this CTA's shared memory
-            if (dead) atomicOr(abort_flag, 1);
-            if (!(ysum <= 3.0e38f)) atomicOr(chain_bad, 1);
+            if (elected) bulk_wait_group<0>();   // (a recomputation below may write the same rows)
+            if (!(ysum <= 3.0e38f)) atomicOr(const_cast<int *>(bad), 2);
+            if (limit == 1u) atomicOr(const_cast<int *>(bad), 1);
             asm volatile("bar.sync 1, 256;" ::: "memory");
         }
     }
-    __syncthreads();
-    if (tid == 0) {
-        if (*abort_flag) atomicExch(status, (int)kDevTimeout);
-        if (*chain_bad) atomicOr(&flags[chain], 1);
-    }
+    if (limit == 1u) atomicOr(const_cast<int *>(bad), 1);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 128);
+    if (*bad & 1) {
+        if (tid == 0) atomicExch(status, (int)kDevTimeout);
+        return;
+    }
+    // A value beyond fp16 (or a flagged chain that nobody else takes): the chain once more, token by token, from the state
+    // this launch started with, which is still untouched.
+    if (((flagged && resolve_flagged) || (*bad & 2)) && tid < 256)
+        scan_rows_by_token<TIO>(ptrs, v, y, s_in, s_out, bi, h, H, Tlen, chunk0 * kL, t_end);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -1079,8 +1140,7 @@ constexpr size_t kOperatorBudget = (size_t)768 << 20;
 
 // ---- host side ------------------------------------------------------------------------------
 //
-// Workspace: [flags: one int per chain][kMaxSegments work counters][carried fp32 state per chain]
-//            [vectors of buffer 0][vectors of buffer 1][operators of buffer 0][operators of buffer 1].
+// Workspace: [flags: one int per chain][4 KB spare][carried fp32 state per chain][records of buffer 0][records of buffer 1].
 // A call is cut into segments of chunks.  With at most as many chains as SMs the scan of a segment
 // leaves most of the GPU idle (one latency-bound CTA per chain), so it runs on a second stream beside
 // the operator kernel of the next segment, which writes the other buffer.
@@ -1090,7 +1150,7 @@ namespace {
 constexpr int kMaxSegments = 1024;
 
 struct WorkspaceLayout {
-    size_t flags, counters, carry, vectors[2], operators[2], total;
+    size_t flags, carry, records[2], total;
     size_t seg;      // chunks per segment
     int buffers;     // 1 or 2
 };
@@ -1104,16 +1164,11 @@ WorkspaceLayout layout_for(size_t chains, size_t seg, int buffers) {
     l.seg = seg;
     l.buffers = buffers;
     l.flags = 0;
-    l.counters = align_up(chains * sizeof(int));
-    l.carry = l.counters + align_up(kMaxSegments * sizeof(int));
+    l.carry = align_up(chains * sizeof(int)) + align_up(kMaxSegments * sizeof(int));
     size_t off = l.carry + align_up(chains * kN * kN * sizeof(float));
     for (int b = 0; b < 2; ++b) {
-        l.vectors[b] = off;
-        if (b < buffers) off += chains * seg * kVecFloats * sizeof(float);   // (512 bytes per chunk: stays aligned)
-    }
-    for (int b = 0; b < 2; ++b) {
-        l.operators[b] = off;
-        if (b < buffers) off += chains * seg * kOperatorBytes;
+        l.records[b] = off;
+        if (b < buffers) off += chains * seg * kRecord;
     }
     l.total = off;
     return l;
@@ -1123,13 +1178,12 @@ WorkspaceLayout layout_for(size_t chains, size_t seg, int buffers) {
 // overlaps) against the few microseconds a segment boundary costs, within the operator budget.
 //
 // When the scan of a segment may run beside the operator kernel of the next one.  The scan is one latency-bound
-// CTA per chain (0.7 us per chunk with an SM to itself), the operator kernel throughput work that fills every SM
-// twice over (8.7 us per chunk and CTA): with x = chains x 8.7 / (2 SMs x 0.7) the two in sequence take (x + 1)
-// scan times.  On SM partitions (the scans on `chains` SMs rounded up to eight, the operator kernel on the rest)
+// CTA per chain (0.75 us per chunk), the operator kernel throughput work that fills every SM (2.8 us per chunk and SM):
+// with x = chains x 2.8 / (SMs x 0.75) the two in sequence take (x + 1) scan times.  On SM partitions (the scans on `chains` SMs rounded up to eight, the operator kernel on the rest)
 // they take max(x SMs / (SMs - R), 1): a gain while x SMs / (SMs - R) < x + 1, which on 148 SMs is up to about
 // 40 chains.  Measured (B200, 148 SMs; in sequence / on partitions, us): 12 chains x 1024 chunks 945 / 799;
 // 32 x 1024 1489 / 1336; 64 x 512 1195 / 1638.  Without partitions the scan CTAs sit beside operator CTAs (the
-// operator kernel then launches 2 SMs - chains CTAs) and run at half their pace: 32 x 1024 1381-1411, but 12 x 1024
+// operator kernel then leaves as many SMs' worth of CTAs out as there are chains) and run at half their pace: 32 x 1024 1381-1411, but 12 x 1024
 // 1204 and 64 x 512 1424, both worse than in sequence; that schedule is kept for 24 to 40 chains where the driver
 // offers no partitions.  Short sequences do not pay either way (32 chains x 128 chunks 257 against 236 us: the
 // first operator kernel and the last scan overlap nothing; on partitions 32 x 128 216 against 207 us, but 24 x 192
@@ -1151,7 +1205,7 @@ size_t preferred_segment(size_t chains, size_t nchunks, bool overlap) {
         while ((nseg + 1) * (nseg + 1) * 16 <= nchunks && nseg < 32) ++nseg;   // about sqrt(nchunks / 16): measured best (1024 chunks: 8 segments)
         seg = (nchunks + nseg - 1) / nseg;
     }
-    const size_t per_chunk = chains * kOperatorBytes * (overlap ? 2 : 1);
+    const size_t per_chunk = chains * kRecord * (overlap ? 2 : 1);
     if (seg * per_chunk > kOperatorBudget) seg = kOperatorBudget / per_chunk;
     if ((nchunks + seg - 1) / (seg ? seg : 1) > (size_t)kMaxSegments) seg = (nchunks + kMaxSegments - 1) / kMaxSegments;
     return seg < 1 ? 1 : seg;
@@ -1314,7 +1368,8 @@ bool wkv7_split_supported(const Wkv7Args &p) {
 // Enqueues the two kernels, once per segment of chunks, and leaves one flag per chain in the first
 // B*H ints of the workspace: 1 for chains that the caller's next kernel must recompute (their final
 // state is not written: it may alias the initial state that the recomputation starts from).
-int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
+int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes, bool wide_range, bool resolve_flagged,
+                      cudaStream_t stream) {
     EncodeTiledFn encode = encode_fn();
     if (encode == nullptr) return (int)cudaErrorNotSupported;
     const size_t chains = (size_t)(p.B * p.H);
@@ -1339,7 +1394,7 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
     size_t seg = preferred_segment(chains, (size_t)nchunks, overlap);
     const size_t fixed = fixed_part(chains);
     if (workspace_bytes < fixed) return (int)cudaErrorInvalidValue;
-    const size_t per_chunk = chains * ((size_t)kVecFloats * sizeof(float) + kOperatorBytes);
+    const size_t per_chunk = chains * kRecord;
     if (overlap && layout_for(chains, seg, 2).total > workspace_bytes) {
         const size_t fit = (workspace_bytes - fixed) / (2 * per_chunk);
         if (fit >= 8) seg = fit;
@@ -1358,58 +1413,40 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
     const WorkspaceLayout lay = layout_for(chains, seg, overlap ? 2 : 1);
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     int *flags = reinterpret_cast<int *>(ws + lay.flags);
-    int *counters = reinterpret_cast<int *>(ws + lay.counters);
     float *carry = reinterpret_cast<float *>(ws + lay.carry);
 
-    OperatorMaps omaps;
-    ScanMaps smaps;
-    const void *ptrs[5] = {p.r, p.w, p.k, p.a, p.b};
+    OperatorMaps omaps{};
+    ScanMaps smaps{};
+    const OperatorPtrs optrs{{p.a, p.r, p.b, p.k, p.w}};
     const cuuint64_t dims[2] = {(cuuint64_t)(p.H * p.N), (cuuint64_t)(p.B * p.T)};
     const size_t esize = p.bf16 ? 2 : 4;
     const CUtensorMapDataType etype = p.bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const cuuint64_t strides[1] = {(cuuint64_t)(p.H * p.N * esize)};
-    const cuuint32_t box[2] = {(cuuint32_t)kN, (cuuint32_t)kL};
+    const cuuint32_t box[2] = {(cuuint32_t)(128 / esize), (cuuint32_t)kL};   // rows of 128 bytes in shared memory
     const cuuint32_t estr[2] = {1, 1};
-    for (int i = 0; i < 5; ++i) {
-        CUresult r = encode(&omaps.m[i], etype, 2, const_cast<void *>(ptrs[i]), dims, strides,
-                            box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return (int)cudaErrorInvalidValue;
-    }
-    {   // V: bf16 tiles land swizzled and are converted in place; fp32 tiles land row-major beside their fp16 copy
-        CUresult r = encode(&smaps.v, etype, 2, const_cast<void *>(p.v), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, p.bf16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return (int)cudaErrorInvalidValue;
-    }
-    {   // y: rows of 128 bytes in shared memory (64 bf16 channels, or 32 fp32 channels: two stores per chunk)
-        const cuuint32_t ybox[2] = {(cuuint32_t)(p.bf16 ? kN : kN / 2), (cuuint32_t)kL};
-        CUresult r = encode(&smaps.y, etype, 2, p.y, dims, strides, ybox, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return (int)cudaErrorInvalidValue;
-    }
+    auto describe = [&](CUtensorMap *map, const void *ptr) {
+        return encode(map, etype, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    for (int i = 0; p.bf16 && i < 5; ++i)   // (fp32 tensors are read by the threads themselves)
+        if (!describe(&omaps.m[i], optrs.p[i])) return (int)cudaErrorInvalidValue;
+    if (!describe(&smaps.v, p.v) || !describe(&smaps.y, p.y)) return (int)cudaErrorInvalidValue;
     int *status = nullptr;
     if (int e = device_status_ptr(p.device, &status)) return e;
 
     auto k1 = p.bf16 ? wkv7_chunk_operator_kernel<__nv_bfloat16> : wkv7_chunk_operator_kernel<float>;
-    const size_t smem1 = p.bf16 ? kSmem1 : kSmem1F32;
-    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem1);
     if (e != cudaSuccess) return (int)e;
     if (!overlap) part = nullptr;
     cudaStream_t op_stream = part ? part->op_stream : stream;
-    // Beside an operator CTA only the two-stage scan fits; it is also the one for more chains than SMs.  On its own
-    // partition a scan CTA has an SM to itself.
-    const bool small_scan = (overlap && part == nullptr) || (int64_t)chains > (int64_t)p.num_sms;
-    auto launch_scan = [&](cudaStream_t st, int buf, const float *s_in, float *s_out, int c0, int n, int check) -> cudaError_t {
-        const unsigned char *ops = ws + lay.operators[buf];
-        const float *vecs = reinterpret_cast<const float *>(ws + lay.vectors[buf]);
-        auto go = [&](auto kern, auto ytype, size_t smem_bytes, unsigned threads) -> cudaError_t {
+    auto launch_scan = [&](cudaStream_t st, int buf, const float *s_in, float *s_out, int c0, int n) -> cudaError_t {
+        const unsigned char *records = ws + lay.records[buf];
+        auto go = [&](auto kern, auto ytype, size_t smem_bytes, int threads) -> cudaError_t {
             cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
             if (err != cudaSuccess) return err;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)chains);
-            cfg.blockDim = dim3(threads);
+            cfg.blockDim = dim3((unsigned)threads);
             cfg.dynamicSmemBytes = smem_bytes;
             cfg.stream = st;
             cudaLaunchAttribute attr[1];
@@ -1417,41 +1454,34 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
             cfg.numAttrs = st == stream ? 1 : 0;   // directly behind its operator kernel on the caller's stream
-            using YPtr = std::remove_pointer_t<decltype(ytype)> *;
-            err = cudaLaunchKernelEx(&cfg, kern, smaps, ops, vecs, s_in, s_out, reinterpret_cast<YPtr>(p.y), flags,
-                                     (int)p.T, (int)p.H, c0, n, n, check, status);
+            using T = std::remove_pointer_t<decltype(ytype)>;
+            err = cudaLaunchKernelEx(&cfg, kern, smaps, optrs, static_cast<const T *>(p.v), records, s_in, s_out,
+                                     static_cast<T *>(p.y), flags, (int)p.T, (int)p.H, c0, n, resolve_flagged ? 1 : 0, status);
             if (err == cudaSuccess) count_launch();
             return err;
         };
         using bf = __nv_bfloat16;
-        if (!p.bf16) return go(wkv7_state_scan_kernel<3, float>, (float *)nullptr, ScanSmem<3, float>::kBytes, ScanWarps<3>::kThreads);
-        return small_scan ? go(wkv7_state_scan_kernel<2, bf>, (bf *)nullptr, ScanSmem<2, bf>::kBytes, ScanWarps<2>::kThreads)
-                          : go(wkv7_state_scan_kernel<4, bf>, (bf *)nullptr, ScanSmem<4, bf>::kBytes, ScanWarps<4>::kThreads);
+        if (!p.bf16) return go(wkv7_state_scan_kernel<float>, (float *)nullptr, Scan<float>::kBytes, Scan<float>::kThreads);
+        return go(wkv7_state_scan_kernel<bf>, (bf *)nullptr, Scan<bf>::kBytes, Scan<bf>::kThreads);
     };
-    auto launch_operators = [&](int buf, int segment, int c0, int n) -> cudaError_t {
+    auto launch_operators = [&](int buf, int c0, int n) -> cudaError_t {
         const long long units = (long long)chains * n;
-        // (see overlap_applies; on its own partition the kernel fills every SM it has twice over)
-        const long long places = part ? 2LL * part->op_sms
-                                      : (p.bf16 ? 2LL : 1LL) * p.num_sms - (overlap ? (long long)chains : 0);
+        // (see overlap_applies; on its own partition the kernel fills every SM it has)
+        const long long places = part ? 4LL * part->op_sms : overlap ? 4LL * (p.num_sms - (long long)chains) : 4LL * p.num_sms;
         const unsigned grid = (unsigned)(units < places ? units : places);
         // (the operator of (chain, chunk) sits at index chain * n + chunk - c0 of the buffer in both kernels)
-        k1<<<grid, kThreads1, smem1, op_stream>>>(omaps, ws + lay.operators[buf], reinterpret_cast<float *>(ws + lay.vectors[buf]),
-                                                flags, (int)p.T, (int)p.H, c0, n, (int)chains, counters + segment, status);
+        k1<<<grid, kOpThreads, kSmem1, op_stream>>>(omaps, optrs, ws + lay.records[buf], (int)p.T, (int)p.H, c0, n, (int)chains, wide_range ? 1 : 0, status);
         count_launch();
         return cudaGetLastError();
     };
-    // flags and work counters start at zero
-    e = cudaMemsetAsync(ws, 0, lay.carry, stream);
-    if (e != cudaSuccess) return (int)e;
 
     if (!overlap) {
-        int segment = 0;
-        for (int c0 = 0; c0 < nchunks; c0 += (int)seg, ++segment) {
+        for (int c0 = 0; c0 < nchunks; c0 += (int)seg) {
             const int n = (int)((size_t)(nchunks - c0) < seg ? (size_t)(nchunks - c0) : seg);
-            e = launch_operators(0, segment, c0, n);
+            e = launch_operators(0, c0, n);
             if (e != cudaSuccess) return (int)e;
             const bool first = c0 == 0, last = c0 + n >= nchunks;
-            e = launch_scan(stream, 0, first ? p.s0 : carry, last ? p.s_out : carry, c0, n, last ? 1 : 0);
+            e = launch_scan(stream, 0, first ? p.s0 : carry, last ? p.s_out : carry, c0, n);
             if (e != cudaSuccess) return (int)e;
         }
         return 0;
@@ -1475,12 +1505,12 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
             e = cudaStreamWaitEvent(op_stream, scanned[buf], 0);
             if (e != cudaSuccess) return (int)e;
         }
-        e = launch_operators(buf, segment, c0, n);
+        e = launch_operators(buf, c0, n);
         if (e == cudaSuccess) e = cudaEventRecord(built[buf], op_stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(scan_stream, built[buf], 0);
         if (e != cudaSuccess) return (int)e;
         const bool first = c0 == 0, last = c0 + n >= nchunks;
-        e = launch_scan(scan_stream, buf, first ? p.s0 : carry, last ? p.s_out : carry, c0, n, last ? 1 : 0);
+        e = launch_scan(scan_stream, buf, first ? p.s0 : carry, last ? p.s_out : carry, c0, n);
         if (e == cudaSuccess) e = cudaEventRecord(scanned[buf], scan_stream);
         if (e != cudaSuccess) return (int)e;
     }
