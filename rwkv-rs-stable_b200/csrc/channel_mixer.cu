@@ -65,7 +65,8 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__rest
     uint64_t *tmem_empty = tmem_full + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (uniform, for elect_one)
     const int ksteps = (K + kBK - 1) / kBK;   // the K tail is zero-filled by TMA
 
     if (tid == 0) {
@@ -83,7 +84,7 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__rest
     bool timed_out = false;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             for (int tile = blockIdx.x; tile < total_tiles && !timed_out; tile += gridDim.x) {
                 const int nt = tile % n_tiles, mt = tile / n_tiles;
@@ -98,7 +99,7 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__rest
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(kFmtBF16, kBM, kBN, false, false);
             uint32_t it = 0, local = 0;
             for (int tile = blockIdx.x; tile < total_tiles && !timed_out; tile += gridDim.x, ++local) {

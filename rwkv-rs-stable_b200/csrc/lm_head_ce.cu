@@ -63,7 +63,8 @@ lm_head_ce_kernel(const __grid_constant__ LmMaps maps, const void *__restrict__ 
     uint64_t *tmem_empty = tmem_full + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (uniform, for elect_one)
     // consecutive CTAs share a vocabulary split and differ in the row block
     const int rb = blockIdx.x % row_blocks, split = blockIdx.x / row_blocks;
     const int total_tiles = (V + kBN - 1) / kBN;
@@ -86,7 +87,7 @@ lm_head_ce_kernel(const __grid_constant__ LmMaps maps, const void *__restrict__ 
     bool timed_out = false;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             for (int t = 0; t < ntiles && !timed_out; ++t) {
                 for (int ks = 0; ks < ksteps; ++ks, ++it) {
@@ -100,7 +101,7 @@ lm_head_ce_kernel(const __grid_constant__ LmMaps maps, const void *__restrict__ 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(kFmtBF16, kBM, kBN, false, false);
             uint32_t it = 0;
             for (int t = 0; t < ntiles && !timed_out; ++t) {

@@ -234,6 +234,8 @@ wkv7_chunked_kernel(const __grid_constant__ TmaMaps maps, const float *s0,
     int *unsafe = reinterpret_cast<int *>(exp_cl + 128);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // (uniform for the warp, and one lane by election: see elect_one for what `tid == 0` costs)
+    const bool issuer = __shfl_sync(0xffffffffu, tid >> 5, 0) == 0;
     const int quarter = warp & 3;   // TMEM lane quarter this warp may read
     const int cgrp = warp >> 2;     // column group among the four warps of a quarter
     static_assert(!(SAVE && K > 1), "the cluster variant does not write the training tensors");
@@ -396,7 +398,7 @@ wkv7_chunked_kernel(const __grid_constant__ TmaMaps maps, const float *s0,
         // that left here would keep its successors waiting for a state.
         if (K > 1 ? (*unsafe & 2) : *unsafe) { failed = true; break; }
         // ---------------- M1: G = [At;Rt] [Bh;Kh]^T
-        if (tid == 0) {
+        if (issuer && elect_one()) {
             tc_fence_after();
             mma_k64<128, 128, 128>(tmem + kColG, dAR, dBK, false);
             umma_commit(bar_mma);
@@ -473,7 +475,7 @@ wkv7_chunked_kernel(const __grid_constant__ TmaMaps maps, const float *s0,
         if (K > 1 ? (*unsafe & 2) : *unsafe) { failed = true; break; }
         // ---------------- state path, part 2: the products with the masked A_ak, A_rk just
         // staged; they run on the tensor core while the diagonal blocks are inverted below.
-        if (tid == 0) {
+        if (issuer && elect_one()) {
             tc_fence_after();
             // (K > 1: the state has not arrived yet, these products start the accumulators)
             mma_k64<64, 128, 128>(tmem + kColXT, dVT, dAKRK, K == 1);            // [X^T | Y^T] (+)= V^T [A_ak;A_rk]^T
@@ -564,7 +566,7 @@ wkv7_chunked_kernel(const __grid_constant__ TmaMaps maps, const float *s0,
         } else {
             // ---------------- T^T = I (I - A_ab)^-T by the same block substitution, before the state is
             // needed; the raw-tile region is refilled once the identity tile has been read.
-            if (tid == 0) {
+            if (issuer && elect_one()) {
                 auto dep_commit = [&]() { umma_commit(bar_dep); };
                 auto dep_wait = [&]() {
                     if (!mbar_wait_spin(bar_dep, dep_phase)) atomicOr(unsafe, 2);
@@ -646,7 +648,7 @@ wkv7_chunked_kernel(const __grid_constant__ TmaMaps maps, const float *s0,
         // commit and a wait (MMAs with different accumulators are not guaranteed to execute
         // in issue order); MMAs that do not depend on the pending result are issued between
         // the commit and the wait so that the tensor core stays busy.
-        if (tid == 0) {
+        if (issuer && elect_one()) {
             auto dep_commit = [&]() { umma_commit(bar_dep); };
             auto dep_wait = [&]() {
                 if (!mbar_wait_spin(bar_dep, dep_phase)) atomicOr(unsafe, 2);
