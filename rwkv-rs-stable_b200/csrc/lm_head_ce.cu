@@ -246,14 +246,20 @@ EncodeTiledFn lm_encode_fn() {
 // splits on a tie).  Example, 148 SMs, 256 row blocks x 32 column tiles: one or two splits take 2 x 32 = 4 x 16 = 64
 // tile times, four splits 7 x 8 = 56 (the ideal is 55.4): 1140 -> 1195 TFLOP/s on that shape.  (Persistent CTAs that
 // walk the work items themselves measured no better: 1167.)
-constexpr int kMaxSplits = 16;
+// Most splits per row block: 16, and with few row blocks as many as give every SM of a large device a CTA of its own
+// (a call of up to 128 rows is one row block: with 16 splits, 16 SMs read the whole weight matrix: 188 us for 16 rows
+// at C = 2048, V = 65 536, against 73).
+int max_splits(int64_t R) {
+    const int64_t rbs = (R + kBM - 1) / kBM, fill = rbs > 0 ? 160 / rbs : 160;
+    return (int)(fill > 16 ? fill : 16);
+}
 void plan(int64_t R, int64_t V, int num_sms, int *row_blocks, int *splits, int *tiles_per_split) {
     const int rbs = (int)((R + kBM - 1) / kBM);
     const int tiles = (int)((V + kBN - 1) / kBN);
     const int sms = num_sms > 0 ? num_sms : 1;
     int best_sp = 1, best_tps = tiles;
     double best_cost = 0.0;
-    for (int want = 1; want <= kMaxSplits && want <= tiles; ++want) {
+    for (int want = 1; want <= max_splits(R) && want <= tiles; ++want) {
         const int tps = (tiles + want - 1) / want;
         const int sp = (tiles + tps - 1) / tps;
         const long long ctas = (long long)rbs * sp;
@@ -274,9 +280,9 @@ void plan(int64_t R, int64_t V, int num_sms, int *row_blocks, int *splits, int *
 
 size_t lm_head_ce_workspace_bytes(int64_t R, int64_t C, int64_t V) {
     (void)C;
-    // Upper bound for any device: one triple per row per vocabulary split, at most kMaxSplits of them.
-    const int64_t tiles = (V + kBN - 1) / kBN;
-    const int64_t sp = tiles < kMaxSplits ? tiles : kMaxSplits;
+    // Upper bound for any device: one triple per row per vocabulary split, at most max_splits of them.
+    const int64_t tiles = (V + kBN - 1) / kBN, most = max_splits(R);
+    const int64_t sp = tiles < most ? tiles : most;
     return sp > 1 ? (size_t)sp * (size_t)R * 3 * sizeof(float) : 0;
 }
 
