@@ -48,12 +48,12 @@ struct GemmMaps {
     CUtensorMap b;  // [N, K] bf16, box 256 x 64
 };
 
-enum { kEpiNone = 0, kEpiReluSquare = 1 };
+enum { kEpiNone = 0, kEpiReluSquare = 1, kEpiPartial = 2 };   // partial: fp32 sums over one piece of K
 
 template <int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__restrict__ out, int64_t M, int N,
-                    int K, int n_tiles, int total_tiles, int *status) {
+gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, void *__restrict__ out, int64_t M, int N,
+                    int K, int n_tiles, int mn_tiles, int splits, int *status) {
     extern __shared__ __align__(1024) unsigned char smem[];   // swizzled TMA tiles need 1024-byte alignment
     if (smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0) atomicExch(status, (int)kDevInternal);
@@ -67,7 +67,11 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__rest
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (uniform, for elect_one)
-    const int ksteps = (K + kBK - 1) / kBK;   // the K tail is zero-filled by TMA
+    const int all_ksteps = (K + kBK - 1) / kBK;   // the K tail is zero-filled by TMA
+    // A work item is an output tile, or (splits > 1) one of `splits` pieces of K of it.
+    const int total_tiles = mn_tiles * splits, per_split = (all_ksteps + splits - 1) / splits;
+    auto first_kstep = [&](int item) { return item / mn_tiles * per_split; };
+    auto count_ksteps = [&](int item) { return max(0, min(per_split, all_ksteps - first_kstep(item))); };
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -82,13 +86,16 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__rest
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool timed_out = false;
+    // (launched with programmatic stream serialization: set up while the kernel before it finishes)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (warp == 0) {
         if (elect_one()) {
             uint32_t it = 0;
             for (int tile = blockIdx.x; tile < total_tiles && !timed_out; tile += gridDim.x) {
-                const int nt = tile % n_tiles, mt = tile / n_tiles;
-                for (int ks = 0; ks < ksteps; ++ks, ++it) {
+                const int nt = tile % mn_tiles % n_tiles, mt = tile % mn_tiles / n_tiles, k0 = first_kstep(tile), ksteps = count_ksteps(tile);
+                for (int ks = k0; ks < k0 + ksteps; ++ks, ++it) {
                     const uint32_t s = it % kStages, ph = (it / kStages) & 1;
                     if (!mbar_wait(&empty[s], ph ^ 1)) { timed_out = true; break; }
                     unsigned char *a = smem + s * kStageBytes, *b = a + kABytes;
@@ -104,6 +111,7 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__rest
             uint32_t it = 0, local = 0;
             for (int tile = blockIdx.x; tile < total_tiles && !timed_out; tile += gridDim.x, ++local) {
                 const uint32_t buf = local & 1, bph = (local >> 1) & 1;
+                const int ksteps = count_ksteps(tile);
                 if (!mbar_wait(&tmem_empty[buf], bph ^ 1)) { timed_out = true; break; }
                 tc_fence_after();
                 for (int ks = 0; ks < ksteps; ++ks, ++it) {
@@ -125,12 +133,13 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__rest
         const int quarter = warp & 3;
         uint32_t local = 0;
         for (int tile = blockIdx.x; tile < total_tiles && !timed_out; tile += gridDim.x, ++local) {
-            const int nt = tile % n_tiles, mt = tile / n_tiles;
+            const int nt = tile % mn_tiles % n_tiles, mt = tile % mn_tiles / n_tiles;
             const uint32_t buf = local & 1, bph = (local >> 1) & 1;
             if (!mbar_wait(&tmem_full[buf], bph)) { timed_out = true; break; }
             tc_fence_after();
             const int64_t row = (int64_t)mt * kBM + quarter * 32 + lane;
-            __nv_bfloat16 *orow = out + row * N + (int64_t)nt * kBN;
+            __nv_bfloat16 *orow = static_cast<__nv_bfloat16 *>(out) + row * N + (int64_t)nt * kBN;
+            float *prow = static_cast<float *>(out) + ((int64_t)(tile / mn_tiles) * M + row) * N + (int64_t)nt * kBN;
 #pragma unroll 1
             for (int ch = 0; ch < kBN / 32; ++ch) {
                 uint32_t v[32];
@@ -139,6 +148,12 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__rest
                 const int c0 = nt * kBN + ch * 32;
                 if (row >= M || c0 >= N) continue;            // padding rows / columns of edge tiles
                 const int nvec = min(32, N - c0) / 8;          // N is a multiple of 8
+                if constexpr (EPI == kEpiPartial) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (q < 2 * nvec) *reinterpret_cast<uint4 *>(prow + ch * 32 + q * 4) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    continue;
+                }
                 uint4 pk[4];
                 unsigned *pw = &pk[0].x;
 #pragma unroll
@@ -166,16 +181,45 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, __nv_bfloat16 *__rest
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
+// Sums the pieces of K and applies the activation; one thread per four columns.
+template <int EPI>
+__global__ void __launch_bounds__(256)
+gemm_reduce_kernel(const float *__restrict__ parts, int splits, __nv_bfloat16 *__restrict__ out, int64_t quads) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= quads) return;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) {
+        const float4 x = __ldcs(reinterpret_cast<const float4 *>(parts) + (int64_t)s * quads + i);
+        a.x += x.x;
+        a.y += x.y;
+        a.z += x.z;
+        a.w += x.w;
+    }
+    if constexpr (EPI == kEpiReluSquare) {
+        a.x = fmaxf(a.x, 0.f); a.x *= a.x;
+        a.y = fmaxf(a.y, 0.f); a.y *= a.y;
+        a.z = fmaxf(a.z, 0.f); a.z *= a.z;
+        a.w = fmaxf(a.w, 0.f); a.w *= a.w;
+    }
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+    reinterpret_cast<uint2 *>(out)[i] = make_uint2(*reinterpret_cast<const unsigned *>(&lo), *reinterpret_cast<const unsigned *>(&hi));
+}
+
 // key_input = x + (shifted - x) * key_scale, shifted = previous token (zero at t == 0)
 // (channel_mixer/kernel.rs:4-25).  A CTA owns 16 consecutive token rows, a thread one
-// 16-byte channel vector; the previous row is carried in registers.
+// 16-byte channel vector; the previous row is carried in registers.  (Few rows: fewer per CTA, so that they are not
+// walked one after the other by one CTA.)
 constexpr int kMixRows = 16;
 __global__ void __launch_bounds__(256)
 channel_mixer_mix_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ scale,
-                         __nv_bfloat16 *__restrict__ out, int64_t rows, int64_t Tlen, int64_t C) {
+                         __nv_bfloat16 *__restrict__ out, int64_t rows, int64_t Tlen, int64_t C, int per_block) {
     const int64_t CV = C / 8;
-    const int64_t row_begin = (int64_t)blockIdx.x * kMixRows;
-    const int64_t row_end = row_begin + kMixRows < rows ? row_begin + kMixRows : rows;
+    const int64_t row_begin = (int64_t)blockIdx.x * per_block;
+    const int64_t row_end = row_begin + per_block < rows ? row_begin + per_block : rows;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     auto unpack = [](const uint4 &u, float (&f)[8]) {
         const unsigned w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -246,8 +290,48 @@ int encode_rows_by_k(EncodeTiledFn encode, CUtensorMap *map, const void *base, i
                : (int)cudaErrorInvalidValue;
 }
 
+// Pieces of K per output tile.  With fewer than half as many tiles as SMs (a decode batch: 128 rows are one row of
+// tiles, 8 of them for 2048 columns) most of the device would idle while a few SMs stream the whole weight matrix, so K is
+// cut until every SM has an item, in pieces of at least four K steps, and a second kernel adds the fp32 sums up.  Measured
+// (B200, C = 2048, F = 8192): one row 91 -> 36 us, 64 rows at C = 4096 172 -> 78 us.
+constexpr int kMaxGemmSplits = 18;
+int gemm_splits(int64_t M, int64_t N, int64_t K, int num_sms) {
+    const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN), ksteps = (K + kBK - 1) / kBK;
+    if (2 * tiles > num_sms) return 1;
+    int64_t sp = num_sms / tiles;
+    if (sp > ksteps / 4) sp = ksteps / 4;
+    if (sp > kMaxGemmSplits) sp = kMaxGemmSplits;
+    if (sp < 2) return 1;
+    const int64_t per = (ksteps + sp - 1) / sp;
+    return (int)((ksteps + per - 1) / per);   // (no piece is empty)
+}
+// fp32 partial sums of any device up to this many SMs.
+constexpr int kMostSms = 160;
+size_t gemm_partial_bytes(int64_t M, int64_t N, int64_t K) {
+    const int sp = gemm_splits(M, N, K, kMostSms);
+    return sp > 1 ? (size_t)sp * M * N * sizeof(float) : 0;
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_serialized(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+    if (e == cudaSuccess) count_launch();
+    return e;
+}
+
 // out[M,N] = act(A[M,K] . B[N,K]^T); K and N multiples of 8, all pointers 16-byte aligned.
-int launch_gemm(const void *a, const void *b, void *out, int64_t M, int64_t N, int64_t K, int epi, int num_sms,
+template <int EPI>
+int launch_gemm(const void *a, const void *b, void *out, float *partials, int64_t M, int64_t N, int64_t K, int num_sms,
                 int *status, cudaStream_t stream) {
     EncodeTiledFn encode = gemm_encode_fn();
     if (encode == nullptr) return (int)cudaErrorNotSupported;
@@ -255,24 +339,18 @@ int launch_gemm(const void *a, const void *b, void *out, int64_t M, int64_t N, i
     if (int e = encode_rows_by_k(encode, &maps.a, a, M, K, kBM)) return e;
     if (int e = encode_rows_by_k(encode, &maps.b, b, N, K, kBN)) return e;
     const int m_tiles = (int)((M + kBM - 1) / kBM), n_tiles = (int)((N + kBN - 1) / kBN);
-    const int total = m_tiles * n_tiles;
-    const unsigned grid = (unsigned)(total < num_sms ? total : num_sms);
-    cudaError_t e;
-    if (epi == kEpiReluSquare) {
-        e = cudaFuncSetAttribute(gemm_tn_bf16_kernel<kEpiReluSquare>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmemBytes);
-        if (e != cudaSuccess) return (int)e;
-        gemm_tn_bf16_kernel<kEpiReluSquare><<<grid, kThreads, kSmemBytes, stream>>>(
-            maps, (__nv_bfloat16 *)out, M, (int)N, (int)K, n_tiles, total, status);
-    } else {
-        e = cudaFuncSetAttribute(gemm_tn_bf16_kernel<kEpiNone>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmemBytes);
-        if (e != cudaSuccess) return (int)e;
-        gemm_tn_bf16_kernel<kEpiNone><<<grid, kThreads, kSmemBytes, stream>>>(
-            maps, (__nv_bfloat16 *)out, M, (int)N, (int)K, n_tiles, total, status);
-    }
-    count_launch();
-    return (int)cudaGetLastError();
+    const int tiles = m_tiles * n_tiles, splits = gemm_splits(M, N, K, num_sms < kMostSms ? num_sms : kMostSms);
+    const int items = tiles * splits;
+    const unsigned grid = (unsigned)(items < num_sms ? items : num_sms);
+    auto kernel = splits > 1 ? gemm_tn_bf16_kernel<kEpiPartial> : gemm_tn_bf16_kernel<EPI>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    if (e == cudaSuccess)
+        e = launch_serialized(kernel, grid, kThreads, kSmemBytes, stream, maps, splits > 1 ? (void *)partials : out, M, (int)N, (int)K,
+                              n_tiles, tiles, splits, status);
+    if (e != cudaSuccess || splits == 1) return (int)e;
+    const int64_t quads = M * N / 4;
+    return (int)launch_serialized(gemm_reduce_kernel<EPI>, (unsigned)((quads + 255) / 256), 256u, 0, stream, (const float *)partials, splits,
+                                  (__nv_bfloat16 *)out, quads);
 }
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -281,7 +359,8 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 size_t channel_mixer_workspace_bytes(int64_t rows, int64_t C, int64_t F) {
     if (rows <= 0 || C <= 0 || F <= 0) return 0;
-    return align256((size_t)rows * C * 2) + align256((size_t)rows * F * 2);   // key_input, hidden
+    const size_t p1 = gemm_partial_bytes(rows, F, C), p2 = gemm_partial_bytes(rows, C, F);
+    return align256((size_t)rows * C * 2) + align256((size_t)rows * F * 2) + align256(p1 > p2 ? p1 : p2);   // key_input, hidden, partial sums
 }
 
 int launch_channel_mixer(const ChannelMixerArgs &p, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
@@ -291,15 +370,17 @@ int launch_channel_mixer(const ChannelMixerArgs &p, void *workspace, size_t work
     __nv_bfloat16 *key_input = static_cast<__nv_bfloat16 *>(workspace);
     __nv_bfloat16 *hidden = reinterpret_cast<__nv_bfloat16 *>(static_cast<unsigned char *>(workspace) +
                                                               align256((size_t)rows * p.C * 2));
+    float *partials = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(hidden) + align256((size_t)rows * p.F * 2));
     int threads = 32;
     while (threads < 256 && threads < p.C / 8) threads <<= 1;
-    channel_mixer_mix_kernel<<<(unsigned)((rows + kMixRows - 1) / kMixRows), threads, 0, stream>>>(
-        (const __nv_bfloat16 *)p.x, (const __nv_bfloat16 *)p.key_scale, key_input, rows, p.T, p.C);
+    const int per_block = rows >= 2 * kMixRows * (int64_t)p.num_sms ? kMixRows : 2;
+    channel_mixer_mix_kernel<<<(unsigned)((rows + per_block - 1) / per_block), threads, 0, stream>>>(
+        (const __nv_bfloat16 *)p.x, (const __nv_bfloat16 *)p.key_scale, key_input, rows, p.T, p.C, per_block);
     count_launch();
     if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return (int)e;
-    if (int e = launch_gemm(key_input, p.key_weight, hidden, rows, p.F, p.C, kEpiReluSquare, p.num_sms, p.status, stream))
+    if (int e = launch_gemm<kEpiReluSquare>(key_input, p.key_weight, hidden, partials, rows, p.F, p.C, p.num_sms, p.status, stream))
         return e;
-    return launch_gemm(hidden, p.value_weight, p.out, rows, p.C, p.F, kEpiNone, p.num_sms, p.status, stream);
+    return launch_gemm<kEpiNone>(hidden, p.value_weight, p.out, partials, rows, p.C, p.F, p.num_sms, p.status, stream);
 }
 
 }  // namespace rwkv7

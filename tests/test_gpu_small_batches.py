@@ -1,0 +1,38 @@
+"""GPU parity of the paths that only small batches take: the channel mixer's products cut along K (few rows), and the
+LM head with more vocabulary splits than row blocks."""
+import numpy as np
+import pytest
+import torch
+
+import parity
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 512, 1032), (2, 65, 1032, 2056), (1, 128, 520, 4096), (3, 1, 2048, 8192)])
+def test_channel_mixer_split_along_k(pkg, workloads, cuda, shape):
+    """Rows on both sides of one 128-row tile, K with a partial last step and a partial last piece, N with partial tiles;
+    against a restatement that rounds where the kernels round."""
+    B, T, C, F = shape
+    x, ks, kw, vw = workloads.channel_mixer_inputs(B, T, C, F, seed=17)
+    out = pkg.channel_mixer_custom(x.to(cuda), ks.to(cuda), kw.to(cuda), vw.to(cuda))
+    torch.cuda.synchronize()
+    assert pkg.read_device_status(0) == 0
+    got = out.float().cpu().numpy().astype(np.float64)
+    prev = torch.cat([torch.zeros(B, 1, C), x.float()[:, :-1]], 1)
+    ki = (x.float() + (prev - x.float()) * ks.float()).to(torch.bfloat16).double().reshape(B * T, C)
+    hid = (torch.relu(ki @ kw.double().T) ** 2).to(torch.bfloat16).double()
+    fine = (hid @ vw.double().T).reshape(B, T, C).numpy()
+    tol = 2e-3 * np.abs(fine).max() + 2 * parity.BF16_ULP * np.abs(fine)
+    assert (np.abs(got - fine) <= tol).all(), float((np.abs(got - fine) - tol).max())
+
+
+@pytest.mark.parametrize("R,C,V", [(1, 64, 20000), (127, 128, 40000), (129, 64, 9000)])
+def test_lm_head_with_many_splits(pkg, oracle, workloads, cuda, R, C, V):
+    x, w, tg = workloads.lm_head_inputs(R, C, V, seed=19)
+    lse_ref, loss_ref = oracle.lm_head_ce(x.float().numpy(), w.float().numpy(), tg.numpy())
+    lse, loss = pkg.lm_head_ce(x.to(cuda), w.to(cuda), tg.to(cuda))
+    torch.cuda.synchronize()
+    assert pkg.read_device_status(0) == 0
+    np.testing.assert_allclose(lse.cpu().numpy(), lse_ref, rtol=0, atol=2e-4)
+    np.testing.assert_allclose(loss.cpu().numpy(), loss_ref, rtol=0, atol=2e-4)
