@@ -359,6 +359,30 @@ int rwkv7_fused_wkv7_backward_parallel(const rwkv7_tensor *initial_state, const 
                                        rwkv7_tensor *initial_state_grad, void *workspace,
                                        size_t workspace_bytes, rwkv7_stream stream);
 
+/*
+ * A training step as two calls that agree on what is kept between them, for callers that need the gradients and not the
+ * reference's saved tensors: the forward pass leaves the linear operator of every 64-token chunk and the state in
+ * front of it in `saved`, the backward pass only reads it (and may run more than once).  Gradients are those of
+ * rwkv7_fused_wkv7_backward.  For BF16 tensors with N = 64, chunk_len 16 and T >= 64 while the WKV7 path is AUTO or
+ * SPLIT; rwkv7_wkv7_training_saved_bytes returns 0 for what the calls do not cover.  saved, workspace:
+ * rwkv7_wkv7_training_saved_bytes / _workspace_bytes bytes, 256-byte aligned; workspace is borrowed until
+ * the enqueued work has finished.
+ */
+size_t rwkv7_wkv7_training_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int32_t dtype, int64_t chunk_len);
+size_t rwkv7_wkv7_training_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t N);
+int rwkv7_fused_wkv7_training_forward(const rwkv7_tensor *initial_state, const rwkv7_tensor *receptance,
+                                      const rwkv7_tensor *weight_decay, const rwkv7_tensor *replacement_key,
+                                      const rwkv7_tensor *value, const rwkv7_tensor *removal_key_normalized,
+                                      const rwkv7_tensor *replacement, int64_t chunk_len, rwkv7_tensor *output,
+                                      rwkv7_tensor *next_state, void *saved, size_t saved_bytes, rwkv7_stream stream);
+int rwkv7_fused_wkv7_training_backward(const rwkv7_tensor *receptance, const rwkv7_tensor *weight_decay,
+                                       const rwkv7_tensor *replacement_key, const rwkv7_tensor *value,
+                                       const rwkv7_tensor *removal_key_normalized, const rwkv7_tensor *replacement,
+                                       int64_t chunk_len, const void *saved, size_t saved_bytes,
+                                       const rwkv7_tensor *output_grad, const rwkv7_tensor *next_state_grad,
+                                       rwkv7_tensor *const sequence_grads[6], rwkv7_tensor *initial_state_grad,
+                                       void *workspace, size_t workspace_bytes, rwkv7_stream stream);
+
 /* ------------------------------------------------------------------ mix6 -- */
 /* Replaces Mix6Backend::fused_mix6 (mix6/mod.rs:25-28, impl :42-73; kernel
  * mix6/kernel.rs:25-57): prev = x[b,t-1,:] (0 at t == 0);

@@ -326,12 +326,22 @@ def wkv7_backward(inputs: Wkv7PretrainForwardInputs, saved: Wkv7SavedForward, ou
 
 
 class _Wkv7Function(torch.autograd.Function):
-    """The autodiff node of the reference (``Wkv7StatepassBackward``, ``wkv7/backward.rs:381-533``):
-    forward saves snapshots and state_replacement, backward runs the reverse kernel."""
+    """The autodiff node of the reference (``Wkv7StatepassBackward``, ``wkv7/backward.rs:381-533``).  bf16 sequences
+    with 64-element heads keep what the tensor-core training step needs (``rwkv7_fused_wkv7_training_forward``);
+    for everything else forward saves snapshots and state_replacement, and backward runs the reverse kernel."""
 
     @staticmethod
     def forward(ctx, r, w, k, v, a, b, s0, chunk_len):
         inputs = Wkv7PretrainForwardInputs(r, w, k, v, a, b, chunk_len=chunk_len)
+        inputs.check(True)
+        ctx.set_materialize_grads(False)
+        step = (_native or native()).wkv7_training_forward(s0, r, w, k, v, a, b, chunk_len)
+        ctx.step = step is not None
+        if ctx.step:
+            y, s_out, kept = step
+            ctx.save_for_backward(r, w, k, v, a, b, kept)
+            ctx.has_state, ctx.chunk_len = s0 is not None, chunk_len
+            return y, s_out
         saved = wkv7_forward_saved(inputs, s0, want_state=True)
         # Only what the backward pass reads is kept, and through save_for_backward: the node then
         # holds no reference to its own outputs (no cycle) and autograd's version counters catch an
@@ -346,6 +356,12 @@ class _Wkv7Function(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, ds):
         t = ctx.saved_tensors
+        if dy is None:
+            dy = torch.zeros_like(t[0])
+        if ctx.step:
+            *grads, ds0 = (_native or native()).wkv7_training_backward(
+                *t[:6], ctx.chunk_len, t[6], dy, None if ds is None else ds.contiguous(), ctx.has_state)
+            return (*grads, ds0, None)
         inputs = Wkv7PretrainForwardInputs(*t[:6], chunk_len=ctx.chunk_len)
         saved = Wkv7SavedForward(output=None, next_state=None, snapshots=t[6], state_replacement=t[7])
         s0 = t[8] if ctx.has_state else None

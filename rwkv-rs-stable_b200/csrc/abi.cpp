@@ -20,14 +20,17 @@ std::atomic<int> g_wkv7_path{RWKV7_WKV7_AUTO};
 constexpr int kMaxDevices = 64;
 std::atomic<int> g_num_sms[kMaxDevices] = {};
 
-// Makes `device` current for the duration of a call and restores the caller's.
+// Makes `device` current for the duration of a call and restores the caller's.  A thread's first call sets the device in any
+// case: until a thread has done something with its device it has no current context, and a tensor map cannot be encoded.
 class DeviceGuard {
    public:
     explicit DeviceGuard(int device) {
+        static thread_local int bound = -1;
         err_ = cudaGetDevice(&prev_);
-        if (err_ == cudaSuccess && prev_ != device) {
+        if (err_ == cudaSuccess && (prev_ != device || bound != device)) {
             err_ = cudaSetDevice(device);
-            switched_ = err_ == cudaSuccess;
+            switched_ = err_ == cudaSuccess && prev_ != device;
+            if (err_ == cudaSuccess) bound = device;
         }
     }
     ~DeviceGuard() {
@@ -707,6 +710,110 @@ static int wkv7_backward_impl(const rwkv7_tensor *s0, const rwkv7_tensor *r_t, c
         return RWKV7_OK;
     }
     if (int e = launch_wkv7_backward(p, (cudaStream_t)stream)) return cuda_fail("wkv7 backward launch", e);
+    return RWKV7_OK;
+}
+
+size_t rwkv7_wkv7_training_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int32_t dtype, int64_t chunk_len) {
+    const int path = g_wkv7_path.load();
+    if (B <= 0 || T <= 0 || H <= 0 || chunk_len != 16 || (path != RWKV7_WKV7_AUTO && path != RWKV7_WKV7_SPLIT)) return 0;
+    return wkv7_training_supported(B, T, H, N, dtype == RWKV7_BF16) ? wkv7_training_saved_bytes(B, T, H) : 0;
+}
+
+size_t rwkv7_wkv7_training_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t N) {
+    if (B <= 0 || T <= 0 || H <= 0 || !wkv7_training_supported(B, T, H, N, true)) return 0;
+    return wkv7_training_workspace_bytes(B, T, H);
+}
+
+namespace {
+
+// Contract of both halves of a training step beyond that of the tensors themselves.
+int check_training_step(const TensorInfo &r, int64_t chunk_len, const void *saved, size_t saved_bytes) {
+    RWKV7_TRY(check_training_chunks(r, chunk_len));
+    if (chunk_len != 16 || !wkv7_training_supported(r.dim(0), r.dim(1), r.dim(2), r.dim(3), r.t->dtype == RWKV7_BF16))
+        return fail(RWKV7_ERR_UNSUPPORTED, "Unsupported: the training step computes BF16 tensors with N = 64, chunk_len 16 and T >= 64");
+    const size_t need = wkv7_training_saved_bytes(r.dim(0), r.dim(1), r.dim(2));
+    if (saved == nullptr || saved_bytes < need)
+        return fail(RWKV7_ERR_WORKSPACE_TOO_SMALL, "WorkspaceTooSmall: the wkv7 training step keeps %zu bytes, got %zu", need,
+                    saved == nullptr ? (size_t)0 : saved_bytes);
+    if ((reinterpret_cast<uintptr_t>(saved) & 255u) != 0)
+        return fail(RWKV7_ERR_UNSUPPORTED, "Unsupported: what a training step keeps must be 256-byte aligned");
+    return RWKV7_OK;
+}
+
+}  // namespace
+
+int rwkv7_fused_wkv7_training_forward(const rwkv7_tensor *s0, const rwkv7_tensor *r_t, const rwkv7_tensor *w, const rwkv7_tensor *k,
+                                      const rwkv7_tensor *v, const rwkv7_tensor *a, const rwkv7_tensor *b, int64_t chunk_len,
+                                      rwkv7_tensor *output, rwkv7_tensor *next_state, void *saved, size_t saved_bytes,
+                                      rwkv7_stream stream) {
+    RWKV7_TRACE("rwkv.train.model.time_mixer.wkv7_forward");
+    clear_error();
+    const rwkv7_tensor *six_t[6] = {r_t, w, k, v, a, b};
+    TensorInfo six[6];
+    for (int i = 0; i < 6; ++i) six[i] = TensorInfo{kSixNames[i], six_t[i]};
+    RWKV7_TRY(check_wkv7_sequence(six, chunk_len));
+    const TensorInfo &r = six[0];
+    if (s0 != nullptr) RWKV7_TRY(check_wkv7_state(TensorInfo{"initial_state", s0}, r));
+    RWKV7_TRY(check_output_like(r, TensorInfo{"output", output}));
+    if (next_state != nullptr) RWKV7_TRY(check_wkv7_state(TensorInfo{"next_state", next_state}, r));
+    if (r.dim(0) == 0 || r.dim(2) == 0) return RWKV7_OK;
+    RWKV7_TRY(check_training_step(r, chunk_len, saved, saved_bytes));
+    Wkv7Args p{};
+    p.r = r_t->data; p.w = w->data; p.k = k->data; p.v = v->data; p.a = a->data; p.b = b->data;
+    p.s0 = s0 ? static_cast<const float *>(s0->data) : nullptr;
+    p.y = output->data;
+    p.s_out = next_state ? static_cast<float *>(next_state->data) : nullptr;
+    p.B = r.dim(0); p.T = r.dim(1); p.H = r.dim(2); p.N = r.dim(3);
+    p.bf16 = true;
+    p.device = r_t->device;
+    DeviceGuard guard(p.device);
+    if (guard.error() != cudaSuccess) return cuda_fail("cudaSetDevice", (int)guard.error());
+    RWKV7_TRY(num_sms(p.device, &p.num_sms));
+    if (int e = launch_wkv7_training_forward(p, saved, (cudaStream_t)stream)) return cuda_fail("wkv7 training forward launch", e);
+    return RWKV7_OK;
+}
+
+int rwkv7_fused_wkv7_training_backward(const rwkv7_tensor *r_t, const rwkv7_tensor *w, const rwkv7_tensor *k, const rwkv7_tensor *v,
+                                       const rwkv7_tensor *a, const rwkv7_tensor *b, int64_t chunk_len, const void *saved,
+                                       size_t saved_bytes, const rwkv7_tensor *output_grad, const rwkv7_tensor *next_state_grad,
+                                       rwkv7_tensor *const sequence_grads[6], rwkv7_tensor *initial_state_grad, void *workspace,
+                                       size_t workspace_bytes, rwkv7_stream stream) {
+    RWKV7_TRACE("rwkv.train.model.time_mixer.wkv7_backward");
+    clear_error();
+    const rwkv7_tensor *six_t[6] = {r_t, w, k, v, a, b};
+    TensorInfo six[6];
+    for (int i = 0; i < 6; ++i) six[i] = TensorInfo{kSixNames[i], six_t[i]};
+    RWKV7_TRY(check_wkv7_sequence(six, chunk_len));
+    const TensorInfo &r = six[0];
+    RWKV7_TRY(check_output_like(r, TensorInfo{"output_grad", output_grad}));
+    if (next_state_grad != nullptr) RWKV7_TRY(check_wkv7_state(TensorInfo{"next_state_grad", next_state_grad}, r));
+    if (sequence_grads == nullptr) return fail(RWKV7_ERR_NULL_POINTER, "NullPointer: sequence_grads array is null");
+    static const char *grad_names[6] = {"receptance_grad", "weight_decay_grad", "replacement_key_grad",
+                                        "value_grad", "removal_key_normalized_grad", "replacement_grad"};
+    for (int i = 0; i < 6; ++i) RWKV7_TRY(check_output_like(r, TensorInfo{grad_names[i], sequence_grads[i]}));
+    if (initial_state_grad != nullptr) RWKV7_TRY(check_wkv7_state(TensorInfo{"initial_state_grad", initial_state_grad}, r));
+    if (r.dim(0) == 0 || r.dim(2) == 0) return RWKV7_OK;
+    RWKV7_TRY(check_training_step(r, chunk_len, saved, saved_bytes));
+    const size_t need = wkv7_training_workspace_bytes(r.dim(0), r.dim(1), r.dim(2));
+    if (workspace == nullptr || workspace_bytes < need)
+        return fail(RWKV7_ERR_WORKSPACE_TOO_SMALL, "WorkspaceTooSmall: wkv7 backward needs %zu workspace bytes, got %zu", need,
+                    workspace == nullptr ? (size_t)0 : workspace_bytes);
+    if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
+        return fail(RWKV7_ERR_UNSUPPORTED, "Unsupported: the backward workspace must be 256-byte aligned");
+    Wkv7TrainingBackwardArgs p{};
+    p.r = r_t->data; p.w = w->data; p.k = k->data; p.v = v->data; p.a = a->data; p.b = b->data;
+    p.dy = output_grad->data;
+    p.next_state_grad = next_state_grad ? static_cast<const float *>(next_state_grad->data) : nullptr;
+    p.dr = sequence_grads[0]->data; p.dw = sequence_grads[1]->data; p.dk = sequence_grads[2]->data;
+    p.dv = sequence_grads[3]->data; p.da = sequence_grads[4]->data; p.db = sequence_grads[5]->data;
+    p.initial_state_grad = initial_state_grad ? static_cast<float *>(initial_state_grad->data) : nullptr;
+    p.B = r.dim(0); p.T = r.dim(1); p.H = r.dim(2);
+    p.device = r_t->device;
+    DeviceGuard guard(p.device);
+    if (guard.error() != cudaSuccess) return cuda_fail("cudaSetDevice", (int)guard.error());
+    RWKV7_TRY(num_sms(p.device, &p.num_sms));
+    if (int e = launch_wkv7_training_backward(p, saved, workspace, (cudaStream_t)stream))
+        return cuda_fail("wkv7 training backward launch", e);
     return RWKV7_OK;
 }
 

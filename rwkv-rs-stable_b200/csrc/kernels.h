@@ -94,6 +94,25 @@ int launch_wkv7_chunked_flagged(const Wkv7Args &p, void *workspace, cudaStream_t
 // Sequential recomputation of the chains whose flag is set (exits at once for the others).
 int launch_wkv7_sequential_flagged(const Wkv7Args &p, const int *flags, cudaStream_t stream);
 
+// A training step on the two-kernel prefill (N == 64, bf16 tensors, T a multiple of 16 and at least 64).  The forward pass
+// keeps the operator of every chunk and the state in front of it in `saved` (wkv7_training_saved_bytes); the backward pass is
+// the same scan over the transposed operators, then every chunk on its own (wkv7_train_chunks.cu).  Both only read `saved`.
+struct Wkv7TrainingBackwardArgs {
+    const void *r, *w, *k, *v, *a, *b, *dy;      // [B,T,H,64] bf16
+    const float *next_state_grad;                // [B,H,64,64] or null (zero)
+    void *dr, *dw, *dk, *dv, *da, *db;           // [B,T,H,64] bf16
+    float *initial_state_grad;                   // [B,H,64,64] or null
+    int64_t B, T, H;
+    int device;
+    int num_sms;
+};
+bool wkv7_training_supported(int64_t B, int64_t T, int64_t H, int64_t N, bool bf16);
+size_t wkv7_training_saved_bytes(int64_t B, int64_t T, int64_t H);
+size_t wkv7_training_workspace_bytes(int64_t B, int64_t T, int64_t H);
+int launch_wkv7_training_forward(const Wkv7Args &p, void *saved, cudaStream_t stream);
+int launch_wkv7_training_backward(const Wkv7TrainingBackwardArgs &p, const void *saved, void *workspace, cudaStream_t stream);
+int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const float *states, const float *gradients, cudaStream_t stream);
+
 // Cluster size of the chunked kernel: 0 = by the number of chains (default), else 1, 2 or 4.
 int wkv7_cluster_override();
 void wkv7_set_cluster_override(int k);

@@ -29,6 +29,8 @@ namespace {
     X(rwkv7_last_error_message) X(rwkv7_wkv7_workspace_bytes) X(rwkv7_fused_wkv7_pretrain)                       \
     X(rwkv7_fused_wkv7_statetune) X(rwkv7_fused_wkv7_statepass) X(rwkv7_fused_wkv7_statepass_noalloc)            \
     X(rwkv7_fused_wkv7_forward_saved) X(rwkv7_fused_wkv7_backward) X(rwkv7_fused_wkv7_backward_parallel)         \
+    X(rwkv7_wkv7_training_saved_bytes) X(rwkv7_wkv7_training_workspace_bytes)                                    \
+    X(rwkv7_fused_wkv7_training_forward) X(rwkv7_fused_wkv7_training_backward)                                   \
     X(rwkv7_wkv7_backward_workspace_bytes) X(rwkv7_fused_mix6) X(rwkv7_fused_mix6_stacked)                       \
     X(rwkv7_fused_addcmul) X(rwkv7_fused_addcmul5) X(rwkv7_fused_token_shift_diff)                               \
     X(rwkv7_fused_weight_prepare) X(rwkv7_fused_gated_readout) X(rwkv7_channel_mixer_workspace_bytes)            \
@@ -304,6 +306,58 @@ PyObject *wkv7_backward(PyObject *const *a) {
     return pair(list, ds0.defined() ? wrap(ds0) : Py_NewRef(Py_None));
 }
 
+// wkv7_training_forward(initial_state|None, r, w, k, v, a, b, chunk_len) -> (output, next_state, saved), or None for what
+// the training step does not cover
+PyObject *wkv7_training_forward(PyObject *const *a) {
+    const at::Tensor &r = tensor(a[1]);
+    Desc s0(a[0]), six[6];
+    for (int i = 0; i < 6; ++i) six[i].set(tensor(a[1 + i]));
+    const int64_t chunk_len = integer(a[7]);
+    const size_t keep = r.dim() != 4 || !r.is_cuda()
+                            ? 0 : abi.rwkv7_wkv7_training_saved_bytes(r.size(0), r.size(1), r.size(2), r.size(3), six[0].d.dtype, chunk_len);
+    if (keep == 0) return Py_NewRef(Py_None);
+    at::Tensor out[3] = {like(r), empty({r.size(0), r.size(2), r.size(3), r.size(3)}, at::kFloat, r), empty({(int64_t)keep}, at::kByte, r)};
+    Desc yd(out[0]), sd(out[1]);
+    const rwkv7_stream st = stream_of(r);
+    call([&] {
+        return abi.rwkv7_fused_wkv7_training_forward(s0.p, six[0].p, six[1].p, six[2].p, six[3].p, six[4].p, six[5].p, chunk_len,
+                                                     yd.p, sd.p, out[2].data_ptr(), keep, st);
+    });
+    return tuple_of(out, 3);
+}
+
+// wkv7_training_backward(r, w, k, v, a, b, chunk_len, saved, output_grad, next_state_grad|None, want_state_grad)
+//   -> (six gradients, state gradient|None)
+PyObject *wkv7_training_backward(PyObject *const *a) {
+    const at::Tensor &r = tensor(a[0]);
+    Desc six[6];
+    for (int i = 0; i < 6; ++i) six[i].set(tensor(a[i]));
+    const int64_t chunk_len = integer(a[6]);
+    const at::Tensor &saved = tensor(a[7]);
+    const at::Tensor dy_t = tensor(a[8]).contiguous();
+    Desc dy(dy_t), ds(a[9]), gd[6], ds0d;
+    at::Tensor grads[7];
+    rwkv7_tensor *gp[6];
+    for (int i = 0; i < 6; ++i) {
+        grads[i] = like(r);
+        gd[i].set(grads[i]);
+        gp[i] = gd[i].p;
+    }
+    if (truth(a[10])) {
+        grads[6] = empty({r.size(0), r.size(2), r.size(3), r.size(3)}, at::kFloat, r);
+        ds0d.set(grads[6]);
+    }
+    Workspace ws;
+    ws.allocate(abi.rwkv7_wkv7_training_workspace_bytes(r.size(0), r.size(1), r.size(2), r.size(3)), r);
+    const rwkv7_stream st = stream_of(r);
+    call([&] {
+        return abi.rwkv7_fused_wkv7_training_backward(six[0].p, six[1].p, six[2].p, six[3].p, six[4].p, six[5].p, chunk_len,
+                                                      saved.data_ptr(), (size_t)saved.numel(), dy.p, ds.p, gp, ds0d.p, ws.ptr,
+                                                      ws.bytes, st);
+    });
+    return tuple_of(grads, 7);
+}
+
 // mix6(x, six scales) -> six outputs
 PyObject *mix6(PyObject *const *a) {
     const at::Tensor &x = tensor(a[0]);
@@ -534,7 +588,7 @@ PyObject *open_library(PyObject *, PyObject *const *args, Py_ssize_t n) {
     {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<name, nargs>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"open", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&open_library)), METH_FASTCALL, nullptr},
-    RWKV7_METHOD(wkv7, 12), RWKV7_METHOD(wkv7_noalloc, 10), RWKV7_METHOD(wkv7_saved, 9), RWKV7_METHOD(wkv7_backward, 15),
+    RWKV7_METHOD(wkv7, 12), RWKV7_METHOD(wkv7_noalloc, 10), RWKV7_METHOD(wkv7_saved, 9), RWKV7_METHOD(wkv7_backward, 15), RWKV7_METHOD(wkv7_training_forward, 8), RWKV7_METHOD(wkv7_training_backward, 11),
     RWKV7_METHOD(mix6, 7), RWKV7_METHOD(mix6_stacked, 7), RWKV7_METHOD(addcmul, 4), RWKV7_METHOD(addcmul5, 7),
     RWKV7_METHOD(token_shift_diff, 4), RWKV7_METHOD(weight_prepare, 9), RWKV7_METHOD(gated_readout, 10),
     RWKV7_METHOD(channel_mixer, 5), RWKV7_METHOD(lm_head_ce_partial, 4), RWKV7_METHOD(lm_head_ce_finalize, 2),

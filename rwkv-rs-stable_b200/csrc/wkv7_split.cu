@@ -48,6 +48,7 @@
 #include "sm100_mma.cuh"
 #include "sm100_umma.cuh"
 #include "trace.h"
+#include "wkv7_tiles.cuh"
 
 namespace rwkv7 {
 
@@ -57,16 +58,12 @@ namespace {
 
 using namespace sm100;
 
-constexpr int kN = 64;
-constexpr int kL = 64;
 constexpr float kMildDecay = 9.118820e-4f;    // e^-7: both halves of the chunk at or above it take one reference point
                                               // (factors up to 2200: room for entries of 29 and, below, down to 6e-2)
-constexpr float kBlockDecay = 6.144212e-6f;   // e^-12: a block below it (or a NaN) marks the chunk
 constexpr float kNarrowDecay = 1.522998e-8f;  // e^-18: least decay over a chunk when the wide range is switched off
 constexpr int kWideShift = 6;                 // block-wise references: operands are stored times 2^6, because there the
 constexpr float kWideScale = 64.f;            // factors reach down to e^-12 and a typical entry has to stay a normal number
-constexpr uint32_t kPanel = 8192;             // one [64][64] 16-bit tile, 128-byte rows, 16-byte pieces XOR-ed with (row & 7)
-constexpr uint32_t kBlk = 512;                // one 16 x 16 fp16 block: two halves of 8 columns, each [16 rows][16 bytes]
+__host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
 
 // What the builder leaves of a chunk in global memory: the 128 x 128 fp16 operator O[n][k], n = (j' | t), as the core
 // matrices (eight rows n, eight k, 128 bytes) of a K-major tcgen05 operand without swizzle, 16 of them along k and 16 along n.
@@ -79,51 +76,6 @@ constexpr uint32_t kDecayAt = kOperatorBytes, kExpAt = kDecayAt + 256;
 constexpr uint32_t kVectorBytes = 256 + 128;
 constexpr uint32_t kMarkAt = kDecayAt + kVectorBytes;   // int: the chunk is beyond what fp16 operands resolve
 constexpr size_t kRecord = 33280;                        // bytes per chunk in the workspace
-__host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
-
-__device__ __forceinline__ uint32_t off16(int row, int col) {
-    return (uint32_t)row * 128u + ((((uint32_t)col >> 3) ^ ((uint32_t)row & 7u)) << 4) + ((uint32_t)col & 7u) * 2u;
-}
-__device__ __forceinline__ float2 unpack_bf2(uint32_t u) {
-    return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
-}
-
-// Lane addresses of ldmatrix.x4 for a 16 x 16 block, as byte offsets.  In a swizzled tile the block starts at (row0,
-// column 16 c); in a compact block the rows are 16 bytes and the halves 256.  "plain" gives A order; "cols" swaps the
-// two middle matrices: B order for a block stored [column][k], and, with .trans, A order of the transposed block.
-__device__ __forceinline__ uint32_t tile_plain(int lane, int row0, int c) {
-    const int r = row0 + (lane & 15), ch = 2 * c + (lane >> 4);
-    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
-}
-__device__ __forceinline__ uint32_t tile_cols(int lane, int row0, int c) {
-    const int r = row0 + (lane & 7) + ((lane >> 4) << 3), ch = 2 * c + ((lane >> 3) & 1);
-    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
-}
-__device__ __forceinline__ uint32_t blk_plain(int lane) { return (uint32_t)lane * 16u; }
-__device__ __forceinline__ uint32_t blk_cols(int lane) {
-    return (uint32_t)((lane >> 3) & 1) * 256u + (uint32_t)((lane & 7) + ((lane >> 4) << 3)) * 16u;
-}
-
-// Bounded wait for a whole warp without compiler-made divergence handling around the loop.
-__device__ __forceinline__ bool mbar_wait_tight(uint64_t *bar, uint32_t parity, uint32_t limit) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p, r;\n\t.reg .u32 n;\n\t"
-        "mov.u32 n, %3;\n"
-        "POLL_%=:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra DONE_%=;\n\t"
-        "sub.u32 n, n, 1;\n\t"
-        "setp.ne.u32 r, n, 0;\n\t"
-        "@r bra POLL_%=;\n"
-        "DONE_%=:\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(limit)
-        : "memory");
-    return ok != 0;
-}
-
 // ------------------------------------------------------------------------------------------
 // Kernel 1: the operator of every chunk.  One CTA of four warps per chunk at a time, four CTAs per SM.
 //
@@ -167,28 +119,6 @@ struct OperatorPtrs {
     const void *p[5];   // the same tensors
 };
 
-// d = exp(-exp(w)) of a channel pair
-// (subnormal results flushed: without that every exponential costs a compare and two more multiplications)
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float rcp(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float2 decay2(float2 w) {
-    constexpr float kLog2e = 1.4426950408889634f;
-    const float2 x = mul2(w, make_float2(kLog2e, kLog2e));
-    const float2 z = mul2(make_float2(ex2(x.x), ex2(x.y)), make_float2(-kLog2e, -kLog2e));
-    return make_float2(ex2(z.x), ex2(z.y));
-}
-__device__ __forceinline__ uint32_t pack2(float2 v) { return pack_half2(v.x, v.y); }
-__device__ __forceinline__ int exponent_of(float v) { return (int)(__float_as_uint(v) >> 23); }   // biased; v > 0
-__device__ __forceinline__ float exp2_of(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }   // -126 <= e <= 127
 __device__ __forceinline__ int lds_s8(uint32_t addr) {
     int v;
     asm volatile("ld.shared.s8 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
@@ -740,7 +670,7 @@ struct Scan {
     static constexpr uint32_t kYTile = kL * kN * sizeof(TIO);
     static constexpr uint32_t kY = kZV + 2 * 2 * kPanel;          // two output tiles (fp32: each two panels of 32 channels)
     static constexpr uint32_t kBars = kY + 2 * kYTile;
-    static constexpr uint32_t kBytes = kBars + 128;
+    static constexpr uint32_t kBytes = kBars + 256;
     static_assert(kBytes <= 232448, "the scan exceeds an SM");
 };
 
@@ -754,10 +684,18 @@ __device__ __forceinline__ int k_position(int j) {
     return ((j >> 5) * 4 + ((j & 7) >> 1)) * 8 + ((j >> 4) & 1) * 4 + (j & 1) + (((j & 15) >> 3) << 1);
 }
 
-// Descriptor of the operator as K-major A operand without swizzle: 8 x 16-byte core matrices, 128 bytes apart along k, 2048
-// along n; one K-step is two of them.
+// ... and the state column or token of a position.
+__device__ __forceinline__ int k_at_position(int p) {
+    return (p >> 5) * 32 + ((p >> 2) & 1) * 16 + ((p >> 1) & 1) * 8 + ((p >> 3) & 3) * 2 + (p & 1);
+}
+
+// Descriptor of the operator as A operand without swizzle: 8 x 16-byte core matrices, 128 bytes apart along k, 2048
+// along n.  Forwards the rows are n and a K-step is two core matrices along k; for gradients the operator is transposed: the
+// rows are k (contiguous, "MN-major") and a K-step is two core matrices along n.
+template <bool kTransposed>
 __device__ __forceinline__ uint64_t desc_operator(uint32_t addr, int ks) {
-    return (uint64_t)(((addr + (uint32_t)ks * 256u) >> 4) & 0x3fffu) | (uint64_t)(128u >> 4) << 16 | (uint64_t)(2048u >> 4) << 32 | (uint64_t)1 << 46;
+    const uint32_t step = kTransposed ? 4096u : 256u, along_k = kTransposed ? 2048u : 128u, along_m = kTransposed ? 128u : 2048u;
+    return (uint64_t)(((addr + (uint32_t)ks * step) >> 4) & 0x3fffu) | (uint64_t)(along_k >> 4) << 16 | (uint64_t)(along_m >> 4) << 32 | (uint64_t)1 << 46;
 }
 
 // Token-by-token recomputation of one chain over tokens t0 .. t1 - 1, fp32 throughout: what a
@@ -765,7 +703,7 @@ __device__ __forceinline__ uint64_t desc_operator(uint32_t addr, int ks) {
 // lanes per row; columns and sums in the order of the sequential scan (wkv7_seq.cu), whose bits it reproduces.
 template <typename TIO>
 __device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TIO *v, TIO *y, const float *s_in, float *s_out,
-                                                int bi, int h, int H, int Tlen, int t0, int t1) {
+                                                float *snapshots, int bi, int h, int H, int Tlen, int t0, int t1) {
     const int row = (int)threadIdx.x >> 2, c0 = ((int)threadIdx.x & 3) * 4;   // columns c0 + 16 kk + e
     float S[4][4];
 #pragma unroll
@@ -773,6 +711,12 @@ __device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TI
 #pragma unroll
         for (int e = 0; e < 4; ++e) S[kk][e] = s_in ? s_in[row * kN + c0 + 16 * kk + e] : 0.f;
     for (int t = t0; t < t1; ++t) {
+        if (snapshots != nullptr && t % kL == 0) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) snapshots[(size_t)(t / kL) * kN * kN + row * kN + c0 + 16 * kk + e] = S[kk][e];
+        }
         const size_t o = (((size_t)bi * Tlen + t) * H + h) * kN;
         auto f = [&](int x, int kk, int e) -> float { return static_cast<float>(static_cast<const TIO *>(in.p[x])[o + c0 + 16 * kk + e]); };
         float p[4] = {}, yy[4] = {};
@@ -807,11 +751,70 @@ __device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TI
     }
 }
 
-template <typename TIO>
+// The same for the gradient of the state, backwards over a whole chain; dv comes with it.  Snapshots: the gradient of the state
+// at the end of every chunk.
+__device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, const __nv_bfloat16 *dy, __nv_bfloat16 *dv, const float *g_in,
+                                                     float *g_out, float *snapshots, int bi, int h, int H, int Tlen) {
+    const int row = (int)threadIdx.x >> 2, c0 = ((int)threadIdx.x & 3) * 4;
+    float G[4][4];
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) G[kk][e] = g_in ? g_in[row * kN + c0 + 16 * kk + e] : 0.f;
+    for (int t = Tlen - 1; t >= 0; --t) {
+        if (t == Tlen - 1 || t % kL == kL - 1) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) snapshots[(size_t)(t / kL) * kN * kN + row * kN + c0 + 16 * kk + e] = G[kk][e];
+        }
+        const size_t o = (((size_t)bi * Tlen + t) * H + h) * kN;
+        auto f = [&](int x, int kk, int e) -> float { return __bfloat162float(static_cast<const __nv_bfloat16 *>(in.p[x])[o + c0 + 16 * kk + e]); };
+        const float dyi = __bfloat162float(dy[o + row]);
+        float dsa = 0.f, out = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                G[kk][e] = fmaf(dyi, f(XR, kk, e), G[kk][e]);
+                dsa = fmaf(G[kk][e], f(XB, kk, e), dsa);
+                out = fmaf(G[kk][e], f(XK, kk, e), out);
+            }
+#pragma unroll
+        for (int x = 1; x <= 2; x <<= 1) {
+            dsa += __shfl_xor_sync(0xffffffffu, dsa, x);
+            out += __shfl_xor_sync(0xffffffffu, out, x);
+        }
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) G[kk][e] = fmaf(G[kk][e], expf(-expf(f(XW, kk, e))), dsa * f(XA, kk, e));
+        if (c0 == 0) dv[o + row] = __float2bfloat16_rn(out);
+    }
+    if (g_out != nullptr) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) g_out[row * kN + c0 + 16 * kk + e] = G[kk][e];
+    }
+}
+
+// What a scan is for.  Training needs the state every chunk starts with (kForTraining); its backward pass is the same scan
+// over the transposed operators, last chunk first (kGradients): with G[j'][i] the gradient of the state behind a chunk and
+// dY[t][i] that of its output,
+//     D'[k][i] = sum_n O[n][k] [G; dY][n][i]
+// has the rows j of the gradient in front of the chunk and the rows s of dV.  Gradients may be far smaller than fp16 resolves
+// well (or larger than it holds), so G and dY of a chunk are scaled by a power of two, chosen by the converting warps from the largest magnitudes
+// of dY in this chunk and the three after it and of G as the state warps last published it.
+enum ScanKind { kPrefill, kForTraining, kGradients };
+
+template <typename TIO, int kKind>
 __global__ void __launch_bounds__(Scan<TIO>::kThreads, 1)
 wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs, const TIO *__restrict__ v,
                        const unsigned char *__restrict__ records, const float *state_in, float *state_out,
-                       TIO *__restrict__ y, int *flags, int Tlen, int H, int chunk0, int n, int resolve_flagged, int *status) {
+                       TIO *__restrict__ y, float *__restrict__ snapshots, int *flags, int Tlen, int H, int chunk0, int n, int resolve_flagged,
+                       int *status) {
+    constexpr bool kGrad = kKind == kGradients;
     using SM = Scan<TIO>;
     constexpr int NS = SM::kStages;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -827,6 +830,14 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     uint64_t *bar_acc = bar_empty + NS;                                    // [2] an accumulator is complete
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_acc + 2);
     volatile int *bad = reinterpret_cast<volatile int *>(tmem_slot + 1);   // bit 0: a wait expired, bit 1: a value is not finite
+    // (gradients) [2] the scale of a chunk is known; its exponent by chunk mod 4; largest magnitudes as float bits: of G by chunk
+    // mod 4 (and at the start) and state warp, of dY by chunk mod 2 and converting warp
+    uint64_t *bar_scale = bar_acc + 3;
+    volatile int *scale_exp = reinterpret_cast<volatile int *>(smem + SM::kBars + 128);
+    volatile uint32_t *top_g = reinterpret_cast<volatile uint32_t *>(smem + SM::kBars + 144), *top_dy = top_g + 20;
+    static_assert(8 * (2 * NS + 5) <= 128, "the barriers' place");
+    // chunk of step c (gradients run from the last to the first)
+    auto at_step = [&](int c) { return kGrad ? n - 1 - c : c; };
     const int chain = blockIdx.x;
     const int bi = chain / H, h = chain % H;
     if (tid == 0) {
@@ -836,6 +847,10 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         }
         mbar_init(bar_acc, 1);
         mbar_init(bar_acc + 1, 1);
+        if (kGrad) {
+            mbar_init(bar_scale, 1);
+            mbar_init(bar_scale + 1, 1);
+        }
         mbar_fence_init();
         *bad = 0;
         tma_prefetch_desc(&maps.v);
@@ -876,14 +891,14 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 if (limit == 1u) break;
                 const uint32_t st = sb + s * SM::kStage;
                 mbar_expect_tx(bar_full + s, kOperatorBytes + kVectorBytes + SM::kVBytes);
-                const unsigned char *src = rec + (size_t)c * kRecord;
+                const unsigned char *src = rec + (size_t)at_step(c) * kRecord;
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                              ::"r"(st), "l"(src), "r"(kOperatorBytes), "r"(smem_u32(bar_full + s))
                              : "memory");
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                              ::"r"(st + SM::kVec), "l"(src + kDecayAt), "r"(kVectorBytes), "r"(smem_u32(bar_full + s))
                              : "memory");
-                const int trow = bi * Tlen + (chunk0 + c) * kL;
+                const int trow = bi * Tlen + (chunk0 + at_step(c)) * kL;
                 tma_load_2d(smem + s * SM::kStage + SM::kV, &maps.v, h * kN, trow, bar_full + s);
                 if (SM::kF32) tma_load_2d(smem + s * SM::kStage + SM::kV + SM::kVBytes / 2, &maps.v, h * kN + 32, trow, bar_full + s);
             }
@@ -893,7 +908,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         __syncwarp();
     } else if (warp == 9) {
         // ---------------- issuing warp
-        constexpr uint32_t id = make_idesc(kFmtF16, 128, 64, false, true);
+        constexpr uint32_t id = make_idesc(kFmtF16, 128, 64, kGrad, true);
         auto v_products = [&](int c) {
             const int s = c % NS, a = c & 1;
             wait(bar_full + s, (uint32_t)((c / NS) & 1));
@@ -903,7 +918,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 const uint32_t op = sb + s * SM::kStage, vt = sb + SM::kZV + a * 2 * kPanel + kPanel;
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                    umma_f16(tmem + a * 64, desc_operator(op, 4 + ks), make_smem_desc(vt + ks * 2048u, kPanel, 1024u), id, ks > 0);
+                    umma_f16(tmem + a * 64, desc_operator<kGrad>(op, 4 + ks), make_smem_desc(vt + ks * 2048u, kPanel, 1024u), id, ks > 0);
             }
             __syncwarp();
         };
@@ -916,7 +931,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 const uint32_t op = sb + s * SM::kStage, zt = sb + SM::kZV + a * 2 * kPanel;
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                    umma_f16(tmem + a * 64, desc_operator(op, ks), make_smem_desc(zt + ks * 2048u, kPanel, 1024u), id, true);
+                    umma_f16(tmem + a * 64, desc_operator<kGrad>(op, ks), make_smem_desc(zt + ks * 2048u, kPanel, 1024u), id, true);
                 umma_commit(bar_acc + a);
                 umma_commit(bar_empty + s);
             }
@@ -927,12 +942,51 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         // ---------------- V converters: tile -> fp16 rows in the order of the contraction index, 16-byte pieces; rows past the sequence's end belong to
         // another one, whatever they hold stays out of the sums
         constexpr int kShare = kL * kN / 8 / 32 / 2;
+        uint32_t dy_before[3] = {0u, 0u, 0u};   // (gradients)
+        if constexpr (kGrad) asm volatile("bar.sync 7, 192;" ::: "memory");   // the state warps have published the start
         for (int c = 0; c < n; ++c) {
             const int s = c % NS, a = c & 1;
             wait(bar_full + s, (uint32_t)((c / NS) & 1));
             if (c >= 2) wait(bar_acc + a, (uint32_t)(((c >> 1) - 1) & 1));   // the products that last read this tile
             const uint32_t vt = sb + s * SM::kStage + SM::kV, out = sb + SM::kZV + a * 2 * kPanel + kPanel;
-            const int valid = Tlen - (chunk0 + c) * kL;
+            const int valid = Tlen - (chunk0 + at_step(c)) * kL;
+            if constexpr (kGrad) {
+                // dY of a chunk: rows in token order, scaled
+                uint32_t x[kShare][4];
+                __nv_bfloat162 m = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < kShare; ++k) {
+                    const int p = ((warp - 10) * kShare + k) * 32 + lane, t = p >> 3;
+                    lds128(x[k], vt + off16(t, (p & 7) * 8));
+                    if (t >= valid) x[k][0] = x[k][1] = x[k][2] = x[k][3] = 0;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&x[k][e])));
+                }
+                const uint32_t own = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(__low2float(m), __high2float(m))));
+                if (lane == 0) top_dy[a * 2 + warp - 10] = own;
+                asm volatile("bar.sync 6, 64;" ::: "memory");
+                const uint32_t dy_now = max(top_dy[a * 2], top_dy[a * 2 + 1]);
+                const volatile uint32_t *tg = top_g + (c < 3 ? 4 : (c - 3) & 3) * 4;
+                // (entries of G gather a chunk's dY times r: eight times dY leaves room on both sides)
+                const float dy_most = 8.f * __uint_as_float(max(max(dy_now, dy_before[0]), max(dy_before[1], dy_before[2])));
+                const float most = fmaxf(dy_most, __uint_as_float(max(max(tg[0], tg[1]), max(tg[2], tg[3]))));
+                const int ex = most > 0.f ? min(max(exponent_of(most) - 127 - 5, -96), 96) : 0;
+                dy_before[2] = dy_before[1];
+                dy_before[1] = dy_before[0];
+                dy_before[0] = dy_now;
+                if (warp == 10 && lane == 0) {
+                    scale_exp[c & 3] = ex;
+                    mbar_arrive(bar_scale + a);
+                }
+                const float2 f = make_float2(exp2_of(-ex), exp2_of(-ex));
+#pragma unroll
+                for (int k = 0; k < kShare; ++k) {
+                    const int p = ((warp - 10) * kShare + k) * 32 + lane;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) x[k][e] = pack2(mul2(unpack_bf2(x[k][e]), f));
+                    sts128(out + off16(p >> 3, (p & 7) * 8), x[k]);
+                }
+            } else {
 #pragma unroll
             for (int k0 = 0; k0 < kShare; k0 += 4) {
                 uint32_t x[4][4];
@@ -959,6 +1013,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                     sts128(out + off16(k_position(p >> 3), (p & 7) * 8), x[k]);
                 }
             }
+            }
             fence_proxy_async();
             v_arrive(c);
         }
@@ -968,22 +1023,49 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         const int i0 = hf * 32;                       // this thread's 32 value channels
         if (quarter < 2) {
             // ---------------- state rows j'
-            const int jp = quarter * 32 + lane;
-            const uint32_t zrow = sb + SM::kZV + off16(k_position(jp), 0);
-            const uint32_t sw = ((uint32_t)k_position(jp) & 7u) << 4;
+            // (gradients: this accumulator row is the channel at its position of the contraction index, and operand rows are in order)
+            const int jp = kGrad ? k_at_position(quarter * 32 + lane) : quarter * 32 + lane;
+            const int zr = kGrad ? jp : k_position(jp);
+            const uint32_t zrow = sb + SM::kZV + off16(zr, 0);
+            const uint32_t sw = ((uint32_t)zr & 7u) << 4;
             float2 Z[16];
 #pragma unroll
             for (int e = 0; e < 16; ++e)
                 Z[e] = s_in ? make_float2(s_in[(i0 + 2 * e) * kN + jp], s_in[(i0 + 2 * e + 1) * kN + jp]) : make_float2(0.f, 0.f);
-            // this row's scalars of a chunk: e^{c_L}, fx, factor of P and Kt
+            // this row's scalars of a chunk: e^{c_L}, and what the operand and the product are multiplied by: fx and the factor of P
+            // and Kt, or, for gradients, the other way round with the chunk's scale
             auto load_vec = [&](int c, float &gx, float &fx, float &g2) {
                 const int s = c % NS;
                 wait(bar_full + s, (uint32_t)((c / NS) & 1));
                 const unsigned char *vec = smem + s * SM::kStage + SM::kVec;
                 gx = *reinterpret_cast<const float *>(vec + jp * 4);
                 const int ef = *reinterpret_cast<const signed char *>(vec + 256 + jp), eg = *reinterpret_cast<const signed char *>(vec + 320 + jp);
-                fx = gx * exp2_of(ef);
-                g2 = exp2_of(-eg);
+                if constexpr (kGrad) {
+                    wait(bar_scale + (c & 1), (uint32_t)((c >> 1) & 1));
+                    const int ex = scale_exp[c & 3];
+                    fx = exp2_of(-eg) * exp2_of(-ex);
+                    g2 = gx * exp2_of(ef) * exp2_of(ex);
+                } else {
+                    fx = gx * exp2_of(ef);
+                    g2 = exp2_of(-eg);
+                }
+            };
+            // largest magnitude of the state in this warp's share, for the converting warps
+            auto publish = [&](int slot) {
+                float m[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int e = 0; e < 16; ++e) m[e & 3] = fmaxf(m[e & 3], fmaxf(fabsf(Z[e].x), fabsf(Z[e].y)));
+                const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]))));
+                if (lane == 0) top_g[slot * 4 + quarter * 2 + hf] = most;
+            };
+            auto keep = [&](int c) {   // the state that step c starts from
+                float *dst = snapshots + ((size_t)chain * n + at_step(c)) * kN * kN + jp;
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                    if (RWKV7_IN_RANGE(c < n && i0 + 2 * e + 1 < kN && jp < kN, status)) {
+                        dst[(i0 + 2 * e) * kN] = Z[e].x;
+                        dst[(i0 + 2 * e + 1) * kN] = Z[e].y;
+                    }
             };
             // the state a chunk starts with, as operand: times fx, fp16
             auto put_z = [&](int c, float fx) {
@@ -999,10 +1081,16 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 z_arrive();
             };
             float gx, fx, g2, gxn = 1.f, fxn = 1.f, g2n = 0.f;
+            if constexpr (kGrad) {
+                publish(4);
+                asm volatile("bar.sync 7, 192;" ::: "memory");
+            }
             load_vec(0, gx, fx, g2);
             put_z(0, fx);
             for (int c = 0; c < n; ++c) {
                 const int a = c & 1;
+                if constexpr (kGrad) publish(c & 3);
+                if constexpr (kKind != kPrefill) keep(c);
                 if (c + 1 < n) load_vec(c + 1, gxn, fxn, g2n);   // (while the products run)
                 wait(bar_acc + a, (uint32_t)((c >> 1) & 1));
                 tc_fence_after();
@@ -1036,7 +1124,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         } else {
             // ---------------- output tokens t.  A chunk's y tile is staged in shared memory (one of two buffers) and leaves
             // by a bulk tensor store; a partial last chunk is stored by the threads themselves.
-            const int tq = (quarter - 2) * 32 + lane;     // token within the chunk
+            const int tq = kGrad ? k_at_position((quarter - 2) * 32 + lane) : (quarter - 2) * 32 + lane;   // token within the chunk
             const bool elected = warp == 2 && lane == 0;
             float ysum = 0.f;    // a non-finite output makes the sum non-finite for good
             v_arrive(0);
@@ -1048,9 +1136,14 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 uint32_t d[32];
                 tmem_ld32(acc + a * 64, d);
                 tmem_ld_wait();
+                if constexpr (kGrad) {
+                    const float up = exp2_of(scale_exp[c & 3]);
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) d[e] = __float_as_uint(__uint_as_float(d[e]) * up);
+                }
                 tc_fence_before();
                 if (c + 2 < n) v_arrive(c + 2);
-                const int t0 = (chunk0 + c) * kL;
+                const int t0 = (chunk0 + at_step(c)) * kL;
                 float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int e = 0; e < 32; ++e) sum[e & 3] += fabsf(__uint_as_float(d[e]));
@@ -1109,8 +1202,11 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     }
     // A value beyond fp16 (or a flagged chain that nobody else takes): the chain once more, token by token, from the state
     // this launch started with, which is still untouched.
-    if (((flagged && resolve_flagged) || (*bad & 2)) && tid < 256)
-        scan_rows_by_token<TIO>(ptrs, v, y, s_in, s_out, bi, h, H, Tlen, chunk0 * kL, t_end);
+    if (((flagged && resolve_flagged) || (*bad & 2)) && tid < 256) {
+        float *own = snapshots + (kKind == kPrefill ? 0 : (size_t)chain * n * kN * kN);
+        if constexpr (kGrad) scan_gradients_by_token(ptrs, v, y, s_in, s_out, own, bi, h, H, Tlen);
+        else scan_rows_by_token<TIO>(ptrs, v, y, s_in, s_out, kKind == kPrefill ? nullptr : own, bi, h, H, Tlen, chunk0 * kL, t_end);
+    }
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -1129,6 +1225,20 @@ EncodeTiledFn encode_fn() {
             fn = reinterpret_cast<EncodeTiledFn>(p);
     });
     return fn;
+}
+
+// A [B,T,H,64] tensor as rows of channels, in tiles of 64 tokens by 128 bytes.
+bool describe_rows(CUtensorMap *map, const void *ptr, int64_t B, int64_t T, int64_t H, bool bf16) {
+    const EncodeTiledFn encode = encode_fn();
+    const size_t esize = bf16 ? 2 : 4;
+    const cuuint64_t dims[2] = {(cuuint64_t)(H * kN), (cuuint64_t)(B * T)};
+    const cuuint64_t strides[1] = {(cuuint64_t)(H * kN * esize)};
+    const cuuint32_t box[2] = {(cuuint32_t)(128 / esize), (cuuint32_t)kL};
+    const cuuint32_t estr[2] = {1, 1};
+    return encode != nullptr &&
+           encode(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(ptr), dims, strides, box,
+                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 constexpr size_t kAlign = 256;
@@ -1370,8 +1480,7 @@ bool wkv7_split_supported(const Wkv7Args &p) {
 // state is not written: it may alias the initial state that the recomputation starts from).
 int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes, bool wide_range, bool resolve_flagged,
                       cudaStream_t stream) {
-    EncodeTiledFn encode = encode_fn();
-    if (encode == nullptr) return (int)cudaErrorNotSupported;
+    if (encode_fn() == nullptr) return (int)cudaErrorNotSupported;
     const size_t chains = (size_t)(p.B * p.H);
     const int nchunks = (int)((p.T + kL - 1) / kL);
     // The plan: overlapped (two buffers) when it applies and the workspace holds two segments of a useful
@@ -1418,16 +1527,7 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
     OperatorMaps omaps{};
     ScanMaps smaps{};
     const OperatorPtrs optrs{{p.a, p.r, p.b, p.k, p.w}};
-    const cuuint64_t dims[2] = {(cuuint64_t)(p.H * p.N), (cuuint64_t)(p.B * p.T)};
-    const size_t esize = p.bf16 ? 2 : 4;
-    const CUtensorMapDataType etype = p.bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    const cuuint64_t strides[1] = {(cuuint64_t)(p.H * p.N * esize)};
-    const cuuint32_t box[2] = {(cuuint32_t)(128 / esize), (cuuint32_t)kL};   // rows of 128 bytes in shared memory
-    const cuuint32_t estr[2] = {1, 1};
-    auto describe = [&](CUtensorMap *map, const void *ptr) {
-        return encode(map, etype, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    };
+    auto describe = [&](CUtensorMap *map, const void *ptr) { return describe_rows(map, ptr, p.B, p.T, p.H, p.bf16); };
     for (int i = 0; p.bf16 && i < 5; ++i)   // (fp32 tensors are read by the threads themselves)
         if (!describe(&omaps.m[i], optrs.p[i])) return (int)cudaErrorInvalidValue;
     if (!describe(&smaps.v, p.v) || !describe(&smaps.y, p.y)) return (int)cudaErrorInvalidValue;
@@ -1456,13 +1556,13 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
             cfg.numAttrs = st == stream ? 1 : 0;   // directly behind its operator kernel on the caller's stream
             using T = std::remove_pointer_t<decltype(ytype)>;
             err = cudaLaunchKernelEx(&cfg, kern, smaps, optrs, static_cast<const T *>(p.v), records, s_in, s_out,
-                                     static_cast<T *>(p.y), flags, (int)p.T, (int)p.H, c0, n, resolve_flagged ? 1 : 0, status);
+                                     static_cast<T *>(p.y), (float *)nullptr, flags, (int)p.T, (int)p.H, c0, n, resolve_flagged ? 1 : 0, status);
             if (err == cudaSuccess) count_launch();
             return err;
         };
         using bf = __nv_bfloat16;
-        if (!p.bf16) return go(wkv7_state_scan_kernel<float>, (float *)nullptr, Scan<float>::kBytes, Scan<float>::kThreads);
-        return go(wkv7_state_scan_kernel<bf>, (bf *)nullptr, Scan<bf>::kBytes, Scan<bf>::kThreads);
+        if (!p.bf16) return go(wkv7_state_scan_kernel<float, kPrefill>, (float *)nullptr, Scan<float>::kBytes, Scan<float>::kThreads);
+        return go(wkv7_state_scan_kernel<bf, kPrefill>, (bf *)nullptr, Scan<bf>::kBytes, Scan<bf>::kThreads);
     };
     auto launch_operators = [&](int buf, int c0, int n) -> cudaError_t {
         const long long units = (long long)chains * n;
@@ -1518,6 +1618,98 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
     // operator kernel is ordered before the scan of its segment)
     e = cudaStreamWaitEvent(stream, scanned[(segment - 1) & 1], 0);
     return (int)e;
+}
+
+// ---- a training step ------------------------------------------------------------------------------
+//
+// Kept between the passes: [records of all chunks][state in front of every chunk][one int per chain]; workspace of the backward
+// pass: [gradient of the state behind every chunk][one int per chain].
+
+namespace {
+
+struct TrainingLayout {
+    size_t chains, nchunks, states, flags, total;
+};
+TrainingLayout training_layout(int64_t B, int64_t T, int64_t H, bool with_records) {
+    TrainingLayout l{};
+    l.chains = (size_t)(B * H);
+    l.nchunks = (size_t)((T + kL - 1) / kL);
+    l.states = with_records ? align_up(l.chains * l.nchunks * kRecord) : 0;
+    l.flags = l.states + l.chains * l.nchunks * kN * kN * sizeof(float);
+    l.total = l.flags + align_up(l.chains * sizeof(int));
+    return l;
+}
+
+template <int kKind>
+int launch_training_scan(const ScanMaps &maps, const OperatorPtrs &ptrs, const void *in, const unsigned char *records, const float *s_in,
+                         float *s_out, void *out, float *states, int *flags, const TrainingLayout &l, int64_t T, int64_t H, int *status,
+                         cudaStream_t stream) {
+    using bf = __nv_bfloat16;
+    auto kern = wkv7_state_scan_kernel<bf, kKind>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Scan<bf>::kBytes);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)l.chains);
+    cfg.blockDim = dim3((unsigned)Scan<bf>::kThreads);
+    cfg.dynamicSmemBytes = Scan<bf>::kBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, maps, ptrs, static_cast<const bf *>(in), records, s_in, s_out, static_cast<bf *>(out), states, flags,
+                           (int)T, (int)H, 0, (int)l.nchunks, 1, status);
+    if (e == cudaSuccess) count_launch();
+    return (int)e;
+}
+
+}  // namespace
+
+bool wkv7_training_supported(int64_t B, int64_t T, int64_t H, int64_t N, bool bf16) {
+    return bf16 && N == kN && T >= kL && T % 16 == 0 && B * T < (int64_t(1) << 31) && B * H < (int64_t(1) << 24);
+}
+size_t wkv7_training_saved_bytes(int64_t B, int64_t T, int64_t H) { return training_layout(B, T, H, true).total; }
+size_t wkv7_training_workspace_bytes(int64_t B, int64_t T, int64_t H) { return training_layout(B, T, H, false).total; }
+
+int launch_wkv7_training_forward(const Wkv7Args &p, void *saved, cudaStream_t stream) {
+    const TrainingLayout l = training_layout(p.B, p.T, p.H, true);
+    unsigned char *base = static_cast<unsigned char *>(saved);
+    OperatorMaps omaps{};
+    ScanMaps smaps{};
+    const OperatorPtrs optrs{{p.a, p.r, p.b, p.k, p.w}};
+    for (int i = 0; i < 5; ++i)
+        if (!describe_rows(&omaps.m[i], optrs.p[i], p.B, p.T, p.H, true)) return (int)cudaErrorInvalidValue;
+    if (!describe_rows(&smaps.v, p.v, p.B, p.T, p.H, true) || !describe_rows(&smaps.y, p.y, p.B, p.T, p.H, true)) return (int)cudaErrorInvalidValue;
+    int *status = nullptr;
+    if (int e = device_status_ptr(p.device, &status)) return e;
+    auto k1 = wkv7_chunk_operator_kernel<__nv_bfloat16>;
+    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem1);
+    if (e != cudaSuccess) return (int)e;
+    const long long units = (long long)(l.chains * l.nchunks), places = 4LL * p.num_sms;
+    k1<<<(unsigned)(units < places ? units : places), kOpThreads, kSmem1, stream>>>(omaps, optrs, base, (int)p.T, (int)p.H, 0, (int)l.nchunks, (int)l.chains, 1,
+                                                                                     status);
+    count_launch();
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+    return launch_training_scan<kForTraining>(smaps, optrs, p.v, base, p.s0, p.s_out, p.y, reinterpret_cast<float *>(base + l.states),
+                                              reinterpret_cast<int *>(base + l.flags), l, p.T, p.H, status, stream);
+}
+
+int launch_wkv7_training_backward(const Wkv7TrainingBackwardArgs &p, const void *saved, void *workspace, cudaStream_t stream) {
+    const TrainingLayout ls = training_layout(p.B, p.T, p.H, true), lw = training_layout(p.B, p.T, p.H, false);
+    const unsigned char *base = static_cast<const unsigned char *>(saved);
+    unsigned char *ws = static_cast<unsigned char *>(workspace);
+    float *gradients = reinterpret_cast<float *>(ws + lw.states);
+    ScanMaps smaps{};
+    const OperatorPtrs optrs{{p.a, p.r, p.b, p.k, p.w}};
+    if (!describe_rows(&smaps.v, p.dy, p.B, p.T, p.H, true) || !describe_rows(&smaps.y, p.dv, p.B, p.T, p.H, true)) return (int)cudaErrorInvalidValue;
+    int *status = nullptr;
+    if (int e = device_status_ptr(p.device, &status)) return e;
+    if (int e = launch_training_scan<kGradients>(smaps, optrs, p.dy, base, p.next_state_grad, p.initial_state_grad, p.dv, gradients,
+                                                 reinterpret_cast<int *>(ws + lw.flags), lw, p.T, p.H, status, stream))
+        return e;
+    return launch_wkv7_chunk_gradients(p, reinterpret_cast<const float *>(base + ls.states), gradients, stream);
 }
 
 }  // namespace rwkv7

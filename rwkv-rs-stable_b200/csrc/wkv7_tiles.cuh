@@ -1,0 +1,88 @@
+// What the tensor-core kernels of a 64-token chunk share: tiles of [64][64] 16-bit elements and 16 x 16 blocks in shared
+// memory, the lane addresses of matrix loads on them, and the arithmetic of the decays.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "sm100_mma.cuh"
+#include "sm100_umma.cuh"
+
+namespace rwkv7 {
+namespace sm100 {
+
+constexpr int kN = 64;   // head size
+constexpr int kL = 64;   // tokens per chunk
+constexpr float kBlockDecay = 6.144212e-6f;   // e^-12: a block below it (or a NaN) marks the chunk
+constexpr uint32_t kPanel = 8192;             // one [64][64] 16-bit tile, 128-byte rows, 16-byte pieces XOR-ed with (row & 7)
+constexpr uint32_t kBlk = 512;                // one 16 x 16 fp16 block: two halves of 8 columns, each [16 rows][16 bytes]
+
+__device__ __forceinline__ uint32_t off16(int row, int col) {
+    return (uint32_t)row * 128u + ((((uint32_t)col >> 3) ^ ((uint32_t)row & 7u)) << 4) + ((uint32_t)col & 7u) * 2u;
+}
+__device__ __forceinline__ float2 unpack_bf2(uint32_t u) {
+    return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+
+// Lane addresses of ldmatrix.x4 for a 16 x 16 block, as byte offsets.  In a swizzled tile the block starts at (row0,
+// column 16 c); in a compact block the rows are 16 bytes and the halves 256.  "plain" gives A order; "cols" swaps the
+// two middle matrices: B order for a block stored [column][k], and, with .trans, A order of the transposed block.
+__device__ __forceinline__ uint32_t tile_plain(int lane, int row0, int c) {
+    const int r = row0 + (lane & 15), ch = 2 * c + (lane >> 4);
+    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
+}
+__device__ __forceinline__ uint32_t tile_cols(int lane, int row0, int c) {
+    const int r = row0 + (lane & 7) + ((lane >> 4) << 3), ch = 2 * c + ((lane >> 3) & 1);
+    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
+}
+__device__ __forceinline__ uint32_t blk_plain(int lane) { return (uint32_t)lane * 16u; }
+__device__ __forceinline__ uint32_t blk_cols(int lane) {
+    return (uint32_t)((lane >> 3) & 1) * 256u + (uint32_t)((lane & 7) + ((lane >> 4) << 3)) * 16u;
+}
+
+// Bounded wait for a whole warp without compiler-made divergence handling around the loop.
+__device__ __forceinline__ bool mbar_wait_tight(uint64_t *bar, uint32_t parity, uint32_t limit) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, r;\n\t.reg .u32 n;\n\t"
+        "mov.u32 n, %3;\n"
+        "POLL_%=:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE_%=;\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 r, n, 0;\n\t"
+        "@r bra POLL_%=;\n"
+        "DONE_%=:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(limit)
+        : "memory");
+    return ok != 0;
+}
+
+// d = exp(-exp(w)) of a channel pair
+// (subnormal results flushed: without that every exponential costs a compare and two more multiplications)
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float2 decay2(float2 w) {
+    constexpr float kLog2e = 1.4426950408889634f;
+    const float2 x = mul2(w, make_float2(kLog2e, kLog2e));
+    const float2 z = mul2(make_float2(ex2(x.x), ex2(x.y)), make_float2(-kLog2e, -kLog2e));
+    return make_float2(ex2(z.x), ex2(z.y));
+}
+__device__ __forceinline__ uint32_t pack2(float2 v) { return pack_half2(v.x, v.y); }
+__device__ __forceinline__ int exponent_of(float v) { return (int)(__float_as_uint(v) >> 23); }   // biased; v > 0
+__device__ __forceinline__ float exp2_of(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }   // -126 <= e <= 127
+
+}  // namespace sm100
+}  // namespace rwkv7

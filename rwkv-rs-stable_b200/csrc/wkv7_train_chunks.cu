@@ -1,0 +1,732 @@
+// Last part of the WKV7 training step (N == 64, bf16 tensors, 64-token chunks): from the state S in front of every chunk
+// (kept by the forward scan) and the gradient G of the state behind it (kept by the gradient scan) the gradients of
+// receptance, decay, keys, removal key and replacement, all chunks in parallel.
+//
+// Gradient definitions: the reference's wkv7_backward_kernel (crates/rwkv-nn/src/kernels/train/time_mixer/wkv7/kernel.rs:395-690).
+// In matrices over a 16-token block, with the decay D_t from the block's start to token t (inclusive), D its value at the
+// end, and a reference point mu per channel, the power of two nearest sqrt(D) (so that no factor leaves e^+-6):
+//     a~_t = a_t D_{t-1} / mu   r~_t = r_t D_t / mu   b^_s = b_s mu / D_s   k^_s = k_s mu / D_s
+//     A_ab[t][s] = a~_t . b^_s (s < t)   A_ak = a~_t . k^_s (s < t)   A_rb[t][s] = r~_t . b^_s (s <= t)
+//     U = T (a~ (S mu)^T + A_ak V)                         T = (I - A_ab)^-1,  u_t = S_{t-1} a_t
+//     S' = (D / mu) (S mu + U^T b^ + V^T k^)               state at the block's end
+//     dU = T^T (b^ (G rho)^T + A_rb^T dY)                  rho = D / mu
+//     G' = mu (G rho + dY^T r~ + dU^T a~)                  gradient of the state at the block's start
+//     dr = (D_t / mu) (dY (S mu) + B_rb b^ + B_rk k^)      B_rb = dY U^T, B_rk = dY V^T   (s <= t)
+//     da = (D_{t-1} / mu) (dU (S mu) + B_ab b^ + B_ak k^)  B_ab = dU U^T, B_ak = dU V^T   (s < t)
+//     db = (mu / D_s) (U (G rho) + B_rb^T r~ + B_ab^T a~)  dk = (mu / D_s) (V (G rho) + B_rk^T r~ + B_ak^T a~)
+// The decay's gradient follows from phi_t = colsum(Gh_t . S_t) at a block's boundary: with x_t = b_t db_t + k_t dk_t - r_t dr_t
+//     d_t dd_t = phi_t - x_t,   phi_{t-1} = phi_t - x_t + a_t da_t,   dw_t = -exp(w_t) d_t dd_t.
+// dv is an output of the gradient scan.
+//
+// States, accumulators, decays and sums are fp32; matrix operands are fp16 (11 significant bits), S with V and G with dY scaled
+// by a power of two per chunk.  A chunk whose decay leaves the range of the reference points, or where a value leaves that of
+// fp16, is recomputed token by token in fp32.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "kernels.h"
+#include "sm100_mma.cuh"
+#include "sm100_umma.cuh"
+#include "trace.h"
+#include "wkv7_tiles.cuh"
+
+namespace rwkv7 {
+namespace {
+
+using namespace sm100;
+
+constexpr int kThreads = 256;
+enum { TA = 0, TR, TB, TK, TV, TY, TW, kTensors };
+constexpr uint32_t kTilesBytes = kTensors * kPanel;             // one of two buffers of input tiles
+constexpr uint32_t kFStride = 288;                               // D_t / mu in fp32, [64 tokens][64 channels]; rows 8 banks apart
+constexpr uint32_t kF = 2 * kTilesBytes;
+constexpr uint32_t kS = kF + 64 * kFStride;                      // [4] S mu of block q, fp16 tiles [value row][channel]
+constexpr uint32_t kG = kS + 4 * kPanel;                         // [4] G rho, the same
+constexpr uint32_t kU = kG + 4 * kPanel;                         // U and dU, tiles [token][value row]
+constexpr uint32_t kDU = kU + kPanel;
+constexpr uint32_t kAak = kDU + kPanel;                          // [4] blocks each of A_ak, A_rb, T
+constexpr uint32_t kArb = kAak + 4 * kBlk;
+constexpr uint32_t kT = kArb + 4 * kBlk;
+constexpr uint32_t kDiag = kT + 4 * kBlk;                        // [4] A_ab in fp32
+constexpr uint32_t kMu = kDiag + 4 * 1024;                       // [4][64] fp32 each
+constexpr uint32_t kRho = kMu + 1024;
+constexpr uint32_t kE = kRho + 1024;                             // [8][64] fp32: decay over half a block
+constexpr uint32_t kTop = kE + 2048;                             // [16] largest magnitudes: of S and V, of G and dY, by warp
+constexpr uint32_t kBars = kTop + 64;
+constexpr uint32_t kSmem = kBars + 64;
+static_assert(kS % 1024 == 0 && kSmem <= 232448, "shared memory");
+
+struct ChunkMaps {
+    CUtensorMap in[kTensors];   // [B*T, H*N] bf16, box 64 x 64, 128-byte swizzle
+    CUtensorMap out[5];         // da, dr, db, dk, dw, box 64 x 16
+};
+struct ChunkArgs {
+    const __nv_bfloat16 *in[kTensors];
+    __nv_bfloat16 *out[5];
+    const float *states, *gradients;   // [chain][chunk][64][64]
+    int T, H, nchunks;
+    long long units;
+    int *status;
+};
+
+__device__ __forceinline__ void stsm4(uint32_t addr, const uint32_t (&r)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+// transposed 16 x 16 block, A order to A order
+__device__ __forceinline__ void transpose16(uint32_t (&y)[4], const uint32_t (&x)[4]) {
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y[0]) : "r"(x[0]));
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y[1]) : "r"(x[2]));
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y[2]) : "r"(x[1]));
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y[3]) : "r"(x[3]));
+}
+__device__ __forceinline__ void pack_block(uint32_t (&x)[4], const float (&c0)[4], const float (&c1)[4]) {
+    x[0] = pack_half2(c0[0], c0[1]);
+    x[1] = pack_half2(c0[2], c0[3]);
+    x[2] = pack_half2(c1[0], c1[1]);
+    x[3] = pack_half2(c1[2], c1[3]);
+}
+__device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&b);
+}
+
+// One chunk in fp32, token by token.  `scratch`: 36 KB, `sums`: 64 KB of shared memory.  Four lanes per value row, columns
+// c0 + 16 kk + e; sums over rows go through the warps' partial sums.
+__device__ __noinline__ void chunk_by_token(const ChunkArgs &p, long long unit, float *scratch, float *sums) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row = tid >> 2, c0 = (tid & 3) * 4;
+    const int chain = (int)(unit / p.nchunks), chunk = (int)(unit % p.nchunks);
+    const int valid = min(kL, p.T - chunk * kL);
+    const size_t base = (((size_t)(chain / p.H) * p.T + chunk * kL) * p.H + chain % p.H) * kN, step = (size_t)p.H * kN;
+    float *u = scratch, *du = u + kL * kN, *part = du + kL * kN;   // [token][row]; [2][8 warps][64]
+    float *dr = sums, *da = dr + kL * kN, *db = da + kL * kN, *dk = db + kL * kN;
+    auto in = [&](int x, int t, int i) -> float { return __bfloat162float(p.in[x][base + t * step + i]); };
+    auto decay = [&](int t, int j) -> float { return expf(-expf(in(TW, t, j))); };
+    // column sums of two products over all rows
+    auto column_sums = [&](float (&m)[2][16], float *out0, float *out1) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                float v = m[x][i];
+                for (int o = 4; o <= 16; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane < 4) part[(x * 8 + warp) * kN + c0 + 16 * (i >> 2) + (i & 3)] = v;
+            }
+        __syncthreads();
+        if (tid < 2 * kN) {
+            float v = 0.f;
+            for (int w = 0; w < 8; ++w) v += part[((tid >> 6) * 8 + w) * kN + (tid & 63)];
+            (tid < kN ? out0 : out1)[tid & 63] = v;
+        }
+        __syncthreads();
+    };
+    float M[16];
+    auto load = [&](const float *src) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) M[i] = src[(size_t)unit * kN * kN + row * kN + c0 + 16 * (i >> 2) + (i & 3)];
+    };
+    auto col = [&](int i) { return c0 + 16 * (i >> 2) + (i & 3); };
+    __syncthreads();
+    load(p.states);
+    for (int t = 0; t < valid; ++t) {
+        float sa = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sa = fmaf(M[i], in(TA, t, col(i)), sa);
+        sa += __shfl_xor_sync(0xffffffffu, sa, 1);
+        sa += __shfl_xor_sync(0xffffffffu, sa, 2);
+        if ((tid & 3) == 0) u[t * kN + row] = sa;
+        const float vi = in(TV, t, row);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) M[i] = fmaf(M[i], decay(t, col(i)), fmaf(sa, in(TB, t, col(i)), vi * in(TK, t, col(i))));
+    }
+    __syncthreads();
+    load(p.gradients);
+    for (int t = valid - 1; t >= 0; --t) {
+        const float dy = in(TY, t, row), vi = in(TV, t, row), ui = u[t * kN + row];
+        float m[2][16], dsa = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            M[i] = fmaf(dy, in(TR, t, col(i)), M[i]);
+            dsa = fmaf(M[i], in(TB, t, col(i)), dsa);
+            m[0][i] = M[i] * vi;
+            m[1][i] = M[i] * ui;
+        }
+        dsa += __shfl_xor_sync(0xffffffffu, dsa, 1);
+        dsa += __shfl_xor_sync(0xffffffffu, dsa, 2);
+        if ((tid & 3) == 0) du[t * kN + row] = dsa;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) M[i] = fmaf(M[i], decay(t, col(i)), dsa * in(TA, t, col(i)));
+        column_sums(m, dk + t * kN, db + t * kN);
+    }
+    load(p.states);
+    for (int t = 0; t < valid; ++t) {
+        const float sa = u[t * kN + row], dsa = du[t * kN + row], vi = in(TV, t, row), dy = in(TY, t, row);
+        float m[2][16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            m[0][i] = M[i] * dsa;
+            M[i] = fmaf(M[i], decay(t, col(i)), fmaf(sa, in(TB, t, col(i)), vi * in(TK, t, col(i))));
+            m[1][i] = M[i] * dy;
+        }
+        column_sums(m, da + t * kN, dr + t * kN);
+    }
+    float m[2][16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        m[0][i] = M[i] * p.gradients[(size_t)unit * kN * kN + row * kN + col(i)];
+        m[1][i] = 0.f;
+    }
+    column_sums(m, u, du);   // (u is no longer needed: its first row takes phi at the chunk's end)
+    if (tid < kN) {
+        float phi = u[tid];
+        for (int t = valid - 1; t >= 0; --t) {
+            const int i = t * kN + tid;
+            const size_t o = base + t * step + tid;
+            const float x = in(TB, t, tid) * db[i] + in(TK, t, tid) * dk[i] - in(TR, t, tid) * dr[i];
+            p.out[TA][o] = __float2bfloat16_rn(da[i]);
+            p.out[TR][o] = __float2bfloat16_rn(dr[i]);
+            p.out[TB][o] = __float2bfloat16_rn(db[i]);
+            p.out[TK][o] = __float2bfloat16_rn(dk[i]);
+            p.out[4][o] = __float2bfloat16_rn(-expf(in(TW, t, tid)) * (phi - x));
+            phi -= x - in(TA, t, tid) * da[i];
+        }
+    }
+    __syncthreads();
+}
+
+// One CTA of eight warps per SM, chunk after chunk; the next chunk's tiles arrive in the other buffer meanwhile.  Warp = 16 value
+// rows of S (warps 0-3) or G (warps 4-7): a row of the state never needs another row, so the state stays in the matrix
+// instructions' accumulators over the four blocks of the chunk, S forwards and G backwards, without a barrier.  What the gradients need of
+// it (S mu, G rho, U, dU) is left in shared memory, and then warp = (block, half of the channels) sums over value rows.
+__global__ void __launch_bounds__(kThreads, 1)
+wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ ChunkArgs p) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    if (smem_u32(smem) & 1023u) {
+        if (threadIdx.x == 0) atomicExch(p.status, (int)kDevInternal);
+        return;
+    }
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int g = lane >> 2, c2 = 2 * (lane & 3);
+    const uint32_t sb = smem_u32(smem);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + kBars);   // [2] a buffer's tiles have landed
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + kBars + 16);
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        mbar_init(bar + 1, 1);
+        mbar_fence_init();
+        *abort_flag = 0;
+    }
+    auto coordinates = [&](long long unit, int &x, int &y) {
+        const int chain = (int)(unit / p.nchunks);
+        x = (chain % p.H) * kN;
+        y = (chain / p.H) * p.T + (int)(unit % p.nchunks) * kL;
+    };
+    auto request = [&](long long unit, int buf) {
+        int x, y;
+        coordinates(unit, x, y);
+        mbar_expect_tx(bar + buf, kTilesBytes);
+#pragma unroll
+        for (int i = 0; i < kTensors; ++i) tma_load_2d(smem + buf * kTilesBytes + i * kPanel, &maps.in[i], x, y, bar + buf);
+    };
+    __syncthreads();
+    if (tid == 0 && blockIdx.x < p.units) request(blockIdx.x, 0);
+    // (launched behind the gradient scan with programmatic stream serialization)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    int seq = 0;
+    for (long long unit = blockIdx.x; unit < p.units; unit += gridDim.x, ++seq) {
+        const int buf = seq & 1;
+        const uint32_t tiles = sb + buf * kTilesBytes;
+        const int valid = min(kL, p.T - (int)(unit % p.nchunks) * kL), nblk = valid / 16;
+        // ---- this warp's 16 rows of S or G, in accumulator order: c[n] = rows g, g + 8, columns 8 n + c2, + 1
+        const int wr = warp & 3;
+        const bool g_side = warp >= 4;
+        float c[8][4];
+        {
+            const float *src = (g_side ? p.gradients : p.states) + (size_t)unit * kN * kN + (16 * wr + g) * kN + c2;
+            if (RWKV7_IN_RANGE(unit >= 0 && unit < p.units, p.status)) {
+#pragma unroll
+                for (int n = 0; n < 8; ++n) {
+                    const float2 lo = __ldcs(reinterpret_cast<const float2 *>(src + 8 * n)), hi = __ldcs(reinterpret_cast<const float2 *>(src + 8 * kN + 8 * n));
+                    c[n][0] = lo.x; c[n][1] = lo.y; c[n][2] = hi.x; c[n][3] = hi.y;
+                }
+            }
+        }
+        if (!mbar_wait(bar + buf, (uint32_t)((seq >> 1) & 1))) *abort_flag = 1;
+        __syncwarp();
+        // ---------------- 1. decays of half a block per warp, lane = channel pair; largest magnitudes
+        const int tb = wr, hf = warp >> 2, ch = 2 * lane, t_first = 16 * tb + 8 * hf;
+        const int nv = min(8, max(0, valid - t_first));       // 0 or 8
+        auto at = [&](int x, int u) -> uint32_t { return tiles + x * kPanel + off16(t_first + u, ch); };
+        uint32_t rv[8], ry[8];
+        float2 d[8], e = make_float2(1.f, 1.f);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const uint32_t w = lds32(at(TW, u));
+            rv[u] = nv ? lds32(at(TV, u)) : 0u;
+            ry[u] = nv ? lds32(at(TY, u)) : 0u;
+            d[u] = nv ? decay2(unpack_bf2(w)) : make_float2(1.f, 1.f);
+            e = mul2(e, d[u]);
+        }
+        sts_f2(sb + kE + ((2 * tb + hf) * 64 + ch) * 4, e.x, e.y);
+        {
+            float ms = 0.f, mg = 0.f, mc = 0.f;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float2 a = unpack_bf2(rv[u]), b = unpack_bf2(ry[u]);
+                ms = fmaxf(ms, fmaxf(fabsf(a.x), fabsf(a.y)));
+                mg = fmaxf(mg, fmaxf(fabsf(b.x), fabsf(b.y)));
+            }
+#pragma unroll
+            for (int n = 0; n < 8; ++n) mc = fmaxf(mc, fmaxf(fmaxf(fabsf(c[n][0]), fabsf(c[n][1])), fmaxf(fabsf(c[n][2]), fabsf(c[n][3]))));
+            if (g_side) mg = fmaxf(mg, mc);
+            else ms = fmaxf(ms, mc);
+            const uint32_t a = __reduce_max_sync(0xffffffffu, __float_as_uint(ms)), b = __reduce_max_sync(0xffffffffu, __float_as_uint(mg));
+            if (lane == 0) {
+                sts32(sb + kTop + warp * 4, a);
+                sts32(sb + kTop + 32 + warp * 4, b);
+            }
+        }
+        __syncthreads();
+        if (*abort_flag) break;
+        if (tid == 0 && unit + gridDim.x < p.units) {
+            bulk_wait_group_read<0>();   // the other buffer's gradients have left
+            request(unit + gridDim.x, buf ^ 1);
+        }
+        // ---------------- 2. scaled fp16 operands, in place; D_t / mu
+        float scale_s, scale_g;
+        int ex;
+        {
+            float ms = 0.f, mg = 0.f;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float4 a = lds_f4(sb + kTop + 16 * i), b = lds_f4(sb + kTop + 32 + 16 * i);
+                ms = fmaxf(ms, fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)));
+                mg = fmaxf(mg, fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
+            }
+            const int es = ms > 0.f ? min(max(exponent_of(ms) - 127, -60), 60) : 0, eg = mg > 0.f ? min(max(exponent_of(mg) - 127, -60), 60) : 0;
+            scale_s = exp2_of(-es);
+            scale_g = exp2_of(-eg);
+            ex = es + eg;
+        }
+        bool over;
+        {
+            const float2 e0 = lds_f2(sb + kE + (2 * tb * 64 + ch) * 4), e1 = lds_f2(sb + kE + ((2 * tb + 1) * 64 + ch) * 4);
+            const float2 D = mul2(e0, e1);
+            over = !(D.x >= kBlockDecay && D.y >= kBlockDecay);
+            // mu = 2^-h, h half of D's exponent
+            const int hx = (127 - exponent_of(D.x)) >> 1, hy = (127 - exponent_of(D.y)) >> 1;
+            const float2 mu = make_float2(exp2_of(-hx), exp2_of(-hy)), up = make_float2(exp2_of(hx), exp2_of(hy));
+            const float2 rho = mul2(D, up);
+            if (hf == 0) {
+                sts_f2(sb + kMu + (tb * 64 + ch) * 4, mu.x, mu.y);
+                sts_f2(sb + kRho + (tb * 64 + ch) * 4, rho.x, rho.y);
+            }
+            float2 f = hf ? mul2(e0, up) : up;
+            uint32_t x0[8], x1[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                x0[u] = nv ? lds32(at(TA, u)) : 0u;
+                x1[u] = nv ? lds32(at(TR, u)) : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                sts32(at(TA, u), pack2(mul2(unpack_bf2(x0[u]), f)));
+                f = mul2(f, d[u]);
+                sts32(at(TR, u), pack2(mul2(unpack_bf2(x1[u]), f)));
+                sts_f2(sb + kF + (t_first + u) * kFStride + ch * 4, f.x, f.y);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                x0[u] = nv ? lds32(at(TB, u)) : 0u;
+                x1[u] = nv ? lds32(at(TK, u)) : 0u;
+            }
+            f = make_float2(rcp(rho.x), rcp(rho.y));
+            if (!hf) f = mul2(f, e1);
+            const float2 vs = make_float2(scale_s, scale_s), ys = make_float2(scale_g, scale_g);
+#pragma unroll
+            for (int u = 7; u >= 0; --u) {
+                sts32(at(TB, u), pack2(mul2(unpack_bf2(x0[u]), f)));
+                sts32(at(TK, u), pack2(mul2(unpack_bf2(x1[u]), f)));
+                f = mul2(f, d[u]);
+                sts32(at(TV, u), pack2(mul2(unpack_bf2(rv[u]), vs)));
+                sts32(at(TY, u), pack2(mul2(unpack_bf2(ry[u]), ys)));
+            }
+        }
+        over = __syncthreads_or(over);
+        bool bad = false;
+        if (!over) {
+            // ---------------- 3. warps 0-3: A_ab of a block and T; warps 4-7: A_ak, A_rb
+            {
+                const int q = wr;
+                float m[2][2][4] = {};
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    uint32_t A[4], B[4];
+                    ldsm4(A, tiles + TA * kPanel + tile_plain(lane, 16 * q, kk));
+                    ldsm4(B, tiles + (g_side ? TK : TB) * kPanel + tile_cols(lane, 16 * q, kk));
+                    mma16816(m[0][0], A, B[0], B[1]);
+                    mma16816(m[0][1], A, B[2], B[3]);
+                    if (g_side) {
+                        ldsm4(A, tiles + TR * kPanel + tile_plain(lane, 16 * q, kk));
+                        ldsm4(B, tiles + TB * kPanel + tile_cols(lane, 16 * q, kk));
+                        mma16816(m[1][0], A, B[0], B[1]);
+                        mma16816(m[1][1], A, B[2], B[3]);
+                    }
+                }
+                if (g_side) {
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        const uint32_t o = sb + (x ? kArb : kAak) + q * kBlk + lane * 4;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int r = 0; r < 2; ++r) {
+                                const int t = g + 8 * r + x, s = 8 * h + c2;   // kept: s < t (A_ak), s <= t (A_rb)
+                                sts32(o + h * 256 + r * 128, pack_half2(s < t ? m[x][h][2 * r] : 0.f, s + 1 < t ? m[x][h][2 * r + 1] : 0.f));
+                            }
+                    }
+                } else {
+                    const uint32_t src = sb + kDiag + q * 1024;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) {
+                            const int t = g + 8 * r, piece = 2 * h + (c2 >> 2);
+                            sts_f2(src + t * 64 + ((piece ^ ((t >> 1) & 3)) << 4) + (c2 & 2) * 4, m[0][h][2 * r], m[0][h][2 * r + 1]);
+                        }
+                    __syncwarp();
+                    // forward substitution, a column per lane (both half-warps the same)
+                    const int cc = lane & 15;
+                    float x[16];
+#pragma unroll
+                    for (int t = 0; t < 16; ++t) {
+                        float acc0 = 0.f, acc1 = 0.f;
+#pragma unroll
+                        for (int s4 = 0; s4 < (t + 3) / 4; ++s4) {
+                            const float4 a4 = lds_f4(src + t * 64 + ((s4 ^ ((t >> 1) & 3)) << 4));
+                            if (4 * s4 + 0 < t) acc0 = fmaf(a4.x, x[4 * s4 + 0], acc0);
+                            if (4 * s4 + 1 < t) acc1 = fmaf(a4.y, x[4 * s4 + 1], acc1);
+                            if (4 * s4 + 2 < t) acc0 = fmaf(a4.z, x[4 * s4 + 2], acc0);
+                            if (4 * s4 + 3 < t) acc1 = fmaf(a4.w, x[4 * s4 + 3], acc1);
+                        }
+                        x[t] = (t == cc) ? 1.f : acc0 + acc1;
+                    }
+                    if (lane < 16) {
+                        unsigned char *dst = smem + kT + q * kBlk + (cc >> 3) * 256 + (cc & 7) * 2;
+#pragma unroll
+                        for (int t = 0; t < 16; ++t) *reinterpret_cast<__half *>(dst + t * 16) = __float2half_rn(x[t]);
+                    }
+                }
+            }
+            __syncthreads();
+            // ---------------- 4. the state, block by block: S forwards, G backwards
+            {
+                const uint32_t own = sb + (g_side ? kG : kS), rows = sb + (g_side ? kDU : kU);
+                const uint32_t left = tiles + (g_side ? TY : TV) * kPanel;      // V or dY
+                const uint32_t with = tiles + (g_side ? TB : TA) * kPanel;      // what S or G is multiplied with: a~ or b^
+                const uint32_t mat = sb + (g_side ? kArb : kAak);
+                const uint32_t up_u = tiles + (g_side ? TA : TB) * kPanel, up_l = tiles + (g_side ? TR : TK) * kPanel;
+                const float scale = g_side ? scale_g : scale_s;
+#pragma unroll 1
+                for (int i = 0; i < 4; ++i) {
+                    const int q = g_side ? 3 - i : i, before = g_side ? q + 1 : q - 1;
+                    // from the block before to this one's reference: S (D / mu) mu', G mu rho'
+                    {
+                        const uint32_t f0 = sb + (g_side ? kRho : kMu) + (q * 64 + c2) * 4, f1 = sb + (g_side ? kMu : kRho) + (before * 64 + c2) * 4;
+#pragma unroll
+                        for (int n = 0; n < 8; ++n) {
+                            float2 f = lds_f2(f0 + n * 32);
+                            f = mul2(f, i == 0 ? make_float2(scale, scale) : lds_f2(f1 + n * 32));
+                            c[n][0] *= f.x; c[n][1] *= f.y; c[n][2] *= f.x; c[n][3] *= f.y;
+                        }
+                    }
+                    uint32_t L[4], M[4];
+                    float o[2][2][4] = {};
+                    ldsm4_t(L, left + tile_cols(lane, 16 * q, wr));
+                    if (g_side) ldsm4_t(M, mat + q * kBlk + blk_plain(lane));
+                    else ldsm4(M, mat + q * kBlk + blk_cols(lane));
+                    mma16816(o[0][0], L, M[0], M[1]);
+                    mma16816(o[0][1], L, M[2], M[3]);
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk) {
+                        uint32_t A[4], B[4];
+                        pack_block(A, c[2 * kk], c[2 * kk + 1]);
+                        stsm4(own + q * kPanel + tile_plain(lane, 16 * wr, kk), A);
+                        ldsm4(B, with + tile_cols(lane, 16 * q, kk));
+                        mma16816(o[kk & 1][0], A, B[0], B[1]);
+                        mma16816(o[kk & 1][1], A, B[2], B[3]);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) o[0][h][x] += o[1][h][x];
+                    uint32_t X[4], U[4];
+                    pack_block(X, o[0][0], o[0][1]);
+                    if (g_side) ldsm4_t(M, sb + kT + q * kBlk + blk_plain(lane));
+                    else ldsm4(M, sb + kT + q * kBlk + blk_cols(lane));
+                    mma16816_first(o[0][0], X, M[0], M[1]);
+                    mma16816_first(o[0][1], X, M[2], M[3]);
+                    pack_block(U, o[0][0], o[0][1]);
+                    stsm4_t(rows + tile_cols(lane, 16 * q, wr), U[0], U[1], U[2], U[3]);
+                    if (i < 3) {
+#pragma unroll
+                        for (int jj = 0; jj < 4; ++jj) {
+                            uint32_t B[4];
+                            ldsm4_t(B, up_l + tile_plain(lane, 16 * q, jj));
+                            mma16816(c[2 * jj], L, B[0], B[1]);
+                            mma16816(c[2 * jj + 1], L, B[2], B[3]);
+                            ldsm4_t(B, up_u + tile_plain(lane, 16 * q, jj));
+                            mma16816(c[2 * jj], U, B[0], B[1]);
+                            mma16816(c[2 * jj + 1], U, B[2], B[3]);
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            // ---------------- 5. gradients of block q, channels 32 jh ..
+            const int q = wr, jh = warp >> 2;
+            if (q < nblk) {
+                float acc[4][4][4] = {}, sc[4][2][4] = {};   // dr, da, db, dk; B_rb, B_rk, B_ab, B_ak
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    uint32_t Y[4], D[4], U[4], V[4], X[2][4];
+                    const uint32_t o = tile_plain(lane, 16 * q, kk);
+                    ldsm4(Y, tiles + TY * kPanel + o);
+                    ldsm4(D, sb + kDU + o);
+                    ldsm4(U, sb + kU + o);
+                    ldsm4(V, tiles + TV * kPanel + o);
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) ldsm4_t(X[x], sb + kS + q * kPanel + tile_plain(lane, 16 * kk, 2 * jh + x));
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        mma16816(acc[0][n], Y, X[n >> 1][(n & 1) * 2], X[n >> 1][(n & 1) * 2 + 1]);
+                        mma16816(acc[1][n], D, X[n >> 1][(n & 1) * 2], X[n >> 1][(n & 1) * 2 + 1]);
+                    }
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) ldsm4_t(X[x], sb + kG + q * kPanel + tile_plain(lane, 16 * kk, 2 * jh + x));
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        mma16816(acc[2][n], U, X[n >> 1][(n & 1) * 2], X[n >> 1][(n & 1) * 2 + 1]);
+                        mma16816(acc[3][n], V, X[n >> 1][(n & 1) * 2], X[n >> 1][(n & 1) * 2 + 1]);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        mma16816(sc[0][h], Y, U[h], U[2 + h]);
+                        mma16816(sc[1][h], Y, V[h], V[2 + h]);
+                        mma16816(sc[2][h], D, U[h], U[2 + h]);
+                        mma16816(sc[3][h], D, V[h], V[2 + h]);
+                    }
+                }
+                uint32_t P[4][4], Q[4][4];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int x = 0; x < 4; ++x)
+                            if (8 * h + c2 + (x & 1) > g + 8 * (x >> 1) - (m >> 1)) sc[m][h][x] = 0.f;
+                    pack_block(P[m], sc[m][0], sc[m][1]);
+                    transpose16(Q[m], P[m]);
+                }
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    uint32_t B[4];
+                    const uint32_t o = tile_plain(lane, 16 * q, 2 * jh + x);
+                    auto both = [&](int i0, const uint32_t (&A0)[4], int i1, const uint32_t (&A1)[4]) {
+#pragma unroll
+                        for (int n = 0; n < 2; ++n) {
+                            mma16816(acc[i0][2 * x + n], A0, B[2 * n], B[2 * n + 1]);
+                            mma16816(acc[i1][2 * x + n], A1, B[2 * n], B[2 * n + 1]);
+                        }
+                    };
+                    ldsm4_t(B, tiles + TB * kPanel + o);
+                    both(0, P[0], 1, P[2]);
+                    ldsm4_t(B, tiles + TK * kPanel + o);
+                    both(0, P[1], 1, P[3]);
+                    ldsm4_t(B, tiles + TR * kPanel + o);
+                    both(2, Q[0], 3, Q[1]);
+                    ldsm4_t(B, tiles + TA * kPanel + o);
+                    both(2, Q[2], 3, Q[3]);
+                }
+                // phi at a block boundary: between this block and the next, or, for the last block, the one before
+                const int bd = min(q + 1, 3);
+                float2 phi[4] = {};
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        uint32_t A[4], B[4];
+                        const uint32_t o = tile_plain(lane, 16 * kk, 2 * jh + x);
+                        ldsm4(A, sb + kS + bd * kPanel + o);
+                        ldsm4(B, sb + kG + (bd - 1) * kPanel + o);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) phi[2 * x + (i >> 1)] = __ffma2_rn(unpack_half2(A[i]), unpack_half2(B[i]), phi[2 * x + (i >> 1)]);
+                    }
+                const float sigma = exp2_of(min(max(ex, -126), 127));
+                float finite = 0.f;
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const uint32_t o = tile_plain(lane, 16 * q, 2 * jh + x);
+                    uint32_t ta[4], tr[4], tbb[4], tk[4], tw[4], out[5][4];
+                    ldsm4(ta, tiles + TA * kPanel + o);
+                    ldsm4(tr, tiles + TR * kPanel + o);
+                    ldsm4(tbb, tiles + TB * kPanel + o);
+                    ldsm4(tk, tiles + TK * kPanel + o);
+                    ldsm4(tw, tiles + TW * kPanel + o);
+#pragma unroll
+                    for (int n2 = 0; n2 < 2; ++n2) {
+                        const int n = 2 * x + n2, j = 32 * jh + 8 * n + c2;
+                        float2 xs[2], z[2], suf[2];
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) {
+                            const int i = n2 * 2 + r;
+                            const float2 dr = make_float2(acc[0][n][2 * r], acc[0][n][2 * r + 1]), da = make_float2(acc[1][n][2 * r], acc[1][n][2 * r + 1]);
+                            const float2 db = make_float2(acc[2][n][2 * r], acc[2][n][2 * r + 1]), dk = make_float2(acc[3][n][2 * r], acc[3][n][2 * r + 1]);
+                            const float2 rr = unpack_half2(tr[i]), aa = unpack_half2(ta[i]);
+                            xs[r] = __ffma2_rn(unpack_half2(tbb[i]), db, __ffma2_rn(unpack_half2(tk[i]), dk, mul2(make_float2(-rr.x, -rr.y), dr)));
+                            z[r] = __ffma2_rn(make_float2(-aa.x, -aa.y), da, xs[r]);
+                            suf[r] = z[r];
+                            finite += (fabsf(xs[r].x) + fabsf(xs[r].y)) + (fabsf(z[r].x) + fabsf(z[r].y));
+                        }
+                        // sums of z over this token and the later ones of its half of the block (over g), then the block
+#pragma unroll
+                        for (int s = 4; s <= 16; s <<= 1)
+#pragma unroll
+                            for (int r = 0; r < 2; ++r) {
+                                const float vx = __shfl_down_sync(0xffffffffu, suf[r].x, s), vy = __shfl_down_sync(0xffffffffu, suf[r].y, s);
+                                if (lane + s < 32) { suf[r].x += vx; suf[r].y += vy; }
+                            }
+                        const float hx = __shfl_sync(0xffffffffu, suf[1].x, lane & 3), hy = __shfl_sync(0xffffffffu, suf[1].y, lane & 3);
+                        suf[0].x += hx;
+                        suf[0].y += hy;
+#pragma unroll
+                        for (int s = 4; s <= 16; s <<= 1) {
+                            phi[n].x += __shfl_xor_sync(0xffffffffu, phi[n].x, s);
+                            phi[n].y += __shfl_xor_sync(0xffffffffu, phi[n].y, s);
+                        }
+                        const float2 m0 = lds_f2(sb + kMu + (bd * 64 + j) * 4), m1 = lds_f2(sb + kRho + ((bd - 1) * 64 + j) * 4);
+                        float2 ph = make_float2(phi[n].x * rcp(m0.x * m1.x), phi[n].y * rcp(m0.y * m1.y));
+                        if (q == 3) {   // from the block's start: the whole block's sum on top
+                            ph.x += __shfl_sync(0xffffffffu, suf[0].x, lane & 3);
+                            ph.y += __shfl_sync(0xffffffffu, suf[0].y, lane & 3);
+                        }
+                        const float2 mu = lds_f2(sb + kMu + (q * 64 + j) * 4);
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) {
+                            const int t = 16 * q + g + 8 * r, i = n2 * 2 + r;
+                            const float2 f = lds_f2(sb + kF + t * kFStride + j * 4);
+                            const bool first = r == 0 && g == 0;
+                            float2 fm = lds_f2(first ? sb + kMu + (q * 64 + j) * 4 : sb + kF + (t - 1) * kFStride + j * 4);
+                            if (first) fm = make_float2(rcp(mu.x), rcp(mu.y));
+                            const float2 fs = make_float2(f.x * sigma, f.y * sigma), fi = make_float2(rcp(f.x) * sigma, rcp(f.y) * sigma);
+                            const float2 w = unpack_bf2(tw[i]);
+                            constexpr float kLog2e = 1.4426950408889634f;
+                            out[TA][i] = pack_bf2(acc[1][n][2 * r] * fm.x * sigma, acc[1][n][2 * r + 1] * fm.y * sigma);
+                            out[TR][i] = pack_bf2(acc[0][n][2 * r] * fs.x, acc[0][n][2 * r + 1] * fs.y);
+                            out[TB][i] = pack_bf2(acc[2][n][2 * r] * fi.x, acc[2][n][2 * r + 1] * fi.y);
+                            out[TK][i] = pack_bf2(acc[3][n][2 * r] * fi.x, acc[3][n][2 * r + 1] * fi.y);
+                            // d_t dd_t = phi_t - x_t, phi_t = phi at the boundary - the later tokens' z
+                            const float px = ph.x - (suf[r].x - z[r].x) - xs[r].x, py = ph.y - (suf[r].y - z[r].y) - xs[r].y;
+                            out[4][i] = pack_bf2(-ex2(w.x * kLog2e) * px * sigma, -ex2(w.y * kLog2e) * py * sigma);
+                        }
+                    }
+                    __syncwarp();
+                    // (the gradients take the place of the operands, which no other warp reads)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) stsm4(tiles + i * kPanel + o, out[i]);
+                    stsm4(tiles + TW * kPanel + o, out[4]);
+                }
+                bad = !(finite <= 3.0e38f);
+            }
+            fence_proxy_async();
+            bad = __syncthreads_or(bad);
+            if (!bad && tid == 0) {
+                int x, y;
+                coordinates(unit, x, y);
+                for (int b = 0; b < nblk; ++b)
+#pragma unroll
+                    for (int i = 0; i < 5; ++i)
+                        tma_store_2d(&maps.out[i], x, y + 16 * b, smem + buf * kTilesBytes + (i < 4 ? i : TW) * kPanel + b * 2048);
+                bulk_commit_group();
+            }
+        }
+        if (over || bad) {
+            chunk_by_token(p, unit, reinterpret_cast<float *>(smem + buf * kTilesBytes), reinterpret_cast<float *>(smem + kS));
+            fence_proxy_async();
+            __syncthreads();
+        }
+    }
+    if (tid == 0) {
+        if (*abort_flag) {   // what is in flight lands before the CTA leaves
+            mbar_wait(bar + (seq & 1), (uint32_t)((seq >> 1) & 1), 100000u);
+            atomicExch(p.status, (int)kDevTimeout);
+        }
+        bulk_wait_group_read<0>();
+    }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+}  // namespace
+
+// Enqueues the chunk kernel behind the gradient scan.
+int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const float *states, const float *gradients, cudaStream_t stream) {
+    static const EncodeTiledFn encode = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
+                   ? reinterpret_cast<EncodeTiledFn>(fn) : nullptr;
+    }();
+    if (encode == nullptr) return (int)cudaErrorNotSupported;
+    ChunkMaps maps{};
+    ChunkArgs args{};
+    const cuuint64_t dims[2] = {(cuuint64_t)(p.H * kN), (cuuint64_t)(p.B * p.T)};
+    const cuuint64_t strides[1] = {(cuuint64_t)(p.H * kN * 2)};
+    const cuuint32_t estr[2] = {1, 1};
+    auto describe = [&](CUtensorMap *map, const void *ptr, cuuint32_t rows) {
+        const cuuint32_t box[2] = {(cuuint32_t)kN, rows};
+        return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    const void *in[kTensors] = {p.a, p.r, p.b, p.k, p.v, p.dy, p.w};
+    void *out[5] = {p.da, p.dr, p.db, p.dk, p.dw};
+    for (int i = 0; i < kTensors; ++i) {
+        if (!describe(&maps.in[i], in[i], (cuuint32_t)kL)) return (int)cudaErrorInvalidValue;
+        args.in[i] = static_cast<const __nv_bfloat16 *>(in[i]);
+    }
+    for (int i = 0; i < 5; ++i) {
+        if (!describe(&maps.out[i], out[i], 16u)) return (int)cudaErrorInvalidValue;
+        args.out[i] = static_cast<__nv_bfloat16 *>(out[i]);
+    }
+    args.states = states;
+    args.gradients = gradients;
+    args.T = (int)p.T;
+    args.H = (int)p.H;
+    args.nchunks = (int)((p.T + kL - 1) / kL);
+    args.units = (long long)(p.B * p.H) * args.nchunks;
+    if (int e = device_status_ptr(p.device, &args.status)) return e;
+    cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_gradients_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(args.units < p.num_sms ? args.units : p.num_sms));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, wkv7_chunk_gradients_kernel, maps, args);
+    if (e == cudaSuccess) count_launch();
+    return (int)e;
+}
+
+}  // namespace rwkv7

@@ -143,6 +143,16 @@ extern "C" {
         state_replacement: T, chunk_len: i64, output_grad: T, next_state_grad: T,
         sequence_grads: *const TM, initial_state_grad: TM, workspace: *mut c_void,
         workspace_bytes: usize, stream: rwkv7_stream) -> c_int;
+    pub fn rwkv7_wkv7_training_saved_bytes(b: i64, t: i64, h: i64, n: i64, dtype: i32, chunk_len: i64) -> usize;
+    pub fn rwkv7_wkv7_training_workspace_bytes(b: i64, t: i64, h: i64, n: i64) -> usize;
+    pub fn rwkv7_fused_wkv7_training_forward(initial_state: T, receptance: T, weight_decay: T,
+        replacement_key: T, value: T, removal_key_normalized: T, replacement: T, chunk_len: i64,
+        output: TM, next_state: TM, saved: *mut c_void, saved_bytes: usize, stream: rwkv7_stream) -> c_int;
+    pub fn rwkv7_fused_wkv7_training_backward(receptance: T, weight_decay: T, replacement_key: T,
+        value: T, removal_key_normalized: T, replacement: T, chunk_len: i64, saved: *const c_void,
+        saved_bytes: usize, output_grad: T, next_state_grad: T, sequence_grads: *const TM,
+        initial_state_grad: TM, workspace: *mut c_void, workspace_bytes: usize,
+        stream: rwkv7_stream) -> c_int;
 
     // ---- Mix6Backend, AddcmulBackend, TokenShiftDiffBackend
     pub fn rwkv7_fused_mix6(embedded_context: T, scales: *const T, outputs: *const TM,
