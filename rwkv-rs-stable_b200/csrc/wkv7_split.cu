@@ -715,7 +715,7 @@ __device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TI
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) snapshots[(size_t)(t / kL) * kN * kN + row * kN + c0 + 16 * kk + e] = S[kk][e];
+                for (int e = 0; e < 4; ++e) snapshots[(size_t)(t / kL) * kN * kN + accumulator_place(row, c0 + 16 * kk + e)] = S[kk][e];
         }
         const size_t o = (((size_t)bi * Tlen + t) * H + h) * kN;
         auto f = [&](int x, int kk, int e) -> float { return static_cast<float>(static_cast<const TIO *>(in.p[x])[o + c0 + 16 * kk + e]); };
@@ -766,7 +766,7 @@ __device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, con
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) snapshots[(size_t)(t / kL) * kN * kN + row * kN + c0 + 16 * kk + e] = G[kk][e];
+                for (int e = 0; e < 4; ++e) snapshots[(size_t)(t / kL) * kN * kN + accumulator_place(row, c0 + 16 * kk + e)] = G[kk][e];
         }
         const size_t o = (((size_t)bi * Tlen + t) * H + h) * kN;
         auto f = [&](int x, int kk, int e) -> float { return __bfloat162float(static_cast<const __nv_bfloat16 *>(in.p[x])[o + c0 + 16 * kk + e]); };
@@ -1058,14 +1058,15 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]))));
                 if (lane == 0) top_g[slot * 4 + quarter * 2 + hf] = most;
             };
-            auto keep = [&](int c) {   // the state that step c starts from
-                float *dst = snapshots + ((size_t)chain * n + at_step(c)) * kN * kN + jp;
+            auto keep = [&](int c) {   // the state that step c starts from, for the kernel of the chunks (see accumulator_place)
+                float *dst = snapshots + ((size_t)chain * n + at_step(c)) * kN * kN + accumulator_place(i0, jp);
 #pragma unroll
-                for (int e = 0; e < 16; ++e)
-                    if (RWKV7_IN_RANGE(c < n && i0 + 2 * e + 1 < kN && jp < kN, status)) {
-                        dst[(i0 + 2 * e) * kN] = Z[e].x;
-                        dst[(i0 + 2 * e + 1) * kN] = Z[e].y;
-                    }
+                for (int m = 0; m < 32; m = m == 7 ? 16 : m + 1) {
+                    if (m >= 24) break;
+                    const float2 lo = Z[m >> 1], hi = Z[(m + 8) >> 1];
+                    if (RWKV7_IN_RANGE(c < n && i0 + m + 8 < kN && jp < kN, status))
+                        *reinterpret_cast<float2 *>(dst + (m >> 4) * 1024 + (m & 7) * 16) = m & 1 ? make_float2(lo.y, hi.y) : make_float2(lo.x, hi.x);
+                }
             };
             // the state a chunk starts with, as operand: times fx, fp16
             auto put_z = [&](int c, float fx) {

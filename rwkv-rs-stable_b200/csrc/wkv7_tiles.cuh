@@ -41,6 +41,12 @@ __device__ __forceinline__ uint32_t blk_cols(int lane) {
     return (uint32_t)((lane >> 3) & 1) * 256u + (uint32_t)((lane & 7) + ((lane >> 4) << 3)) * 16u;
 }
 
+// Place of element (i, j) of a [64][64] fp32 matrix kept in the order of matrix-instruction accumulators: a warp's 16 rows i in
+// turn, in them eight columns j at a time, four elements per lane (rows g and g + 8 of column 2q, then of 2q + 1).
+__device__ __forceinline__ int accumulator_place(int i, int j) {
+    return (((i >> 4) * 8 + (j >> 3)) * 32 + (i & 7) * 4 + ((j & 7) >> 1)) * 4 + (j & 1) * 2 + ((i >> 3) & 1);
+}
+
 // Bounded wait for a whole warp without compiler-made divergence handling around the loop.
 __device__ __forceinline__ bool mbar_wait_tight(uint64_t *bar, uint32_t parity, uint32_t limit) {
     uint32_t ok;

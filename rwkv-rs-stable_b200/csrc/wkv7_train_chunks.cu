@@ -42,9 +42,8 @@ using namespace sm100;
 constexpr int kThreads = 256;
 enum { TA = 0, TR, TB, TK, TV, TY, TW, kTensors };
 constexpr uint32_t kTilesBytes = kTensors * kPanel;             // one of two buffers of input tiles
-constexpr uint32_t kFStride = 288;                               // D_t / mu in fp32, [64 tokens][64 channels]; rows 8 banks apart
-constexpr uint32_t kF = 2 * kTilesBytes;
-constexpr uint32_t kS = kF + 64 * kFStride;                      // [4] S mu of block q, fp16 tiles [value row][channel]
+constexpr uint32_t kF = 2 * kTilesBytes;                         // D_{t-1} / mu and D_t / mu, fp16 tiles [token][channel]
+constexpr uint32_t kS = kF + 2 * kPanel;                         // [4] S mu of block q, fp16 tiles [value row][channel]
 constexpr uint32_t kG = kS + 4 * kPanel;                         // [4] G rho, the same
 constexpr uint32_t kU = kG + 4 * kPanel;                         // U and dU, tiles [token][value row]
 constexpr uint32_t kDU = kU + kPanel;
@@ -54,7 +53,8 @@ constexpr uint32_t kT = kArb + 4 * kBlk;
 constexpr uint32_t kDiag = kT + 4 * kBlk;                        // [4] A_ab in fp32
 constexpr uint32_t kMu = kDiag + 4 * 1024;                       // [4][64] fp32 each
 constexpr uint32_t kRho = kMu + 1024;
-constexpr uint32_t kE = kRho + 1024;                             // [8][64] fp32: decay over half a block
+constexpr uint32_t kFactors = kRho + 1024;                       // [8][64] fp32: from block to block, S then G; channel order of factor_place
+constexpr uint32_t kE = kFactors + 2048;                         // [8][64] fp32: decay over half a block
 constexpr uint32_t kTop = kE + 2048;                             // [16] largest magnitudes: of S and V, of G and dY, by warp
 constexpr uint32_t kBars = kTop + 64;
 constexpr uint32_t kSmem = kBars + 64;
@@ -62,12 +62,13 @@ static_assert(kS % 1024 == 0 && kSmem <= 232448, "shared memory");
 
 struct ChunkMaps {
     CUtensorMap in[kTensors];   // [B*T, H*N] bf16, box 64 x 64, 128-byte swizzle
-    CUtensorMap out[5];         // da, dr, db, dk, dw, box 64 x 16
+    CUtensorMap out[5];         // da, dr, db, dk, dw, the same
+    CUtensorMap block[5];       // and with box 64 x 16, for a chunk that ends early
 };
 struct ChunkArgs {
     const __nv_bfloat16 *in[kTensors];
     __nv_bfloat16 *out[5];
-    const float *states, *gradients;   // [chain][chunk][64][64]
+    const float *states, *gradients;   // [chain][chunk][64 x 64], in the order of accumulator_place
     int T, H, nchunks;
     long long units;
     int *status;
@@ -89,6 +90,8 @@ __device__ __forceinline__ void pack_block(uint32_t (&x)[4], const float (&c0)[4
     x[2] = pack_half2(c1[0], c1[1]);
     x[3] = pack_half2(c1[2], c1[3]);
 }
+// Channels 8 n + 2 q, + 1 of all n next to one another: what lane q of a row group multiplies its accumulators with.
+__device__ __forceinline__ int factor_place(int j) { return ((j & 7) >> 1) * 16 + (j >> 3) * 2 + (j & 1); }
 __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
     const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&b);
@@ -127,7 +130,7 @@ __device__ __noinline__ void chunk_by_token(const ChunkArgs &p, long long unit, 
     float M[16];
     auto load = [&](const float *src) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) M[i] = src[(size_t)unit * kN * kN + row * kN + c0 + 16 * (i >> 2) + (i & 3)];
+        for (int i = 0; i < 16; ++i) M[i] = src[(size_t)unit * kN * kN + accumulator_place(row, c0 + 16 * (i >> 2) + (i & 3))];
     };
     auto col = [&](int i) { return c0 + 16 * (i >> 2) + (i & 3); };
     __syncthreads();
@@ -177,7 +180,7 @@ __device__ __noinline__ void chunk_by_token(const ChunkArgs &p, long long unit, 
     float m[2][16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-        m[0][i] = M[i] * p.gradients[(size_t)unit * kN * kN + row * kN + col(i)];
+        m[0][i] = M[i] * p.gradients[(size_t)unit * kN * kN + accumulator_place(row, col(i))];
         m[1][i] = 0.f;
     }
     column_sums(m, u, du);   // (u is no longer needed: its first row takes phi at the chunk's end)
@@ -234,7 +237,8 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         for (int i = 0; i < kTensors; ++i) tma_load_2d(smem + buf * kTilesBytes + i * kPanel, &maps.in[i], x, y, bar + buf);
     };
     __syncthreads();
-    if (tid == 0 && blockIdx.x < p.units) request(blockIdx.x, 0);
+    if (warp == 7 && elect_one() && blockIdx.x < p.units) request(blockIdx.x, 0);
+    __syncwarp();
     // (launched behind the gradient scan with programmatic stream serialization)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     int seq = 0;
@@ -247,12 +251,12 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         const bool g_side = warp >= 4;
         float c[8][4];
         {
-            const float *src = (g_side ? p.gradients : p.states) + (size_t)unit * kN * kN + (16 * wr + g) * kN + c2;
+            const float *src = (g_side ? p.gradients : p.states) + (size_t)unit * kN * kN + (wr * 256 + lane) * 4;
             if (RWKV7_IN_RANGE(unit >= 0 && unit < p.units, p.status)) {
 #pragma unroll
                 for (int n = 0; n < 8; ++n) {
-                    const float2 lo = __ldcs(reinterpret_cast<const float2 *>(src + 8 * n)), hi = __ldcs(reinterpret_cast<const float2 *>(src + 8 * kN + 8 * n));
-                    c[n][0] = lo.x; c[n][1] = lo.y; c[n][2] = hi.x; c[n][3] = hi.y;
+                    const float4 x = __ldcs(reinterpret_cast<const float4 *>(src + n * 128));
+                    c[n][0] = x.x; c[n][2] = x.y; c[n][1] = x.z; c[n][3] = x.w;
                 }
             }
         }
@@ -293,10 +297,6 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         }
         __syncthreads();
         if (*abort_flag) break;
-        if (tid == 0 && unit + gridDim.x < p.units) {
-            bulk_wait_group_read<0>();   // the other buffer's gradients have left
-            request(unit + gridDim.x, buf ^ 1);
-        }
         // ---------------- 2. scaled fp16 operands, in place; D_t / mu
         float scale_s, scale_g;
         int ex;
@@ -335,10 +335,12 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
+                const uint32_t o = off16(t_first + u, ch);
                 sts32(at(TA, u), pack2(mul2(unpack_bf2(x0[u]), f)));
+                sts32(sb + kF + o, pack2(f));
                 f = mul2(f, d[u]);
                 sts32(at(TR, u), pack2(mul2(unpack_bf2(x1[u]), f)));
-                sts_f2(sb + kF + (t_first + u) * kFStride + ch * 4, f.x, f.y);
+                sts32(sb + kF + kPanel + o, pack2(f));
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -359,6 +361,15 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         }
         over = __syncthreads_or(over);
         bool bad = false;
+        if (unit + gridDim.x < p.units) {   // the next chunk: its tiles into the other buffer, its states into L2
+            const long long next = unit + gridDim.x;
+            if (warp == 7 && elect_one()) {
+                bulk_wait_group_read<0>();   // the other buffer's gradients have left
+                request(next, buf ^ 1);
+            }
+            __syncwarp();
+            asm volatile("prefetch.global.L2 [%0];" ::"l"((tid < 128 ? p.states : p.gradients) + (size_t)next * kN * kN + (tid & 127) * 32));
+        }
         if (!over) {
             // ---------------- 3. warps 0-3: A_ab of a block and T; warps 4-7: A_ak, A_rb
             {
@@ -379,6 +390,14 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                     }
                 }
                 if (g_side) {
+                    {   // factors from the block before (S: mu rho', G: rho mu') to this one
+                        const uint32_t own = sb + (q * 64 + ch) * 4;
+                        const float2 mu = lds_f2(own + kMu), rho = lds_f2(own + kRho);
+                        const float2 fs = q == 0 ? make_float2(scale_s, scale_s) : lds_f2(own + kRho - 256), fg = q == 3 ? make_float2(scale_g, scale_g) : lds_f2(own + kMu + 256);
+                        const uint32_t o = sb + kFactors + q * 256 + factor_place(ch) * 4;
+                        sts_f2(o, mu.x * fs.x, mu.y * fs.y);
+                        sts_f2(o + 1024, rho.x * fg.x, rho.y * fg.y);
+                    }
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
                         const uint32_t o = sb + (x ? kArb : kAak) + q * kBlk + lane * 4;
@@ -431,18 +450,16 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                 const uint32_t with = tiles + (g_side ? TB : TA) * kPanel;      // what S or G is multiplied with: a~ or b^
                 const uint32_t mat = sb + (g_side ? kArb : kAak);
                 const uint32_t up_u = tiles + (g_side ? TA : TB) * kPanel, up_l = tiles + (g_side ? TR : TK) * kPanel;
-                const float scale = g_side ? scale_g : scale_s;
 #pragma unroll 1
                 for (int i = 0; i < 4; ++i) {
-                    const int q = g_side ? 3 - i : i, before = g_side ? q + 1 : q - 1;
-                    // from the block before to this one's reference: S (D / mu) mu', G mu rho'
+                    const int q = g_side ? 3 - i : i;
                     {
-                        const uint32_t f0 = sb + (g_side ? kRho : kMu) + (q * 64 + c2) * 4, f1 = sb + (g_side ? kMu : kRho) + (before * 64 + c2) * 4;
+                        const uint32_t f0 = sb + kFactors + (g_side ? 1024 : 0) + q * 256 + (lane & 3) * 64;
 #pragma unroll
-                        for (int n = 0; n < 8; ++n) {
-                            float2 f = lds_f2(f0 + n * 32);
-                            f = mul2(f, i == 0 ? make_float2(scale, scale) : lds_f2(f1 + n * 32));
+                        for (int n = 0; n < 8; n += 2) {
+                            const float4 f = lds_f4(f0 + n * 8);
                             c[n][0] *= f.x; c[n][1] *= f.y; c[n][2] *= f.x; c[n][3] *= f.y;
+                            c[n + 1][0] *= f.z; c[n + 1][1] *= f.w; c[n + 1][2] *= f.z; c[n + 1][3] *= f.w;
                         }
                     }
                     uint32_t L[4], M[4];
@@ -572,12 +589,14 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
                     const uint32_t o = tile_plain(lane, 16 * q, 2 * jh + x);
-                    uint32_t ta[4], tr[4], tbb[4], tk[4], tw[4], out[5][4];
+                    uint32_t ta[4], tr[4], tbb[4], tk[4], tw[4], fe[4], fi[4], out[5][4];
                     ldsm4(ta, tiles + TA * kPanel + o);
                     ldsm4(tr, tiles + TR * kPanel + o);
                     ldsm4(tbb, tiles + TB * kPanel + o);
                     ldsm4(tk, tiles + TK * kPanel + o);
                     ldsm4(tw, tiles + TW * kPanel + o);
+                    ldsm4(fe, sb + kF + o);
+                    ldsm4(fi, sb + kF + kPanel + o);
 #pragma unroll
                     for (int n2 = 0; n2 < 2; ++n2) {
                         const int n = 2 * x + n2, j = 32 * jh + 8 * n + c2;
@@ -615,21 +634,17 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                             ph.x += __shfl_sync(0xffffffffu, suf[0].x, lane & 3);
                             ph.y += __shfl_sync(0xffffffffu, suf[0].y, lane & 3);
                         }
-                        const float2 mu = lds_f2(sb + kMu + (q * 64 + j) * 4);
 #pragma unroll
                         for (int r = 0; r < 2; ++r) {
-                            const int t = 16 * q + g + 8 * r, i = n2 * 2 + r;
-                            const float2 f = lds_f2(sb + kF + t * kFStride + j * 4);
-                            const bool first = r == 0 && g == 0;
-                            float2 fm = lds_f2(first ? sb + kMu + (q * 64 + j) * 4 : sb + kF + (t - 1) * kFStride + j * 4);
-                            if (first) fm = make_float2(rcp(mu.x), rcp(mu.y));
-                            const float2 fs = make_float2(f.x * sigma, f.y * sigma), fi = make_float2(rcp(f.x) * sigma, rcp(f.y) * sigma);
+                            const int i = n2 * 2 + r;
+                            const float2 s2 = make_float2(sigma, sigma), f = unpack_half2(fi[i]);
+                            const float2 fa = mul2(unpack_half2(fe[i]), s2), fr = mul2(f, s2), fb = mul2(make_float2(rcp(f.x), rcp(f.y)), s2);
                             const float2 w = unpack_bf2(tw[i]);
                             constexpr float kLog2e = 1.4426950408889634f;
-                            out[TA][i] = pack_bf2(acc[1][n][2 * r] * fm.x * sigma, acc[1][n][2 * r + 1] * fm.y * sigma);
-                            out[TR][i] = pack_bf2(acc[0][n][2 * r] * fs.x, acc[0][n][2 * r + 1] * fs.y);
-                            out[TB][i] = pack_bf2(acc[2][n][2 * r] * fi.x, acc[2][n][2 * r + 1] * fi.y);
-                            out[TK][i] = pack_bf2(acc[3][n][2 * r] * fi.x, acc[3][n][2 * r + 1] * fi.y);
+                            out[TA][i] = pack_bf2(acc[1][n][2 * r] * fa.x, acc[1][n][2 * r + 1] * fa.y);
+                            out[TR][i] = pack_bf2(acc[0][n][2 * r] * fr.x, acc[0][n][2 * r + 1] * fr.y);
+                            out[TB][i] = pack_bf2(acc[2][n][2 * r] * fb.x, acc[2][n][2 * r + 1] * fb.y);
+                            out[TK][i] = pack_bf2(acc[3][n][2 * r] * fb.x, acc[3][n][2 * r + 1] * fb.y);
                             // d_t dd_t = phi_t - x_t, phi_t = phi at the boundary - the later tokens' z
                             const float px = ph.x - (suf[r].x - z[r].x) - xs[r].x, py = ph.y - (suf[r].y - z[r].y) - xs[r].y;
                             out[4][i] = pack_bf2(-ex2(w.x * kLog2e) * px * sigma, -ex2(w.y * kLog2e) * py * sigma);
@@ -645,15 +660,21 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
             }
             fence_proxy_async();
             bad = __syncthreads_or(bad);
-            if (!bad && tid == 0) {
+            if (!bad && warp == 7 && elect_one()) {
                 int x, y;
                 coordinates(unit, x, y);
-                for (int b = 0; b < nblk; ++b)
+                const unsigned char *from = smem + buf * kTilesBytes;
+                if (nblk == 4) {
 #pragma unroll
-                    for (int i = 0; i < 5; ++i)
-                        tma_store_2d(&maps.out[i], x, y + 16 * b, smem + buf * kTilesBytes + (i < 4 ? i : TW) * kPanel + b * 2048);
+                    for (int i = 0; i < 5; ++i) tma_store_2d(&maps.out[i], x, y, from + (i < 4 ? i : TW) * kPanel);
+                } else {
+                    for (int b = 0; b < nblk; ++b)
+#pragma unroll
+                        for (int i = 0; i < 5; ++i) tma_store_2d(&maps.block[i], x, y + 16 * b, from + (i < 4 ? i : TW) * kPanel + b * 2048);
+                }
                 bulk_commit_group();
             }
+            __syncwarp();
         }
         if (over || bad) {
             chunk_by_token(p, unit, reinterpret_cast<float *>(smem + buf * kTilesBytes), reinterpret_cast<float *>(smem + kS));
@@ -661,7 +682,7 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
             __syncthreads();
         }
     }
-    if (tid == 0) {
+    if (warp == 7 && elect_one()) {
         if (*abort_flag) {   // what is in flight lands before the CTA leaves
             mbar_wait(bar + (seq & 1), (uint32_t)((seq >> 1) & 1), 100000u);
             atomicExch(p.status, (int)kDevTimeout);
@@ -702,7 +723,7 @@ int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const float *
         args.in[i] = static_cast<const __nv_bfloat16 *>(in[i]);
     }
     for (int i = 0; i < 5; ++i) {
-        if (!describe(&maps.out[i], out[i], 16u)) return (int)cudaErrorInvalidValue;
+        if (!describe(&maps.out[i], out[i], (cuuint32_t)kL) || !describe(&maps.block[i], out[i], 16u)) return (int)cudaErrorInvalidValue;
         args.out[i] = static_cast<__nv_bfloat16 *>(out[i]);
     }
     args.states = states;
