@@ -698,12 +698,21 @@ __device__ __forceinline__ uint64_t desc_operator(uint32_t addr, int ks) {
     return (uint64_t)(((addr + (uint32_t)ks * step) >> 4) & 0x3fffu) | (uint64_t)(along_k >> 4) << 16 | (uint64_t)(along_m >> 4) << 32 | (uint64_t)1 << 46;
 }
 
+// A warp's largest magnitude of a state, as float bits.
+__device__ __forceinline__ void keep_top(uint32_t *tops, const float (&S)[4][4]) {
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m = fmaxf(m, fabsf(S[i >> 2][i & 3]));
+    const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) tops[threadIdx.x >> 5] = most;
+}
+
 // Token-by-token recomputation of one chain over tokens t0 .. t1 - 1, fp32 throughout: what a
 // CTA does when a value overflowed fp16 on the way, or the chain is flagged and no later kernel is there to take it.  Four
 // lanes per row; columns and sums in the order of the sequential scan (wkv7_seq.cu), whose bits it reproduces.
 template <typename TIO>
 __device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TIO *v, TIO *y, const float *s_in, float *s_out,
-                                                float *snapshots, int bi, int h, int H, int Tlen, int t0, int t1) {
+                                                float *snapshots, uint32_t *tops, int bi, int h, int H, int Tlen, int t0, int t1) {
     const int row = (int)threadIdx.x >> 2, c0 = ((int)threadIdx.x & 3) * 4;   // columns c0 + 16 kk + e
     float S[4][4];
 #pragma unroll
@@ -712,6 +721,7 @@ __device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TI
         for (int e = 0; e < 4; ++e) S[kk][e] = s_in ? s_in[row * kN + c0 + 16 * kk + e] : 0.f;
     for (int t = t0; t < t1; ++t) {
         if (snapshots != nullptr && t % kL == 0) {
+            keep_top(tops + t / kL * 8, S);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
@@ -754,7 +764,7 @@ __device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TI
 // The same for the gradient of the state, backwards over a whole chain; dv comes with it.  Snapshots: the gradient of the state
 // at the end of every chunk.
 __device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, const __nv_bfloat16 *dy, __nv_bfloat16 *dv, const float *g_in,
-                                                     float *g_out, float *snapshots, int bi, int h, int H, int Tlen) {
+                                                     float *g_out, float *snapshots, uint32_t *tops, int bi, int h, int H, int Tlen) {
     const int row = (int)threadIdx.x >> 2, c0 = ((int)threadIdx.x & 3) * 4;
     float G[4][4];
 #pragma unroll
@@ -763,6 +773,7 @@ __device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, con
         for (int e = 0; e < 4; ++e) G[kk][e] = g_in ? g_in[row * kN + c0 + 16 * kk + e] : 0.f;
     for (int t = Tlen - 1; t >= 0; --t) {
         if (t == Tlen - 1 || t % kL == kL - 1) {
+            keep_top(tops + t / kL * 8, G);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
@@ -812,7 +823,7 @@ template <typename TIO, int kKind>
 __global__ void __launch_bounds__(Scan<TIO>::kThreads, 1)
 wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs, const TIO *__restrict__ v,
                        const unsigned char *__restrict__ records, const float *state_in, float *state_out,
-                       TIO *__restrict__ y, float *__restrict__ snapshots, int *flags, int Tlen, int H, int chunk0, int n, int resolve_flagged,
+                       TIO *__restrict__ y, float *__restrict__ snapshots, uint32_t *__restrict__ tops, int *flags, int Tlen, int H, int chunk0, int n, int resolve_flagged,
                        int *status) {
     constexpr bool kGrad = kKind == kGradients;
     using SM = Scan<TIO>;
@@ -1050,15 +1061,15 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                     g2 = exp2_of(-eg);
                 }
             };
-            // largest magnitude of the state in this warp's share, for the converting warps
-            auto publish = [&](int slot) {
+            // largest magnitude of the state in this warp's share
+            auto largest = [&] {
                 float m[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int e = 0; e < 16; ++e) m[e & 3] = fmaxf(m[e & 3], fmaxf(fabsf(Z[e].x), fabsf(Z[e].y)));
-                const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]))));
-                if (lane == 0) top_g[slot * 4 + quarter * 2 + hf] = most;
+                return __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]))));
             };
-            auto keep = [&](int c) {   // the state that step c starts from, for the kernel of the chunks (see accumulator_place)
+            auto keep = [&](int c, uint32_t most) {   // the state that step c starts from, for the kernel of the chunks (see accumulator_place)
+                if (lane < 2) tops[((size_t)chain * n + at_step(c)) * 8 + quarter * 2 + hf + 4 * lane] = lane ? 0u : most;
                 float *dst = snapshots + ((size_t)chain * n + at_step(c)) * kN * kN + accumulator_place(i0, jp);
 #pragma unroll
                 for (int m = 0; m < 32; m = m == 7 ? 16 : m + 1) {
@@ -1083,15 +1094,19 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
             };
             float gx, fx, g2, gxn = 1.f, fxn = 1.f, g2n = 0.f;
             if constexpr (kGrad) {
-                publish(4);
+                const uint32_t most = largest();
+                if (lane == 0) top_g[16 + quarter * 2 + hf] = most;
                 asm volatile("bar.sync 7, 192;" ::: "memory");
             }
             load_vec(0, gx, fx, g2);
             put_z(0, fx);
             for (int c = 0; c < n; ++c) {
                 const int a = c & 1;
-                if constexpr (kGrad) publish(c & 3);
-                if constexpr (kKind != kPrefill) keep(c);
+                if constexpr (kKind != kPrefill) {
+                    const uint32_t most = largest();
+                    if (kGrad && lane == 0) top_g[(c & 3) * 4 + quarter * 2 + hf] = most;   // for the converting warps
+                    keep(c, most);
+                }
                 if (c + 1 < n) load_vec(c + 1, gxn, fxn, g2n);   // (while the products run)
                 wait(bar_acc + a, (uint32_t)((c >> 1) & 1));
                 tc_fence_after();
@@ -1205,8 +1220,9 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     // this launch started with, which is still untouched.
     if (((flagged && resolve_flagged) || (*bad & 2)) && tid < 256) {
         float *own = snapshots + (kKind == kPrefill ? 0 : (size_t)chain * n * kN * kN);
-        if constexpr (kGrad) scan_gradients_by_token(ptrs, v, y, s_in, s_out, own, bi, h, H, Tlen);
-        else scan_rows_by_token<TIO>(ptrs, v, y, s_in, s_out, kKind == kPrefill ? nullptr : own, bi, h, H, Tlen, chunk0 * kL, t_end);
+        uint32_t *top = tops + (kKind == kPrefill ? 0 : (size_t)chain * n * 8);
+        if constexpr (kGrad) scan_gradients_by_token(ptrs, v, y, s_in, s_out, own, top, bi, h, H, Tlen);
+        else scan_rows_by_token<TIO>(ptrs, v, y, s_in, s_out, kKind == kPrefill ? nullptr : own, top, bi, h, H, Tlen, chunk0 * kL, t_end);
     }
 }
 
@@ -1557,7 +1573,7 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
             cfg.numAttrs = st == stream ? 1 : 0;   // directly behind its operator kernel on the caller's stream
             using T = std::remove_pointer_t<decltype(ytype)>;
             err = cudaLaunchKernelEx(&cfg, kern, smaps, optrs, static_cast<const T *>(p.v), records, s_in, s_out,
-                                     static_cast<T *>(p.y), (float *)nullptr, flags, (int)p.T, (int)p.H, c0, n, resolve_flagged ? 1 : 0, status);
+                                     static_cast<T *>(p.y), (float *)nullptr, (uint32_t *)nullptr, flags, (int)p.T, (int)p.H, c0, n, resolve_flagged ? 1 : 0, status);
             if (err == cudaSuccess) count_launch();
             return err;
         };
@@ -1623,8 +1639,8 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
 
 // ---- a training step ------------------------------------------------------------------------------
 //
-// Kept between the passes: [records of all chunks][state in front of every chunk][one int per chain]; workspace of the backward
-// pass: [gradient of the state behind every chunk][one int per chain].
+// Kept between the passes: [records of all chunks][state in front of every chunk][eight largest magnitudes for each][one int per
+// chain]; workspace of the backward pass: the same without records, for the gradient of the state behind every chunk.
 
 namespace {
 
@@ -1636,7 +1652,7 @@ TrainingLayout training_layout(int64_t B, int64_t T, int64_t H, bool with_record
     l.chains = (size_t)(B * H);
     l.nchunks = (size_t)((T + kL - 1) / kL);
     l.states = with_records ? align_up(l.chains * l.nchunks * kRecord) : 0;
-    l.flags = l.states + l.chains * l.nchunks * kN * kN * sizeof(float);
+    l.flags = l.states + align_up(l.chains * l.nchunks * (kN * kN * sizeof(float) + 32));
     l.total = l.flags + align_up(l.chains * sizeof(int));
     return l;
 }
@@ -1659,7 +1675,8 @@ int launch_training_scan(const ScanMaps &maps, const OperatorPtrs &ptrs, const v
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kern, maps, ptrs, static_cast<const bf *>(in), records, s_in, s_out, static_cast<bf *>(out), states, flags,
+    e = cudaLaunchKernelEx(&cfg, kern, maps, ptrs, static_cast<const bf *>(in), records, s_in, s_out, static_cast<bf *>(out), states,
+                           reinterpret_cast<uint32_t *>(states + l.chains * l.nchunks * kN * kN), flags,
                            (int)T, (int)H, 0, (int)l.nchunks, 1, status);
     if (e == cudaSuccess) count_launch();
     return (int)e;

@@ -32,6 +32,10 @@ __device__ __forceinline__ uint32_t tile_plain(int lane, int row0, int c) {
     const int r = row0 + (lane & 15), ch = 2 * c + (lane >> 4);
     return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
 }
+__device__ __forceinline__ uint32_t tile_before(int lane, int row0, int c) {   // tile_plain one row up
+    const int r = row0 + (lane & 15) - 1, ch = 2 * c + (lane >> 4);
+    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
+}
 __device__ __forceinline__ uint32_t tile_cols(int lane, int row0, int c) {
     const int r = row0 + (lane & 7) + ((lane >> 4) << 3), ch = 2 * c + ((lane >> 3) & 1);
     return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);

@@ -68,9 +68,10 @@ struct ChunkMaps {
 struct ChunkArgs {
     const __nv_bfloat16 *in[kTensors];
     __nv_bfloat16 *out[5];
-    const float *states, *gradients;   // [chain][chunk][64 x 64], in the order of accumulator_place
+    // [chain][chunk][64 x 64], in the order of accumulator_place; behind them eight largest magnitudes each, as float bits
+    const float *states, *gradients;
     int T, H, nchunks;
-    long long units;
+    int units;
     int *status;
 };
 
@@ -99,10 +100,10 @@ __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
 
 // One chunk in fp32, token by token.  `scratch`: 36 KB, `sums`: 64 KB of shared memory.  Four lanes per value row, columns
 // c0 + 16 kk + e; sums over rows go through the warps' partial sums.
-__device__ __noinline__ void chunk_by_token(const ChunkArgs &p, long long unit, float *scratch, float *sums) {
+__device__ __noinline__ void chunk_by_token(const ChunkArgs &p, int unit, float *scratch, float *sums) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = tid >> 2, c0 = (tid & 3) * 4;
-    const int chain = (int)(unit / p.nchunks), chunk = (int)(unit % p.nchunks);
+    const int chain = unit / p.nchunks, chunk = unit % p.nchunks;
     const int valid = min(kL, p.T - chunk * kL);
     const size_t base = (((size_t)(chain / p.H) * p.T + chunk * kL) * p.H + chain % p.H) * kN, step = (size_t)p.H * kN;
     float *u = scratch, *du = u + kL * kN, *part = du + kL * kN;   // [token][row]; [2][8 warps][64]
@@ -224,12 +225,12 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         mbar_fence_init();
         *abort_flag = 0;
     }
-    auto coordinates = [&](long long unit, int &x, int &y) {
-        const int chain = (int)(unit / p.nchunks);
+    auto coordinates = [&](int unit, int &x, int &y) {
+        const int chain = unit / p.nchunks;
         x = (chain % p.H) * kN;
-        y = (chain / p.H) * p.T + (int)(unit % p.nchunks) * kL;
+        y = (chain / p.H) * p.T + unit % p.nchunks * kL;
     };
-    auto request = [&](long long unit, int buf) {
+    auto request = [&](int unit, int buf) {
         int x, y;
         coordinates(unit, x, y);
         mbar_expect_tx(bar + buf, kTilesBytes);
@@ -237,29 +238,33 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         for (int i = 0; i < kTensors; ++i) tma_load_2d(smem + buf * kTilesBytes + i * kPanel, &maps.in[i], x, y, bar + buf);
     };
     __syncthreads();
-    if (warp == 7 && elect_one() && blockIdx.x < p.units) request(blockIdx.x, 0);
+    if (warp == 7 && elect_one() && (int)blockIdx.x < p.units) request(blockIdx.x, 0);
     __syncwarp();
     // (launched behind the gradient scan with programmatic stream serialization)
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    int seq = 0;
-    for (long long unit = blockIdx.x; unit < p.units; unit += gridDim.x, ++seq) {
-        const int buf = seq & 1;
-        const uint32_t tiles = sb + buf * kTilesBytes;
-        const int valid = min(kL, p.T - (int)(unit % p.nchunks) * kL), nblk = valid / 16;
-        // ---- this warp's 16 rows of S or G, in accumulator order: c[n] = rows g, g + 8, columns 8 n + c2, + 1
-        const int wr = warp & 3;
-        const bool g_side = warp >= 4;
-        float c[8][4];
-        {
-            const float *src = (g_side ? p.gradients : p.states) + (size_t)unit * kN * kN + (wr * 256 + lane) * 4;
-            if (RWKV7_IN_RANGE(unit >= 0 && unit < p.units, p.status)) {
+    // this warp's 16 rows of S or G, in accumulator order: c[n] = rows g, g + 8, columns 8 n + c2, + 1
+    const int wr = warp & 3;
+    const bool g_side = warp >= 4;
+    float c[8][4];
+    auto fetch = [&](int unit) {
+        const float *src = (g_side ? p.gradients : p.states) + (size_t)unit * kN * kN + (wr * 256 + lane) * 4;
+        if (RWKV7_IN_RANGE(unit >= 0 && unit < p.units, p.status)) {
 #pragma unroll
-                for (int n = 0; n < 8; ++n) {
-                    const float4 x = __ldcs(reinterpret_cast<const float4 *>(src + n * 128));
-                    c[n][0] = x.x; c[n][2] = x.y; c[n][1] = x.z; c[n][3] = x.w;
-                }
+            for (int n = 0; n < 8; ++n) {
+                const float4 x = __ldcs(reinterpret_cast<const float4 *>(src + n * 128));
+                c[n][0] = x.x; c[n][2] = x.y; c[n][1] = x.z; c[n][3] = x.w;
             }
         }
+    };
+    if ((int)blockIdx.x < p.units) fetch(blockIdx.x);
+    const uint32_t *tops_s = reinterpret_cast<const uint32_t *>(p.states + (size_t)p.units * kN * kN);
+    const uint32_t *tops_g = reinterpret_cast<const uint32_t *>(p.gradients + (size_t)p.units * kN * kN);
+    int seq = 0;
+    for (int unit = blockIdx.x; unit < p.units; unit += (int)gridDim.x, ++seq) {
+        const int buf = seq & 1;
+        const uint32_t tiles = sb + buf * kTilesBytes;
+        const int valid = min(kL, p.T - unit % p.nchunks * kL), nblk = valid / 16;
+        const uint32_t state_top = lane < 16 ? (lane < 8 ? tops_s : tops_g)[(size_t)unit * 8 + (lane & 7)] : 0u;
         if (!mbar_wait(bar + buf, (uint32_t)((seq >> 1) & 1))) *abort_flag = 1;
         __syncwarp();
         // ---------------- 1. decays of half a block per warp, lane = channel pair; largest magnitudes
@@ -278,18 +283,14 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         }
         sts_f2(sb + kE + ((2 * tb + hf) * 64 + ch) * 4, e.x, e.y);
         {
-            float ms = 0.f, mg = 0.f, mc = 0.f;
+            __nv_bfloat162 m = __floats2bfloat162_rn(0.f, 0.f), my = m;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const float2 a = unpack_bf2(rv[u]), b = unpack_bf2(ry[u]);
-                ms = fmaxf(ms, fmaxf(fabsf(a.x), fabsf(a.y)));
-                mg = fmaxf(mg, fmaxf(fabsf(b.x), fabsf(b.y)));
+                m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&rv[u])));
+                my = __hmax2(my, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&ry[u])));
             }
-#pragma unroll
-            for (int n = 0; n < 8; ++n) mc = fmaxf(mc, fmaxf(fmaxf(fabsf(c[n][0]), fabsf(c[n][1])), fmaxf(fabsf(c[n][2]), fabsf(c[n][3]))));
-            if (g_side) mg = fmaxf(mg, mc);
-            else ms = fmaxf(ms, mc);
-            const uint32_t a = __reduce_max_sync(0xffffffffu, __float_as_uint(ms)), b = __reduce_max_sync(0xffffffffu, __float_as_uint(mg));
+            const uint32_t a = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(__low2float(m), __high2float(m)))),
+                           b = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(__low2float(my), __high2float(my))));
             if (lane == 0) {
                 sts32(sb + kTop + warp * 4, a);
                 sts32(sb + kTop + 32 + warp * 4, b);
@@ -301,14 +302,10 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         float scale_s, scale_g;
         int ex;
         {
-            float ms = 0.f, mg = 0.f;
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float4 a = lds_f4(sb + kTop + 16 * i), b = lds_f4(sb + kTop + 32 + 16 * i);
-                ms = fmaxf(ms, fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)));
-                mg = fmaxf(mg, fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
-            }
-            const int es = ms > 0.f ? min(max(exponent_of(ms) - 127, -60), 60) : 0, eg = mg > 0.f ? min(max(exponent_of(mg) - 127, -60), 60) : 0;
+            const uint32_t ts = lane < 8 ? state_top : lane >= 16 && lane < 24 ? lds32(sb + kTop + (lane - 16) * 4) : 0u;
+            const uint32_t tg = lane >= 8 && lane < 16 ? state_top : lane >= 24 ? lds32(sb + kTop + 32 + (lane - 24) * 4) : 0u;
+            const uint32_t ms = __reduce_max_sync(0xffffffffu, ts), mg = __reduce_max_sync(0xffffffffu, tg);
+            const int es = ms ? min(max((int)(ms >> 23) - 127, -60), 60) : 0, eg = mg ? min(max((int)(mg >> 23) - 127, -60), 60) : 0;
             scale_s = exp2_of(-es);
             scale_g = exp2_of(-eg);
             ex = es + eg;
@@ -361,8 +358,8 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         }
         over = __syncthreads_or(over);
         bool bad = false;
-        if (unit + gridDim.x < p.units) {   // the next chunk: its tiles into the other buffer, its states into L2
-            const long long next = unit + gridDim.x;
+        if (unit + (int)gridDim.x < p.units) {   // the next chunk: its tiles into the other buffer, its states into L2
+            const int next = unit + (int)gridDim.x;
             if (warp == 7 && elect_one()) {
                 bulk_wait_group_read<0>();   // the other buffer's gradients have left
                 request(next, buf ^ 1);
@@ -509,6 +506,10 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
             const int q = wr, jh = warp >> 2;
             if (q < nblk) {
                 float acc[4][4][4] = {}, sc[4][2][4] = {};   // dr, da, db, dk; B_rb, B_rk, B_ab, B_ak
+                // phi at the block's start, from its S and the G of the block before; at the first block's end, the other way round
+                float2 phi[4] = {};
+                const uint32_t other = sb + (q == 0 ? kS + kPanel : kG + (q - 1) * kPanel);
+                const int bd = max(q, 1);
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) {
                     uint32_t Y[4], D[4], U[4], V[4], X[2][4];
@@ -517,15 +518,28 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                     ldsm4(D, sb + kDU + o);
                     ldsm4(U, sb + kU + o);
                     ldsm4(V, tiles + TV * kPanel + o);
+                    uint32_t Z[2][4];
 #pragma unroll
-                    for (int x = 0; x < 2; ++x) ldsm4_t(X[x], sb + kS + q * kPanel + tile_plain(lane, 16 * kk, 2 * jh + x));
+                    for (int x = 0; x < 2; ++x) {
+                        const uint32_t ox = tile_plain(lane, 16 * kk, 2 * jh + x);
+                        ldsm4_t(X[x], sb + kS + q * kPanel + ox);
+                        ldsm4_t(Z[x], other + ox);
+                    }
+                    auto boundary = [&] {
+#pragma unroll
+                        for (int x = 0; x < 2; ++x)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) phi[2 * x + (i >> 1)] = __ffma2_rn(unpack_half2(X[x][i]), unpack_half2(Z[x][i]), phi[2 * x + (i >> 1)]);
+                    };
 #pragma unroll
                     for (int n = 0; n < 4; ++n) {
                         mma16816(acc[0][n], Y, X[n >> 1][(n & 1) * 2], X[n >> 1][(n & 1) * 2 + 1]);
                         mma16816(acc[1][n], D, X[n >> 1][(n & 1) * 2], X[n >> 1][(n & 1) * 2 + 1]);
                     }
+                    if (q > 0) boundary();
 #pragma unroll
                     for (int x = 0; x < 2; ++x) ldsm4_t(X[x], sb + kG + q * kPanel + tile_plain(lane, 16 * kk, 2 * jh + x));
+                    if (q == 0) boundary();
 #pragma unroll
                     for (int n = 0; n < 4; ++n) {
                         mma16816(acc[2][n], U, X[n >> 1][(n & 1) * 2], X[n >> 1][(n & 1) * 2 + 1]);
@@ -570,20 +584,6 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                     ldsm4_t(B, tiles + TA * kPanel + o);
                     both(2, Q[2], 3, Q[3]);
                 }
-                // phi at a block boundary: between this block and the next, or, for the last block, the one before
-                const int bd = min(q + 1, 3);
-                float2 phi[4] = {};
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        uint32_t A[4], B[4];
-                        const uint32_t o = tile_plain(lane, 16 * kk, 2 * jh + x);
-                        ldsm4(A, sb + kS + bd * kPanel + o);
-                        ldsm4(B, sb + kG + (bd - 1) * kPanel + o);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) phi[2 * x + (i >> 1)] = __ffma2_rn(unpack_half2(A[i]), unpack_half2(B[i]), phi[2 * x + (i >> 1)]);
-                    }
                 const float sigma = exp2_of(min(max(ex, -126), 127));
                 float finite = 0.f;
 #pragma unroll
@@ -623,14 +623,13 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                         const float hx = __shfl_sync(0xffffffffu, suf[1].x, lane & 3), hy = __shfl_sync(0xffffffffu, suf[1].y, lane & 3);
                         suf[0].x += hx;
                         suf[0].y += hy;
-#pragma unroll
-                        for (int s = 4; s <= 16; s <<= 1) {
-                            phi[n].x += __shfl_xor_sync(0xffffffffu, phi[n].x, s);
-                            phi[n].y += __shfl_xor_sync(0xffffffffu, phi[n].y, s);
-                        }
+                        // (phi: lane (g, q') holds the rows of its q' of column 8 n + g)
+                        float pc = phi[n].x + phi[n].y;
+                        pc += __shfl_xor_sync(0xffffffffu, pc, 1);
+                        pc += __shfl_xor_sync(0xffffffffu, pc, 2);
                         const float2 m0 = lds_f2(sb + kMu + (bd * 64 + j) * 4), m1 = lds_f2(sb + kRho + ((bd - 1) * 64 + j) * 4);
-                        float2 ph = make_float2(phi[n].x * rcp(m0.x * m1.x), phi[n].y * rcp(m0.y * m1.y));
-                        if (q == 3) {   // from the block's start: the whole block's sum on top
+                        float2 ph = make_float2(__shfl_sync(0xffffffffu, pc, 4 * c2) * rcp(m0.x * m1.x), __shfl_sync(0xffffffffu, pc, 4 * c2 + 4) * rcp(m0.y * m1.y));
+                        if (q > 0) {   // from the block's start: the whole block's sum on top
                             ph.x += __shfl_sync(0xffffffffu, suf[0].x, lane & 3);
                             ph.y += __shfl_sync(0xffffffffu, suf[0].y, lane & 3);
                         }
@@ -658,6 +657,7 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                 }
                 bad = !(finite <= 3.0e38f);
             }
+            if (unit + (int)gridDim.x < p.units) fetch(unit + (int)gridDim.x);
             fence_proxy_async();
             bad = __syncthreads_or(bad);
             if (!bad && warp == 7 && elect_one()) {
@@ -677,6 +677,7 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
             __syncwarp();
         }
         if (over || bad) {
+            if (over && unit + (int)gridDim.x < p.units) fetch(unit + (int)gridDim.x);
             chunk_by_token(p, unit, reinterpret_cast<float *>(smem + buf * kTilesBytes), reinterpret_cast<float *>(smem + kS));
             fence_proxy_async();
             __syncthreads();
@@ -731,7 +732,7 @@ int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const float *
     args.T = (int)p.T;
     args.H = (int)p.H;
     args.nchunks = (int)((p.T + kL - 1) / kL);
-    args.units = (long long)(p.B * p.H) * args.nchunks;
+    args.units = (int)(p.B * p.H * args.nchunks);   // (33 KB are kept for each: far fewer than 2^31)
     if (int e = device_status_ptr(p.device, &args.status)) return e;
     cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_gradients_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return (int)e;
