@@ -424,6 +424,13 @@ int rwkv7_fused_token_shift_diff(const rwkv7_tensor *embedded_context,
                                  rwkv7_tensor *embedded_token_shift,
                                  const rwkv7_tensor *batch_ids, rwkv7_tensor *token_shifted_diff,
                                  rwkv7_stream stream);
+/*
+ * The same without touching embedded_token_shift: next_token_shift [S,C] takes the last token of every sequence at its slot and
+ * the carried token of every other slot (where two sequences name one slot, the later one's).
+ */
+int rwkv7_fused_token_shift_diff_into(const rwkv7_tensor *embedded_context, const rwkv7_tensor *embedded_token_shift,
+                                      const rwkv7_tensor *batch_ids, rwkv7_tensor *next_token_shift,
+                                      rwkv7_tensor *token_shifted_diff, rwkv7_stream stream);
 
 /* -------------------------------------------------- time-mixer epilogues -- */
 /*

@@ -522,9 +522,9 @@ class TokenShiftDiffForwardOutput:
 def token_shift_diff_custom(embedded_context: torch.Tensor, embedded_token_shift: torch.Tensor,
                             batch_ids: torch.Tensor, *, inplace_state: bool = False
                             ) -> TokenShiftDiffForwardOutput:
-    """``token_shift_diff_custom`` (``token_shift_diff/mod.rs:82-111``).  The state
-    buffer is updated in place by the kernel; unless ``inplace_state`` the caller's
-    tensor is cloned first so that the call is functional like the reference's."""
+    """``token_shift_diff_custom`` (``token_shift_diff/mod.rs:82-111``).  With
+    ``inplace_state`` the state buffer is updated in place; otherwise the kernel writes the next state
+    beside it, so that the call is functional like the reference's."""
     diff, state = (_native or native()).token_shift_diff(embedded_context, embedded_token_shift, batch_ids, inplace_state)
     return TokenShiftDiffForwardOutput(token_shifted_diff=diff, next_token_shift=state)
 

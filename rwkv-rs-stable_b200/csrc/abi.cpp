@@ -916,8 +916,8 @@ int rwkv7_fused_addcmul5(const rwkv7_tensor *base, const rwkv7_tensor *diff,
     return addcmul_run(base, diff, scales, outputs, 5, kMixScaleNames, kMixOutNames, stream);
 }
 
-int rwkv7_fused_token_shift_diff(const rwkv7_tensor *x_t, rwkv7_tensor *state_t,
-                                 const rwkv7_tensor *ids_t, rwkv7_tensor *diff_t, rwkv7_stream stream) {
+static int token_shift_diff_impl(const rwkv7_tensor *x_t, const rwkv7_tensor *state_t, const rwkv7_tensor *ids_t,
+                                 rwkv7_tensor *next_t, rwkv7_tensor *diff_t, rwkv7_stream stream) {
     RWKV7_TRACE("rwkv.infer.model.time_mixer.token_shift_diff");
     clear_error();
     const TensorInfo x{"embedded_context", x_t}, state{"embedded_token_shift", state_t},
@@ -939,18 +939,34 @@ int rwkv7_fused_token_shift_diff(const rwkv7_tensor *x_t, rwkv7_tensor *state_t,
     if (ids_t->dtype != RWKV7_I32 && ids_t->dtype != RWKV7_I64 && ids_t->dtype != RWKV7_U32)
         return fail(RWKV7_ERR_DTYPE_MISMATCH, "DTypeMismatch: batch_ids must be I32, I64 or U32, got %s", dtype_name(ids_t->dtype));
     RWKV7_TRY(check_output_like(x, TensorInfo{"token_shifted_diff", diff_t}));
+    if (next_t != state_t) RWKV7_TRY(check_output_like(state, TensorInfo{"next_token_shift", next_t}));
     TokenShiftArgs p{};
-    p.x = x_t->data; p.state = state_t->data; p.ids = ids_t->data; p.ids_dtype = ids_t->dtype;
+    p.x = x_t->data; p.state = state_t->data; p.next = next_t->data; p.ids = ids_t->data; p.ids_dtype = ids_t->dtype;
     p.diff = diff_t->data;
     p.B = x.dim(0); p.T = x.dim(1); p.C = x.dim(2); p.S = state.dim(0);
     p.bf16 = x_t->dtype == RWKV7_BF16;
-    if (p.B == 0 || p.T == 0) return RWKV7_OK;  // token_shift_diff/mod.rs:88-97: T == 0 is a no-op
+    const bool nothing = p.B == 0 || p.T == 0;   // token_shift_diff/mod.rs:88-97: T == 0 is a no-op
+    if (nothing && p.next == p.state) return RWKV7_OK;
     DeviceGuard guard(x_t->device);
     if (guard.error() != cudaSuccess) return cuda_fail("cudaSetDevice", (int)guard.error());
+    if (nothing) {
+        const cudaError_t e = cudaMemcpyAsync(p.next, p.state, (size_t)(p.S * p.C) * dtype_size(x_t->dtype), cudaMemcpyDeviceToDevice, (cudaStream_t)stream);
+        return e == cudaSuccess ? RWKV7_OK : cuda_fail("token_shift_diff state", (int)e);
+    }
     RWKV7_TRY(num_sms(x_t->device, &p.num_sms));
     if (int e = device_status_ptr(x_t->device, &p.status)) return cuda_fail("device status word", e);
     if (int e = launch_token_shift_diff(p, (cudaStream_t)stream)) return cuda_fail("token_shift_diff launch", e);
     return RWKV7_OK;
+}
+
+int rwkv7_fused_token_shift_diff(const rwkv7_tensor *x, rwkv7_tensor *state, const rwkv7_tensor *ids, rwkv7_tensor *diff,
+                                 rwkv7_stream stream) {
+    return token_shift_diff_impl(x, state, ids, state, diff, stream);
+}
+
+int rwkv7_fused_token_shift_diff_into(const rwkv7_tensor *x, const rwkv7_tensor *state, const rwkv7_tensor *ids,
+                                      rwkv7_tensor *next_state, rwkv7_tensor *diff, rwkv7_stream stream) {
+    return token_shift_diff_impl(x, state, ids, next_state, diff, stream);
 }
 
 namespace {

@@ -187,7 +187,8 @@ int launch_channel_mixer(const ChannelMixerArgs &p, void *workspace, size_t work
 
 struct TokenShiftArgs {
     const void *x;     // [B,T,C]
-    void *state;       // [S,C], updated in place
+    const void *state; // [S,C]
+    void *next;        // [S,C]: `state` itself (updated in place) or memory apart from it
     const void *ids;   // [B]
     int ids_dtype;     // RWKV7_I32 / RWKV7_I64 / RWKV7_U32
     void *diff;        // [B,T,C]

@@ -22,7 +22,13 @@
 namespace rwkv7 {
 namespace {
 
-constexpr int kRowsPerBlock = 16;
+// Rows per CTA: 16, or with few rows (a decode step) as few as give every SM two CTAs, since a CTA walks its rows one after the
+// other: five scales over 16 rows of 2048 channels took one CTA 10 us.
+constexpr int kMostRows = 16;
+int rows_per_block(int64_t rows, int num_sms) {
+    const int64_t r = rows / (2 * (int64_t)(num_sms > 0 ? num_sms : 1));
+    return (int)(r < 1 ? 1 : r < kMostRows ? r : kMostRows);
+}
 
 __host__ __device__ __forceinline__ int64_t imin(int64_t a, int64_t b) { return a < b ? a : b; }
 
@@ -77,10 +83,10 @@ struct Mix6Ptrs {
 
 template <typename T, int EPV>
 __global__ void __launch_bounds__(256)
-mix6_kernel(const T *__restrict__ x, Mix6Ptrs ptrs, int64_t rows, int64_t Tlen, int64_t C) {
+mix6_kernel(const T *__restrict__ x, Mix6Ptrs ptrs, int64_t rows, int64_t Tlen, int64_t C, int per_block) {
     const int64_t CV = C / EPV;
-    const int64_t row_begin = (int64_t)blockIdx.x * kRowsPerBlock;
-    const int64_t row_end = imin(rows, row_begin + kRowsPerBlock);
+    const int64_t row_begin = (int64_t)blockIdx.x * per_block;
+    const int64_t row_end = imin(rows, row_begin + per_block);
     for (int64_t cv = threadIdx.x; cv < CV; cv += blockDim.x) {
         const int64_t c = cv * EPV;
         Pack<T, EPV> mu[6];
@@ -114,10 +120,10 @@ struct AddcmulPtrs {
 
 template <typename T, int EPV, int NS>
 __global__ void __launch_bounds__(256)
-addcmul_kernel(const T *base, const T *__restrict__ diff, AddcmulPtrs ptrs, int64_t rows, int64_t C) {
+addcmul_kernel(const T *base, const T *__restrict__ diff, AddcmulPtrs ptrs, int64_t rows, int64_t C, int per_block) {
     const int64_t CV = C / EPV;
-    const int64_t row_begin = (int64_t)blockIdx.x * kRowsPerBlock;
-    const int64_t row_end = imin(rows, row_begin + kRowsPerBlock);
+    const int64_t row_begin = (int64_t)blockIdx.x * per_block;
+    const int64_t row_end = imin(rows, row_begin + per_block);
     for (int64_t cv = threadIdx.x; cv < CV; cv += blockDim.x) {
         const int64_t c = cv * EPV;
         Pack<T, EPV> sc[NS];
@@ -152,16 +158,33 @@ __device__ __forceinline__ int64_t load_id(const void *ids, int dtype, int64_t b
     return (int64_t) reinterpret_cast<const int32_t *>(ids)[b];
 }
 
+// `next` == `state`: the carried tokens are updated in place.  Otherwise the CTAs behind those of the sequences write `next`, a slot
+// each: the last token of the sequence that names it, else what `state` holds.
 template <typename T, int EPV>
 __global__ void __launch_bounds__(256)
-token_shift_diff_kernel(const T *__restrict__ x, T *state, const void *__restrict__ ids,
-                        int ids_dtype, T *__restrict__ diff, int64_t B, int64_t Tlen, int64_t C,
-                        int64_t S, int *status) {
+token_shift_diff_kernel(const T *__restrict__ x, const T *state, T *next, const void *__restrict__ ids, int ids_dtype,
+                        T *__restrict__ diff, int64_t B, int64_t Tlen, int64_t C, int64_t S, int per_block, int *status) {
     const int64_t CV = C / EPV;
-    const int64_t blocks_per_seq = (Tlen + kRowsPerBlock - 1) / kRowsPerBlock;
+    const int64_t blocks_per_seq = (Tlen + per_block - 1) / per_block;
+    if (blockIdx.x >= B * blocks_per_seq) {
+        const int64_t slot = blockIdx.x - B * blocks_per_seq;
+        __shared__ int named_by;
+        if (threadIdx.x == 0) named_by = -1;
+        __syncthreads();
+        for (int64_t b = threadIdx.x; b < B; b += blockDim.x)
+            if (load_id(ids, ids_dtype, b) == slot) atomicMax(&named_by, (int)b);
+        __syncthreads();
+        const T *from = named_by < 0 ? state + slot * C : x + ((int64_t)named_by * Tlen + Tlen - 1) * C;
+        for (int64_t cv = threadIdx.x; cv < CV; cv += blockDim.x) {
+            Pack<T, EPV> v;
+            v.load(from + cv * EPV);
+            v.store(next + slot * C + cv * EPV);
+        }
+        return;
+    }
     const int64_t b = blockIdx.x / blocks_per_seq;
-    const int64_t t_begin = (blockIdx.x % blocks_per_seq) * kRowsPerBlock;
-    const int64_t t_end = imin(Tlen, t_begin + kRowsPerBlock);
+    const int64_t t_begin = (blockIdx.x % blocks_per_seq) * per_block;
+    const int64_t t_end = imin(Tlen, t_begin + per_block);
     const int64_t slot = load_id(ids, ids_dtype, b);
     const bool slot_ok = slot >= 0 && slot < S;
     if (!slot_ok && threadIdx.x == 0 && t_begin == 0) atomicExch(status, (int)kDevBadIndex);
@@ -185,13 +208,13 @@ token_shift_diff_kernel(const T *__restrict__ x, T *state, const void *__restric
             o.store(db + t * C + c);
             prev = cur;
         }
-        // The thread that read the carried token of this (slot, channel vector)
-        // is the only one that overwrites it, after its read.
-        if (t_begin == 0 && slot_ok) {
+        // In place the thread that read the carried token of this (slot, channel vector) is the only one that
+        // overwrites it, after its read.
+        if (t_begin == 0 && slot_ok && next == state) {
             Pack<T, EPV> last;
             if (t_end == Tlen) last = prev;
             else last.load(xb + (Tlen - 1) * C + c);
-            last.store(state + slot * C + c);
+            last.store(next + slot * C + c);
         }
     }
 }
@@ -216,31 +239,32 @@ int launch_mix6(const MixArgs &p, cudaStream_t stream) {
         ptrs.out[s] = p.out[s];
         vec_ok = vec_ok && aligned16(p.mu[s]) && aligned16(p.out[s]);
     }
-    const unsigned grid = (unsigned)((rows + kRowsPerBlock - 1) / kRowsPerBlock);
+    const int per = rows_per_block(rows, p.num_sms);
+    const unsigned grid = (unsigned)((rows + per - 1) / per);
     if (p.bf16) {
         using T = __nv_bfloat16;
         if (vec_ok && p.C % 8 == 0)
-            mix6_kernel<T, 8><<<grid, pick_threads(p.C / 8), 0, stream>>>((const T *)p.x, ptrs, rows, p.T, p.C);
+            mix6_kernel<T, 8><<<grid, pick_threads(p.C / 8), 0, stream>>>((const T *)p.x, ptrs, rows, p.T, p.C, per);
         else
-            mix6_kernel<T, 1><<<grid, pick_threads(p.C), 0, stream>>>((const T *)p.x, ptrs, rows, p.T, p.C);
+            mix6_kernel<T, 1><<<grid, pick_threads(p.C), 0, stream>>>((const T *)p.x, ptrs, rows, p.T, p.C, per);
     } else {
         if (vec_ok && p.C % 4 == 0)
-            mix6_kernel<float, 4><<<grid, pick_threads(p.C / 4), 0, stream>>>((const float *)p.x, ptrs, rows, p.T, p.C);
+            mix6_kernel<float, 4><<<grid, pick_threads(p.C / 4), 0, stream>>>((const float *)p.x, ptrs, rows, p.T, p.C, per);
         else
-            mix6_kernel<float, 1><<<grid, pick_threads(p.C), 0, stream>>>((const float *)p.x, ptrs, rows, p.T, p.C);
+            mix6_kernel<float, 1><<<grid, pick_threads(p.C), 0, stream>>>((const float *)p.x, ptrs, rows, p.T, p.C, per);
     }
     count_launch();
     return (int)cudaGetLastError();
 }
 
 template <typename T, int EPV>
-static void launch_addcmul_t(const AddcmulArgs &p, const AddcmulPtrs &ptrs, unsigned grid,
-                             cudaStream_t stream) {
-    const int threads = pick_threads(p.C / EPV);
+static void launch_addcmul_t(const AddcmulArgs &p, const AddcmulPtrs &ptrs, cudaStream_t stream) {
+    const int threads = pick_threads(p.C / EPV), per = rows_per_block(p.rows, p.num_sms);
+    const unsigned grid = (unsigned)((p.rows + per - 1) / per);
     if (p.nscale == 1)
-        addcmul_kernel<T, EPV, 1><<<grid, threads, 0, stream>>>((const T *)p.base, (const T *)p.diff, ptrs, p.rows, p.C);
+        addcmul_kernel<T, EPV, 1><<<grid, threads, 0, stream>>>((const T *)p.base, (const T *)p.diff, ptrs, p.rows, p.C, per);
     else
-        addcmul_kernel<T, EPV, 5><<<grid, threads, 0, stream>>>((const T *)p.base, (const T *)p.diff, ptrs, p.rows, p.C);
+        addcmul_kernel<T, EPV, 5><<<grid, threads, 0, stream>>>((const T *)p.base, (const T *)p.diff, ptrs, p.rows, p.C, per);
 }
 
 int launch_addcmul(const AddcmulArgs &p, cudaStream_t stream) {
@@ -252,38 +276,34 @@ int launch_addcmul(const AddcmulArgs &p, cudaStream_t stream) {
         ptrs.out[s] = p.out[s];
         vec_ok = vec_ok && aligned16(p.scale[s]) && aligned16(p.out[s]);
     }
-    const unsigned grid = (unsigned)((p.rows + kRowsPerBlock - 1) / kRowsPerBlock);
     if (p.bf16) {
-        if (vec_ok && p.C % 8 == 0) launch_addcmul_t<__nv_bfloat16, 8>(p, ptrs, grid, stream);
-        else launch_addcmul_t<__nv_bfloat16, 1>(p, ptrs, grid, stream);
+        if (vec_ok && p.C % 8 == 0) launch_addcmul_t<__nv_bfloat16, 8>(p, ptrs, stream);
+        else launch_addcmul_t<__nv_bfloat16, 1>(p, ptrs, stream);
     } else {
-        if (vec_ok && p.C % 4 == 0) launch_addcmul_t<float, 4>(p, ptrs, grid, stream);
-        else launch_addcmul_t<float, 1>(p, ptrs, grid, stream);
+        if (vec_ok && p.C % 4 == 0) launch_addcmul_t<float, 4>(p, ptrs, stream);
+        else launch_addcmul_t<float, 1>(p, ptrs, stream);
     }
     count_launch();
     return (int)cudaGetLastError();
 }
 
+template <typename T, int EPV>
+static void launch_token_shift_t(const TokenShiftArgs &p, cudaStream_t stream) {
+    const int per = rows_per_block(p.B * p.T, p.num_sms);
+    const int64_t blocks = p.B * ((p.T + per - 1) / per) + (p.next != p.state ? p.S : 0);
+    token_shift_diff_kernel<T, EPV><<<(unsigned)blocks, pick_threads(p.C / EPV), 0, stream>>>(
+        (const T *)p.x, (const T *)p.state, (T *)p.next, p.ids, p.ids_dtype, (T *)p.diff, p.B, p.T, p.C, p.S, per, p.status);
+}
+
 int launch_token_shift_diff(const TokenShiftArgs &p, cudaStream_t stream) {
     if (p.B == 0 || p.T == 0 || p.C == 0) return 0;  // T == 0: diff empty, state unchanged
-    const int64_t blocks_per_seq = (p.T + kRowsPerBlock - 1) / kRowsPerBlock;
-    const unsigned grid = (unsigned)(p.B * blocks_per_seq);
-    const bool vec_ok = aligned16(p.x) && aligned16(p.state) && aligned16(p.diff);
+    const bool vec_ok = aligned16(p.x) && aligned16(p.state) && aligned16(p.next) && aligned16(p.diff);
     if (p.bf16) {
-        using T = __nv_bfloat16;
-        if (vec_ok && p.C % 8 == 0)
-            token_shift_diff_kernel<T, 8><<<grid, pick_threads(p.C / 8), 0, stream>>>(
-                (const T *)p.x, (T *)p.state, p.ids, p.ids_dtype, (T *)p.diff, p.B, p.T, p.C, p.S, p.status);
-        else
-            token_shift_diff_kernel<T, 1><<<grid, pick_threads(p.C), 0, stream>>>(
-                (const T *)p.x, (T *)p.state, p.ids, p.ids_dtype, (T *)p.diff, p.B, p.T, p.C, p.S, p.status);
+        if (vec_ok && p.C % 8 == 0) launch_token_shift_t<__nv_bfloat16, 8>(p, stream);
+        else launch_token_shift_t<__nv_bfloat16, 1>(p, stream);
     } else {
-        if (vec_ok && p.C % 4 == 0)
-            token_shift_diff_kernel<float, 4><<<grid, pick_threads(p.C / 4), 0, stream>>>(
-                (const float *)p.x, (float *)p.state, p.ids, p.ids_dtype, (float *)p.diff, p.B, p.T, p.C, p.S, p.status);
-        else
-            token_shift_diff_kernel<float, 1><<<grid, pick_threads(p.C), 0, stream>>>(
-                (const float *)p.x, (float *)p.state, p.ids, p.ids_dtype, (float *)p.diff, p.B, p.T, p.C, p.S, p.status);
+        if (vec_ok && p.C % 4 == 0) launch_token_shift_t<float, 4>(p, stream);
+        else launch_token_shift_t<float, 1>(p, stream);
     }
     count_launch();
     return (int)cudaGetLastError();

@@ -33,6 +33,7 @@ namespace {
     X(rwkv7_fused_wkv7_training_forward) X(rwkv7_fused_wkv7_training_backward)                                   \
     X(rwkv7_wkv7_backward_workspace_bytes) X(rwkv7_fused_mix6) X(rwkv7_fused_mix6_stacked)                       \
     X(rwkv7_fused_addcmul) X(rwkv7_fused_addcmul5) X(rwkv7_fused_token_shift_diff)                               \
+    X(rwkv7_fused_token_shift_diff_into)                                                                         \
     X(rwkv7_fused_weight_prepare) X(rwkv7_fused_gated_readout) X(rwkv7_channel_mixer_workspace_bytes)            \
     X(rwkv7_fused_channel_mixer) X(rwkv7_lm_head_ce_workspace_bytes) X(rwkv7_fused_lm_head_ce_partial)           \
     X(rwkv7_lm_head_ce_finalize)
@@ -121,6 +122,36 @@ at::Tensor empty(at::IntArrayRef shape, at::ScalarType dtype, const at::Tensor &
 
 at::Tensor like(const at::Tensor &t) {
     return t.is_contiguous() ? empty(t.sizes(), t.scalar_type(), t) : at::empty_like(t);
+}
+
+// The outputs of a call, each like its own tensor.  Small ones share one allocation (at 512-byte boundaries, as the allocator itself
+// would place them): an output costs 0.9 us to allocate and wrap, and a decode step around WKV7 has thirteen.  Up to 1 MB
+// in all, because up to there the caching allocator cuts blocks from shared 2 MB segments anyway; larger outputs stay
+// separate, so that holding one of them holds no more memory than its own.
+template <typename... Like>
+void outputs_like(at::Tensor *out, const Like &...tensors) {
+    constexpr int n = sizeof...(Like);
+    const at::Tensor *ts[n] = {&tensors...};
+    constexpr size_t kAlign = 512, kMost = (size_t)1 << 20;
+    size_t at_byte[n], total = 0;
+    bool together = true;
+    for (int i = 0; i < n; ++i) {
+        const at::Tensor &t = *ts[i];
+        together = together && t.is_cuda() && t.is_contiguous() && t.device() == ts[0]->device() && t.layout() == at::kStrided && t.numel() > 0;
+        at_byte[i] = total;
+        total += ((size_t)t.numel() * (size_t)t.element_size() + kAlign - 1) / kAlign * kAlign;
+    }
+    if (!together || total > kMost) {
+        for (int i = 0; i < n; ++i) out[i] = like(*ts[i]);
+        return;
+    }
+    const at::Tensor all = empty({(int64_t)total}, at::kByte, *ts[0]);
+    for (int i = 0; i < n; ++i) {
+        const at::Tensor &t = *ts[i];
+        out[i] = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(all.storage()), all.key_set(), t.dtype());
+        out[i].unsafeGetTensorImpl()->set_storage_offset((int64_t)(at_byte[i] / (size_t)t.element_size()));
+        out[i].unsafeGetTensorImpl()->set_sizes_contiguous(t.sizes());
+    }
 }
 
 // Scratch memory of a call: freed when the call has been enqueued, i.e. given back to the allocator's stream order.
@@ -363,12 +394,12 @@ PyObject *mix6(PyObject *const *a) {
     const at::Tensor &x = tensor(a[0]);
     Desc xd(x), sd[6], od[6];
     at::Tensor out[6];
+    outputs_like(out, x, x, x, x, x, x);
     const rwkv7_tensor *sp[6];
     rwkv7_tensor *op[6];
     for (int i = 0; i < 6; ++i) {
         sd[i].set(tensor(a[1 + i]));
         sp[i] = sd[i].p;
-        out[i] = like(x);
         od[i].set(out[i]);
         op[i] = od[i].p;
     }
@@ -412,12 +443,12 @@ PyObject *addcmul5(PyObject *const *a) {
     const at::Tensor &base = tensor(a[0]);
     Desc bd(base), dd(tensor(a[1])), sd[5], od[5];
     at::Tensor out[5];
+    outputs_like(out, base, base, base, base, base);
     const rwkv7_tensor *sp[5];
     rwkv7_tensor *op[5];
     for (int i = 0; i < 5; ++i) {
         sd[i].set(tensor(a[2 + i]));
         sp[i] = sd[i].p;
-        out[i] = like(base);
         od[i].set(out[i]);
         op[i] = od[i].p;
     }
@@ -429,26 +460,20 @@ PyObject *addcmul5(PyObject *const *a) {
 // token_shift_diff(x, state, batch_ids, inplace_state) -> (diff, next state)
 PyObject *token_shift_diff(PyObject *const *a) {
     const at::Tensor &x = tensor(a[0]);
-    const bool inplace = truth(a[3]);
-    const at::Tensor &given = tensor(a[1]);
-    // (a plain contiguous copy is one asynchronous copy into fresh memory: no dispatch through torch)
-    at::Tensor state;
-    if (inplace) state = given;
-    else if (given.is_cuda() && given.is_contiguous() && dtype_code(given.scalar_type()) >= 0) {
-        state = empty(given.sizes(), given.scalar_type(), given);
-        const size_t bytes = (size_t)given.numel() * (size_t)given.element_size();
-        const c10::DeviceGuard guard(given.device());
-        if (bytes && cudaMemcpyAsync(state.data_ptr(), given.data_ptr(), bytes, cudaMemcpyDeviceToDevice,
-                                     (cudaStream_t)stream_of(given)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            raise(PyExc_RuntimeError, "copying the token-shift state failed");
-        }
-    } else state = given.detach().clone();
-    const at::Tensor diff = like(x);
-    Desc xd(x), sd(state), idd(tensor(a[2])), dd(diff);
+    const bool keep = !truth(a[3]), copied = keep && x.numel() == 0;   // (no tokens: nothing to compute, a plain copy)
+    const at::Tensor state = copied ? tensor(a[1]).detach().clone() : tensor(a[1]);
+    const bool inplace = !keep || copied;
+    at::Tensor out[2];   // diff, next state
+    if (inplace) out[0] = like(x);
+    else outputs_like(out, x, state);
+    Desc xd(x), sd(state), idd(tensor(a[2])), dd(out[0]), nd;
+    if (!inplace) nd.set(out[1]);
     const rwkv7_stream st = stream_of(x);
-    call([&] { return abi.rwkv7_fused_token_shift_diff(xd.p, sd.p, idd.p, dd.p, st); });
-    return pair(wrap(diff), inplace ? Py_NewRef(a[1]) : wrap(state));
+    call([&] {
+        return inplace ? abi.rwkv7_fused_token_shift_diff(xd.p, sd.p, idd.p, dd.p, st)
+                       : abi.rwkv7_fused_token_shift_diff_into(xd.p, sd.p, idd.p, nd.p, dd.p, st);
+    });
+    return pair(wrap(out[0]), !keep ? Py_NewRef(a[1]) : wrap(copied ? state : out[1]));
 }
 
 // weight_prepare(key_precursor, learning_rate_lora, weight_decay_lora, key_removal, key_replacement,
@@ -460,11 +485,10 @@ PyObject *weight_prepare(PyObject *const *a) {
     for (int i = 0; i < 8; ++i)
         if (a[i] != Py_None) in[i].set(tensor(a[i]));
     at::Tensor out[5];
-    for (int i = 0; i < 5; ++i) {
-        if (i == 4 && a[5] == Py_None) continue;   // (no value inputs: no value output)
-        out[i] = like(key);
-        od[i].set(out[i]);
-    }
+    if (a[5] == Py_None) outputs_like(out, key, key, key, key);   // (no value inputs: no value output)
+    else outputs_like(out, key, key, key, key, key);
+    for (int i = 0; i < 5; ++i)
+        if (out[i].defined()) od[i].set(out[i]);
     const int64_t heads = integer(a[8]);
     const rwkv7_stream st = stream_of(key);
     call([&] {

@@ -164,6 +164,8 @@ extern "C" {
         stream: rwkv7_stream) -> c_int;
     pub fn rwkv7_fused_token_shift_diff(embedded_context: T, embedded_token_shift: TM, batch_ids: T,
         token_shifted_diff: TM, stream: rwkv7_stream) -> c_int;
+    pub fn rwkv7_fused_token_shift_diff_into(embedded_context: T, embedded_token_shift: T, batch_ids: T,
+        next_token_shift: TM, token_shifted_diff: TM, stream: rwkv7_stream) -> c_int;
 
     // ---- time-mixer epilogues and the channel mixer
     pub fn rwkv7_fused_weight_prepare(key_precursor: T, learning_rate_lora: T, weight_decay_lora: T,
