@@ -28,17 +28,14 @@ __device__ __forceinline__ float2 unpack_bf2(uint32_t u) {
 // Lane addresses of ldmatrix.x4 for a 16 x 16 block, as byte offsets.  In a swizzled tile the block starts at (row0,
 // column 16 c); in a compact block the rows are 16 bytes and the halves 256.  "plain" gives A order; "cols" swaps the
 // two middle matrices: B order for a block stored [column][k], and, with .trans, A order of the transposed block.
+// (row0 is a multiple of eight, so the swizzle depends on the lane alone and the column block is one exclusive or.)
 __device__ __forceinline__ uint32_t tile_plain(int lane, int row0, int c) {
-    const int r = row0 + (lane & 15), ch = 2 * c + (lane >> 4);
-    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
-}
-__device__ __forceinline__ uint32_t tile_before(int lane, int row0, int c) {   // tile_plain one row up
-    const int r = row0 + (lane & 15) - 1, ch = 2 * c + (lane >> 4);
-    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
+    const uint32_t own = (uint32_t)(lane & 15) * 128u + (uint32_t)(((lane >> 4) ^ (lane & 7)) << 4);
+    return (uint32_t)row0 * 128u + (own ^ (uint32_t)(c << 5));
 }
 __device__ __forceinline__ uint32_t tile_cols(int lane, int row0, int c) {
-    const int r = row0 + (lane & 7) + ((lane >> 4) << 3), ch = 2 * c + ((lane >> 3) & 1);
-    return (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4);
+    const uint32_t own = (uint32_t)((lane & 7) + ((lane >> 4) << 3)) * 128u + (uint32_t)((((lane >> 3) & 1) ^ (lane & 7)) << 4);
+    return (uint32_t)row0 * 128u + (own ^ (uint32_t)(c << 5));
 }
 __device__ __forceinline__ uint32_t blk_plain(int lane) { return (uint32_t)lane * 16u; }
 __device__ __forceinline__ uint32_t blk_cols(int lane) {

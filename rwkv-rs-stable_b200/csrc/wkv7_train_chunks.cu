@@ -270,7 +270,8 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         // ---------------- 1. decays of half a block per warp, lane = channel pair; largest magnitudes
         const int tb = wr, hf = warp >> 2, ch = 2 * lane, t_first = 16 * tb + 8 * hf;
         const int nv = min(8, max(0, valid - t_first));       // 0 or 8
-        auto at = [&](int x, int u) -> uint32_t { return tiles + x * kPanel + off16(t_first + u, ch); };
+        // (t_first is a multiple of eight: the swizzle depends on u alone)
+        auto at = [&](int x, int u) -> uint32_t { return tiles + t_first * 128 + x * kPanel + off16(u, ch); };
         uint32_t rv[8], ry[8];
         float2 d[8], e = make_float2(1.f, 1.f);
 #pragma unroll
@@ -332,7 +333,7 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const uint32_t o = off16(t_first + u, ch);
+                const uint32_t o = t_first * 128 + off16(u, ch);
                 sts32(at(TA, u), pack2(mul2(unpack_bf2(x0[u]), f)));
                 sts32(sb + kF + o, pack2(f));
                 f = mul2(f, d[u]);
