@@ -456,8 +456,13 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
 #pragma unroll
                         for (int n = 0; n < 8; n += 2) {
                             const float4 f = lds_f4(f0 + n * 8);
-                            c[n][0] *= f.x; c[n][1] *= f.y; c[n][2] *= f.x; c[n][3] *= f.y;
-                            c[n + 1][0] *= f.z; c[n + 1][1] *= f.w; c[n + 1][2] *= f.z; c[n + 1][3] *= f.w;
+#pragma unroll
+                            for (int r = 0; r < 4; r += 2) {
+                                const float2 a = mul2(make_float2(c[n][r], c[n][r + 1]), make_float2(f.x, f.y));
+                                const float2 b = mul2(make_float2(c[n + 1][r], c[n + 1][r + 1]), make_float2(f.z, f.w));
+                                c[n][r] = a.x; c[n][r + 1] = a.y;
+                                c[n + 1][r] = b.x; c[n + 1][r + 1] = b.y;
+                            }
                         }
                     }
                     uint32_t L[4], M[4];
@@ -546,12 +551,16 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                         mma16816(acc[2][n], U, X[n >> 1][(n & 1) * 2], X[n >> 1][(n & 1) * 2 + 1]);
                         mma16816(acc[3][n], V, X[n >> 1][(n & 1) * 2], X[n >> 1][(n & 1) * 2 + 1]);
                     }
+                    // (as second operands a register pair holds both halves of k: read in that order, not moved)
+                    const uint32_t oc = tile_cols(lane, 16 * q, kk);
+                    ldsm4(X[0], sb + kU + oc);
+                    ldsm4(X[1], tiles + TV * kPanel + oc);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        mma16816(sc[0][h], Y, U[h], U[2 + h]);
-                        mma16816(sc[1][h], Y, V[h], V[2 + h]);
-                        mma16816(sc[2][h], D, U[h], U[2 + h]);
-                        mma16816(sc[3][h], D, V[h], V[2 + h]);
+                        mma16816(sc[0][h], Y, X[0][2 * h], X[0][2 * h + 1]);
+                        mma16816(sc[1][h], Y, X[1][2 * h], X[1][2 * h + 1]);
+                        mma16816(sc[2][h], D, X[0][2 * h], X[0][2 * h + 1]);
+                        mma16816(sc[3][h], D, X[1][2 * h], X[1][2 * h + 1]);
                     }
                 }
                 uint32_t P[4][4], Q[4][4];
@@ -611,7 +620,6 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                             xs[r] = __ffma2_rn(unpack_half2(tbb[i]), db, __ffma2_rn(unpack_half2(tk[i]), dk, mul2(make_float2(-rr.x, -rr.y), dr)));
                             z[r] = __ffma2_rn(make_float2(-aa.x, -aa.y), da, xs[r]);
                             suf[r] = z[r];
-                            finite += (fabsf(xs[r].x) + fabsf(xs[r].y)) + (fabsf(z[r].x) + fabsf(z[r].y));
                         }
                         // sums of z over this token and the later ones of its half of the block (over g), then the block
 #pragma unroll
@@ -647,6 +655,7 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                             out[TK][i] = pack_bf2(acc[3][n][2 * r] * fb.x, acc[3][n][2 * r + 1] * fb.y);
                             // d_t dd_t = phi_t - x_t, phi_t = phi at the boundary - the later tokens' z
                             const float px = ph.x - (suf[r].x - z[r].x) - xs[r].x, py = ph.y - (suf[r].y - z[r].y) - xs[r].y;
+                            finite += fabsf(px) + fabsf(py);   // (every product above is part of it)
                             out[4][i] = pack_bf2(-ex2(w.x * kLog2e) * px * sigma, -ex2(w.y * kLog2e) * py * sigma);
                         }
                     }
