@@ -104,40 +104,38 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
     const int tid = threadIdx.x;
     const int i = tid >> 2, q = tid & 3;
 
-    float S[16];
+    float2 S[4][2];   // columns 16 kk + 4 q + {0, 1}, {2, 3}
     if (s0 != nullptr) {
         const float4 *src =
             reinterpret_cast<const float4 *>(s0 + ((size_t)bh * kN + row0 + i) * kN);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
             const float4 x = src[kk * 4 + q];
-            S[kk * 4 + 0] = x.x; S[kk * 4 + 1] = x.y; S[kk * 4 + 2] = x.z; S[kk * 4 + 3] = x.w;
+            S[kk][0] = make_float2(x.x, x.y);
+            S[kk][1] = make_float2(x.z, x.w);
         }
     } else {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) S[e] = 0.f;
+        for (int kk = 0; kk < 4; ++kk) S[kk][0] = S[kk][1] = make_float2(0.f, 0.f);
     }
 
     const size_t seq_base = ((size_t)bi * Tlen * H + h) * kN;  // element offset of (b, t=0, h, 0)
     const size_t tok_stride = (size_t)H * kN;
     const int ntiles = (Tlen + kTile - 1) / kTile;
 
+    // Vectors of a tile in the order (tensor, token, piece): a thread's n-th is of a tensor known at compile time (or uniform for
+    // its warp).
     uint4 stage[NV];
     auto issue_loads = [&](int tile) {
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
             const int idx = tid + n * THREADS;
             stage[n] = make_uint4(0, 0, 0, 0);
-            if (idx < VECS) {
-                const int c = idx % VPR;
-                const int tensor = (idx / VPR) % 6;
-                const int tok = idx / (VPR * 6);
-                const int t = tile * kTile + tok;
-                if (t < Tlen) {
-                    const T *p = reinterpret_cast<const T *>(ptrs.in[tensor]) + seq_base +
-                                 (size_t)t * tok_stride + c * EPV;
-                    stage[n] = __ldg(reinterpret_cast<const uint4 *>(p));
-                }
+            const int c = idx % VPR, tok = idx / VPR % kTile, tensor = idx / (VPR * kTile);
+            const int t = tile * kTile + tok;
+            if (idx < VECS && t < Tlen) {
+                const T *p = reinterpret_cast<const T *>(ptrs.in[tensor]) + seq_base + (size_t)t * tok_stride + c * EPV;
+                stage[n] = __ldg(reinterpret_cast<const uint4 *>(p));
             }
         }
     };
@@ -145,10 +143,8 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
             const int idx = tid + n * THREADS;
+            const int c = idx % VPR, tok = idx / VPR % kTile, tensor = idx / (VPR * kTile);
             if (idx < VECS) {
-                const int c = idx % VPR;
-                const int tensor = (idx / VPR) % 6;
-                const int tok = idx / (VPR * 6);
                 float f[EPV];
                 Vec16<T>::unpack(stage[n], f);
                 if (tensor == VD) {
@@ -176,44 +172,34 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
         float *yt = ytile + (size_t)buf * kTile * ROWS;
         float *sat = satile + (size_t)buf * kTile * ROWS;
 
-        for (int tt = 0; tt < ntok; ++tt) {
+        // One token: the state's step; returns this thread's part of y.  (Packed multiply-adds: the sums are those of single ones.)
+        auto step = [&](int tt) -> float {
             const float *base = tv + (size_t)tt * 6 * kN;
-            const float4 *a4 = reinterpret_cast<const float4 *>(base + VA * kN);
-            float sa0 = 0.f, sa1 = 0.f, sa2 = 0.f, sa3 = 0.f;
+            auto vec4 = [&](int x, int kk) { return reinterpret_cast<const float4 *>(base + x * kN)[kk * 4 + q]; };
+            float2 s01 = make_float2(0.f, 0.f), s23 = s01;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
-                const float4 x = a4[kk * 4 + q];
-                sa0 = fmaf(S[kk * 4 + 0], x.x, sa0);
-                sa1 = fmaf(S[kk * 4 + 1], x.y, sa1);
-                sa2 = fmaf(S[kk * 4 + 2], x.z, sa2);
-                sa3 = fmaf(S[kk * 4 + 3], x.w, sa3);
+                const float4 x = vec4(VA, kk);
+                s01 = __ffma2_rn(S[kk][0], make_float2(x.x, x.y), s01);
+                s23 = __ffma2_rn(S[kk][1], make_float2(x.z, x.w), s23);
             }
-            float sa = (sa0 + sa1) + (sa2 + sa3);
+            float sa = (s01.x + s01.y) + (s23.x + s23.y);
             sa += __shfl_xor_sync(0xffffffffu, sa, 1);
             sa += __shfl_xor_sync(0xffffffffu, sa, 2);
             if constexpr (SAVE) {
                 if (q == 0) sat[tt * ROWS + i] = sa;
             }
             const float vi = base[VV * kN + row0 + i];
-            const float4 *d4 = reinterpret_cast<const float4 *>(base + VD * kN);
-            const float4 *b4 = reinterpret_cast<const float4 *>(base + VB * kN);
-            const float4 *k4 = reinterpret_cast<const float4 *>(base + VK * kN);
-            const float4 *r4 = reinterpret_cast<const float4 *>(base + VR * kN);
-            float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;
+            const float2 sa2 = make_float2(sa, sa), v2 = make_float2(vi, vi);
+            float2 y01 = make_float2(0.f, 0.f), y23 = y01;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
-                const float4 d = d4[kk * 4 + q], bb = b4[kk * 4 + q], kx = k4[kk * 4 + q],
-                             rr = r4[kk * 4 + q];
-                float s;
-                s = fmaf(S[kk * 4 + 0], d.x, fmaf(sa, bb.x, vi * kx.x)); S[kk * 4 + 0] = s; y0 = fmaf(s, rr.x, y0);
-                s = fmaf(S[kk * 4 + 1], d.y, fmaf(sa, bb.y, vi * kx.y)); S[kk * 4 + 1] = s; y1 = fmaf(s, rr.y, y1);
-                s = fmaf(S[kk * 4 + 2], d.z, fmaf(sa, bb.z, vi * kx.z)); S[kk * 4 + 2] = s; y2 = fmaf(s, rr.z, y2);
-                s = fmaf(S[kk * 4 + 3], d.w, fmaf(sa, bb.w, vi * kx.w)); S[kk * 4 + 3] = s; y3 = fmaf(s, rr.w, y3);
+                const float4 d = vec4(VD, kk), b = vec4(VB, kk), k = vec4(VK, kk), r = vec4(VR, kk);
+                S[kk][0] = __ffma2_rn(S[kk][0], make_float2(d.x, d.y), __ffma2_rn(sa2, make_float2(b.x, b.y), __fmul2_rn(v2, make_float2(k.x, k.y))));
+                S[kk][1] = __ffma2_rn(S[kk][1], make_float2(d.z, d.w), __ffma2_rn(sa2, make_float2(b.z, b.w), __fmul2_rn(v2, make_float2(k.z, k.w))));
+                y01 = __ffma2_rn(S[kk][0], make_float2(r.x, r.y), y01);
+                y23 = __ffma2_rn(S[kk][1], make_float2(r.z, r.w), y23);
             }
-            float yy = (y0 + y1) + (y2 + y3);
-            yy += __shfl_xor_sync(0xffffffffu, yy, 1);
-            yy += __shfl_xor_sync(0xffffffffu, yy, 2);
-            if (q == 0) yt[tt * ROWS + i] = yy;
             if constexpr (SAVE) {
                 const int t = tile * kTile + tt;
                 if ((t + 1) % save.chunk_len == 0) {   // state after the last token of a chunk
@@ -221,10 +207,29 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
                     float4 *dst = reinterpret_cast<float4 *>(
                         save.snapshots + (((size_t)bh * nchunks + chunk) * kN + row0 + i) * kN);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        dst[kk * 4 + q] = make_float4(S[kk * 4 + 0], S[kk * 4 + 1], S[kk * 4 + 2], S[kk * 4 + 3]);
+                    for (int kk = 0; kk < 4; ++kk) dst[kk * 4 + q] = make_float4(S[kk][0].x, S[kk][0].y, S[kk][1].x, S[kk][1].y);
                 }
             }
+            return (y01.x + y01.y) + (y23.x + y23.y);
+        };
+        // Four tokens at a time: their outputs are summed over the four lanes of a row together (lane q ends up with token q's, by the
+        // additions a sum of its own would have) and stored once, so that nothing but the state's own chain lies between
+        // one token and the next.
+        int tt = 0;
+        for (; tt + 4 <= ntok; tt += 4) {
+            float part[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) part[u] = step(tt + u);
+            const bool odd = q & 1, high = q & 2;
+            const float r0 = (odd ? part[1] : part[0]) + __shfl_xor_sync(0xffffffffu, odd ? part[0] : part[1], 1);
+            const float r1 = (odd ? part[3] : part[2]) + __shfl_xor_sync(0xffffffffu, odd ? part[2] : part[3], 1);
+            yt[(tt + q) * ROWS + i] = (high ? r1 : r0) + __shfl_xor_sync(0xffffffffu, high ? r0 : r1, 2);
+        }
+        for (; tt < ntok; ++tt) {
+            float yy = step(tt);
+            yy += __shfl_xor_sync(0xffffffffu, yy, 1);
+            yy += __shfl_xor_sync(0xffffffffu, yy, 2);
+            if (q == 0) yt[tt * ROWS + i] = yy;
         }
 
         if (tile + 1 < ntiles) commit_stage(buf ^ 1);
@@ -241,7 +246,7 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
         float4 *dst = reinterpret_cast<float4 *>(s_out + ((size_t)bh * kN + row0 + i) * kN);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-            dst[kk * 4 + q] = make_float4(S[kk * 4 + 0], S[kk * 4 + 1], S[kk * 4 + 2], S[kk * 4 + 3]);
+            dst[kk * 4 + q] = make_float4(S[kk][0].x, S[kk][0].y, S[kk][1].x, S[kk][1].y);
     }
 }
 
