@@ -23,7 +23,11 @@ namespace rwkv7 {
 namespace {
 
 constexpr int kN = 64;
-constexpr int kTile = 16;  // tokens staged per shared tile
+// Tokens staged per shared tile; fewer where a thread has several rows, so that more CTAs fit an SM.
+__host__ __device__ constexpr int seq_tile(int rows_per_thread) { return rows_per_thread == 1 ? 16 : 8; }
+constexpr size_t seq_smem(int rows, int rows_per_thread) {
+    return sizeof(float) * (size_t)(2 * seq_tile(rows_per_thread) * 6 * 64 + 4 * seq_tile(rows_per_thread) * rows);
+}
 
 enum { VR = 0, VD = 1, VK = 2, VV = 3, VA = 4, VB = 5 };
 
@@ -74,16 +78,22 @@ struct SavePtrs {
     int chunk_len;
 };
 
-template <typename T, int ROWS, bool SAVE = false>
-__global__ void __launch_bounds__(ROWS * 4)
+// ROWS value rows per CTA, RPT of them per group of four threads (RPT 1, 2 or 4).
+template <typename T, int ROWS, int RPT = 1, bool SAVE = false>
+__global__ void __launch_bounds__(ROWS / RPT * 4)
 wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
                   float *s_out, int Tlen, int H, const int *__restrict__ flags, SavePtrs save = SavePtrs{}) {
-    constexpr int THREADS = ROWS * 4;
+    constexpr int THREADS = ROWS / RPT * 4, GROUPS = THREADS / 4;
     constexpr int SPLITS = kN / ROWS;
+    constexpr int kTile = seq_tile(RPT);
+    // fp32 tensors land in shared memory as they are where registers are short.  (With a row per thread the registers a tile
+    // passes through cost nothing, and the compiler then keeps more of a token's loads ahead of its sums: 125 against 146 us, 511 tokens x 32 heads.)
+    constexpr bool kDirect = sizeof(T) == 4 && RPT > 1;
     constexpr int EPV = Vec16<T>::kElems;
     constexpr int VPR = kN / EPV;                 // 16-byte vectors per token row
     constexpr int VECS = kTile * 6 * VPR;         // vectors per tile
     constexpr int NV = (VECS + THREADS - 1) / THREADS;
+    static_assert(RPT == 1 || !SAVE, "the saving variant has a row per thread");
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *vec = reinterpret_cast<float *>(smem_raw);             // [2][kTile][6][kN]
@@ -102,22 +112,18 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
     const int bi = bh / H, h = bh % H;
     const int row0 = split * ROWS;
     const int tid = threadIdx.x;
-    const int i = tid >> 2, q = tid & 3;
+    const int i0 = tid >> 2, q = tid & 3;         // rows i0 + m GROUPS
 
-    float2 S[4][2];   // columns 16 kk + 4 q + {0, 1}, {2, 3}
-    if (s0 != nullptr) {
-        const float4 *src =
-            reinterpret_cast<const float4 *>(s0 + ((size_t)bh * kN + row0 + i) * kN);
+    float2 S[RPT][4][2];   // columns 16 kk + 4 q + {0, 1}, {2, 3}
+#pragma unroll
+    for (int m = 0; m < RPT; ++m)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
-            const float4 x = src[kk * 4 + q];
-            S[kk][0] = make_float2(x.x, x.y);
-            S[kk][1] = make_float2(x.z, x.w);
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (s0 != nullptr) x = reinterpret_cast<const float4 *>(s0 + ((size_t)bh * kN + row0 + i0 + m * GROUPS) * kN)[kk * 4 + q];
+            S[m][kk][0] = make_float2(x.x, x.y);
+            S[m][kk][1] = make_float2(x.z, x.w);
         }
-    } else {
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) S[kk][0] = S[kk][1] = make_float2(0.f, 0.f);
-    }
 
     const size_t seq_base = ((size_t)bi * Tlen * H + h) * kN;  // element offset of (b, t=0, h, 0)
     const size_t tok_stride = (size_t)H * kN;
@@ -125,37 +131,52 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
 
     // Vectors of a tile in the order (tensor, token, piece): a thread's n-th is of a tensor known at compile time (or uniform for
     // its warp).
-    uint4 stage[NV];
+    uint4 stage[kDirect ? 1 : NV];
+    auto place = [&](int n, int &c, int &tok, int &tensor) {
+        const int idx = tid + n * THREADS;
+        c = idx % VPR;
+        tok = idx / VPR % kTile;
+        tensor = idx / (VPR * kTile);
+        return idx < VECS;
+    };
     auto issue_loads = [&](int tile) {
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            const int idx = tid + n * THREADS;
-            stage[n] = make_uint4(0, 0, 0, 0);
-            const int c = idx % VPR, tok = idx / VPR % kTile, tensor = idx / (VPR * kTile);
+            int c, tok, tensor;
+            const bool mine = place(n, c, tok, tensor);
             const int t = tile * kTile + tok;
-            if (idx < VECS && t < Tlen) {
+            if constexpr (!kDirect) stage[n] = make_uint4(0, 0, 0, 0);
+            if (mine && t < Tlen) {
                 const T *p = reinterpret_cast<const T *>(ptrs.in[tensor]) + seq_base + (size_t)t * tok_stride + c * EPV;
-                stage[n] = __ldg(reinterpret_cast<const uint4 *>(p));
+                if constexpr (kDirect) {
+                    const unsigned dst = (unsigned)__cvta_generic_to_shared(vec + (((size_t)(tile & 1) * kTile + tok) * 6 + tensor) * kN + c * EPV);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(p) : "memory");
+                } else {
+                    stage[n] = __ldg(reinterpret_cast<const uint4 *>(p));
+                }
             }
         }
     };
     auto commit_stage = [&](int buf) {
+        if constexpr (kDirect) asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            const int idx = tid + n * THREADS;
-            const int c = idx % VPR, tok = idx / VPR % kTile, tensor = idx / (VPR * kTile);
-            if (idx < VECS) {
+            int c, tok, tensor;
+            if (place(n, c, tok, tensor) && (!kDirect || tensor == VD)) {   // (a thread converts what it fetched itself)
+                float4 *dst = reinterpret_cast<float4 *>(vec + (((size_t)buf * kTile + tok) * 6 + tensor) * kN + c * EPV);
                 float f[EPV];
-                Vec16<T>::unpack(stage[n], f);
+                if constexpr (kDirect) {
+                    const float4 x = *dst;
+                    f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w;
+                } else {
+                    Vec16<T>::unpack(stage[n], f);
+                }
                 if (tensor == VD) {
 #pragma unroll
                     for (int e = 0; e < EPV; ++e) f[e] = expf(-expf(f[e]));
                 }
-                float4 *dst = reinterpret_cast<float4 *>(
-                    vec + (((size_t)buf * kTile + tok) * 6 + tensor) * kN + c * EPV);
 #pragma unroll
-                for (int e = 0; e < EPV / 4; ++e)
-                    dst[e] = make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]);
+                for (int e = 0; e < EPV / 4; ++e) dst[e] = make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]);
             }
         }
     };
@@ -172,64 +193,83 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
         float *yt = ytile + (size_t)buf * kTile * ROWS;
         float *sat = satile + (size_t)buf * kTile * ROWS;
 
-        // One token: the state's step; returns this thread's part of y.  (Packed multiply-adds: the sums are those of single ones.)
-        auto step = [&](int tt) -> float {
+        // One token: the step of the state; this thread's parts of y.  (Packed multiply-adds: the sums are those of single ones.)
+        auto step = [&](int tt, float (&part)[RPT]) {
             const float *base = tv + (size_t)tt * 6 * kN;
             auto vec4 = [&](int x, int kk) { return reinterpret_cast<const float4 *>(base + x * kN)[kk * 4 + q]; };
-            float2 s01 = make_float2(0.f, 0.f), s23 = s01;
+            float2 s01[RPT], s23[RPT], sa[RPT], vi[RPT], y01[RPT], y23[RPT];
+#pragma unroll
+            for (int m = 0; m < RPT; ++m) s01[m] = s23[m] = y01[m] = y23[m] = make_float2(0.f, 0.f);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 const float4 x = vec4(VA, kk);
-                s01 = __ffma2_rn(S[kk][0], make_float2(x.x, x.y), s01);
-                s23 = __ffma2_rn(S[kk][1], make_float2(x.z, x.w), s23);
+#pragma unroll
+                for (int m = 0; m < RPT; ++m) {
+                    s01[m] = __ffma2_rn(S[m][kk][0], make_float2(x.x, x.y), s01[m]);
+                    s23[m] = __ffma2_rn(S[m][kk][1], make_float2(x.z, x.w), s23[m]);
+                }
             }
-            float sa = (s01.x + s01.y) + (s23.x + s23.y);
-            sa += __shfl_xor_sync(0xffffffffu, sa, 1);
-            sa += __shfl_xor_sync(0xffffffffu, sa, 2);
-            if constexpr (SAVE) {
-                if (q == 0) sat[tt * ROWS + i] = sa;
+#pragma unroll
+            for (int m = 0; m < RPT; ++m) {
+                float sum = (s01[m].x + s01[m].y) + (s23[m].x + s23[m].y);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                if constexpr (SAVE) {
+                    if (q == 0) sat[tt * ROWS + i0] = sum;
+                }
+                const float v = base[VV * kN + row0 + i0 + m * GROUPS];
+                sa[m] = make_float2(sum, sum);
+                vi[m] = make_float2(v, v);
             }
-            const float vi = base[VV * kN + row0 + i];
-            const float2 sa2 = make_float2(sa, sa), v2 = make_float2(vi, vi);
-            float2 y01 = make_float2(0.f, 0.f), y23 = y01;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 const float4 d = vec4(VD, kk), b = vec4(VB, kk), k = vec4(VK, kk), r = vec4(VR, kk);
-                S[kk][0] = __ffma2_rn(S[kk][0], make_float2(d.x, d.y), __ffma2_rn(sa2, make_float2(b.x, b.y), __fmul2_rn(v2, make_float2(k.x, k.y))));
-                S[kk][1] = __ffma2_rn(S[kk][1], make_float2(d.z, d.w), __ffma2_rn(sa2, make_float2(b.z, b.w), __fmul2_rn(v2, make_float2(k.z, k.w))));
-                y01 = __ffma2_rn(S[kk][0], make_float2(r.x, r.y), y01);
-                y23 = __ffma2_rn(S[kk][1], make_float2(r.z, r.w), y23);
+#pragma unroll
+                for (int m = 0; m < RPT; ++m) {
+                    float2 &s0 = S[m][kk][0], &s1 = S[m][kk][1];
+                    s0 = __ffma2_rn(s0, make_float2(d.x, d.y), __ffma2_rn(sa[m], make_float2(b.x, b.y), __fmul2_rn(vi[m], make_float2(k.x, k.y))));
+                    s1 = __ffma2_rn(s1, make_float2(d.z, d.w), __ffma2_rn(sa[m], make_float2(b.z, b.w), __fmul2_rn(vi[m], make_float2(k.z, k.w))));
+                    y01[m] = __ffma2_rn(s0, make_float2(r.x, r.y), y01[m]);
+                    y23[m] = __ffma2_rn(s1, make_float2(r.z, r.w), y23[m]);
+                }
             }
             if constexpr (SAVE) {
                 const int t = tile * kTile + tt;
                 if ((t + 1) % save.chunk_len == 0) {   // state after the last token of a chunk
                     const int chunk = t / save.chunk_len, nchunks = Tlen / save.chunk_len;
                     float4 *dst = reinterpret_cast<float4 *>(
-                        save.snapshots + (((size_t)bh * nchunks + chunk) * kN + row0 + i) * kN);
+                        save.snapshots + (((size_t)bh * nchunks + chunk) * kN + row0 + i0) * kN);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) dst[kk * 4 + q] = make_float4(S[kk][0].x, S[kk][0].y, S[kk][1].x, S[kk][1].y);
+                    for (int kk = 0; kk < 4; ++kk) dst[kk * 4 + q] = make_float4(S[0][kk][0].x, S[0][kk][0].y, S[0][kk][1].x, S[0][kk][1].y);
                 }
             }
-            return (y01.x + y01.y) + (y23.x + y23.y);
-        };
-        // Four tokens at a time: their outputs are summed over the four lanes of a row together (lane q ends up with token q's, by the
-        // additions a sum of its own would have) and stored once, so that nothing but the state's own chain lies between
-        // one token and the next.
-        int tt = 0;
-        for (; tt + 4 <= ntok; tt += 4) {
-            float part[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) part[u] = step(tt + u);
+            for (int m = 0; m < RPT; ++m) part[m] = (y01[m].x + y01[m].y) + (y23[m].x + y23[m].y);
+        };
+        // Four outputs at a time (of 4 / RPT tokens) are summed over the four lanes of a row group together: lane q ends up with
+        // the q-th, by the additions a sum of its own would have.  With a row per thread nothing but the state's own chain then
+        // lies between one token and the next three.
+        constexpr int TOKENS = 4 / RPT;
+        int tt = 0;
+        for (; tt + TOKENS <= ntok; tt += TOKENS) {
+            float part[TOKENS][RPT];
+#pragma unroll
+            for (int u = 0; u < TOKENS; ++u) step(tt + u, part[u]);
+            const float p0 = part[0][0], p1 = part[1 / RPT][1 % RPT], p2 = part[2 / RPT][2 % RPT], p3 = part[3 / RPT][3 % RPT];
             const bool odd = q & 1, high = q & 2;
-            const float r0 = (odd ? part[1] : part[0]) + __shfl_xor_sync(0xffffffffu, odd ? part[0] : part[1], 1);
-            const float r1 = (odd ? part[3] : part[2]) + __shfl_xor_sync(0xffffffffu, odd ? part[2] : part[3], 1);
-            yt[(tt + q) * ROWS + i] = (high ? r1 : r0) + __shfl_xor_sync(0xffffffffu, high ? r0 : r1, 2);
+            const float r0 = (odd ? p1 : p0) + __shfl_xor_sync(0xffffffffu, odd ? p0 : p1, 1);
+            const float r1 = (odd ? p3 : p2) + __shfl_xor_sync(0xffffffffu, odd ? p2 : p3, 1);
+            yt[(tt + q / RPT) * ROWS + i0 + q % RPT * GROUPS] = (high ? r1 : r0) + __shfl_xor_sync(0xffffffffu, high ? r0 : r1, 2);
         }
         for (; tt < ntok; ++tt) {
-            float yy = step(tt);
-            yy += __shfl_xor_sync(0xffffffffu, yy, 1);
-            yy += __shfl_xor_sync(0xffffffffu, yy, 2);
-            if (q == 0) yt[tt * ROWS + i] = yy;
+            float part[RPT];
+            step(tt, part);
+#pragma unroll
+            for (int m = 0; m < RPT; ++m) {
+                part[m] += __shfl_xor_sync(0xffffffffu, part[m], 1);
+                part[m] += __shfl_xor_sync(0xffffffffu, part[m], 2);
+                if (q == 0) yt[tt * ROWS + i0 + m * GROUPS] = part[m];
+            }
         }
 
         if (tile + 1 < ntiles) commit_stage(buf ^ 1);
@@ -243,10 +283,12 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
     }
 
     if (s_out != nullptr) {
-        float4 *dst = reinterpret_cast<float4 *>(s_out + ((size_t)bh * kN + row0 + i) * kN);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-            dst[kk * 4 + q] = make_float4(S[kk][0].x, S[kk][0].y, S[kk][1].x, S[kk][1].y);
+        for (int m = 0; m < RPT; ++m) {
+            float4 *dst = reinterpret_cast<float4 *>(s_out + ((size_t)bh * kN + row0 + i0 + m * GROUPS) * kN);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) dst[kk * 4 + q] = make_float4(S[m][kk][0].x, S[m][kk][0].y, S[m][kk][1].x, S[m][kk][1].y);
+        }
     }
 }
 
@@ -310,11 +352,12 @@ __global__ void wkv7_seq_generic_kernel(SeqPtrs ptrs, const float *s0,
         }
 }
 
-template <typename T, int ROWS>
+template <typename T, int ROWS, int RPT>
 int launch_seq64(const Wkv7Args &p, cudaStream_t stream, const int *flags = nullptr) {
     SeqPtrs ptrs{{p.r, p.w, p.k, p.v, p.a, p.b}};
-    const size_t smem = sizeof(float) * (2 * kTile * 6 * kN + 4 * kTile * ROWS);
-    auto kern = wkv7_seq64_kernel<T, ROWS, false>;
+    constexpr size_t smem = seq_smem(ROWS, RPT);
+    constexpr unsigned threads = ROWS / RPT * 4;
+    auto kern = wkv7_seq64_kernel<T, ROWS, RPT, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const unsigned grid = (unsigned)(p.B * p.H * (kN / ROWS));
@@ -323,7 +366,7 @@ int launch_seq64(const Wkv7Args &p, cudaStream_t stream, const int *flags = null
         // dependent launch lets its launch overlap that kernel's tail (the kernel itself waits for the flags).
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(ROWS * 4);
+        cfg.blockDim = dim3(threads);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
         cudaLaunchAttribute attr[1];
@@ -336,7 +379,7 @@ int launch_seq64(const Wkv7Args &p, cudaStream_t stream, const int *flags = null
         if (e == cudaSuccess) count_launch();
         return (int)e;
     }
-    kern<<<grid, ROWS * 4, smem, stream>>>(ptrs, p.s0, reinterpret_cast<T *>(p.y), p.s_out,
+    kern<<<grid, threads, smem, stream>>>(ptrs, p.s0, reinterpret_cast<T *>(p.y), p.s_out,
                                            (int)p.T, (int)p.H, flags, SavePtrs{});
     count_launch();
     return (int)cudaGetLastError();
@@ -345,15 +388,14 @@ int launch_seq64(const Wkv7Args &p, cudaStream_t stream, const int *flags = null
 template <typename T>
 int launch_seq(const Wkv7Args &p, cudaStream_t stream) {
     if (p.N == kN) {
-        // Split the 64 value rows of a (b,h) over several CTAs when there are too
-        // few (b,h) chains to fill the SMs; rows of S never interact.
+        // Rows of S never interact.  A token's five column vectors cost a warp 84 wavefronts of shared memory however many
+        // rows its threads have: 672 cycles of an SM per chain and token with a row per thread, 336 with two, 168 with
+        // four.  The chain of one token to the next takes about 400, so threads take as few rows as keep an SM's
+        // chains below that, and a chain is spread over as many CTAs as that leaves.
         const int64_t chains = p.B * p.H;
-        int rows = 64;
-        if (chains < 2 * (int64_t)p.num_sms) rows = 32;
-        if (chains * 2 < 2 * (int64_t)p.num_sms) rows = 16;
-        if (rows == 64) return launch_seq64<T, 64>(p, stream);
-        if (rows == 32) return launch_seq64<T, 32>(p, stream);
-        return launch_seq64<T, 16>(p, stream);
+        if (chains * 5 <= 3 * (int64_t)p.num_sms) return launch_seq64<T, 16, 1>(p, stream);
+        if (chains * 5 <= 6 * (int64_t)p.num_sms) return launch_seq64<T, 32, 2>(p, stream);
+        return launch_seq64<T, 64, 4>(p, stream);
     }
     SeqPtrs ptrs{{p.r, p.w, p.k, p.v, p.a, p.b}};
     const int N = (int)p.N;
@@ -376,8 +418,8 @@ int launch_seq_saved(const Wkv7Args &p, float *snapshots, void *state_replacemen
     SavePtrs save{snapshots, state_replacement, chunk_len};
     if (p.N == kN) {
         constexpr int ROWS = 16;   // four CTAs per chain: rows of S never interact
-        const size_t smem = sizeof(float) * (2 * kTile * 6 * kN + 4 * kTile * ROWS);
-        auto kern = wkv7_seq64_kernel<T, ROWS, true>;
+        const size_t smem = seq_smem(ROWS, 1);
+        auto kern = wkv7_seq64_kernel<T, ROWS, 1, true>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         kern<<<(unsigned)(p.B * p.H * (kN / ROWS)), ROWS * 4, smem, stream>>>(
@@ -409,17 +451,17 @@ int launch_wkv7_sequential_flagged_saved(const Wkv7Args &p, const int *flags, fl
     SeqPtrs ptrs{{p.r, p.w, p.k, p.v, p.a, p.b}};
     SavePtrs save{snapshots, state_replacement, chunk_len};
     constexpr int ROWS = 16;
-    const size_t smem = sizeof(float) * (2 * kTile * 6 * kN + 4 * kTile * ROWS);
+    const size_t smem = seq_smem(ROWS, 1);
     const unsigned grid = (unsigned)(p.B * p.H * (kN / ROWS));
     cudaError_t e;
     if (p.bf16) {
-        auto kern = wkv7_seq64_kernel<__nv_bfloat16, ROWS, true>;
+        auto kern = wkv7_seq64_kernel<__nv_bfloat16, ROWS, 1, true>;
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         kern<<<grid, ROWS * 4, smem, stream>>>(ptrs, p.s0, reinterpret_cast<__nv_bfloat16 *>(p.y), p.s_out, (int)p.T,
                                                (int)p.H, flags, save);
     } else {
-        auto kern = wkv7_seq64_kernel<float, ROWS, true>;
+        auto kern = wkv7_seq64_kernel<float, ROWS, 1, true>;
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         kern<<<grid, ROWS * 4, smem, stream>>>(ptrs, p.s0, reinterpret_cast<float *>(p.y), p.s_out, (int)p.T, (int)p.H,
@@ -431,7 +473,7 @@ int launch_wkv7_sequential_flagged_saved(const Wkv7Args &p, const int *flags, fl
 
 // N == 64 only: recomputes the chains with flags[b*H+h] != 0, 16 value rows per CTA.
 int launch_wkv7_sequential_flagged(const Wkv7Args &p, const int *flags, cudaStream_t stream) {
-    return p.bf16 ? launch_seq64<__nv_bfloat16, 16>(p, stream, flags) : launch_seq64<float, 16>(p, stream, flags);
+    return p.bf16 ? launch_seq64<__nv_bfloat16, 16, 1>(p, stream, flags) : launch_seq64<float, 16, 1>(p, stream, flags);
 }
 
 int launch_wkv7_sequential(const Wkv7Args &p, cudaStream_t stream) {
