@@ -12,6 +12,10 @@
 // vectors are staged 16 tokens at a time through a double-buffered shared tile,
 // converted to fp32 once (decay computed once per element).
 // Any other N <= 128: one thread per row, state in shared memory.
+//
+// Bound by the chain from one token's state to the next with few chains (0.21 us a token: eight multiply-adds deep, two shuffles,
+// the update) and by shared memory and the packed multiply-adds with many.  Measured (B200), fp32, 511 tokens: 32 chains 108
+// us, 1600 chains 900 us (with a row per thread throughout and the output summed in the chain: 191 and 2385).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -87,7 +91,7 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
     constexpr int SPLITS = kN / ROWS;
     constexpr int kTile = seq_tile(RPT);
     // fp32 tensors land in shared memory as they are where registers are short.  (With a row per thread the registers a tile
-    // passes through cost nothing, and the compiler then keeps more of a token's loads ahead of its sums: 125 against 146 us, 511 tokens x 32 heads.)
+    // passes through cost nothing, and the compiler then keeps more of a token's loads ahead of its sums: 125 against 146 us at 511 tokens x 32 heads.)
     constexpr bool kDirect = sizeof(T) == 4 && RPT > 1;
     constexpr int EPV = Vec16<T>::kElems;
     constexpr int VPR = kN / EPV;                 // 16-byte vectors per token row
@@ -193,6 +197,12 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
         float *yt = ytile + (size_t)buf * kTile * ROWS;
         float *sat = satile + (size_t)buf * kTile * ROWS;
 
+        // (the removal key of the next token is fetched while this one's is used, which takes its latency out of the chain from state
+        // to state: 125 -> 108 us at 511 fp32 tokens x 32 heads; fetching the other vectors as early cost registers, 117.  Behind a
+        // tile's last token it reads what follows the tile and nobody uses it.)
+        float4 ahead[4];
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) ahead[kk] = reinterpret_cast<const float4 *>(tv + VA * kN)[kk * 4 + q];
         // One token: the step of the state; this thread's parts of y.  (Packed multiply-adds: the sums are those of single ones.)
         auto step = [&](int tt, float (&part)[RPT]) {
             const float *base = tv + (size_t)tt * 6 * kN;
@@ -202,7 +212,8 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
             for (int m = 0; m < RPT; ++m) s01[m] = s23[m] = y01[m] = y23[m] = make_float2(0.f, 0.f);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
-                const float4 x = vec4(VA, kk);
+                const float4 x = ahead[kk];
+                ahead[kk] = vec4(6 + VA, kk);   // the next token's
 #pragma unroll
                 for (int m = 0; m < RPT; ++m) {
                     s01[m] = __ffma2_rn(S[m][kk][0], make_float2(x.x, x.y), s01[m]);
