@@ -326,22 +326,13 @@ def wkv7_backward(inputs: Wkv7PretrainForwardInputs, saved: Wkv7SavedForward, ou
 
 
 class _Wkv7Function(torch.autograd.Function):
-    """The autodiff node of the reference (``Wkv7StatepassBackward``, ``wkv7/backward.rs:381-533``).  bf16 sequences
-    with 64-element heads keep what the tensor-core training step needs (``rwkv7_fused_wkv7_training_forward``);
-    for everything else forward saves snapshots and state_replacement, and backward runs the reverse kernel."""
+    """The autodiff node of the reference (``Wkv7StatepassBackward``, ``wkv7/backward.rs:381-533``):
+    forward saves snapshots and state_replacement, backward runs the reverse kernel."""
 
     @staticmethod
     def forward(ctx, r, w, k, v, a, b, s0, chunk_len):
         inputs = Wkv7PretrainForwardInputs(r, w, k, v, a, b, chunk_len=chunk_len)
-        inputs.check(True)
         ctx.set_materialize_grads(False)
-        step = (_native or native()).wkv7_training_forward(s0, r, w, k, v, a, b, chunk_len)
-        ctx.step = step is not None
-        if ctx.step:
-            y, s_out, kept = step
-            ctx.save_for_backward(r, w, k, v, a, b, kept)
-            ctx.has_state, ctx.chunk_len = s0 is not None, chunk_len
-            return y, s_out
         saved = wkv7_forward_saved(inputs, s0, want_state=True)
         # Only what the backward pass reads is kept, and through save_for_backward: the node then
         # holds no reference to its own outputs (no cycle) and autograd's version counters catch an
@@ -358,10 +349,6 @@ class _Wkv7Function(torch.autograd.Function):
         t = ctx.saved_tensors
         if dy is None:
             dy = torch.zeros_like(t[0])
-        if ctx.step:
-            *grads, ds0 = (_native or native()).wkv7_training_backward(
-                *t[:6], ctx.chunk_len, t[6], dy, None if ds is None else ds.contiguous(), ctx.has_state)
-            return (*grads, ds0, None)
         inputs = Wkv7PretrainForwardInputs(*t[:6], chunk_len=ctx.chunk_len)
         saved = Wkv7SavedForward(output=None, next_state=None, snapshots=t[6], state_replacement=t[7])
         s0 = t[8] if ctx.has_state else None
@@ -372,8 +359,13 @@ class _Wkv7Function(torch.autograd.Function):
 
 def wkv7_statepass_autograd(initial_state: Optional[torch.Tensor], sequence: Wkv7PretrainForwardInputs):
     """Differentiable statepass: ``(output, next_state)`` with gradients to the six sequence tensors and
-    the initial state, like ``wkv7_statepass_custom`` on the reference's Autodiff backend."""
-    return _Wkv7Function.apply(*[t.contiguous() for t in sequence.six()], initial_state, sequence.chunk_len)
+    the initial state, like ``wkv7_statepass_custom`` on the reference's Autodiff backend.  bf16 sequences with
+    64-element heads go through the tensor-core training step (``rwkv7_fused_wkv7_training_forward``), whose node is
+    native code; everything else keeps the reference's saved tensors (:class:`_Wkv7Function`)."""
+    sequence.check(True)
+    six = [t.contiguous() for t in sequence.six()]
+    step = (_native or native()).wkv7_training_step(initial_state, *six, sequence.chunk_len)
+    return step if step is not None else _Wkv7Function.apply(*six, initial_state, sequence.chunk_len)
 
 
 class Wkv7HostStatepass:

@@ -17,6 +17,7 @@
 #include <cuda_runtime_api.h>
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "rwkv7_b200.h"
@@ -337,56 +338,84 @@ PyObject *wkv7_backward(PyObject *const *a) {
     return pair(list, ds0.defined() ? wrap(ds0) : Py_NewRef(Py_None));
 }
 
-// wkv7_training_forward(initial_state|None, r, w, k, v, a, b, chunk_len) -> (output, next_state, saved), or None for what
-// the training step does not cover
-PyObject *wkv7_training_forward(PyObject *const *a) {
+// The node of a training step (see rwkv7_fused_wkv7_training_forward).  In native code because a short step is bound by its host
+// path: with the node in Python a step of 1 x 128 tokens x 12 heads took 130 us of it, now 117 (the engine is most of that).
+struct TrainingStep : torch::autograd::Function<TrainingStep> {
+    using Tensors = torch::autograd::variable_list;
+
+    static Tensors forward(torch::autograd::AutogradContext *ctx, const at::Tensor &r, const at::Tensor &w, const at::Tensor &k, const at::Tensor &v,
+                           const at::Tensor &a, const at::Tensor &b, const std::optional<at::Tensor> &s0, int64_t chunk_len, int64_t keep) {
+        const Desc in[6] = {Desc(r), Desc(w), Desc(k), Desc(v), Desc(a), Desc(b)};
+        Desc sd0;
+        if (s0) sd0.set(*s0);
+        Tensors out{like(r), empty({r.size(0), r.size(2), r.size(3), r.size(3)}, at::kFloat, r)};
+        const at::Tensor kept = empty({keep}, at::kByte, r);
+        Desc yd(out[0]), sd(out[1]);
+        const rwkv7_stream st = stream_of(r);
+        call([&] {
+            return abi.rwkv7_fused_wkv7_training_forward(sd0.p, in[0].p, in[1].p, in[2].p, in[3].p, in[4].p, in[5].p, chunk_len, yd.p, sd.p,
+                                                         kept.data_ptr(), (size_t)keep, st);
+        });
+        // (what the backward pass reads, and only that: the version counters catch a change in place before it)
+        ctx->save_for_backward({r, w, k, v, a, b, kept});
+        ctx->saved_data["chunk_len"] = chunk_len;
+        ctx->saved_data["has_state"] = s0.has_value();
+        ctx->set_materialize_grads(false);
+        return out;
+    }
+
+    // On a thread of the autograd engine, without the interpreter lock.
+    static Tensors backward(torch::autograd::AutogradContext *ctx, Tensors grad) {
+        const Tensors t = ctx->get_saved_variables();
+        const at::Tensor &r = t[0], &kept = t[6];
+        const int64_t chunk_len = ctx->saved_data["chunk_len"].toInt();
+        const Desc in[6] = {Desc(t[0]), Desc(t[1]), Desc(t[2]), Desc(t[3]), Desc(t[4]), Desc(t[5])};
+        const at::Tensor dy_t = grad[0].defined() ? grad[0].contiguous() : at::zeros_like(r), ds_t = grad[1].defined() ? grad[1].contiguous() : grad[1];
+        Desc dy(dy_t), ds, gd[6], ds0d;
+        if (ds_t.defined()) ds.set(ds_t);
+        Tensors out(9);
+        rwkv7_tensor *gp[6];
+        for (int i = 0; i < 6; ++i) {
+            out[i] = like(r);
+            gd[i].set(out[i]);
+            gp[i] = gd[i].p;
+        }
+        if (ctx->saved_data["has_state"].toBool()) {
+            out[6] = empty({r.size(0), r.size(2), r.size(3), r.size(3)}, at::kFloat, r);
+            ds0d.set(out[6]);
+        }
+        Workspace ws;
+        ws.allocate(abi.rwkv7_wkv7_training_workspace_bytes(r.size(0), r.size(1), r.size(2), r.size(3)), r);
+        const int status = abi.rwkv7_fused_wkv7_training_backward(in[0].p, in[1].p, in[2].p, in[3].p, in[4].p, in[5].p, chunk_len,
+                                                                  kept.data_ptr(), (size_t)kept.numel(), dy.p, ds.p, gp, ds0d.p, ws.ptr,
+                                                                  ws.bytes, stream_of(r));
+        if (status != 0) {
+            const PyGILState_STATE gil = PyGILState_Ensure();
+            python_error error;
+            try {
+                check(status);
+            } catch (const PythonError &) {
+                error.persist();
+            }
+            PyGILState_Release(gil);
+            throw error;
+        }
+        return out;
+    }
+};
+
+// wkv7_training_step(initial_state|None, r, w, k, v, a, b, chunk_len) -> (output, next_state), part of the autograd graph, or
+// None for what the training step does not cover
+PyObject *wkv7_training_step(PyObject *const *a) {
     const at::Tensor &r = tensor(a[1]);
-    Desc s0(a[0]), six[6];
-    for (int i = 0; i < 6; ++i) six[i].set(tensor(a[1 + i]));
+    for (int i = 2; i < 7; ++i) tensor(a[i]);
     const int64_t chunk_len = integer(a[7]);
     const size_t keep = r.dim() != 4 || !r.is_cuda()
-                            ? 0 : abi.rwkv7_wkv7_training_saved_bytes(r.size(0), r.size(1), r.size(2), r.size(3), six[0].d.dtype, chunk_len);
+                            ? 0 : abi.rwkv7_wkv7_training_saved_bytes(r.size(0), r.size(1), r.size(2), r.size(3), dtype_code(r.scalar_type()), chunk_len);
     if (keep == 0) return Py_NewRef(Py_None);
-    at::Tensor out[3] = {like(r), empty({r.size(0), r.size(2), r.size(3), r.size(3)}, at::kFloat, r), empty({(int64_t)keep}, at::kByte, r)};
-    Desc yd(out[0]), sd(out[1]);
-    const rwkv7_stream st = stream_of(r);
-    call([&] {
-        return abi.rwkv7_fused_wkv7_training_forward(s0.p, six[0].p, six[1].p, six[2].p, six[3].p, six[4].p, six[5].p, chunk_len,
-                                                     yd.p, sd.p, out[2].data_ptr(), keep, st);
-    });
-    return tuple_of(out, 3);
-}
-
-// wkv7_training_backward(r, w, k, v, a, b, chunk_len, saved, output_grad, next_state_grad|None, want_state_grad)
-//   -> (six gradients, state gradient|None)
-PyObject *wkv7_training_backward(PyObject *const *a) {
-    const at::Tensor &r = tensor(a[0]);
-    Desc six[6];
-    for (int i = 0; i < 6; ++i) six[i].set(tensor(a[i]));
-    const int64_t chunk_len = integer(a[6]);
-    const at::Tensor &saved = tensor(a[7]);
-    const at::Tensor dy_t = tensor(a[8]).contiguous();
-    Desc dy(dy_t), ds(a[9]), gd[6], ds0d;
-    at::Tensor grads[7];
-    rwkv7_tensor *gp[6];
-    for (int i = 0; i < 6; ++i) {
-        grads[i] = like(r);
-        gd[i].set(grads[i]);
-        gp[i] = gd[i].p;
-    }
-    if (truth(a[10])) {
-        grads[6] = empty({r.size(0), r.size(2), r.size(3), r.size(3)}, at::kFloat, r);
-        ds0d.set(grads[6]);
-    }
-    Workspace ws;
-    ws.allocate(abi.rwkv7_wkv7_training_workspace_bytes(r.size(0), r.size(1), r.size(2), r.size(3)), r);
-    const rwkv7_stream st = stream_of(r);
-    call([&] {
-        return abi.rwkv7_fused_wkv7_training_backward(six[0].p, six[1].p, six[2].p, six[3].p, six[4].p, six[5].p, chunk_len,
-                                                      saved.data_ptr(), (size_t)saved.numel(), dy.p, ds.p, gp, ds0d.p, ws.ptr,
-                                                      ws.bytes, st);
-    });
-    return tuple_of(grads, 7);
+    const auto out = TrainingStep::apply(r, tensor(a[2]), tensor(a[3]), tensor(a[4]), tensor(a[5]), tensor(a[6]),
+                                         a[0] == Py_None ? std::nullopt : std::make_optional(tensor(a[0])), chunk_len, (int64_t)keep);
+    return pair(wrap(out[0]), wrap(out[1]));
 }
 
 // mix6(x, six scales) -> six outputs
@@ -612,7 +641,7 @@ PyObject *open_library(PyObject *, PyObject *const *args, Py_ssize_t n) {
     {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<name, nargs>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"open", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&open_library)), METH_FASTCALL, nullptr},
-    RWKV7_METHOD(wkv7, 12), RWKV7_METHOD(wkv7_noalloc, 10), RWKV7_METHOD(wkv7_saved, 9), RWKV7_METHOD(wkv7_backward, 15), RWKV7_METHOD(wkv7_training_forward, 8), RWKV7_METHOD(wkv7_training_backward, 11),
+    RWKV7_METHOD(wkv7, 12), RWKV7_METHOD(wkv7_noalloc, 10), RWKV7_METHOD(wkv7_saved, 9), RWKV7_METHOD(wkv7_backward, 15), RWKV7_METHOD(wkv7_training_step, 8),
     RWKV7_METHOD(mix6, 7), RWKV7_METHOD(mix6_stacked, 7), RWKV7_METHOD(addcmul, 4), RWKV7_METHOD(addcmul5, 7),
     RWKV7_METHOD(token_shift_diff, 4), RWKV7_METHOD(weight_prepare, 9), RWKV7_METHOD(gated_readout, 10),
     RWKV7_METHOD(channel_mixer, 5), RWKV7_METHOD(lm_head_ce_partial, 4), RWKV7_METHOD(lm_head_ce_finalize, 2),
