@@ -158,12 +158,15 @@ int wkv7_dispatch(Wkv7Args &p, void *workspace, size_t workspace_bytes, rwkv7_st
     // The two-kernel prefill first, where it applies and the workspace holds at least one segment of
     // operators; chains it leaves flagged (decay beyond what fp16 operands resolve, non-finite values)
     // go to the tf32 chunked kernel, and from there to the sequential scan.
-    const bool split_fits = wkv7_split_supported(p) && workspace != nullptr &&
+    // (The operators lie in the workspace and are read by bulk copies, which need 16-byte boundaries; the tf32 kernel only keeps
+    // ints there, so an odd workspace takes that one.)
+    const bool bulk_ws = (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0;
+    const bool split_fits = wkv7_split_supported(p) && workspace != nullptr && bulk_ws &&
                             workspace_bytes >= wkv7_split_min_workspace_bytes(p.B, p.T, p.H, p.N);
     if (path == RWKV7_WKV7_SPLIT && !split_fits) {
-        if (!wkv7_split_supported(p))
+        if (!wkv7_split_supported(p) || !bulk_ws)
             return fail(RWKV7_ERR_UNSUPPORTED,
-                        "Unsupported: the two-kernel WKV7 prefill needs N == 64 and 16-byte aligned tensors (got N=%lld)", (long long)p.N);
+                        "Unsupported: the two-kernel WKV7 prefill needs N == 64 and 16-byte aligned tensors and workspace (got N=%lld)", (long long)p.N);
         return fail(RWKV7_ERR_WORKSPACE_TOO_SMALL, "WorkspaceTooSmall: wkv7 needs %zu workspace bytes, got %zu",
                     wkv7_split_min_workspace_bytes(p.B, p.T, p.H, p.N), workspace == nullptr ? (size_t)0 : workspace_bytes);
     }
@@ -192,6 +195,8 @@ int wkv7_dispatch(Wkv7Args &p, void *workspace, size_t workspace_bytes, rwkv7_st
             return fail(RWKV7_ERR_WORKSPACE_TOO_SMALL,
                         "WorkspaceTooSmall: wkv7 needs %zu workspace bytes, got %zu", need,
                         workspace == nullptr ? (size_t)0 : workspace_bytes);
+        if (need > 0 && (reinterpret_cast<uintptr_t>(workspace) & 3u) != 0)
+            return fail(RWKV7_ERR_UNSUPPORTED, "Unsupported: the wkv7 workspace must be 4-byte aligned");
         if (int e = launch_wkv7_chunked(p, workspace, workspace_bytes, (cudaStream_t)stream))
             return cuda_fail("wkv7 chunked launch", e);
         return RWKV7_OK;
