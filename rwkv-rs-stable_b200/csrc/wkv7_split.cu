@@ -481,7 +481,8 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                     }
                     x[t] = (t == cc) ? 1.f : acc0 + acc1;   // (zero above: every term up to there is)
                 }
-                unsigned char *dst = smem + kDiag + b * 1024 + (cc >> 3) * 256 + (cc & 7) * 2;   // (every lane has read the block)
+                __syncwarp();   // (every lane has read the block that the inverse replaces)
+                unsigned char *dst = smem + kDiag + b * 1024 + (cc >> 3) * 256 + (cc & 7) * 2;
 #pragma unroll
                 for (int t = 0; t < 16; ++t) *reinterpret_cast<__half *>(dst + t * 16) = __float2half_rn(x[t]);
             }
