@@ -489,8 +489,12 @@ PyObject *addcmul5(PyObject *const *a) {
 // token_shift_diff(x, state, batch_ids, inplace_state) -> (diff, next state)
 PyObject *token_shift_diff(PyObject *const *a) {
     const at::Tensor &x = tensor(a[0]);
-    const bool keep = !truth(a[3]), copied = keep && x.numel() == 0;   // (no tokens: nothing to compute, a plain copy)
-    const at::Tensor state = copied ? tensor(a[1]).detach().clone() : tensor(a[1]);
+    // (Copied first, and the copy updated in place: a state the kernel does not take as it is, such as some columns of a wider
+    // table, a broadcast row or rows from an odd offset on, which its copy mends; and nothing to compute, T = 0.)
+    const at::Tensor &given = tensor(a[1]);
+    const bool keep = !truth(a[3]);
+    const bool copied = keep && (x.numel() == 0 || !given.is_contiguous() || (reinterpret_cast<uintptr_t>(given.data_ptr()) & 15u) != 0);
+    const at::Tensor state = copied ? given.detach().clone() : given;
     const bool inplace = !keep || copied;
     at::Tensor out[2];   // diff, next state
     if (inplace) out[0] = like(x);

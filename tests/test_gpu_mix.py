@@ -85,3 +85,28 @@ def test_token_shift_diff_bad_id_is_reported_not_faulted(pkg, cuda):
     assert pkg.read_device_status(0) == 0   # cleared by the read
     assert torch.equal(out.next_token_shift[0], before[0]) and torch.equal(out.next_token_shift[2], before[2])
     assert torch.equal(out.next_token_shift[1], x[0, 3])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("layout", ["columns", "broadcast", "odd_offset"])
+def test_token_shift_diff_state_of_another_layout(pkg, oracle, cuda, layout, dtype):
+    """A state that is not dense or not aligned: the functional call works on a copy, which is; in place it is refused."""
+    B, T, C, S = 2, 5, 24, 4
+    g = torch.Generator().manual_seed(7)
+    x = torch.randn(B, T, C, generator=g).to(dtype)
+    table = torch.randn(S, 2 * C, generator=g).to(dtype).to(cuda)
+    if layout == "columns":
+        state = table[:, :C]
+    elif layout == "broadcast":
+        state = table[:1, :C].expand(S, C)
+    else:
+        state = table.view(-1)[1:1 + S * C].view(S, C)
+    before = table.clone()
+    ids = torch.tensor([3, 1], dtype=torch.int32)
+    d_ref, s_ref = oracle.token_shift_diff(x.float().numpy(), state.float().cpu().numpy(), ids.numpy())
+    out = pkg.token_shift_diff_custom(x.to(cuda), state, ids.to(cuda))
+    torch.cuda.synchronize()
+    _check(out.token_shifted_diff, d_ref.astype(np.float64), dtype)
+    assert torch.equal(out.next_token_shift.float().cpu(), torch.from_numpy(s_ref)) and torch.equal(table, before)
+    with pytest.raises(pkg.KernelInputsError):
+        pkg.token_shift_diff_custom(x.to(cuda), state, ids.to(cuda), inplace_state=True)
