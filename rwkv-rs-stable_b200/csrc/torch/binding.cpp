@@ -88,9 +88,12 @@ struct Desc {
     rwkv7_tensor *p = nullptr;
     Desc() = default;
     explicit Desc(const at::Tensor &t) { set(t); }
-    explicit Desc(PyObject *o) { if (o != Py_None) set(tensor(o)); }
+    explicit Desc(PyObject *o) { set(o); }
     Desc(const Desc &) = delete;
     Desc &operator=(const Desc &) = delete;
+    void set(PyObject *o) {   // (None: the library says which tensor is missing)
+        if (o != Py_None) set(tensor(o));
+    }
     void set(const at::Tensor &t) {
         const int32_t dt = dtype_code(t.scalar_type());
         if (dt < 0) {
@@ -226,7 +229,7 @@ bool truth(PyObject *o) {
 //   -> (output, next_state|None)
 PyObject *wkv7(PyObject *const *a) {
     Desc s0(a[0]), six[6];
-    for (int i = 0; i < 6; ++i) six[i].set(tensor(a[1 + i]));
+    for (int i = 0; i < 6; ++i) six[i].set(a[1 + i]);
     const at::Tensor &r = tensor(a[1]);
     const int64_t chunk_len = integer(a[7]);
     const bool has_state = a[0] != Py_None, want_state = has_state && truth(a[8]);
@@ -259,7 +262,7 @@ PyObject *wkv7(PyObject *const *a) {
 // wkv7_noalloc(initial_state, r, w, k, v, a, b, chunk_len, output, next_state)
 PyObject *wkv7_noalloc(PyObject *const *a) {
     Desc s0(a[0]), six[6];
-    for (int i = 0; i < 6; ++i) six[i].set(tensor(a[1 + i]));
+    for (int i = 0; i < 6; ++i) six[i].set(a[1 + i]);
     const int64_t chunk_len = integer(a[7]);
     Desc yd(a[8]), sd(a[9]);
     const rwkv7_stream st = stream_of(tensor(a[1]));
@@ -274,7 +277,7 @@ PyObject *wkv7_noalloc(PyObject *const *a) {
 //   -> (output, next_state|None, snapshots, state_replacement)
 PyObject *wkv7_saved(PyObject *const *a) {
     Desc s0(a[0]), six[6];
-    for (int i = 0; i < 6; ++i) six[i].set(tensor(a[1 + i]));
+    for (int i = 0; i < 6; ++i) six[i].set(a[1 + i]);
     const at::Tensor &r = tensor(a[1]);
     if (r.dim() != 4) raise(PyExc_ValueError, "not enough values to unpack (expected 4)");
     const int64_t B = r.size(0), T = r.size(1), H = r.size(2), N = r.size(3), chunk_len = integer(a[7]);
@@ -297,7 +300,7 @@ PyObject *wkv7_saved(PyObject *const *a) {
 //               next_state_grad|None, want_state_grad, parallel, workspace|None) -> (six gradients, state gradient|None)
 PyObject *wkv7_backward(PyObject *const *a) {
     Desc s0(a[0]), six[6], snap(a[7]), sa(a[8]);
-    for (int i = 0; i < 6; ++i) six[i].set(tensor(a[1 + i]));
+    for (int i = 0; i < 6; ++i) six[i].set(a[1 + i]);
     const at::Tensor &r = tensor(a[1]);
     if (r.dim() != 4) raise(PyExc_ValueError, "not enough values to unpack (expected 4)");
     const int64_t B = r.size(0), T = r.size(1), H = r.size(2), N = r.size(3), chunk_len = integer(a[9]);
@@ -427,7 +430,7 @@ PyObject *mix6(PyObject *const *a) {
     const rwkv7_tensor *sp[6];
     rwkv7_tensor *op[6];
     for (int i = 0; i < 6; ++i) {
-        sd[i].set(tensor(a[1 + i]));
+        sd[i].set(a[1 + i]);
         sp[i] = sd[i].p;
         od[i].set(out[i]);
         op[i] = od[i].p;
@@ -443,7 +446,7 @@ PyObject *mix6_stacked(PyObject *const *a) {
     Desc xd(x), sd[6];
     const rwkv7_tensor *sp[6];
     for (int i = 0; i < 6; ++i) {
-        sd[i].set(tensor(a[1 + i]));
+        sd[i].set(a[1 + i]);
         sp[i] = sd[i].p;
     }
     std::vector<int64_t> shape{6};
@@ -459,7 +462,7 @@ PyObject *mix6_stacked(PyObject *const *a) {
 PyObject *addcmul(PyObject *const *a) {
     const at::Tensor &base = tensor(a[0]);
     const bool inplace = truth(a[3]);
-    Desc bd(base), dd(tensor(a[1])), sd(tensor(a[2]));
+    Desc bd(base), dd(a[1]), sd(a[2]);
     const at::Tensor out = inplace ? base : like(base);
     Desc od(out);
     const rwkv7_stream st = stream_of(base);
@@ -470,13 +473,13 @@ PyObject *addcmul(PyObject *const *a) {
 // addcmul5(base, diff, five scales) -> five outputs
 PyObject *addcmul5(PyObject *const *a) {
     const at::Tensor &base = tensor(a[0]);
-    Desc bd(base), dd(tensor(a[1])), sd[5], od[5];
+    Desc bd(base), dd(a[1]), sd[5], od[5];
     at::Tensor out[5];
     outputs_like(out, base, base, base, base, base);
     const rwkv7_tensor *sp[5];
     rwkv7_tensor *op[5];
     for (int i = 0; i < 5; ++i) {
-        sd[i].set(tensor(a[2 + i]));
+        sd[i].set(a[2 + i]);
         sp[i] = sd[i].p;
         od[i].set(out[i]);
         op[i] = od[i].p;
@@ -499,7 +502,7 @@ PyObject *token_shift_diff(PyObject *const *a) {
     at::Tensor out[2];   // diff, next state
     if (inplace) out[0] = like(x);
     else outputs_like(out, x, state);
-    Desc xd(x), sd(state), idd(tensor(a[2])), dd(out[0]), nd;
+    Desc xd(x), sd(state), idd(a[2]), dd(out[0]), nd;
     if (!inplace) nd.set(out[1]);
     const rwkv7_stream st = stream_of(x);
     call([&] {
@@ -515,8 +518,7 @@ PyObject *token_shift_diff(PyObject *const *a) {
 PyObject *weight_prepare(PyObject *const *a) {
     const at::Tensor &key = tensor(a[0]);
     Desc in[8], od[5];
-    for (int i = 0; i < 8; ++i)
-        if (a[i] != Py_None) in[i].set(tensor(a[i]));
+    for (int i = 0; i < 8; ++i) in[i].set(a[i]);
     at::Tensor out[5];
     if (a[5] == Py_None) outputs_like(out, key, key, key, key);   // (no value inputs: no value output)
     else outputs_like(out, key, key, key, key, key);
@@ -535,7 +537,7 @@ PyObject *weight_prepare(PyObject *const *a) {
 PyObject *gated_readout(PyObject *const *a) {
     const at::Tensor &y = tensor(a[0]);
     Desc in[8];
-    for (int i = 0; i < 8; ++i) in[i].set(tensor(a[i]));
+    for (int i = 0; i < 8; ++i) in[i].set(a[i]);
     const int64_t heads = integer(a[8]);
     const double eps = PyFloat_AsDouble(a[9]);
     if (eps == -1.0 && PyErr_Occurred()) throw PythonError{};
@@ -552,7 +554,7 @@ PyObject *gated_readout(PyObject *const *a) {
 // channel_mixer(x, key_scale, key_weight, value_weight, workspace|None) -> output
 PyObject *channel_mixer(PyObject *const *a) {
     const at::Tensor &x = tensor(a[0]), &kw = tensor(a[2]);
-    Desc xd(x), sd(tensor(a[1])), kd(kw), vd(tensor(a[3]));
+    Desc xd(x), sd(a[1]), kd(kw), vd(a[3]);
     const at::Tensor out = like(x);
     Desc od(out);
     Workspace ws;
@@ -565,7 +567,7 @@ PyObject *channel_mixer(PyObject *const *a) {
     return wrap(out);
 }
 
-at::Tensor lm_head_partial_of(const at::Tensor &x, const at::Tensor &w, const at::Tensor &targets, int64_t offset) {
+at::Tensor lm_head_partial_of(const at::Tensor &x, const at::Tensor &w, PyObject *targets, int64_t offset) {
     if (x.dim() < 2 || w.dim() < 1) raise(PyExc_IndexError, "tuple index out of range");
     const at::Tensor partials = empty({x.size(0), 3}, at::kFloat, x);
     Workspace ws;
@@ -577,7 +579,7 @@ at::Tensor lm_head_partial_of(const at::Tensor &x, const at::Tensor &w, const at
     return partials;
 }
 
-PyObject *lm_head_finalize_of(const at::Tensor &partials_all, const at::Tensor &targets) {
+PyObject *lm_head_finalize_of(const at::Tensor &partials_all, PyObject *targets) {
     if (partials_all.dim() < 2) raise(PyExc_IndexError, "tuple index out of range");
     const int64_t R = partials_all.size(1);
     const at::Tensor out[2] = {empty({R}, at::kFloat, partials_all), empty({R}, at::kFloat, partials_all)};
@@ -589,14 +591,14 @@ PyObject *lm_head_finalize_of(const at::Tensor &partials_all, const at::Tensor &
 
 // lm_head_ce_partial(x, weight_shard, targets, vocab_offset) -> partials
 PyObject *lm_head_ce_partial(PyObject *const *a) {
-    return wrap(lm_head_partial_of(tensor(a[0]), tensor(a[1]), tensor(a[2]), integer(a[3])));
+    return wrap(lm_head_partial_of(tensor(a[0]), tensor(a[1]), a[2], integer(a[3])));
 }
 // lm_head_ce_finalize(partials_all, targets) -> (lse, loss)
-PyObject *lm_head_ce_finalize(PyObject *const *a) { return lm_head_finalize_of(tensor(a[0]), tensor(a[1])); }
+PyObject *lm_head_ce_finalize(PyObject *const *a) { return lm_head_finalize_of(tensor(a[0]), a[1]); }
 // lm_head_ce(x, weight, targets) -> (lse, loss)
 PyObject *lm_head_ce(PyObject *const *a) {
-    const at::Tensor p = lm_head_partial_of(tensor(a[0]), tensor(a[1]), tensor(a[2]), 0);
-    return lm_head_finalize_of(p.unsqueeze(0), tensor(a[2]));
+    const at::Tensor p = lm_head_partial_of(tensor(a[0]), tensor(a[1]), a[2], 0);
+    return lm_head_finalize_of(p.unsqueeze(0), a[2]);
 }
 
 // ---- module ---------------------------------------------------------------------------------------

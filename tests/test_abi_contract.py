@@ -251,3 +251,27 @@ def test_host_statepass_contract(pkg):
     on_device = [pkg.describe(t, device=0) for t in six]
     dev_arr = (ctypes.POINTER(pkg.Tensor) * 6)(*[ctypes.pointer(d) for d in on_device])
     assert L.rwkv7_status_string(call(2, 1 << 30, dev_arr)) == b"DeviceMismatch"
+
+
+def test_a_missing_tensor_is_named(pkg):
+    """None where an operator needs a tensor is the contract's NullPointer, with the tensor's name."""
+    x, c, ids = torch.zeros(1, 16, 8), torch.zeros(1, 1, 8), torch.zeros(1, dtype=torch.int32)
+    seq = _seq(pkg, (1, 16, 1, 8))
+    seq.value = None
+    w = torch.zeros(8, 64, dtype=torch.bfloat16)
+    calls = [
+        ("value", lambda: pkg.wkv7_pretrain_custom(seq)),
+        ("key_scale", lambda: pkg.mix6_custom(x, c, c, None, c, c, c)),
+        ("gate_scale", lambda: pkg.mix6_custom(x, c, c, c, c, c, None, stacked=True)),
+        ("diff", lambda: pkg.addcmul_custom(x, None, c)),
+        ("value_scale", lambda: pkg.addcmul5_custom(x, x, c, c, c, None, c)),
+        ("batch_ids", lambda: pkg.token_shift_diff_custom(x, torch.zeros(2, 8), None)),
+        ("learning_rate_lora", lambda: pkg.weight_prepare_epilogue(x, None, x, c, c, 1)),
+        ("group_norm_gamma", lambda: pkg.gated_readout_epilogue(x, x, x, x, x, None, c, c, 1)),
+        ("value_weight", lambda: pkg.channel_mixer_custom(x, torch.zeros(8), torch.zeros(32, 8), None)),
+        ("targets", lambda: pkg.lm_head_ce(torch.zeros(2, 64, dtype=torch.bfloat16), w, None)),
+    ]
+    for name, call in calls:
+        with pytest.raises(pkg.KernelInputsError) as e:
+            call()
+        assert e.value.kind == "NullPointer" and name in str(e.value), (name, str(e.value))
