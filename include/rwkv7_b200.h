@@ -490,7 +490,9 @@ int rwkv7_fused_gated_readout(const rwkv7_tensor *wkv7_output, const rwkv7_tenso
  * Both projections run on the tensor cores in BF16 with fp32 accumulation; the
  * activation is part of the first projection's epilogue.  BF16 tensors only (F32 returns
  * RWKV7_ERR_UNSUPPORTED); C and F must be multiples of 8.  The workspace holds key_input
- * and the activated hidden tensor: rwkv7_channel_mixer_workspace_bytes(B, T, C, F).
+ * and the activated hidden tensor (B*T*C and B*T*F elements, each rounded up to 256 bytes) and, for few rows, partial
+ * sums of the projections: rwkv7_channel_mixer_workspace_bytes(B, T, C, F).  Without room for the partial sums the call
+ * takes fewer of them, or none.
  */
 size_t rwkv7_channel_mixer_workspace_bytes(int64_t B, int64_t T, int64_t C, int64_t F);
 

@@ -1157,7 +1157,7 @@ int rwkv7_fused_channel_mixer(const rwkv7_tensor *x_t, const rwkv7_tensor *scale
     for (const void *ptr : {p.x, p.key_scale, p.key_weight, p.value_weight, (const void *)p.out, (const void *)workspace})
         if (reinterpret_cast<uintptr_t>(ptr) & 15u)
             return fail(RWKV7_ERR_BAD_ARGUMENT, "BadArgument: channel_mixer tensors and workspace must be 16-byte aligned");
-    const size_t need = channel_mixer_workspace_bytes(p.B * p.T, p.C, p.F);
+    const size_t need = channel_mixer_min_workspace_bytes(p.B * p.T, p.C, p.F);
     if (workspace == nullptr) return fail(RWKV7_ERR_NULL_POINTER, "NullPointer: channel_mixer needs a workspace of %zu bytes", need);
     if (workspace_bytes < need)
         return fail(RWKV7_ERR_WORKSPACE_TOO_SMALL, "WorkspaceTooSmall: channel_mixer needs %zu workspace bytes, got %zu", need,

@@ -294,13 +294,18 @@ int encode_rows_by_k(EncodeTiledFn encode, CUtensorMap *map, const void *base, i
 // tiles, 8 of them for 2048 columns) most of the device would idle while a few SMs stream the whole weight matrix, so K is
 // cut until every SM has an item, in pieces of at least four K steps, and a second kernel adds the fp32 sums up.  Measured
 // (B200, C = 2048, F = 8192): one row 91 -> 36 us, 64 rows at C = 4096 172 -> 78 us.
+// (At most 18, the 148 SMs over the 8 tiles of 2048 columns: a bound on the partial sums of narrower products, whose K is short
+// enough at the widths in use that the four K steps of a piece bind first.)
+// `room`: bytes for the sums; with less than the pieces take there are fewer of them.
 constexpr int kMaxGemmSplits = 18;
-int gemm_splits(int64_t M, int64_t N, int64_t K, int num_sms) {
+int gemm_splits(int64_t M, int64_t N, int64_t K, int num_sms, size_t room) {
     const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN), ksteps = (K + kBK - 1) / kBK;
     if (2 * tiles > num_sms) return 1;
     int64_t sp = num_sms / tiles;
     if (sp > ksteps / 4) sp = ksteps / 4;
     if (sp > kMaxGemmSplits) sp = kMaxGemmSplits;
+    const int64_t fit = (int64_t)(room / ((size_t)M * N * sizeof(float)));
+    if (sp > fit) sp = fit;
     if (sp < 2) return 1;
     const int64_t per = (ksteps + sp - 1) / sp;
     return (int)((ksteps + per - 1) / per);   // (no piece is empty)
@@ -308,7 +313,7 @@ int gemm_splits(int64_t M, int64_t N, int64_t K, int num_sms) {
 // fp32 partial sums of any device up to this many SMs.
 constexpr int kMostSms = 160;
 size_t gemm_partial_bytes(int64_t M, int64_t N, int64_t K) {
-    const int sp = gemm_splits(M, N, K, kMostSms);
+    const int sp = gemm_splits(M, N, K, kMostSms, SIZE_MAX);
     return sp > 1 ? (size_t)sp * M * N * sizeof(float) : 0;
 }
 
@@ -331,7 +336,7 @@ cudaError_t launch_serialized(void (*kernel)(Params...), unsigned grid, unsigned
 
 // out[M,N] = act(A[M,K] . B[N,K]^T); K and N multiples of 8, all pointers 16-byte aligned.
 template <int EPI>
-int launch_gemm(const void *a, const void *b, void *out, float *partials, int64_t M, int64_t N, int64_t K, int num_sms,
+int launch_gemm(const void *a, const void *b, void *out, float *partials, size_t room, int64_t M, int64_t N, int64_t K, int num_sms,
                 int *status, cudaStream_t stream) {
     EncodeTiledFn encode = gemm_encode_fn();
     if (encode == nullptr) return (int)cudaErrorNotSupported;
@@ -339,7 +344,7 @@ int launch_gemm(const void *a, const void *b, void *out, float *partials, int64_
     if (int e = encode_rows_by_k(encode, &maps.a, a, M, K, kBM)) return e;
     if (int e = encode_rows_by_k(encode, &maps.b, b, N, K, kBN)) return e;
     const int m_tiles = (int)((M + kBM - 1) / kBM), n_tiles = (int)((N + kBN - 1) / kBN);
-    const int tiles = m_tiles * n_tiles, splits = gemm_splits(M, N, K, num_sms < kMostSms ? num_sms : kMostSms);
+    const int tiles = m_tiles * n_tiles, splits = gemm_splits(M, N, K, num_sms < kMostSms ? num_sms : kMostSms, room);
     const int items = tiles * splits;
     const unsigned grid = (unsigned)(items < num_sms ? items : num_sms);
     auto kernel = splits > 1 ? gemm_tn_bf16_kernel<kEpiPartial> : gemm_tn_bf16_kernel<EPI>;
@@ -357,20 +362,28 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace
 
+// key_input and hidden; the partial sums behind them take what room there is (a workspace laid out for the largest batch serves a
+// smaller one, which may cut K into more pieces).
+size_t channel_mixer_min_workspace_bytes(int64_t rows, int64_t C, int64_t F) {
+    if (rows <= 0 || C <= 0 || F <= 0) return 0;
+    return align256((size_t)rows * C * 2) + align256((size_t)rows * F * 2);
+}
+
 size_t channel_mixer_workspace_bytes(int64_t rows, int64_t C, int64_t F) {
     if (rows <= 0 || C <= 0 || F <= 0) return 0;
     const size_t p1 = gemm_partial_bytes(rows, F, C), p2 = gemm_partial_bytes(rows, C, F);
-    return align256((size_t)rows * C * 2) + align256((size_t)rows * F * 2) + align256(p1 > p2 ? p1 : p2);   // key_input, hidden, partial sums
+    return channel_mixer_min_workspace_bytes(rows, C, F) + align256(p1 > p2 ? p1 : p2);
 }
 
 int launch_channel_mixer(const ChannelMixerArgs &p, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
     const int64_t rows = p.B * p.T;
     if (rows == 0) return 0;
-    if (workspace_bytes < channel_mixer_workspace_bytes(rows, p.C, p.F)) return (int)cudaErrorInvalidValue;
+    if (workspace_bytes < channel_mixer_min_workspace_bytes(rows, p.C, p.F)) return (int)cudaErrorInvalidValue;
     __nv_bfloat16 *key_input = static_cast<__nv_bfloat16 *>(workspace);
     __nv_bfloat16 *hidden = reinterpret_cast<__nv_bfloat16 *>(static_cast<unsigned char *>(workspace) +
                                                               align256((size_t)rows * p.C * 2));
-    float *partials = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(hidden) + align256((size_t)rows * p.F * 2));
+    const size_t least = channel_mixer_min_workspace_bytes(rows, p.C, p.F), room = workspace_bytes - least;
+    float *partials = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + least);
     int threads = 32;
     while (threads < 256 && threads < p.C / 8) threads <<= 1;
     const int per_block = rows >= 2 * kMixRows * (int64_t)p.num_sms ? kMixRows : 2;
@@ -378,9 +391,9 @@ int launch_channel_mixer(const ChannelMixerArgs &p, void *workspace, size_t work
         (const __nv_bfloat16 *)p.x, (const __nv_bfloat16 *)p.key_scale, key_input, rows, p.T, p.C, per_block);
     count_launch();
     if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return (int)e;
-    if (int e = launch_gemm<kEpiReluSquare>(key_input, p.key_weight, hidden, partials, rows, p.F, p.C, p.num_sms, p.status, stream))
+    if (int e = launch_gemm<kEpiReluSquare>(key_input, p.key_weight, hidden, partials, room, rows, p.F, p.C, p.num_sms, p.status, stream))
         return e;
-    return launch_gemm<kEpiNone>(hidden, p.value_weight, p.out, partials, rows, p.C, p.F, p.num_sms, p.status, stream);
+    return launch_gemm<kEpiNone>(hidden, p.value_weight, p.out, partials, room, rows, p.C, p.F, p.num_sms, p.status, stream);
 }
 
 }  // namespace rwkv7

@@ -183,6 +183,7 @@ struct ChannelMixerArgs {
     int num_sms;
 };
 size_t channel_mixer_workspace_bytes(int64_t rows, int64_t C, int64_t F);
+size_t channel_mixer_min_workspace_bytes(int64_t rows, int64_t C, int64_t F);
 int launch_channel_mixer(const ChannelMixerArgs &p, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 
 struct TokenShiftArgs {

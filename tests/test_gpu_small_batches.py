@@ -36,3 +36,25 @@ def test_lm_head_with_many_splits(pkg, oracle, workloads, cuda, R, C, V):
     assert pkg.read_device_status(0) == 0
     np.testing.assert_allclose(lse.cpu().numpy(), lse_ref, rtol=0, atol=2e-4)
     np.testing.assert_allclose(loss.cpu().numpy(), loss_ref, rtol=0, atol=2e-4)
+
+
+@pytest.mark.parametrize("rows,room", [(1, "least"), (128, "least"), (128, 200), (128, 129)])
+def test_channel_mixer_takes_a_workspace_for_another_batch(pkg, workloads, cuda, rows, room):
+    """Room for key_input and hidden alone (no partial sums), or what a larger batch asks for (whose products are cut
+    into fewer pieces of K): the same call with fewer pieces, within a rounding of the hidden tensor and one of the output."""
+    C, F = 2048, 8192
+    x, ks, kw, vw = (t.to(cuda) for t in workloads.channel_mixer_inputs(1, rows, C, F, seed=23))
+    L = pkg.lib()
+    least = sum((rows * n * 2 + 255) // 256 * 256 for n in (C, F))
+    nbytes = least if room == "least" else L.rwkv7_channel_mixer_workspace_bytes(1, room, C, F)
+    assert least <= nbytes < L.rwkv7_channel_mixer_workspace_bytes(1, rows, C, F)
+    ws = torch.empty(nbytes + 4096, dtype=torch.uint8, device=cuda)
+    ws[nbytes:] = 77
+    got = pkg.channel_mixer_custom(x, ks, kw, vw, workspace=ws[:nbytes])
+    want = pkg.channel_mixer_custom(x, ks, kw, vw)
+    torch.cuda.synchronize()
+    assert pkg.read_device_status(0) == 0 and (ws[nbytes:] == 77).all()
+    got, want = got.float(), want.float()
+    assert ((got - want).abs() <= 2e-3 * want.abs().max() + 2 * parity.BF16_ULP * want.abs()).all()
+    with pytest.raises(pkg.KernelInputsError):
+        pkg.channel_mixer_custom(x, ks, kw, vw, workspace=ws[:least - 256])
