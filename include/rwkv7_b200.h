@@ -512,7 +512,9 @@ int rwkv7_fused_channel_mixer(const rwkv7_tensor *embedded_context, const rwkv7_
  *   row_target = z[target - vocab_offset] if the target falls in the shard else 0.
  * Logits are never written to memory.  targets [R] are I32 or I64; a negative
  * target marks an ignored row.  L2Wrap is a backward-only regulariser and is the
- * identity here.  partials is [R,3] F32 (max, sumexp, target logit).
+ * identity here.  partials is [R,3] F32 (max, sumexp, target logit).  With a workspace smaller than
+ * rwkv7_lm_head_ce_workspace_bytes, down to 16 triples per row (one per 256 columns if V_shard has fewer), the call takes fewer
+ * vocabulary splits.
  */
 size_t rwkv7_lm_head_ce_workspace_bytes(int64_t R, int64_t C, int64_t V_shard);
 

@@ -1211,7 +1211,7 @@ int rwkv7_fused_lm_head_ce_partial(const rwkv7_tensor *x_t, const rwkv7_tensor *
     if (p.R == 0) return RWKV7_OK;
     if (p.C % 64 != 0)
         return fail(RWKV7_ERR_UNSUPPORTED, "Unsupported: lm_head_ce needs C %% 64 == 0 (got C=%lld)", (long long)p.C);
-    const size_t need = lm_head_ce_workspace_bytes(p.R, p.C, p.V);
+    const size_t need = lm_head_ce_min_workspace_bytes(p.R, p.C, p.V);
     if (need > 0 && (workspace == nullptr || workspace_bytes < need))
         return fail(RWKV7_ERR_WORKSPACE_TOO_SMALL, "WorkspaceTooSmall: lm_head_ce needs %zu workspace bytes, got %zu",
                     need, workspace == nullptr ? (size_t)0 : workspace_bytes);

@@ -213,6 +213,7 @@ struct LmHeadArgs {
     int *status;
 };
 size_t lm_head_ce_workspace_bytes(int64_t R, int64_t C, int64_t V);
+size_t lm_head_ce_min_workspace_bytes(int64_t R, int64_t C, int64_t V);
 int launch_lm_head_ce_partial(const LmHeadArgs &p, void *workspace, size_t workspace_bytes,
                               cudaStream_t stream);
 int launch_lm_head_ce_finalize(const float *partials_all, int num_shards, const void *targets,

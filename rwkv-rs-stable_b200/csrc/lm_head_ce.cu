@@ -249,17 +249,23 @@ EncodeTiledFn lm_encode_fn() {
 // Most splits per row block: 16, and with few row blocks as many as give every SM of a large device a CTA of its own
 // (a call of up to 128 rows is one row block: with 16 splits, 16 SMs read the whole weight matrix: 188 us for 16 rows
 // at C = 2048, V = 65 536, against 73).
+constexpr int kFewSplits = 16;
 int max_splits(int64_t R) {
     const int64_t rbs = (R + kBM - 1) / kBM, fill = rbs > 0 ? 160 / rbs : 160;
-    return (int)(fill > 16 ? fill : 16);
+    return (int)(fill > kFewSplits ? fill : kFewSplits);
 }
-void plan(int64_t R, int64_t V, int num_sms, int *row_blocks, int *splits, int *tiles_per_split) {
+size_t split_bytes(int64_t R, int64_t V, int most) {
+    const int64_t tiles = (V + kBN - 1) / kBN, sp = tiles < most ? tiles : most;
+    return sp > 1 ? (size_t)sp * (size_t)R * 3 * sizeof(float) : 0;
+}
+// `most`: splits that the workspace has room for.
+void plan(int64_t R, int64_t V, int num_sms, int64_t most, int *row_blocks, int *splits, int *tiles_per_split) {
     const int rbs = (int)((R + kBM - 1) / kBM);
     const int tiles = (int)((V + kBN - 1) / kBN);
     const int sms = num_sms > 0 ? num_sms : 1;
     int best_sp = 1, best_tps = tiles;
     double best_cost = 0.0;
-    for (int want = 1; want <= max_splits(R) && want <= tiles; ++want) {
+    for (int want = 1; want <= max_splits(R) && want <= tiles && want <= most; ++want) {
         const int tps = (tiles + want - 1) / want;
         const int sp = (tiles + tps - 1) / tps;
         const long long ctas = (long long)rbs * sp;
@@ -278,12 +284,15 @@ void plan(int64_t R, int64_t V, int num_sms, int *row_blocks, int *splits, int *
 
 }  // namespace
 
+// Upper bound for any device: one triple per row per vocabulary split, at most max_splits of them.  (Fewer rows may have more
+// splits: a workspace laid out for the largest batch serves a smaller one with as many as it has room for.)
 size_t lm_head_ce_workspace_bytes(int64_t R, int64_t C, int64_t V) {
     (void)C;
-    // Upper bound for any device: one triple per row per vocabulary split, at most max_splits of them.
-    const int64_t tiles = (V + kBN - 1) / kBN, most = max_splits(R);
-    const int64_t sp = tiles < most ? tiles : most;
-    return sp > 1 ? (size_t)sp * (size_t)R * 3 * sizeof(float) : 0;
+    return split_bytes(R, V, max_splits(R));
+}
+size_t lm_head_ce_min_workspace_bytes(int64_t R, int64_t C, int64_t V) {
+    (void)C;
+    return split_bytes(R, V, kFewSplits);
 }
 
 int launch_lm_head_ce_partial(const LmHeadArgs &p, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
@@ -312,9 +321,9 @@ int launch_lm_head_ce_partial(const LmHeadArgs &p, void *workspace, size_t works
             return (int)cudaErrorInvalidValue;
     }
     int row_blocks, splits, tps;
-    plan(p.R, p.V, p.num_sms, &row_blocks, &splits, &tps);
+    const int64_t room = workspace == nullptr ? 1 : (int64_t)(workspace_bytes / ((size_t)p.R * 3 * sizeof(float)));
+    plan(p.R, p.V, p.num_sms, room > 1 ? room : 1, &row_blocks, &splits, &tps);
     float *parts = splits == 1 ? p.partials : static_cast<float *>(workspace);
-    if (splits > 1 && workspace_bytes < (size_t)splits * p.R * 3 * sizeof(float)) return (int)cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(lm_head_ce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     lm_head_ce_kernel<<<(unsigned)(row_blocks * splits), kThreads, kSmemBytes, stream>>>(

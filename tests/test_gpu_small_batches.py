@@ -58,3 +58,26 @@ def test_channel_mixer_takes_a_workspace_for_another_batch(pkg, workloads, cuda,
     assert ((got - want).abs() <= 2e-3 * want.abs().max() + 2 * parity.BF16_ULP * want.abs()).all()
     with pytest.raises(pkg.KernelInputsError):
         pkg.channel_mixer_custom(x, ks, kw, vw, workspace=ws[:least - 256])
+
+
+@pytest.mark.parametrize("rows,room", [(1, None), (128, None), (128, 129), (128, 200)])
+def test_lm_head_takes_a_workspace_for_another_batch(pkg, workloads, cuda, rows, room):
+    """16 triples per row, or what a larger batch asks for: fewer vocabulary splits, the same sums to fp32 rounding."""
+    import ctypes
+    C, V = 128, 65536
+    x, w, tg = (t.to(cuda) for t in workloads.lm_head_inputs(rows, C, V, seed=29))
+    L = pkg.lib()
+    nbytes = 16 * rows * 12 if room is None else L.rwkv7_lm_head_ce_workspace_bytes(room, C, V)
+    assert nbytes < L.rwkv7_lm_head_ce_workspace_bytes(rows, C, V)
+    want = pkg.lm_head_ce_partial(x, w, tg)
+    got = torch.empty_like(want)
+    ws = torch.full((nbytes + 4096,), 77, dtype=torch.uint8, device=cuda)
+    d = [pkg.describe(t) for t in (x, w, tg, got)]
+    call = lambda n: L.rwkv7_fused_lm_head_ce_partial(  # noqa: E731
+        *[ctypes.byref(t) for t in d[:3]], ctypes.c_int64(0), ctypes.byref(d[3]), ctypes.c_void_p(ws.data_ptr()), ctypes.c_size_t(n),
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert call(nbytes) == 0
+    torch.cuda.synchronize()
+    assert pkg.read_device_status(0) == 0 and (ws[nbytes:] == 77).all()
+    torch.testing.assert_close(got, want, rtol=1e-5, atol=0)     # 256 sums of 256 terms in fp32
+    assert L.rwkv7_status_string(call(16 * rows * 12 - 4)) == b"WorkspaceTooSmall"
