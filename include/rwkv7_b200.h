@@ -95,8 +95,8 @@ typedef struct rwkv7_tensor {
  * chain) from 64 tokens (BF16) or 512 (F32) on when the workspace holds at least one chunk of operators per chain;
  * for BF16 tensors otherwise the fused tf32 chunked kernel (CHUNKED) from 64 tokens on; the sequential kernel for everything else
  * (F32 tensors under 512 tokens, other head sizes).  Chains that the fp16 operators of SPLIT cannot resolve (a
- * log-decay beyond 12 in 16 tokens in some channel; beyond 18 in 64 tokens when the path is selected explicitly) are
- * recomputed by CHUNKED (BF16 tensors), and chains beyond its range (80), or flagged chains of F32 tensors, by
+ * log-decay beyond 12 in 16 tokens in some channel; beyond 18 in 64 tokens for F32 tensors and when the path is selected
+ * explicitly) are recomputed by CHUNKED (BF16 tensors), and chains beyond its range (80), or flagged chains of F32 tensors, by
  * SEQUENTIAL, inside the same call; under 512 tokens, and where a value overflows fp16, token by token by the scan; a final
  * state that aliases the initial state is only written once a chain's result is final. */
 typedef enum rwkv7_wkv7_path {

@@ -172,7 +172,9 @@ int wkv7_dispatch(Wkv7Args &p, void *workspace, size_t workspace_bytes, rwkv7_st
     }
     if (path == RWKV7_WKV7_SPLIT || (path == RWKV7_WKV7_AUTO && split_fits && p.T >= split_min_tokens(p.bf16))) {
         const bool own_tier = path == RWKV7_WKV7_AUTO && p.T < kSplitTiersTokens;
-        if (int e = launch_wkv7_split(p, workspace, workspace_bytes, path == RWKV7_WKV7_AUTO, own_tier, (cudaStream_t)stream))
+        // (fp32 tensors keep the narrow range: a chain beyond it is computed in fp32 by the sequential scan, error 6e-7 over 1000 tokens
+        // with a model's decays; fp16 operands would resolve it, but to 5e-4)
+        if (int e = launch_wkv7_split(p, workspace, workspace_bytes, path == RWKV7_WKV7_AUTO && p.bf16, own_tier, (cudaStream_t)stream))
             return cuda_fail("wkv7 split launch", e);
         if (own_tier) return RWKV7_OK;
         // (the tf32 chunked kernel reads bf16 tiles: flagged chains of fp32 tensors go straight to the sequential scan)
