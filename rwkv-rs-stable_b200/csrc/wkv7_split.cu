@@ -21,6 +21,9 @@
 // matrix instructions (see sm100_mma.cuh for why not tcgen05).  fp16 has a narrow exponent range, and the factors of the
 // four A matrices, e^{c_t} and e^{-c_s}, do not.  A chunk whose decay exceeds what the references below resolve is marked
 // and its chain flagged; non-finite values (keys or values beyond fp16) are detected in the scan.
+// Small values do not lose bits below fp16's normal numbers: r and k rows go in times a power of two where a 16-token block of
+// them stays below 2 (the factor comes out again in the scan), and the scan scales V and the state likewise per chunk.
+// Without, values of 1e-5 came out with an error of 1.1e-2 (tf32 operands: 1.7e-3, the rounding of y to bf16).
 //
 // References.  The factor e^{c_t - c_s} of an A matrix is split between its two operands at a reference point, per
 // channel, chosen as e^{c_L} times a power of two.  Then
@@ -65,17 +68,6 @@ constexpr int kWideShift = 6;                 // block-wise references: operands
 constexpr float kWideScale = 64.f;            // factors reach down to e^-12 and a typical entry has to stay a normal number
 __host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
 
-// What the builder leaves of a chunk in global memory: the 128 x 128 fp16 operator O[n][k], n = (j' | t), as the core
-// matrices (eight rows n, eight k, 128 bytes) of a K-major tcgen05 operand without swizzle, 16 of them along k and 16 along n.
-// The contraction index (64 j, then 64 s) is ordered so that a lane of the builder holds four neighbouring k of a row in its
-// accumulators: the eight of core 4 c + q are {2q, 2q+1, 2q+8, 2q+9} of the 16-block 2 c, then the same of 2 c + 1.  Behind
-// the operator e^{c_L}[64] in fp32, two signed exponents per channel (fx = e^{c_L} 2^ef; P and Kt are stored times 2^eg), and
-// the mark.
-constexpr uint32_t kOperatorBytes = 4 * kPanel;
-constexpr uint32_t kDecayAt = kOperatorBytes, kExpAt = kDecayAt + 256;
-constexpr uint32_t kVectorBytes = 256 + 128;
-constexpr uint32_t kMarkAt = kDecayAt + kVectorBytes;   // int: the chunk is beyond what fp16 operands resolve
-constexpr size_t kRecord = 33280;                        // bytes per chunk in the workspace
 // ------------------------------------------------------------------------------------------
 // Kernel 1: the operator of every chunk.  One CTA of four warps per chunk at a time, four CTAs per SM.
 //
@@ -267,7 +259,12 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
 #pragma unroll
                     for (int x = 0; x < 4; ++x) sts32(sb + kTiles + x * kPanel + off16(16 * tb + u, ch), 0u);
         }
+        auto note = [&](int er, int ek) {
+            if (lane == 0 && RWKV7_IN_RANGE(unit >= 0 && unit < units, status))
+                *reinterpret_cast<char2 *>(record + kDecayAt + kRowExpAt + 2 * tb) = make_char2((signed char)er, (signed char)ek);
+        };
         if (over) {   // the chain is recomputed elsewhere: nothing more to do for this chunk
+            note(0, 0);   // (read by the kernel of the chunk gradients, whose range may differ by a rounding)
             if (kTma) fence_proxy_async();
             __syncthreads();   // (everyone has read the decays)
             if (kTma && tid == 0 && more) request(unit + gridDim.x);
@@ -313,8 +310,39 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                 *reinterpret_cast<char2 *>(record + kExpAt + 64 + ch) = make_char2((signed char)eg[0], (signed char)eg[1]);
             }
             Raw v0[16], v1[16];
+            // Rows of small values (largest magnitude below 2) times the power of two that brings it to [2, 4); its exponent.
+            auto raise_small = [&](Raw (&v)[16]) -> int {
+                uint32_t bits = 0u;   // (a magnitude of 2 and above has the top bit of its exponent)
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    if constexpr (kTma) bits |= v[u];
+                    else bits |= __float_as_uint(v[u].x) | __float_as_uint(v[u].y);
+                }
+                if (__any_sync(0xffffffffu, (bits & (kTma ? 0x40004000u : 0x40000000u)) != 0u)) return 0;
+                uint32_t most;
+                if constexpr (kTma) {
+                    __nv_bfloat162 m = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v[u])));
+                    most = __float_as_uint(fmaxf(__low2float(m), __high2float(m)));
+                } else {
+                    float m = 0.f;
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) m = fmaxf(m, fmaxf(fabsf(v[u].x), fabsf(v[u].y)));
+                    most = __float_as_uint(m);
+                }
+                const int x = (int)(__reduce_max_sync(0xffffffffu, most) >> 23);
+                const int ex = max(min(x - 128, 0), -60);   // (rows of zeros: whatever)
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    if constexpr (kTma) v[u] = raise_bf2(v[u], -ex);
+                    else v[u] = mul2(v[u], make_float2(exp2_of(-ex), exp2_of(-ex)));
+                }
+                return ex;
+            };
             load16(XA, v0);
             load16(XR, v1);
+            const int er = raise_small(v1);
             float2 f = make_float2(mA[0], mA[1]);
 #pragma unroll
             for (int u = 0; u < 16; ++u) {
@@ -324,6 +352,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
             }
             load16(XB, v0);
             load16(XK, v1);
+            note(er, raise_small(v1));
             f = make_float2(mB[0], mB[1]);
 #pragma unroll
             for (int u = 15; u >= 0; --u) {
@@ -649,7 +678,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
 // Kernel 2: the scan, one CTA per chain.  D[n][i] = sum_k O[n][k] [Z; V][k][i] per chunk, four tcgen05 products of M = 128,
 // N = 64, K = 16 over V, issued a chunk ahead, and four over Z: TMEM lanes 0-63 are the rows j' of the next state (fp32 state Z[j'][i] = S[i][j'] in registers, two
 // warps per column half), lanes 64-127 the output tokens.  Warps 0-7 own the lanes twice over (two column halves), warp 8
-// streams records and V tiles into a ring, warp 9 issues, warps 10 and 11 turn V tiles into fp16 rows of [Z; V] ahead of time.
+// streams records and V tiles into a ring, warp 9 issues, warps 10 to 13 turn V tiles into scaled fp16 rows of [Z; V] ahead of time.
 //
 // Bound by the serial step of a chain: TMEM read, multiply-add with the decays, fp16 rows of Z, hand-over to the issuing
 // warp, the products over Z, their completion.  Hand-overs are hardware barriers (16 cycles; a satisfied mbarrier wait
@@ -659,10 +688,11 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
 // accumulators, was bound by shared-memory bandwidth: each warp reads its operator columns and all of Z and V, 1.8 k
 // cycles a chunk.)  Measured: 1.35 k cycles a chunk, 53 us for 64 chunks of up to 148 chains; 512 chains 6.1 TB/s, the roof.
 // ------------------------------------------------------------------------------------------
+constexpr int kConverters = 4;                    // (one per token block of a chunk; with two the prefill's scan took 60.5 us, not 58.8)
+constexpr int kScanThreads = (10 + kConverters) * 32;
 template <typename TIO>
 struct Scan {
     static constexpr bool kF32 = sizeof(TIO) == 4;
-    static constexpr int kThreads = 12 * 32;
     static constexpr int kStages = kF32 ? 3 : 4;
     static constexpr uint32_t kVBytes = kL * kN * sizeof(TIO);
     static constexpr uint32_t kV = kOperatorBytes;                // stage: operator, V tile, vectors
@@ -672,7 +702,7 @@ struct Scan {
     static constexpr uint32_t kYTile = kL * kN * sizeof(TIO);
     static constexpr uint32_t kY = kZV + 2 * 2 * kPanel;          // two output tiles (fp32: each two panels of 32 channels)
     static constexpr uint32_t kBars = kY + 2 * kYTile;
-    static constexpr uint32_t kBytes = kBars + 256;
+    static constexpr uint32_t kBytes = kBars + 320;
     static_assert(kBytes <= 232448, "the scan exceeds an SM");
 };
 
@@ -698,6 +728,12 @@ template <bool kTransposed>
 __device__ __forceinline__ uint64_t desc_operator(uint32_t addr, int ks) {
     const uint32_t step = kTransposed ? 4096u : 256u, along_k = kTransposed ? 2048u : 128u, along_m = kTransposed ? 128u : 2048u;
     return (uint64_t)(((addr + (uint32_t)ks * step) >> 4) & 0x3fffu) | (uint64_t)(along_k >> 4) << 16 | (uint64_t)(along_m >> 4) << 32 | (uint64_t)1 << 46;
+}
+
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+    float y;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
 }
 
 // A warp's largest magnitude of a state, as float bits.
@@ -816,14 +852,17 @@ __device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, con
 // over the transposed operators, last chunk first (kGradients): with G[j'][i] the gradient of the state behind a chunk and
 // dY[t][i] that of its output,
 //     D'[k][i] = sum_n O[n][k] [G; dY][n][i]
-// has the rows j of the gradient in front of the chunk and the rows s of dV.  Gradients may be far smaller than fp16 resolves
-// well (or larger than it holds), so G and dY of a chunk are scaled by a power of two, chosen by the converting warps from the largest magnitudes
-// of dY in this chunk and the three after it and of G as the state warps last published it.  Measured, 96 chains x 64 chunks: 65
-// and 75 us; the tf32 kernel that ran both passes before took 560 us for each.
+// has the rows j of the gradient in front of the chunk and the rows s of dV.
+//
+// Scales.  Values and states may be far smaller than fp16 resolves well, and gradients also larger than it holds: the state and V of a
+// chunk (G and dY) go in times a power of two, chosen by the converting warps from the largest magnitudes of V in this chunk and the three
+// before it in the scan's order and of the state as it entered the chunk three steps back, which the state warps publish.
+// Forwards values are only scaled up: a chain that overflows fp16 is recomputed in fp32.  The choice does not depend on where a call
+// is cut into segments: what the first three chunks of the next segment look back on is handed on with the chain's flag.
 enum ScanKind { kPrefill, kForTraining, kGradients };
 
 template <typename TIO, int kKind>
-__global__ void __launch_bounds__(Scan<TIO>::kThreads, 1)
+__global__ void __launch_bounds__(kScanThreads, 1)
 wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs, const TIO *__restrict__ v,
                        const unsigned char *__restrict__ records, const float *state_in, float *state_out,
                        TIO *__restrict__ y, float *__restrict__ snapshots, uint32_t *__restrict__ tops, int *flags, int Tlen, int H, int chunk0, int n, int resolve_flagged,
@@ -844,11 +883,14 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     uint64_t *bar_acc = bar_empty + NS;                                    // [2] an accumulator is complete
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_acc + 2);
     volatile int *bad = reinterpret_cast<volatile int *>(tmem_slot + 1);   // bit 0: a wait expired, bit 1: a value is not finite
-    // (gradients) [2] the scale of a chunk is known; its exponent by chunk mod 4; largest magnitudes as float bits: of G by chunk
-    // mod 4 (and at the start) and state warp, of dY by chunk mod 2 and converting warp
-    uint64_t *bar_scale = bar_acc + 3;
+    uint64_t *bar_scale = bar_acc + 3;                                     // [2] the scale of a chunk is known
+    // Its exponent, by chunk mod 4; largest magnitude of the state as float bits, by chunk mod 4
+    // (and at the start) and state warp; exponent of the largest V by chunk mod 2 and converting warp; what an output row of each
+    // 16-token block is multiplied by, by chunk mod 4
     volatile int *scale_exp = reinterpret_cast<volatile int *>(smem + SM::kBars + 128);
-    volatile uint32_t *top_g = reinterpret_cast<volatile uint32_t *>(smem + SM::kBars + 144), *top_dy = top_g + 20;
+    volatile uint32_t *top_z = reinterpret_cast<volatile uint32_t *>(smem + SM::kBars + 144);
+    volatile int *top_v = reinterpret_cast<volatile int *>(smem + SM::kBars + 224);
+    volatile float *row_up = reinterpret_cast<volatile float *>(smem + SM::kBars + 256);
     static_assert(8 * (2 * NS + 5) <= 128, "the barriers' place");
     // chunk of step c (gradients run from the last to the first)
     auto at_step = [&](int c) { return kGrad ? n - 1 - c : c; };
@@ -861,12 +903,11 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         }
         mbar_init(bar_acc, 1);
         mbar_init(bar_acc + 1, 1);
-        if (kGrad) {
-            mbar_init(bar_scale, 1);
-            mbar_init(bar_scale + 1, 1);
-        }
+        mbar_init(bar_scale, 1);
+        mbar_init(bar_scale + 1, 1);
         mbar_fence_init();
         *bad = 0;
+        for (int i = 0; i < 8; ++i) top_v[i] = 0;
         tma_prefetch_desc(&maps.v);
         tma_prefetch_desc(&maps.y);
     }
@@ -881,16 +922,19 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     const float *s_in = state_in ? state_in + (size_t)chain * kN * kN : nullptr;
     float *s_out = state_out ? state_out + (size_t)chain * kN * kN : nullptr;
     const unsigned char *rec = records + (size_t)chain * n * kRecord;
-    // A chain is flagged by any of its chunks, in this segment or (as the scan of that segment left it) an earlier one.
-    int mark = chunk0 > 0 && tid == 0 ? *reinterpret_cast<volatile int *>(&flags[chain]) : 0;
-    for (int c = tid; c < n; c += SM::kThreads) mark |= *reinterpret_cast<const int *>(rec + (size_t)c * kRecord + kMarkAt);
+    // A chain is flagged by any of its chunks, in this segment or (as the scan of that segment left it, bit 0) an earlier one.
+    // Above it, for the first three chunks of a segment: the exponent of what their scales have to cover from before it, 0 where
+    // that is not known (then it is the state's at the start).
+    const uint32_t left = chunk0 > 0 ? *reinterpret_cast<volatile uint32_t *>(&flags[chain]) : 0u;
+    int mark = (int)(left & 1u);
+    for (int c = tid; c < n; c += kScanThreads) mark |= *reinterpret_cast<const int *>(rec + (size_t)c * kRecord + kMarkAt);
     const bool flagged = __syncthreads_or(mark) != 0;
-    if (tid == 0) flags[chain] = flagged && !resolve_flagged;
+    uint32_t leave = flagged && !resolve_flagged ? 1u : 0u;   // (warp 10 writes it at the end)
     const int t_end = min(Tlen, (chunk0 + n) * kL);
     // Z of a chunk is written: four state warps arrive, the issuing warp waits.  V of chunk c is converted and the chunk's
-    // accumulator, the one of two chunks before, read back: two converters and four output warps arrive.
+    // accumulator, the one of two chunks before, read back: four converters and four output warps arrive.
     auto z_arrive = [] { asm volatile("bar.arrive 3, 160;" ::: "memory"); };
-    auto v_arrive = [](int c) { asm volatile("bar.arrive %0, 224;" ::"r"(4 + (c & 1)) : "memory"); };
+    auto v_arrive = [](int c) { asm volatile("bar.arrive %0, 288;" ::"r"(4 + (c & 1)) : "memory"); };
     uint32_t limit = 4000000u;   // polls a wait may take; after the first that expires this thread stops waiting, and the call reports it
     auto wait = [&](uint64_t *b, uint32_t parity) { limit = mbar_wait_tight(b, parity, limit) ? limit : 1u; };
     if (flagged) {
@@ -926,7 +970,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         auto v_products = [&](int c) {
             const int s = c % NS, a = c & 1;
             wait(bar_full + s, (uint32_t)((c / NS) & 1));
-            asm volatile("bar.sync %0, 224;" ::"r"(4 + a) : "memory");
+            asm volatile("bar.sync %0, 288;" ::"r"(4 + a) : "memory");
             if (elect_one()) {
                 tc_fence_after();
                 const uint32_t op = sb + s * SM::kStage, vt = sb + SM::kZV + a * 2 * kPanel + kPanel;
@@ -955,81 +999,105 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     } else if (warp >= 10) {
         // ---------------- V converters: tile -> fp16 rows in the order of the contraction index, 16-byte pieces; rows past the sequence's end belong to
         // another one, whatever they hold stays out of the sums
-        constexpr int kShare = kL * kN / 8 / 32 / 2;
-        uint32_t dy_before[3] = {0u, 0u, 0u};   // (gradients)
-        if constexpr (kGrad) asm volatile("bar.sync 7, 192;" ::: "memory");   // the state warps have published the start
+        constexpr int kShare = kL * kN / 8 / 32 / kConverters;
+        // What is largest, the state or eight times V (a state gathers a chunk's V times k; a gradient dY times r), comes to lie in
+        // [32, 64): eleven binary orders to overflow, and a state that falls by nineteen within three chunks is still resolved.
+        constexpr int kAbove = 3, kUnscaled = 127 + 5;
+        const int own = warp - 10;                  // this warp's token block
+        int carried[3], before[3] = {0, 0, 0};      // exponents; of V (dY) one, two and three chunks ago
+        auto most_at = [&](uint32_t at) {   // of four words
+            uint32_t x[4];
+            lds128(x, sb + SM::kBars + at);
+            return max(max(x[0], x[1]), max(x[2], x[3]));
+        };
+        auto top_state = [&](int slot) { return (int)(most_at(144 + slot * 16) >> 23); };
+        asm volatile("bar.sync 7, 256;" ::: "memory");   // the state warps have published the start
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int x = (int)(left >> (8 + 8 * i)) & 255;
+            carried[i] = x ? x : top_state(4);
+        }
         for (int c = 0; c < n; ++c) {
             const int s = c % NS, a = c & 1;
             wait(bar_full + s, (uint32_t)((c / NS) & 1));
-            if (c >= 2) wait(bar_acc + a, (uint32_t)(((c >> 1) - 1) & 1));   // the products that last read this tile
             const uint32_t vt = sb + s * SM::kStage + SM::kV, out = sb + SM::kZV + a * 2 * kPanel + kPanel;
             const int valid = Tlen - (chunk0 + at_step(c)) * kL;
-            if constexpr (kGrad) {
-                // dY of a chunk: rows in token order, scaled
-                uint32_t x[kShare][4];
-                __nv_bfloat162 m = __floats2bfloat162_rn(0.f, 0.f);
+            const signed char *row_exp = reinterpret_cast<const signed char *>(smem + s * SM::kStage + SM::kVec + kRowExpAt);
+            const int e_in = row_exp[2 * own + (kGrad ? 0 : 1)];
+            auto token = [&](int k) { return ((own * kShare + k) * 32 + lane) >> 3; };
+            // eight channels of a token (fp32: two pieces of a panel of 32 channels)
+            constexpr int kWords = SM::kF32 ? 8 : 4;
+            uint32_t x[kShare][kWords];
+            __nv_bfloat162 m[4];
+            float m32[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int k = 0; k < kShare; ++k) {
-                    const int p = ((warp - 10) * kShare + k) * 32 + lane, t = p >> 3;
-                    lds128(x[k], vt + off16(t, (p & 7) * 8));
-                    if (t >= valid) x[k][0] = x[k][1] = x[k][2] = x[k][3] = 0;
+            for (int e = 0; e < 4; ++e) m[e] = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&x[k][e])));
-                }
-                const uint32_t own = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(__low2float(m), __high2float(m))));
-                if (lane == 0) top_dy[a * 2 + warp - 10] = own;
-                asm volatile("bar.sync 6, 64;" ::: "memory");
-                const uint32_t dy_now = max(top_dy[a * 2], top_dy[a * 2 + 1]);
-                const volatile uint32_t *tg = top_g + (c < 3 ? 4 : (c - 3) & 3) * 4;
-                // (entries of G gather a chunk's dY times r: eight times dY leaves room on both sides)
-                const float dy_most = 8.f * __uint_as_float(max(max(dy_now, dy_before[0]), max(dy_before[1], dy_before[2])));
-                const float most = fmaxf(dy_most, __uint_as_float(max(max(tg[0], tg[1]), max(tg[2], tg[3]))));
-                const int ex = most > 0.f ? min(max(exponent_of(most) - 127 - 5, -96), 96) : 0;
-                dy_before[2] = dy_before[1];
-                dy_before[1] = dy_before[0];
-                dy_before[0] = dy_now;
-                if (warp == 10 && lane == 0) {
-                    scale_exp[c & 3] = ex;
-                    mbar_arrive(bar_scale + a);
-                }
-                const float2 f = make_float2(exp2_of(-ex), exp2_of(-ex));
+            for (int k = 0; k < kShare; ++k) {
+                const int t = token(k), cg = lane & 7;
+                if constexpr (!SM::kF32) lds128(x[k], vt + off16(t, cg * 8));
+                else {
+                    const uint32_t row = vt + (cg >> 2) * (SM::kVBytes / 2) + t * 128;
 #pragma unroll
-                for (int k = 0; k < kShare; ++k) {
-                    const int p = ((warp - 10) * kShare + k) * 32 + lane;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) x[k][e] = pack2(mul2(unpack_bf2(x[k][e]), f));
-                    sts128(out + off16(p >> 3, (p & 7) * 8), x[k]);
-                }
-            } else {
-#pragma unroll
-            for (int k0 = 0; k0 < kShare; k0 += 4) {
-                uint32_t x[4][4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int p = ((warp - 10) * kShare + k0 + k) * 32 + lane, t = p >> 3, cg = p & 7;
-                    if constexpr (!SM::kF32) {
-                        lds128(x[k], vt + off16(t, cg * 8));
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) x[k][e] = bf2_to_half2(x[k][e]);
-                    } else {                                // two pieces of a panel of 32 channels
-                        const uint32_t row = vt + (cg >> 2) * (SM::kVBytes / 2) + t * 128;
-                        const float4 lo = lds_f4(row + (((2 * cg & 7) ^ (t & 7)) << 4)), hi = lds_f4(row + (((2 * cg & 7) + 1) ^ (t & 7)) * 16);
-                        x[k][0] = pack_half2(lo.x, lo.y);
-                        x[k][1] = pack_half2(lo.z, lo.w);
-                        x[k][2] = pack_half2(hi.x, hi.y);
-                        x[k][3] = pack_half2(hi.z, hi.w);
+                    for (int i = 0; i < 2; ++i) {
+                        const float4 f = lds_f4(row + (((2 * cg & 7) + i) ^ (t & 7)) * 16);
+                        x[k][4 * i] = __float_as_uint(f.x); x[k][4 * i + 1] = __float_as_uint(f.y);
+                        x[k][4 * i + 2] = __float_as_uint(f.z); x[k][4 * i + 3] = __float_as_uint(f.w);
                     }
-                    if (t >= valid) x[k][0] = x[k][1] = x[k][2] = x[k][3] = 0;
                 }
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int p = ((warp - 10) * kShare + k0 + k) * 32 + lane;
-                    sts128(out + off16(k_position(p >> 3), (p & 7) * 8), x[k]);
+                for (int e = 0; e < kWords; ++e) {
+                    if (t >= valid) x[k][e] = 0;
+                    if constexpr (!SM::kF32) m[e] = __hmax2(m[e], __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&x[k][e])));
+                    else m32[e & 3] = fmaxf(m32[e & 3], fabsf(__uint_as_float(x[k][e])));
                 }
             }
+            const __nv_bfloat162 mm = __hmax2(__hmax2(m[0], m[1]), __hmax2(m[2], m[3]));
+            const float most = SM::kF32 ? fmaxf(fmaxf(m32[0], m32[1]), fmaxf(m32[2], m32[3])) : fmaxf(__low2float(mm), __high2float(mm));
+            int top = (int)(__reduce_max_sync(0xffffffffu, __float_as_uint(most)) >> 23);
+            if (top > 0) top = max(top + e_in, 1);
+            if (lane == 0) top_v[a * 4 + own] = top;
+            asm volatile("bar.sync 6, 128;" ::: "memory");
+            if (c >= 2) wait(bar_acc + a, (uint32_t)(((c >> 1) - 1) & 1));   // the products that last read this tile
+            const int now = (int)most_at(224 + a * 16);
+            const int v_most = max(max(now, before[0]), max(before[1], before[2]));
+            const int all = max(c < 3 ? (c == 0 ? carried[0] : c == 1 ? carried[1] : carried[2]) : top_state((c - 3) & 3), v_most > 0 ? v_most + kAbove : 0);
+            const int ex = all > 0 ? min(max(all - kUnscaled, -96), kGrad ? 96 : 0) : 0;
+            before[2] = before[1];
+            before[1] = before[0];
+            before[0] = now;
+            if (own == 0) {
+                if (lane < 4) row_up[(c & 3) * 4 + lane] = exp2_of(ex) * exp2_of(row_exp[2 * lane + (kGrad ? 1 : 0)]);
+                if (lane == 0) scale_exp[c & 3] = ex;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_scale + a);   // (a hardware barrier would have the state warps wait for one another too)
+            }
+#pragma unroll
+            for (int k = 0; k < kShare; ++k) {
+                const float f1 = exp2_of(max(e_in - ex, -126));
+                uint32_t y[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float2 v2;
+                    if constexpr (!SM::kF32) v2 = unpack_bf2(x[k][e]);
+                    else v2 = make_float2(__uint_as_float(x[k][2 * e]), __uint_as_float(x[k][2 * e + 1]));
+                    y[e] = pack2(mul2(v2, make_float2(f1, f1)));
+                }
+                // (dY of a chunk: rows in token order)
+                sts128(out + off16(kGrad ? token(k) : k_position(token(k)), (lane & 7) * 8), y);
             }
             fence_proxy_async();
             v_arrive(c);
+        }
+        if ((chunk0 + n) * kL < Tlen) {   // what the next segment's first chunks look back on
+            asm volatile("bar.sync 7, 256;" ::: "memory");   // (the state warps have published every chunk)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                int x = n + i >= 3 ? top_state((n + i - 3) & 3) : n + i == 1 ? carried[1] : carried[2];
+#pragma unroll
+                for (int k = 0; k < 3 - i; ++k) x = max(x, before[k] > 0 ? before[k] + kAbove : 0);
+                leave |= (uint32_t)min(x, 255) << (8 + 8 * i);
+            }
         }
     } else {
         const int quarter = warp & 3, hf = warp >> 2;
@@ -1047,28 +1115,28 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
             for (int e = 0; e < 16; ++e)
                 Z[e] = s_in ? make_float2(s_in[(i0 + 2 * e) * kN + jp], s_in[(i0 + 2 * e + 1) * kN + jp]) : make_float2(0.f, 0.f);
             // this row's scalars of a chunk: e^{c_L}, and what the operand and the product are multiplied by: fx and the factor of P
-            // and Kt, or, for gradients, the other way round with the chunk's scale
+            // and Kt, or, for gradients, the other way round; both with the chunk's scale
             auto load_vec = [&](int c, float &gx, float &fx, float &g2) {
                 const int s = c % NS;
                 wait(bar_full + s, (uint32_t)((c / NS) & 1));
                 const unsigned char *vec = smem + s * SM::kStage + SM::kVec;
                 gx = *reinterpret_cast<const float *>(vec + jp * 4);
                 const int ef = *reinterpret_cast<const signed char *>(vec + 256 + jp), eg = *reinterpret_cast<const signed char *>(vec + 320 + jp);
+                wait(bar_scale + (c & 1), (uint32_t)((c >> 1) & 1));
+                const float up = exp2_of(scale_exp[c & 3]), down = exp2_of(-scale_exp[c & 3]);
                 if constexpr (kGrad) {
-                    wait(bar_scale + (c & 1), (uint32_t)((c >> 1) & 1));
-                    const int ex = scale_exp[c & 3];
-                    fx = exp2_of(-eg) * exp2_of(-ex);
-                    g2 = gx * exp2_of(ef) * exp2_of(ex);
+                    fx = exp2_of(-eg) * down;
+                    g2 = gx * exp2_of(ef) * up;
                 } else {
-                    fx = gx * exp2_of(ef);
-                    g2 = exp2_of(-eg);
+                    fx = gx * exp2_of(ef) * down;
+                    g2 = exp2_of(-eg) * up;
                 }
             };
             // largest magnitude of the state in this warp's share
             auto largest = [&] {
                 float m[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int e = 0; e < 16; ++e) m[e & 3] = fmaxf(m[e & 3], fmaxf(fabsf(Z[e].x), fabsf(Z[e].y)));
+                for (int e = 0; e < 16; ++e) m[e & 3] = max3_abs(m[e & 3], Z[e].x, Z[e].y);
                 return __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]))));
             };
             auto keep = [&](int c, uint32_t most) {   // the state that step c starts from, for the kernel of the chunks (see accumulator_place)
@@ -1096,20 +1164,18 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 z_arrive();
             };
             float gx, fx, g2, gxn = 1.f, fxn = 1.f, g2n = 0.f;
-            if constexpr (kGrad) {
+            {
                 const uint32_t most = largest();
-                if (lane == 0) top_g[16 + quarter * 2 + hf] = most;
-                asm volatile("bar.sync 7, 192;" ::: "memory");
+                if (lane == 0) top_z[16 + quarter * 2 + hf] = most;
+                asm volatile("bar.sync 7, 256;" ::: "memory");
             }
             load_vec(0, gx, fx, g2);
             put_z(0, fx);
             for (int c = 0; c < n; ++c) {
                 const int a = c & 1;
-                if constexpr (kKind != kPrefill) {
-                    const uint32_t most = largest();
-                    if (kGrad && lane == 0) top_g[(c & 3) * 4 + quarter * 2 + hf] = most;   // for the converting warps
-                    keep(c, most);
-                }
+                const uint32_t most = largest();
+                if (lane == 0) top_z[(c & 3) * 4 + quarter * 2 + hf] = most;   // for the converting warps
+                if constexpr (kKind != kPrefill) keep(c, most);
                 if (c + 1 < n) load_vec(c + 1, gxn, fxn, g2n);   // (while the products run)
                 wait(bar_acc + a, (uint32_t)((c >> 1) & 1));
                 tc_fence_after();
@@ -1124,6 +1190,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 gx = gxn;
                 g2 = g2n;
             }
+            if ((chunk0 + n) * kL < Tlen) asm volatile("bar.sync 7, 256;" ::: "memory");
             bool off = false;   // a non-finite operand upstream stays in the state for good
 #pragma unroll
             for (int e = 0; e < 16; ++e) off |= !(fabsf(Z[e].x) <= 3.0e38f) | !(fabsf(Z[e].y) <= 3.0e38f);
@@ -1155,10 +1222,12 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 uint32_t d[32];
                 tmem_ld32(acc + a * 64, d);
                 tmem_ld_wait();
-                if constexpr (kGrad) {
-                    const float up = exp2_of(scale_exp[c & 3]);
+                const float up = row_up[(c & 3) * 4 + (tq >> 4)];
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) d[e] = __float_as_uint(__uint_as_float(d[e]) * up);
+                for (int e = 0; e < 32; e += 2) {
+                    const float2 y2 = mul2(make_float2(__uint_as_float(d[e]), __uint_as_float(d[e + 1])), make_float2(up, up));
+                    d[e] = __float_as_uint(y2.x);
+                    d[e + 1] = __float_as_uint(y2.y);
                 }
                 tc_fence_before();
                 if (c + 2 < n) v_arrive(c + 2);
@@ -1215,6 +1284,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 128);
+    if (warp == 10 && lane == 0) flags[chain] = (int)(*bad ? leave & 1u : leave);   // (a chain redone below starts afresh)
     if (*bad & 1) {
         if (tid == 0) atomicExch(status, (int)kDevTimeout);
         return;
@@ -1561,12 +1631,12 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
     cudaStream_t op_stream = part ? part->op_stream : stream;
     auto launch_scan = [&](cudaStream_t st, int buf, const float *s_in, float *s_out, int c0, int n) -> cudaError_t {
         const unsigned char *records = ws + lay.records[buf];
-        auto go = [&](auto kern, auto ytype, size_t smem_bytes, int threads) -> cudaError_t {
+        auto go = [&](auto kern, auto ytype, size_t smem_bytes) -> cudaError_t {
             cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
             if (err != cudaSuccess) return err;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)chains);
-            cfg.blockDim = dim3((unsigned)threads);
+            cfg.blockDim = dim3((unsigned)kScanThreads);
             cfg.dynamicSmemBytes = smem_bytes;
             cfg.stream = st;
             cudaLaunchAttribute attr[1];
@@ -1581,8 +1651,8 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
             return err;
         };
         using bf = __nv_bfloat16;
-        if (!p.bf16) return go(wkv7_state_scan_kernel<float, kPrefill>, (float *)nullptr, Scan<float>::kBytes, Scan<float>::kThreads);
-        return go(wkv7_state_scan_kernel<bf, kPrefill>, (bf *)nullptr, Scan<bf>::kBytes, Scan<bf>::kThreads);
+        if (!p.bf16) return go(wkv7_state_scan_kernel<float, kPrefill>, (float *)nullptr, Scan<float>::kBytes);
+        return go(wkv7_state_scan_kernel<bf, kPrefill>, (bf *)nullptr, Scan<bf>::kBytes);
     };
     auto launch_operators = [&](int buf, int c0, int n) -> cudaError_t {
         const long long units = (long long)chains * n;
@@ -1670,7 +1740,7 @@ int launch_training_scan(const ScanMaps &maps, const OperatorPtrs &ptrs, const v
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)l.chains);
-    cfg.blockDim = dim3((unsigned)Scan<bf>::kThreads);
+    cfg.blockDim = dim3((unsigned)kScanThreads);
     cfg.dynamicSmemBytes = Scan<bf>::kBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];

@@ -2,6 +2,7 @@
 // memory, the lane addresses of matrix loads on them, and the arithmetic of the decays.
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -48,6 +49,19 @@ __device__ __forceinline__ int accumulator_place(int i, int j) {
     return (((i >> 4) * 8 + (j >> 3)) * 32 + (i & 7) * 4 + ((j & 7) >> 1)) * 4 + (j & 1) * 2 + ((i >> 3) & 1);
 }
 
+// What the builder leaves of a chunk in global memory: the 128 x 128 fp16 operator O[n][k], n = (j' | t), as the core
+// matrices (eight rows n, eight k, 128 bytes) of a K-major tcgen05 operand without swizzle, 16 of them along k and 16 along n.
+// The contraction index (64 j, then 64 s) is ordered so that a lane of the builder holds four neighbouring k of a row in its
+// accumulators: the eight of core 4 c + q are {2q, 2q+1, 2q+8, 2q+9} of the 16-block 2 c, then the same of 2 c + 1.  Behind
+// the operator e^{c_L}[64] in fp32, two signed exponents per channel (fx = e^{c_L} 2^ef; P and Kt are stored times 2^eg), two
+// per 16-token block (its r rows were taken times 2^-er, its k rows times 2^-ek), and the mark.
+constexpr uint32_t kOperatorBytes = 4 * kPanel;
+constexpr uint32_t kDecayAt = kOperatorBytes, kExpAt = kDecayAt + 256;
+constexpr uint32_t kVectorBytes = 256 + 128 + 16;
+constexpr uint32_t kRowExpAt = 384;                      // of er, ek of every block in turn, from kDecayAt on
+constexpr uint32_t kMarkAt = kDecayAt + kVectorBytes;   // int: the chunk is beyond what fp16 operands resolve
+constexpr size_t kRecord = 33280;                        // bytes per chunk in the workspace
+
 // Bounded wait for a whole warp without compiler-made divergence handling around the loop.
 __device__ __forceinline__ bool mbar_wait_tight(uint64_t *bar, uint32_t parity, uint32_t limit) {
     uint32_t ok;
@@ -86,6 +100,12 @@ __device__ __forceinline__ float2 decay2(float2 w) {
     const float2 x = mul2(w, make_float2(kLog2e, kLog2e));
     const float2 z = mul2(make_float2(ex2(x.x), ex2(x.y)), make_float2(-kLog2e, -kLog2e));
     return make_float2(ex2(z.x), ex2(z.y));
+}
+// A bf16 pair times 2^e, 0 <= e <= 60: exact
+__device__ __forceinline__ uint32_t raise_bf2(uint32_t v, int e) {
+    const uint32_t f = (uint32_t)(127 + e) * 0x00800080u;
+    const __nv_bfloat162 y = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&v), *reinterpret_cast<const __nv_bfloat162 *>(&f));
+    return *reinterpret_cast<const uint32_t *>(&y);
 }
 __device__ __forceinline__ uint32_t pack2(float2 v) { return pack_half2(v.x, v.y); }
 __device__ __forceinline__ int exponent_of(float v) { return (int)(__float_as_uint(v) >> 23); }   // biased; v > 0
