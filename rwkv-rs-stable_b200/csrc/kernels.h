@@ -111,7 +111,7 @@ size_t wkv7_training_saved_bytes(int64_t B, int64_t T, int64_t H);
 size_t wkv7_training_workspace_bytes(int64_t B, int64_t T, int64_t H);
 int launch_wkv7_training_forward(const Wkv7Args &p, void *saved, cudaStream_t stream);
 int launch_wkv7_training_backward(const Wkv7TrainingBackwardArgs &p, const void *saved, void *workspace, cudaStream_t stream);
-int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const float *states, const float *gradients, cudaStream_t stream);
+int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const unsigned char *records, const float *states, const float *gradients, cudaStream_t stream);
 
 // Cluster size of the chunked kernel: 0 = by the number of chains (default), else 1, 2 or 4.
 int wkv7_cluster_override();

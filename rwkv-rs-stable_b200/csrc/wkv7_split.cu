@@ -1800,7 +1800,7 @@ int launch_wkv7_training_backward(const Wkv7TrainingBackwardArgs &p, const void 
     if (int e = launch_training_scan<kGradients>(smaps, optrs, p.dy, base, p.next_state_grad, p.initial_state_grad, p.dv, gradients,
                                                  reinterpret_cast<int *>(ws + lw.flags), lw, p.T, p.H, status, stream))
         return e;
-    return launch_wkv7_chunk_gradients(p, reinterpret_cast<const float *>(base + ls.states), gradients, stream);
+    return launch_wkv7_chunk_gradients(p, base, reinterpret_cast<const float *>(base + ls.states), gradients, stream);
 }
 
 }  // namespace rwkv7

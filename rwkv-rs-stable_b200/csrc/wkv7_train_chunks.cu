@@ -19,8 +19,9 @@
 // dv is an output of the gradient scan.
 //
 // States, accumulators, decays and sums are fp32; matrix operands are fp16 (11 significant bits), S with V and G with dY scaled
-// by a power of two per chunk.  A chunk whose decay leaves the range of the reference points, or where a value leaves that of
-// fp16, is recomputed token by token in fp32.
+// by a power of two per chunk, k and r by what then is between the two (see below).  A chunk whose decay leaves the range of the
+// reference points, where a value leaves that of fp16, or with rows of a or b that are all below 2^-12 (u and du are as small, and
+// db and da are made of them; a model's are of length one), is recomputed token by token in fp32.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -40,6 +41,7 @@ namespace {
 using namespace sm100;
 
 constexpr int kThreads = 256;
+constexpr float kTiny = 2.44140625e-4f;   // 2^-12
 enum { TA = 0, TR, TB, TK, TV, TY, TW, kTensors };
 constexpr uint32_t kTilesBytes = kTensors * kPanel;             // one of two buffers of input tiles
 constexpr uint32_t kF = 2 * kTilesBytes;                         // D_{t-1} / mu and D_t / mu, fp16 tiles [token][channel]
@@ -68,6 +70,7 @@ struct ChunkMaps {
 struct ChunkArgs {
     const __nv_bfloat16 *in[kTensors];
     __nv_bfloat16 *out[5];
+    const unsigned char *records;   // [chain][chunk], of which the exponents of r and k rows are read
     // [chain][chunk][64 x 64], in the order of accumulator_place; behind them eight largest magnitudes each, as float bits
     const float *states, *gradients;
     int T, H, nchunks;
@@ -96,6 +99,19 @@ __device__ __forceinline__ int factor_place(int j) { return ((j & 7) >> 1) * 16 
 __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
     const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&b);
+}
+
+// Largest of four signed bytes.
+__device__ __forceinline__ int most_of_four(uint32_t x) {
+    return max(max((int)(signed char)x, (int)(signed char)(x >> 8)), max((int)(signed char)(x >> 16), (int)(signed char)(x >> 24)));
+}
+// Whether eight rows of a removal key or replacement are below what its products keep their bits at, but not zero.
+__device__ __forceinline__ bool tiny(const uint32_t (&x)[8]) {
+    __nv_bfloat162 m = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&x[u])));
+    const float most = fmaxf(__low2float(m), __high2float(m));
+    return !__any_sync(0xffffffffu, most >= kTiny) && __any_sync(0xffffffffu, most > 0.f);
 }
 
 // One chunk in fp32, token by token.  `scratch`: 36 KB, `sums`: 64 KB of shared memory.  Four lanes per value row, columns
@@ -264,11 +280,15 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
     if ((int)blockIdx.x < p.units) fetch(blockIdx.x);
     const uint32_t *tops_s = reinterpret_cast<const uint32_t *>(p.states + (size_t)p.units * kN * kN);
     const uint32_t *tops_g = reinterpret_cast<const uint32_t *>(p.gradients + (size_t)p.units * kN * kN);
+    auto row_exponents = [&](int unit) { return *reinterpret_cast<const uint2 *>(p.records + (size_t)unit * kRecord + kDecayAt + kRowExpAt); };
+    uint2 row_exp_next = (int)blockIdx.x < p.units ? row_exponents(blockIdx.x) : make_uint2(0u, 0u);
     int seq = 0;
     for (int unit = blockIdx.x; unit < p.units; unit += (int)gridDim.x, ++seq) {
         const int buf = seq & 1;
         const uint32_t tiles = sb + buf * kTilesBytes;
         const int valid = min(kL, p.T - unit % p.nchunks * kL), nblk = valid / 16;
+        const uint2 row_exp = row_exp_next;   // (a line of its own in memory for every chunk: fetched a chunk ahead)
+        if (unit + (int)gridDim.x < p.units) row_exp_next = row_exponents(unit + (int)gridDim.x);
         const uint32_t state_top = lane < 16 ? (lane < 8 ? tops_s : tops_g)[(size_t)unit * 8 + (lane & 7)] : 0u;
         if (!mbar_wait(bar + buf, (uint32_t)((seq >> 1) & 1))) *abort_flag = 1;
         __syncwarp();
@@ -305,17 +325,25 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         __syncthreads();
         if (*abort_flag) break;
         // ---------------- 2. scaled fp16 operands, in place; D_t / mu
-        float scale_s, scale_g;
-        int ex;
+        // V and dY are scaled alone (dk, dr are made of them); S and G with what V k^T and dY r^T add to them, and k and r by
+        // what is left between the two: V 2^-ev, S 2^-es, k 2^(ev - es), dY 2^-ey, G 2^-eg, r 2^(ey - eg).
+        int es, ev, eg, ey;
         {
-            const uint32_t ts = lane < 8 ? state_top : lane >= 16 && lane < 24 ? lds32(sb + kTop + (lane - 16) * 4) : 0u;
-            const uint32_t tg = lane >= 8 && lane < 16 ? state_top : lane >= 24 ? lds32(sb + kTop + 32 + (lane - 24) * 4) : 0u;
-            const uint32_t ms = __reduce_max_sync(0xffffffffu, ts), mg = __reduce_max_sync(0xffffffffu, tg);
-            const int es = ms ? min(max((int)(ms >> 23) - 127, -60), 60) : 0, eg = mg ? min(max((int)(mg >> 23) - 127, -60), 60) : 0;
-            scale_s = exp2_of(-es);
-            scale_g = exp2_of(-eg);
-            ex = es + eg;
+            const int er = most_of_four(__byte_perm(row_exp.x, row_exp.y, 0x6420)), ek = most_of_four(__byte_perm(row_exp.x, row_exp.y, 0x7531));
+            const uint32_t own = lane < 16 ? 0u : lds32(sb + kTop + (lane - 16) * 4);
+            auto largest = [&](uint32_t x, int &e) {
+                const uint32_t m = __reduce_max_sync(0xffffffffu, x);
+                e = min(max((int)(m >> 23) - 127, -60), 60);
+                return m != 0u;
+            };
+            const bool has_s = largest(lane < 8 ? state_top : 0u, es), has_v = largest(lane >= 16 && lane < 24 ? own : 0u, ev);
+            const bool has_g = largest(lane >= 8 && lane < 16 ? state_top : 0u, eg), has_y = largest(lane >= 24 ? own : 0u, ey);
+            es = has_v ? max(has_s ? es : -60, max(ev + ek, -60)) : has_s ? es : 0;
+            eg = has_y ? max(has_g ? eg : -60, max(ey + er, -60)) : has_g ? eg : 0;
+            if (!has_v) ev = es;
+            if (!has_y) ey = eg;
         }
+        const float scale_s = exp2_of(-es), scale_g = exp2_of(-eg);
         bool over;
         {
             const float2 e0 = lds_f2(sb + kE + (2 * tb * 64 + ch) * 4), e1 = lds_f2(sb + kE + ((2 * tb + 1) * 64 + ch) * 4);
@@ -330,19 +358,21 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                 sts_f2(sb + kRho + (tb * 64 + ch) * 4, rho.x, rho.y);
             }
             float2 f = hf ? mul2(e0, up) : up;
+            const float2 rs = make_float2(exp2_of(ey - eg), exp2_of(ey - eg)), ks = make_float2(exp2_of(ev - es), exp2_of(ev - es));
             uint32_t x0[8], x1[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 x0[u] = nv ? lds32(at(TA, u)) : 0u;
                 x1[u] = nv ? lds32(at(TR, u)) : 0u;
             }
+            over |= tiny(x0);
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const uint32_t o = t_first * 128 + off16(u, ch);
                 sts32(at(TA, u), pack2(mul2(unpack_bf2(x0[u]), f)));
                 sts32(sb + kF + o, pack2(f));
                 f = mul2(f, d[u]);
-                sts32(at(TR, u), pack2(mul2(unpack_bf2(x1[u]), f)));
+                sts32(at(TR, u), pack2(mul2(mul2(unpack_bf2(x1[u]), rs), f)));
                 sts32(sb + kF + kPanel + o, pack2(f));
             }
 #pragma unroll
@@ -350,13 +380,14 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                 x0[u] = nv ? lds32(at(TB, u)) : 0u;
                 x1[u] = nv ? lds32(at(TK, u)) : 0u;
             }
+            over |= tiny(x0);
             f = make_float2(rcp(rho.x), rcp(rho.y));
             if (!hf) f = mul2(f, e1);
-            const float2 vs = make_float2(scale_s, scale_s), ys = make_float2(scale_g, scale_g);
+            const float2 vs = make_float2(exp2_of(-ev), exp2_of(-ev)), ys = make_float2(exp2_of(-ey), exp2_of(-ey));
 #pragma unroll
             for (int u = 7; u >= 0; --u) {
                 sts32(at(TB, u), pack2(mul2(unpack_bf2(x0[u]), f)));
-                sts32(at(TK, u), pack2(mul2(unpack_bf2(x1[u]), f)));
+                sts32(at(TK, u), pack2(mul2(mul2(unpack_bf2(x1[u]), ks), f)));
                 f = mul2(f, d[u]);
                 sts32(at(TV, u), pack2(mul2(unpack_bf2(rv[u]), vs)));
                 sts32(at(TY, u), pack2(mul2(unpack_bf2(ry[u]), ys)));
@@ -599,7 +630,7 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                     ldsm4_t(B, tiles + TA * kPanel + o);
                     both(2, Q[2], 3, Q[3]);
                 }
-                const float sigma = exp2_of(min(max(ex, -126), 127));
+                const float sigma = exp2_of(es + eg), sigma_r = exp2_of(ey + es), sigma_k = exp2_of(ev + eg);
                 float finite = 0.f;
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
@@ -651,13 +682,14 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                         for (int r = 0; r < 2; ++r) {
                             const int i = n2 * 2 + r;
                             const float2 s2 = make_float2(sigma, sigma), f = unpack_half2(fi[i]);
-                            const float2 fa = mul2(unpack_half2(fe[i]), s2), fr = mul2(f, s2), fb = mul2(make_float2(rcp(f.x), rcp(f.y)), s2);
+                            const float2 inv = make_float2(rcp(f.x), rcp(f.y));
+                            const float2 fa = mul2(unpack_half2(fe[i]), s2), fr = mul2(f, make_float2(sigma_r, sigma_r)), fb = mul2(inv, s2), fk = mul2(inv, make_float2(sigma_k, sigma_k));
                             const float2 w = unpack_bf2(tw[i]);
                             constexpr float kLog2e = 1.4426950408889634f;
                             out[TA][i] = pack_bf2(acc[1][n][2 * r] * fa.x, acc[1][n][2 * r + 1] * fa.y);
                             out[TR][i] = pack_bf2(acc[0][n][2 * r] * fr.x, acc[0][n][2 * r + 1] * fr.y);
                             out[TB][i] = pack_bf2(acc[2][n][2 * r] * fb.x, acc[2][n][2 * r + 1] * fb.y);
-                            out[TK][i] = pack_bf2(acc[3][n][2 * r] * fb.x, acc[3][n][2 * r + 1] * fb.y);
+                            out[TK][i] = pack_bf2(acc[3][n][2 * r] * fk.x, acc[3][n][2 * r + 1] * fk.y);
                             // d_t dd_t = phi_t - x_t, phi_t = phi at the boundary - the later tokens' z
                             const float px = ph.x - (suf[r].x - z[r].x) - xs[r].x, py = ph.y - (suf[r].y - z[r].y) - xs[r].y;
                             finite += fabsf(px) + fabsf(py);   // (every product above is part of it)
@@ -714,7 +746,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
 }  // namespace
 
 // Enqueues the chunk kernel behind the gradient scan.
-int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const float *states, const float *gradients, cudaStream_t stream) {
+int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const unsigned char *records, const float *states, const float *gradients,
+                                cudaStream_t stream) {
     static const EncodeTiledFn encode = [] {
         void *fn = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -742,6 +775,7 @@ int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const float *
         if (!describe(&maps.out[i], out[i], (cuuint32_t)kL) || !describe(&maps.block[i], out[i], 16u)) return (int)cudaErrorInvalidValue;
         args.out[i] = static_cast<__nv_bfloat16 *>(out[i]);
     }
+    args.records = records;
     args.states = states;
     args.gradients = gradients;
     args.T = (int)p.T;

@@ -69,3 +69,28 @@ def test_segments_scale_alike(pkg, workloads, cuda, dtype):
     assert pkg.read_device_status(0) == 0
     for o in outs[1:]:
         assert torch.equal(o.output, outs[0].output) and torch.equal(o.next_state, outs[0].next_state)
+
+
+@pytest.mark.parametrize("scales", SCALES + [dict(a=1e-5), dict(b=1e-5)], ids=str)
+@pytest.mark.parametrize("model", [False, True])
+def test_training_step(pkg, oracle, workloads, cuda, scales, model):
+    B, T, H = 1, 208, 2
+    inp = _inputs(workloads, (B, T, H, 64), scales, torch.bfloat16, 113, model)
+    gen = torch.Generator().manual_seed(13)
+    dy = torch.randn(B, T, H, 64, generator=gen).to(torch.bfloat16)
+    ds = torch.randn(B, H, 64, 64, generator=gen) * scales.get("r", 1.0)
+    f = {n: inp[n].float().numpy() for n in inp}
+    y_ref, s_ref = oracle.wkv7_train(*[f[n] for n in "rwkvab"], s0=f["s0"], chunk_len=16)[:2]
+    ref = oracle.wkv7_backward(*[f[n] for n in "rwkvab"], dy.float().numpy(), s0=f["s0"], ds_out=ds.numpy())
+    leaves = {n: t.to(cuda).requires_grad_(True) for n, t in inp.items()}
+    y, s = pkg.wkv7_statepass_autograd(leaves["s0"], pkg.Wkv7PretrainForwardInputs(*[leaves[n] for n in "rwkvab"]))
+    grads = torch.autograd.grad((y, s), list(leaves.values()), (dy.to(cuda), ds.to(cuda)))
+    torch.cuda.synchronize()
+    assert pkg.read_device_status(0) == 0
+    parity.assert_close_bf16_store(y.detach().float().cpu().numpy(), y_ref, 1e-3, "y")
+    parity.assert_close_f32(s.detach().cpu().numpy(), s_ref, 1e-3, "next_state")
+    worst = {}
+    for n, got in zip(leaves, grads):
+        worst[n] = np.abs(got.float().cpu().numpy().astype(np.float64) - ref[n]).max() / np.abs(ref[n]).max()
+    print(scales, {n: f"{e:.1e}" for n, e in worst.items()})
+    assert all(e <= (1e-3 if n == "s0" else 5e-3) for n, e in worst.items()), worst
