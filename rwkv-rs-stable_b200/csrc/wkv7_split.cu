@@ -745,50 +745,115 @@ __device__ __forceinline__ void keep_top(uint32_t *tops, const float (&S)[4][4])
     if ((threadIdx.x & 31) == 0) tops[threadIdx.x >> 5] = most;
 }
 
+// Tiles of 32 tokens of a chain's tensors (a, r, b, k, w, and v or dY) in shared memory, one fetched while the one before is
+// used, with the decays of the current one.  For the 256 threads that recompute a chain.
+template <typename TIO>
+struct TokenTiles {
+    static constexpr int kTokens = 32, kPiece = 16 / (int)sizeof(TIO), kPieces = kN / kPiece, kTile = kTokens * kN;
+    const OperatorPtrs &in;
+    const TIO *x;
+    size_t base, step;   // of token 0, from token to token
+    TIO *room;
+    float *d;
+    __device__ TokenTiles(const OperatorPtrs &in, const TIO *x, unsigned char *smem, int bi, int h, int H, int Tlen)
+        : in(in), x(x), base(((size_t)bi * Tlen * H + h) * kN), step((size_t)H * kN), room(reinterpret_cast<TIO *>(smem)), d(reinterpret_cast<float *>(room + 12 * kTile)) {}
+    static __device__ void together() { asm volatile("bar.sync 9, 256;" ::: "memory"); }
+    __device__ const TIO *tile(int i, int tensor) const { return room + ((i & 1) * 6 + tensor) * kTile; }
+    __device__ void fetch(int i, int t0, int t1) const {
+#pragma unroll
+        for (int tensor = 0; tensor < 6; ++tensor)
+#pragma unroll
+            for (int idx = threadIdx.x; idx < kTokens * kPieces; idx += 256) {
+                const int tok = idx / kPieces, at = idx % kPieces * kPiece;
+                if (t0 + tok < t1) {
+                    const TIO *src = (tensor < 5 ? static_cast<const TIO *>(in.p[tensor]) : x) + base + (size_t)(t0 + tok) * step + at;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(tile(i, tensor) + tok * kN + at)), "l"(src) : "memory");
+                }
+            }
+    }
+    // tile i is there and its decays are known
+    __device__ void arrived(int i) const {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        together();
+        const TIO *w = tile(i, XW) + threadIdx.x * 8;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) d[threadIdx.x * 8 + e] = expf(-expf(static_cast<float>(w[e])));
+        together();
+    }
+    // four neighbouring channels of a token
+    static __device__ float4 four(const TIO *at) {
+        if constexpr (sizeof(TIO) == 4) return *reinterpret_cast<const float4 *>(at);
+        else {
+            const uint2 u = *reinterpret_cast<const uint2 *>(at);
+            const float2 lo = unpack_bf2(u.x), hi = unpack_bf2(u.y);
+            return make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+    }
+};
+constexpr size_t kTokenTilesBytes = 12 * 32 * kN * sizeof(float) + 32 * kN * sizeof(float);   // fp32
+static_assert(kTokenTilesBytes <= Scan<float>::kBars && kTokenTilesBytes <= Scan<__nv_bfloat16>::kBars, "the tiles lie where the stages were");
+
 // Token-by-token recomputation of one chain over tokens t0 .. t1 - 1, fp32 throughout: what a
 // CTA does when a value overflowed fp16 on the way, or the chain is flagged and no later kernel is there to take it.  Four
 // lanes per row; columns and sums in the order of the sequential scan (wkv7_seq.cu), whose bits it reproduces.
 template <typename TIO>
-__device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TIO *v, TIO *y, const float *s_in, float *s_out,
-                                                float *snapshots, uint32_t *tops, int bi, int h, int H, int Tlen, int t0, int t1) {
+__device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TIO *v, TIO *y, const float *s_in, float *s_out, float *snapshots,
+                                                uint32_t *tops, unsigned char *smem, int bi, int h, int H, int Tlen, int t0, int t1) {
+    using Tiles = TokenTiles<TIO>;
+    const Tiles tiles(in, v, smem, bi, h, H, Tlen);
     const int row = (int)threadIdx.x >> 2, c0 = ((int)threadIdx.x & 3) * 4;   // columns c0 + 16 kk + e
+    tiles.fetch(0, t0, t1);
     float S[4][4];
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
         for (int e = 0; e < 4; ++e) S[kk][e] = s_in ? s_in[row * kN + c0 + 16 * kk + e] : 0.f;
-    for (int t = t0; t < t1; ++t) {
-        if (snapshots != nullptr && t % kL == 0) {
-            keep_top(tops + t / kL * 8, S);
+    for (int i = 0, first = t0; first < t1; ++i, first += Tiles::kTokens) {
+        tiles.arrived(i);
+        tiles.fetch(i + 1, first + Tiles::kTokens, t1);
+        if (snapshots != nullptr && first % kL == 0) {
+            keep_top(tops + first / kL * 8, S);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) snapshots[(size_t)(t / kL) * kN * kN + accumulator_place(row, c0 + 16 * kk + e)] = S[kk][e];
+                for (int e = 0; e < 4; ++e) snapshots[(size_t)(first / kL) * kN * kN + accumulator_place(row, c0 + 16 * kk + e)] = S[kk][e];
         }
-        const size_t o = (((size_t)bi * Tlen + t) * H + h) * kN;
-        auto f = [&](int x, int kk, int e) -> float { return static_cast<float>(static_cast<const TIO *>(in.p[x])[o + c0 + 16 * kk + e]); };
-        float p[4] = {}, yy[4] = {};
+        const int count = min(Tiles::kTokens, t1 - first);
+        for (int u = 0; u < count; ++u) {
+            auto f = [&](int x, int kk) { return Tiles::four(tiles.tile(i, x) + u * kN + c0 + 16 * kk); };
+            float p[4] = {}, yy[4] = {};
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) p[e] = fmaf(S[kk][e], f(XA, kk, e), p[e]);
-        float sa = (p[0] + p[1]) + (p[2] + p[3]);
-        sa += __shfl_xor_sync(0xffffffffu, sa, 1);
-        sa += __shfl_xor_sync(0xffffffffu, sa, 2);
-        const float vi = static_cast<float>(v[o + row]);
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                S[kk][e] = fmaf(S[kk][e], expf(-expf(f(XW, kk, e))), fmaf(sa, f(XB, kk, e), vi * f(XK, kk, e)));
-                yy[e] = fmaf(S[kk][e], f(XR, kk, e), yy[e]);
+            for (int kk = 0; kk < 4; ++kk) {
+                const float4 a = f(XA, kk);
+                p[0] = fmaf(S[kk][0], a.x, p[0]);
+                p[1] = fmaf(S[kk][1], a.y, p[1]);
+                p[2] = fmaf(S[kk][2], a.z, p[2]);
+                p[3] = fmaf(S[kk][3], a.w, p[3]);
             }
-        float out = (yy[0] + yy[1]) + (yy[2] + yy[3]);
-        out += __shfl_xor_sync(0xffffffffu, out, 1);
-        out += __shfl_xor_sync(0xffffffffu, out, 2);
-        if (c0 == 0) {
-            if constexpr (sizeof(TIO) == 4) y[o + row] = out;
-            else y[o + row] = __float2bfloat16_rn(out);
+            float sa = (p[0] + p[1]) + (p[2] + p[3]);
+            sa += __shfl_xor_sync(0xffffffffu, sa, 1);
+            sa += __shfl_xor_sync(0xffffffffu, sa, 2);
+            const float vi = static_cast<float>(tiles.tile(i, 5)[u * kN + row]);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                const float4 d = *reinterpret_cast<const float4 *>(tiles.d + u * kN + c0 + 16 * kk), b = f(XB, kk), k = f(XK, kk), r = f(XR, kk);
+                S[kk][0] = fmaf(S[kk][0], d.x, fmaf(sa, b.x, vi * k.x));
+                S[kk][1] = fmaf(S[kk][1], d.y, fmaf(sa, b.y, vi * k.y));
+                S[kk][2] = fmaf(S[kk][2], d.z, fmaf(sa, b.z, vi * k.z));
+                S[kk][3] = fmaf(S[kk][3], d.w, fmaf(sa, b.w, vi * k.w));
+                yy[0] = fmaf(S[kk][0], r.x, yy[0]);
+                yy[1] = fmaf(S[kk][1], r.y, yy[1]);
+                yy[2] = fmaf(S[kk][2], r.z, yy[2]);
+                yy[3] = fmaf(S[kk][3], r.w, yy[3]);
+            }
+            float out = (yy[0] + yy[1]) + (yy[2] + yy[3]);
+            out += __shfl_xor_sync(0xffffffffu, out, 1);
+            out += __shfl_xor_sync(0xffffffffu, out, 2);
+            if (c0 == 0) {
+                TIO *o = y + tiles.base + (size_t)(first + u) * tiles.step + row;
+                if constexpr (sizeof(TIO) == 4) *o = out;
+                else *o = __float2bfloat16_rn(out);
+            }
         }
     }
     if (s_out != nullptr) {
@@ -801,44 +866,58 @@ __device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TI
 
 // The same for the gradient of the state, backwards over a whole chain; dv comes with it.  Snapshots: the gradient of the state
 // at the end of every chunk.
-__device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, const __nv_bfloat16 *dy, __nv_bfloat16 *dv, const float *g_in,
-                                                     float *g_out, float *snapshots, uint32_t *tops, int bi, int h, int H, int Tlen) {
+__device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, const __nv_bfloat16 *dy, __nv_bfloat16 *dv, const float *g_in, float *g_out,
+                                                     float *snapshots, uint32_t *tops, unsigned char *smem, int bi, int h, int H, int Tlen) {
+    using Tiles = TokenTiles<__nv_bfloat16>;
+    const Tiles tiles(in, dy, smem, bi, h, H, Tlen);
     const int row = (int)threadIdx.x >> 2, c0 = ((int)threadIdx.x & 3) * 4;
+    const int last = (Tlen - 1) / Tiles::kTokens * Tiles::kTokens;
+    tiles.fetch(0, last, Tlen);
     float G[4][4];
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
         for (int e = 0; e < 4; ++e) G[kk][e] = g_in ? g_in[row * kN + c0 + 16 * kk + e] : 0.f;
-    for (int t = Tlen - 1; t >= 0; --t) {
-        if (t == Tlen - 1 || t % kL == kL - 1) {
-            keep_top(tops + t / kL * 8, G);
+    for (int i = 0, first = last; first >= 0; ++i, first -= Tiles::kTokens) {
+        tiles.arrived(i);
+        if (first > 0) tiles.fetch(i + 1, first - Tiles::kTokens, Tlen);
+        for (int u = min(Tiles::kTokens, Tlen - first) - 1; u >= 0; --u) {
+            const int t = first + u;
+            if (t == Tlen - 1 || t % kL == kL - 1) {
+                keep_top(tops + t / kL * 8, G);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
+                for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) snapshots[(size_t)(t / kL) * kN * kN + accumulator_place(row, c0 + 16 * kk + e)] = G[kk][e];
-        }
-        const size_t o = (((size_t)bi * Tlen + t) * H + h) * kN;
-        auto f = [&](int x, int kk, int e) -> float { return __bfloat162float(static_cast<const __nv_bfloat16 *>(in.p[x])[o + c0 + 16 * kk + e]); };
-        const float dyi = __bfloat162float(dy[o + row]);
-        float dsa = 0.f, out = 0.f;
+                    for (int e = 0; e < 4; ++e) snapshots[(size_t)(t / kL) * kN * kN + accumulator_place(row, c0 + 16 * kk + e)] = G[kk][e];
+            }
+            auto f = [&](int x, int kk) { return Tiles::four(tiles.tile(i, x) + u * kN + c0 + 16 * kk); };
+            const float dyi = __bfloat162float(tiles.tile(i, 5)[u * kN + row]);
+            float dsa = 0.f, out = 0.f;
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
+            for (int kk = 0; kk < 4; ++kk) {
+                const float4 r = f(XR, kk), b = f(XB, kk), k = f(XK, kk);
+                const float rr[4] = {r.x, r.y, r.z, r.w}, bb[4] = {b.x, b.y, b.z, b.w}, kv[4] = {k.x, k.y, k.z, k.w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                G[kk][e] = fmaf(dyi, f(XR, kk, e), G[kk][e]);
-                dsa = fmaf(G[kk][e], f(XB, kk, e), dsa);
-                out = fmaf(G[kk][e], f(XK, kk, e), out);
+                for (int e = 0; e < 4; ++e) {
+                    G[kk][e] = fmaf(dyi, rr[e], G[kk][e]);
+                    dsa = fmaf(G[kk][e], bb[e], dsa);
+                    out = fmaf(G[kk][e], kv[e], out);
+                }
             }
 #pragma unroll
-        for (int x = 1; x <= 2; x <<= 1) {
-            dsa += __shfl_xor_sync(0xffffffffu, dsa, x);
-            out += __shfl_xor_sync(0xffffffffu, out, x);
+            for (int x = 1; x <= 2; x <<= 1) {
+                dsa += __shfl_xor_sync(0xffffffffu, dsa, x);
+                out += __shfl_xor_sync(0xffffffffu, out, x);
+            }
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                const float4 d = *reinterpret_cast<const float4 *>(tiles.d + u * kN + c0 + 16 * kk), a = f(XA, kk);
+                const float dd[4] = {d.x, d.y, d.z, d.w}, aa[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) G[kk][e] = fmaf(G[kk][e], dd[e], dsa * aa[e]);
+            }
+            if (c0 == 0) dv[tiles.base + (size_t)t * tiles.step + row] = __float2bfloat16_rn(out);
         }
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) G[kk][e] = fmaf(G[kk][e], expf(-expf(f(XW, kk, e))), dsa * f(XA, kk, e));
-        if (c0 == 0) dv[o + row] = __float2bfloat16_rn(out);
     }
     if (g_out != nullptr) {
 #pragma unroll
@@ -1294,8 +1373,8 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     if (((flagged && resolve_flagged) || (*bad & 2)) && tid < 256) {
         float *own = snapshots + (kKind == kPrefill ? 0 : (size_t)chain * n * kN * kN);
         uint32_t *top = tops + (kKind == kPrefill ? 0 : (size_t)chain * n * 8);
-        if constexpr (kGrad) scan_gradients_by_token(ptrs, v, y, s_in, s_out, own, top, bi, h, H, Tlen);
-        else scan_rows_by_token<TIO>(ptrs, v, y, s_in, s_out, kKind == kPrefill ? nullptr : own, top, bi, h, H, Tlen, chunk0 * kL, t_end);
+        if constexpr (kGrad) scan_gradients_by_token(ptrs, v, y, s_in, s_out, own, top, smem, bi, h, H, Tlen);
+        else scan_rows_by_token<TIO>(ptrs, v, y, s_in, s_out, kKind == kPrefill ? nullptr : own, top, smem, bi, h, H, Tlen, chunk0 * kL, t_end);
     }
 }
 

@@ -114,106 +114,150 @@ __device__ __forceinline__ bool tiny(const uint32_t (&x)[8]) {
     return !__any_sync(0xffffffffu, most >= kTiny) && __any_sync(0xffffffffu, most > 0.f);
 }
 
-// One chunk in fp32, token by token.  `scratch`: 36 KB, `sums`: 64 KB of shared memory.  Four lanes per value row, columns
-// c0 + 16 kk + e; sums over rows go through the warps' partial sums.
-__device__ __noinline__ void chunk_by_token(const ChunkArgs &p, int unit, float *scratch, float *sums) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int row = tid >> 2, c0 = (tid & 3) * 4;
+// One chunk in fp32, token by token.  Four lanes per value row, columns c0 + 16 kk + e, for u = S a and du = G b; then four lanes per
+// column, rows c0 + 16 kk + e, where with u and du known the state and its gradient need no sum over a row any more, and the sums over
+// rows that the gradients are stay within four lanes.  `raw`: 56 KB of shared memory for the chunk's tensors, `d`: 16 KB, `sums`: 64 KB.
+__device__ __noinline__ void chunk_by_token(const ChunkArgs &p, int unit, __nv_bfloat16 *raw, float *d, float *sums) {
+    const int tid = threadIdx.x;
+    const int own = tid >> 2, c0 = (tid & 3) * 4;   // row, or column; of the other
     const int chain = unit / p.nchunks, chunk = unit % p.nchunks;
     const int valid = min(kL, p.T - chunk * kL);
     const size_t base = (((size_t)(chain / p.H) * p.T + chunk * kL) * p.H + chain % p.H) * kN, step = (size_t)p.H * kN;
-    float *u = scratch, *du = u + kL * kN, *part = du + kL * kN;   // [token][row]; [2][8 warps][64]
-    float *dr = sums, *da = dr + kL * kN, *db = da + kL * kN, *dk = db + kL * kN;
-    auto in = [&](int x, int t, int i) -> float { return __bfloat162float(p.in[x][base + t * step + i]); };
-    auto decay = [&](int t, int j) -> float { return expf(-expf(in(TW, t, j))); };
-    // column sums of two products over all rows
-    auto column_sums = [&](float (&m)[2][16], float *out0, float *out1) {
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float v = m[x][i];
-                for (int o = 4; o <= 16; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lane < 4) part[(x * 8 + warp) * kN + c0 + 16 * (i >> 2) + (i & 3)] = v;
-            }
-        __syncthreads();
-        if (tid < 2 * kN) {
-            float v = 0.f;
-            for (int w = 0; w < 8; ++w) v += part[((tid >> 6) * 8 + w) * kN + (tid & 63)];
-            (tid < kN ? out0 : out1)[tid & 63] = v;
-        }
-        __syncthreads();
-    };
-    float M[16];
-    auto load = [&](const float *src) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) M[i] = src[(size_t)unit * kN * kN + accumulator_place(row, c0 + 16 * (i >> 2) + (i & 3))];
-    };
-    auto col = [&](int i) { return c0 + 16 * (i >> 2) + (i & 3); };
+    float *u = sums, *du = u + kL * kN, *dr = du + kL * kN, *da = dr + kL * kN;
+    __syncthreads();   // (the tiles and the operands are no longer read)
+    for (int idx = tid; idx < kTensors * kL * 8; idx += kThreads) {
+        const int x = idx / (kL * 8), t = idx / 8 % kL, c = idx % 8 * 8;
+        if (t < valid) *reinterpret_cast<uint4 *>(raw + (x * kL + t) * kN + c) = *reinterpret_cast<const uint4 *>(p.in[x] + base + t * step + c);
+    }
     __syncthreads();
-    load(p.states);
+    for (int i = tid; i < valid * kN; i += kThreads) d[i] = expf(-expf(__bfloat162float(raw[TW * kL * kN + i])));
+    __syncthreads();
+    auto one = [&](int x, int t) -> float { return __bfloat162float(raw[(x * kL + t) * kN + own]); };
+    struct Four { float v[4]; };
+    auto four = [&](int x, int t, int kk) {
+        const uint2 w = *reinterpret_cast<const uint2 *>(raw + (x * kL + t) * kN + c0 + 16 * kk);
+        const float2 lo = unpack_bf2(w.x), hi = unpack_bf2(w.y);
+        return Four{{lo.x, lo.y, hi.x, hi.y}};
+    };
+    auto four_f32 = [&](const float *v, int t, int kk) {
+        const float4 w = *reinterpret_cast<const float4 *>(v + t * kN + c0 + 16 * kk);
+        return Four{{w.x, w.y, w.z, w.w}};
+    };
+    auto over_four = [](float x) {
+        x += __shfl_xor_sync(0xffffffffu, x, 1);
+        return x + __shfl_xor_sync(0xffffffffu, x, 2);
+    };
+    float M[4][4];
+    auto load = [&](const float *src, bool by_row) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int other = c0 + 16 * kk + e;
+                M[kk][e] = src[(size_t)unit * kN * kN + (by_row ? accumulator_place(own, other) : accumulator_place(other, own))];
+            }
+    };
+    // rows: u, then du
+    load(p.states, true);
     for (int t = 0; t < valid; ++t) {
         float sa = 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) sa = fmaf(M[i], in(TA, t, col(i)), sa);
-        sa += __shfl_xor_sync(0xffffffffu, sa, 1);
-        sa += __shfl_xor_sync(0xffffffffu, sa, 2);
-        if ((tid & 3) == 0) u[t * kN + row] = sa;
-        const float vi = in(TV, t, row);
+        for (int kk = 0; kk < 4; ++kk) {
+            const Four a = four(TA, t, kk);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) M[i] = fmaf(M[i], decay(t, col(i)), fmaf(sa, in(TB, t, col(i)), vi * in(TK, t, col(i))));
+            for (int e = 0; e < 4; ++e) sa = fmaf(M[kk][e], a.v[e], sa);
+        }
+        sa = over_four(sa);
+        if (c0 == 0) u[t * kN + own] = sa;
+        const float vi = one(TV, t);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const Four dd = four_f32(d, t, kk), b = four(TB, t, kk), k = four(TK, t, kk);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) M[kk][e] = fmaf(M[kk][e], dd.v[e], fmaf(sa, b.v[e], vi * k.v[e]));
+        }
+    }
+    load(p.gradients, true);
+    for (int t = valid - 1; t >= 0; --t) {
+        const float dy = one(TY, t);
+        float dsa = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const Four r = four(TR, t, kk), b = four(TB, t, kk);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                M[kk][e] = fmaf(dy, r.v[e], M[kk][e]);
+                dsa = fmaf(M[kk][e], b.v[e], dsa);
+            }
+        }
+        dsa = over_four(dsa);
+        if (c0 == 0) du[t * kN + own] = dsa;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const Four dd = four_f32(d, t, kk), a = four(TA, t, kk);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) M[kk][e] = fmaf(M[kk][e], dd.v[e], dsa * a.v[e]);
+        }
     }
     __syncthreads();
-    load(p.gradients);
-    for (int t = valid - 1; t >= 0; --t) {
-        const float dy = in(TY, t, row), vi = in(TV, t, row), ui = u[t * kN + row];
-        float m[2][16], dsa = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            M[i] = fmaf(dy, in(TR, t, col(i)), M[i]);
-            dsa = fmaf(M[i], in(TB, t, col(i)), dsa);
-            m[0][i] = M[i] * vi;
-            m[1][i] = M[i] * ui;
-        }
-        dsa += __shfl_xor_sync(0xffffffffu, dsa, 1);
-        dsa += __shfl_xor_sync(0xffffffffu, dsa, 2);
-        if ((tid & 3) == 0) du[t * kN + row] = dsa;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) M[i] = fmaf(M[i], decay(t, col(i)), dsa * in(TA, t, col(i)));
-        column_sums(m, dk + t * kN, db + t * kN);
-    }
-    load(p.states);
+    // columns: da and dr forwards, then the rest backwards
+    load(p.states, false);
     for (int t = 0; t < valid; ++t) {
-        const float sa = u[t * kN + row], dsa = du[t * kN + row], vi = in(TV, t, row), dy = in(TY, t, row);
-        float m[2][16];
+        const float dj = d[t * kN + own], b = one(TB, t), k = one(TK, t);
+        float sum_a = 0.f, sum_r = 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            m[0][i] = M[i] * dsa;
-            M[i] = fmaf(M[i], decay(t, col(i)), fmaf(sa, in(TB, t, col(i)), vi * in(TK, t, col(i))));
-            m[1][i] = M[i] * dy;
-        }
-        column_sums(m, da + t * kN, dr + t * kN);
-    }
-    float m[2][16];
+        for (int kk = 0; kk < 4; ++kk) {
+            const Four ui = four_f32(u, t, kk), dui = four_f32(du, t, kk), v = four(TV, t, kk), dy = four(TY, t, kk);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        m[0][i] = M[i] * p.gradients[(size_t)unit * kN * kN + accumulator_place(row, col(i))];
-        m[1][i] = 0.f;
-    }
-    column_sums(m, u, du);   // (u is no longer needed: its first row takes phi at the chunk's end)
-    if (tid < kN) {
-        float phi = u[tid];
-        for (int t = valid - 1; t >= 0; --t) {
-            const int i = t * kN + tid;
-            const size_t o = base + t * step + tid;
-            const float x = in(TB, t, tid) * db[i] + in(TK, t, tid) * dk[i] - in(TR, t, tid) * dr[i];
-            p.out[TA][o] = __float2bfloat16_rn(da[i]);
-            p.out[TR][o] = __float2bfloat16_rn(dr[i]);
-            p.out[TB][o] = __float2bfloat16_rn(db[i]);
-            p.out[TK][o] = __float2bfloat16_rn(dk[i]);
-            p.out[4][o] = __float2bfloat16_rn(-expf(in(TW, t, tid)) * (phi - x));
-            phi -= x - in(TA, t, tid) * da[i];
+            for (int e = 0; e < 4; ++e) {
+                sum_a = fmaf(M[kk][e], dui.v[e], sum_a);
+                M[kk][e] = fmaf(M[kk][e], dj, fmaf(ui.v[e], b, v.v[e] * k));
+                sum_r = fmaf(M[kk][e], dy.v[e], sum_r);
+            }
         }
+        sum_a = over_four(sum_a);
+        sum_r = over_four(sum_r);
+        if (c0 == 0) {
+            da[t * kN + own] = sum_a;
+            dr[t * kN + own] = sum_r;
+        }
+    }
+    float phi = 0.f, end[4][4];
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) end[kk][e] = M[kk][e];
+    load(p.gradients, false);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) phi = fmaf(end[kk][e], M[kk][e], phi);
+    phi = over_four(phi);
+    __syncwarp();   // (da and dr are this quad's own)
+    for (int t = valid - 1; t >= 0; --t) {
+        const float dj = d[t * kN + own], r = one(TR, t), a = one(TA, t);
+        float sum_k = 0.f, sum_b = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const Four ui = four_f32(u, t, kk), dui = four_f32(du, t, kk), v = four(TV, t, kk), dy = four(TY, t, kk);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                M[kk][e] = fmaf(dy.v[e], r, M[kk][e]);
+                sum_k = fmaf(M[kk][e], v.v[e], sum_k);
+                sum_b = fmaf(M[kk][e], ui.v[e], sum_b);
+                M[kk][e] = fmaf(M[kk][e], dj, dui.v[e] * a);
+            }
+        }
+        sum_k = over_four(sum_k);
+        sum_b = over_four(sum_b);
+        const float sum_a = da[t * kN + own], sum_r = dr[t * kN + own];
+        const float x = one(TB, t) * sum_b + one(TK, t) * sum_k - r * sum_r;
+        const size_t o = base + t * step + own;
+        const int q = tid & 3;   // (a lane of the four stores one of the gradients)
+        (q == 0 ? p.out[TA] : q == 1 ? p.out[TR] : q == 2 ? p.out[TB] : p.out[TK])[o] =
+            __float2bfloat16_rn(q == 0 ? sum_a : q == 1 ? sum_r : q == 2 ? sum_b : sum_k);
+        if (q == 0) p.out[4][o] = __float2bfloat16_rn(-expf(one(TW, t)) * (phi - x));
+        phi -= x - a * sum_a;
     }
     __syncthreads();
 }
@@ -725,7 +769,7 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         }
         if (over || bad) {
             if (over && unit + (int)gridDim.x < p.units) fetch(unit + (int)gridDim.x);
-            chunk_by_token(p, unit, reinterpret_cast<float *>(smem + buf * kTilesBytes), reinterpret_cast<float *>(smem + kS));
+            chunk_by_token(p, unit, reinterpret_cast<__nv_bfloat16 *>(smem + buf * kTilesBytes), reinterpret_cast<float *>(smem + kF), reinterpret_cast<float *>(smem + kS));
             fence_proxy_async();
             __syncthreads();
         }
