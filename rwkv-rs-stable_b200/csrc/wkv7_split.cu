@@ -702,7 +702,7 @@ struct Scan {
     static constexpr uint32_t kYTile = kL * kN * sizeof(TIO);
     static constexpr uint32_t kY = kZV + 2 * 2 * kPanel;          // two output tiles (fp32: each two panels of 32 channels)
     static constexpr uint32_t kBars = kY + 2 * kYTile;
-    static constexpr uint32_t kBytes = kBars + 320;
+    static constexpr uint32_t kBytes = kBars + 384;
     static_assert(kBytes <= 232448, "the scan exceeds an SM");
 };
 
@@ -790,8 +790,9 @@ struct TokenTiles {
         }
     }
 };
-constexpr size_t kTokenTilesBytes = 12 * 32 * kN * sizeof(float) + 32 * kN * sizeof(float);   // fp32
-static_assert(kTokenTilesBytes <= Scan<float>::kBars && kTokenTilesBytes <= Scan<__nv_bfloat16>::kBars, "the tiles lie where the stages were");
+// (the tiles, and behind them the state that the recomputation goes on from, lie where the stages were)
+constexpr uint32_t kStateThen = 12 * 32 * kN * sizeof(float) + 32 * kN * sizeof(float);
+static_assert(kStateThen + kN * kN * sizeof(float) <= Scan<float>::kZV && kStateThen + kN * kN * sizeof(float) <= Scan<__nv_bfloat16>::kZV, "shared memory");
 
 // Token-by-token recomputation of one chain over tokens t0 .. t1 - 1, fp32 throughout: what a
 // CTA does when a value overflowed fp16 on the way, or the chain is flagged and no later kernel is there to take it.  Four
@@ -864,15 +865,15 @@ __device__ __noinline__ void scan_rows_by_token(const OperatorPtrs &in, const TI
     }
 }
 
-// The same for the gradient of the state, backwards over a whole chain; dv comes with it.  Snapshots: the gradient of the state
+// The same for the gradient of the state, backwards from token t_end - 1 on; dv comes with it.  Snapshots: the gradient of the state
 // at the end of every chunk.
 __device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, const __nv_bfloat16 *dy, __nv_bfloat16 *dv, const float *g_in, float *g_out,
-                                                     float *snapshots, uint32_t *tops, unsigned char *smem, int bi, int h, int H, int Tlen) {
+                                                     float *snapshots, uint32_t *tops, unsigned char *smem, int bi, int h, int H, int Tlen, int t_end) {
     using Tiles = TokenTiles<__nv_bfloat16>;
     const Tiles tiles(in, dy, smem, bi, h, H, Tlen);
     const int row = (int)threadIdx.x >> 2, c0 = ((int)threadIdx.x & 3) * 4;
-    const int last = (Tlen - 1) / Tiles::kTokens * Tiles::kTokens;
-    tiles.fetch(0, last, Tlen);
+    const int last = (t_end - 1) / Tiles::kTokens * Tiles::kTokens;
+    tiles.fetch(0, last, t_end);
     float G[4][4];
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
@@ -880,10 +881,10 @@ __device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, con
         for (int e = 0; e < 4; ++e) G[kk][e] = g_in ? g_in[row * kN + c0 + 16 * kk + e] : 0.f;
     for (int i = 0, first = last; first >= 0; ++i, first -= Tiles::kTokens) {
         tiles.arrived(i);
-        if (first > 0) tiles.fetch(i + 1, first - Tiles::kTokens, Tlen);
-        for (int u = min(Tiles::kTokens, Tlen - first) - 1; u >= 0; --u) {
+        if (first > 0) tiles.fetch(i + 1, first - Tiles::kTokens, t_end);
+        for (int u = min(Tiles::kTokens, t_end - first) - 1; u >= 0; --u) {
             const int t = first + u;
-            if (t == Tlen - 1 || t % kL == kL - 1) {
+            if (t == t_end - 1 || t % kL == kL - 1) {
                 keep_top(tops + t / kL * 8, G);
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk)
@@ -970,6 +971,8 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     volatile uint32_t *top_z = reinterpret_cast<volatile uint32_t *>(smem + SM::kBars + 144);
     volatile int *top_v = reinterpret_cast<volatile int *>(smem + SM::kBars + 224);
     volatile float *row_up = reinterpret_cast<volatile float *>(smem + SM::kBars + 256);
+    int *first_marked = reinterpret_cast<int *>(smem + SM::kBars + 320);
+    float *state_then = reinterpret_cast<float *>(smem + kStateThen);   // behind the last step run, if the chain goes on token by token
     static_assert(8 * (2 * NS + 5) <= 128, "the barriers' place");
     // chunk of step c (gradients run from the last to the first)
     auto at_step = [&](int c) { return kGrad ? n - 1 - c : c; };
@@ -986,6 +989,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         mbar_init(bar_scale + 1, 1);
         mbar_fence_init();
         *bad = 0;
+        *first_marked = n;
         for (int i = 0; i < 8; ++i) top_v[i] = 0;
         tma_prefetch_desc(&maps.v);
         tma_prefetch_desc(&maps.y);
@@ -1006,8 +1010,22 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     // that is not known (then it is the state's at the start).
     const uint32_t left = chunk0 > 0 ? *reinterpret_cast<volatile uint32_t *>(&flags[chain]) : 0u;
     int mark = (int)(left & 1u);
-    for (int c = tid; c < n; c += kScanThreads) mark |= *reinterpret_cast<const int *>(rec + (size_t)c * kRecord + kMarkAt);
+    int first = n;   // step of the first marked chunk
+    for (int c = tid; c < n; c += kScanThreads)
+        if (*reinterpret_cast<const int *>(rec + (size_t)at_step(c) * kRecord + kMarkAt)) {
+            mark = 1;
+            first = min(first, c);
+        }
     const bool flagged = __syncthreads_or(mark) != 0;
+    // Steps to run here: all; none for a chain that later kernels take; those in front of the first marked chunk for one that is
+    // continued token by token below.
+    int run = flagged ? 0 : n;
+    if (flagged && resolve_flagged) {
+        if (first < n) atomicMin(first_marked, first);
+        __syncthreads();
+        run = *reinterpret_cast<volatile int *>(first_marked);
+    }
+    run = __shfl_sync(0xffffffffu, run, 0);   // (uniform, as the warp's number)
     uint32_t leave = flagged && !resolve_flagged ? 1u : 0u;   // (warp 10 writes it at the end)
     const int t_end = min(Tlen, (chunk0 + n) * kL);
     // Z of a chunk is written: four state warps arrive, the issuing warp waits.  V of chunk c is converted and the chunk's
@@ -1016,13 +1034,13 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     auto v_arrive = [](int c) { asm volatile("bar.arrive %0, 288;" ::"r"(4 + (c & 1)) : "memory"); };
     uint32_t limit = 4000000u;   // polls a wait may take; after the first that expires this thread stops waiting, and the call reports it
     auto wait = [&](uint64_t *b, uint32_t parity) { limit = mbar_wait_tight(b, parity, limit) ? limit : 1u; };
-    if (flagged) {
+    if (run == 0) {
         // (recomputed below, or by the next kernel in line)
     } else if (warp == 8) {
         // ---------------- loader
         if (lane == 0) {
             int issued = 0;
-            for (int c = 0; c < n; ++c, ++issued) {
+            for (int c = 0; c < run; ++c, ++issued) {
                 const int s = c % NS;
                 if (c >= NS) wait(bar_empty + s, (uint32_t)((c / NS - 1) & 1));
                 if (limit == 1u) break;
@@ -1059,8 +1077,8 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
             }
             __syncwarp();
         };
-        if (n > 0) v_products(0);
-        for (int c = 0; c < n; ++c) {
+        v_products(0);
+        for (int c = 0; c < run; ++c) {
             const int s = c % NS, a = c & 1;
             asm volatile("bar.sync 3, 160;" ::: "memory");
             if (elect_one()) {
@@ -1073,7 +1091,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                 umma_commit(bar_empty + s);
             }
             __syncwarp();
-            if (c + 1 < n) v_products(c + 1);
+            if (c + 1 < run) v_products(c + 1);
         }
     } else if (warp >= 10) {
         // ---------------- V converters: tile -> fp16 rows in the order of the contraction index, 16-byte pieces; rows past the sequence's end belong to
@@ -1096,7 +1114,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
             const int x = (int)(left >> (8 + 8 * i)) & 255;
             carried[i] = x ? x : top_state(4);
         }
-        for (int c = 0; c < n; ++c) {
+        for (int c = 0; c < run; ++c) {
             const int s = c % NS, a = c & 1;
             wait(bar_full + s, (uint32_t)((c / NS) & 1));
             const uint32_t vt = sb + s * SM::kStage + SM::kV, out = sb + SM::kZV + a * 2 * kPanel + kPanel;
@@ -1168,7 +1186,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
             fence_proxy_async();
             v_arrive(c);
         }
-        if ((chunk0 + n) * kL < Tlen) {   // what the next segment's first chunks look back on
+        if (!flagged && (chunk0 + n) * kL < Tlen) {   // what the next segment's first chunks look back on
             asm volatile("bar.sync 7, 256;" ::: "memory");   // (the state warps have published every chunk)
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -1250,12 +1268,12 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
             }
             load_vec(0, gx, fx, g2);
             put_z(0, fx);
-            for (int c = 0; c < n; ++c) {
+            for (int c = 0; c < run; ++c) {
                 const int a = c & 1;
                 const uint32_t most = largest();
                 if (lane == 0) top_z[(c & 3) * 4 + quarter * 2 + hf] = most;   // for the converting warps
                 if constexpr (kKind != kPrefill) keep(c, most);
-                if (c + 1 < n) load_vec(c + 1, gxn, fxn, g2n);   // (while the products run)
+                if (c + 1 < run) load_vec(c + 1, gxn, fxn, g2n);   // (while the products run)
                 wait(bar_acc + a, (uint32_t)((c >> 1) & 1));
                 tc_fence_after();
                 uint32_t d[32];
@@ -1265,11 +1283,11 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
 #pragma unroll
                 for (int e = 0; e < 16; ++e)
                     Z[e] = __ffma2_rn(gx2, Z[e], mul2(gg, make_float2(__uint_as_float(d[2 * e]), __uint_as_float(d[2 * e + 1]))));
-                if (c + 1 < n) put_z(c + 1, fxn);
+                if (c + 1 < run) put_z(c + 1, fxn);
                 gx = gxn;
                 g2 = g2n;
             }
-            if ((chunk0 + n) * kL < Tlen) asm volatile("bar.sync 7, 256;" ::: "memory");
+            if (!flagged && (chunk0 + n) * kL < Tlen) asm volatile("bar.sync 7, 256;" ::: "memory");
             bool off = false;   // a non-finite operand upstream stays in the state for good
 #pragma unroll
             for (int e = 0; e < 16; ++e) off |= !(fabsf(Z[e].x) <= 3.0e38f) | !(fabsf(Z[e].y) <= 3.0e38f);
@@ -1278,7 +1296,13 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
             // the eight compute warps have all reported before the state is written: it may alias what a recomputation
             // starts from
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (*bad == 0 && s_out != nullptr) {
+            if (flagged) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    state_then[(i0 + 2 * e) * kN + jp] = Z[e].x;
+                    state_then[(i0 + 2 * e + 1) * kN + jp] = Z[e].y;
+                }
+            } else if (*bad == 0 && s_out != nullptr) {
 #pragma unroll
                 for (int e = 0; e < 16; ++e)
                     if (RWKV7_IN_RANGE(i0 + 2 * e + 1 < kN && jp < kN, status)) {
@@ -1293,8 +1317,8 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
             const bool elected = warp == 2 && lane == 0;
             float ysum = 0.f;    // a non-finite output makes the sum non-finite for good
             v_arrive(0);
-            if (n > 1) v_arrive(1);
-            for (int c = 0; c < n; ++c) {
+            if (run > 1) v_arrive(1);
+            for (int c = 0; c < run; ++c) {
                 const int a = c & 1;
                 wait(bar_acc + a, (uint32_t)((c >> 1) & 1));
                 tc_fence_after();
@@ -1309,7 +1333,7 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
                     d[e + 1] = __float_as_uint(y2.y);
                 }
                 tc_fence_before();
-                if (c + 2 < n) v_arrive(c + 2);
+                if (c + 2 < run) v_arrive(c + 2);
                 const int t0 = (chunk0 + at_step(c)) * kL;
                 float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -1368,13 +1392,15 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         if (tid == 0) atomicExch(status, (int)kDevTimeout);
         return;
     }
-    // A value beyond fp16 (or a flagged chain that nobody else takes): the chain once more, token by token, from the state
-    // this launch started with, which is still untouched.
+    // A value beyond fp16: the chain once more, token by token, from the state this launch started with, which is still
+    // untouched.  A flagged chain that nobody else takes: on from its first marked chunk.
     if (((flagged && resolve_flagged) || (*bad & 2)) && tid < 256) {
         float *own = snapshots + (kKind == kPrefill ? 0 : (size_t)chain * n * kN * kN);
         uint32_t *top = tops + (kKind == kPrefill ? 0 : (size_t)chain * n * 8);
-        if constexpr (kGrad) scan_gradients_by_token(ptrs, v, y, s_in, s_out, own, top, smem, bi, h, H, Tlen);
-        else scan_rows_by_token<TIO>(ptrs, v, y, s_in, s_out, kKind == kPrefill ? nullptr : own, top, smem, bi, h, H, Tlen, chunk0 * kL, t_end);
+        const int done = (*bad & 2) ? 0 : run;
+        const float *from = done > 0 ? state_then : s_in;
+        if constexpr (kGrad) scan_gradients_by_token(ptrs, v, y, from, s_out, own, top, smem, bi, h, H, Tlen, min(Tlen, (n - done) * kL));
+        else scan_rows_by_token<TIO>(ptrs, v, y, from, s_out, kKind == kPrefill ? nullptr : own, top, smem, bi, h, H, Tlen, (chunk0 + done) * kL, t_end);
     }
 }
 

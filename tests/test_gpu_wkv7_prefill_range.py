@@ -57,3 +57,27 @@ def test_fp32_chains_of_a_models_decays_stay_fp32(pkg, oracle, workloads, cuda, 
             tol = 1e-3 if b == h == 0 else 2e-5
             parity.assert_close_f32(y[b, :, h], y_ref[b, :, h], tol, f"y, chain {b},{h}")
             parity.assert_close_f32(s[b, h], s_ref[b, h], tol, f"state, chain {b},{h}")
+
+
+@pytest.mark.parametrize("alias", [False, True])
+def test_recomputation_goes_on_from_the_first_marked_chunk(pkg, oracle, workloads, cuda, alias):
+    """Chains under 512 tokens with a decay out of range in one chunk: the scan runs up to it and goes on token by token from the state
+    there; where a value in front of it overflows fp16, from the beginning.  The state may be updated in place."""
+    T, H = 500, 8
+    inp = workloads.wkv7_inputs(1, T, H, 64, seed=71, dtype=torch.bfloat16, state="normal")
+    for h, t in ((0, 0), (1, 63), (2, 64), (3, 200), (4, 499), (5, 320)):
+        inp["w"][0, t, h] = 2.8
+    inp["r"][0, 100, 5] *= 1e5      # (marked and overflowing)
+    inp["r"][0, 400, 3] *= 1e5      # (only behind the mark: token by token by then)
+    inp["r"][0, 10, 6] *= 1e5
+    f = {n: t.float().numpy() for n, t in inp.items()}
+    y_ref, s_ref = oracle.wkv7(*[f[n] for n in "rwkvab"], f["s0"])
+    d = {n: t.to(cuda) for n, t in inp.items()}
+    out = pkg.wkv7_statepass(d["s0"], pkg.Wkv7PretrainForwardInputs(*[d[n] for n in "rwkvab"]), reference_contract=False,
+                             next_state=d["s0"] if alias else None)
+    torch.cuda.synchronize()
+    assert pkg.read_device_status(0) == 0
+    y, s = out.output.float().cpu().numpy(), out.next_state.cpu().numpy()
+    for h in range(H):
+        parity.assert_close_bf16_store(y[:, :, h], y_ref[:, :, h], 1e-3, f"y, head {h}")
+        parity.assert_close_f32(s[:, h], s_ref[:, h], 1e-3, f"state, head {h}")

@@ -64,6 +64,7 @@ def test_training_step_of_many_chunks(pkg, oracle, workloads, cuda, B, T, H):
     inp["w"][0, :, 1] = 0.5                              # every chunk of a chain out of range
     inp["w"][1, -16:, 3] = 0.5                           # the last chunk
     inp["w"][0, :64, H - 1] = 0.5                        # the first
+    inp["w"][1, 64, 4] = 2.8                             # the second
     inp["r"][0, 16:32, 2] *= 1e5                         # a chunk whose receptances overflow
     inp["r"][1, -20:, 5] *= 1e5
     gen = torch.Generator().manual_seed(29)
@@ -85,7 +86,7 @@ def test_training_step_of_many_chunks(pkg, oracle, workloads, cuda, B, T, H):
             for n, whole, alone in zip(what, got, own):
                 assert torch.equal(chain(whole, b, h), alone), (n, b, h)
     assert pkg.read_device_status(0) == 0
-    for b, h in [(0, 0), (0, 1), (1, 3), (0, H - 1), (0, 2), (1, 5), (1, H - 1)]:
+    for b, h in [(0, 0), (0, 1), (1, 3), (0, H - 1), (0, 2), (1, 5), (1, 4), (1, H - 1)]:
         f = {n: chain(inp[n], b, h).float().numpy() for n in names}
         y_ref, s_ref = oracle.wkv7_train(*[f[n] for n in "rwkvab"], s0=f["s0"], chunk_len=16)[:2]
         ref = oracle.wkv7_backward(*[f[n] for n in "rwkvab"], chain(dy, b, h).float().numpy(), s0=f["s0"], ds_out=chain(ds, b, h).numpy())
