@@ -178,8 +178,9 @@ int rwkv7_selftest_bounded_wait(int device, int64_t max_polls, rwkv7_stream stre
  */
 
 /* Scratch bytes the WKV7 entry points prefer for this shape (0 for the sequential and decode kernels; B*H*4
- * for the tf32 chunked kernel; for the two-kernel prefill the flags, a carried state per
- * chain and 32.5 KB per 64-token chunk of a segment of the call, at most 768 MB of operators).  A smaller
+ * for the tf32 chunked kernel; for the two-kernel prefill the flags and 32.5 KB per 64-token chunk of a segment of the call, at most 768 MB of
+ * operators, and a carried state per chain where a call has several segments; for BF16 calls under 512 tokens of so many chains
+ * that one chunk of each is more, B*H*4 for the tf32 kernel).  A smaller
  * workspace is accepted: the call is cut into more segments, and below one chunk per chain the tf32 kernel
  * (BF16 tensors) or the sequential scan runs instead.  The size depends on the SM count of the calling thread's
  * current device. */

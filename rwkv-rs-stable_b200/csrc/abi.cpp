@@ -348,7 +348,10 @@ int rwkv7_selftest_bounded_wait(int device, int64_t max_polls, rwkv7_stream stre
 size_t rwkv7_wkv7_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int32_t dtype) {
     const int path = g_wkv7_path.load();
     if (path == RWKV7_WKV7_SEQUENTIAL) return 0;
-    if ((path == RWKV7_WKV7_SPLIT || (path == RWKV7_WKV7_AUTO && T >= split_min_tokens(dtype == RWKV7_BF16))) &&
+    // (Short calls of very many chains: their operators would be several times the call's own tensors, 1.4 GB for 1024 x 64 tokens x 40
+    // heads; such a call is not asked for that much and takes the tf32 kernel, unless its workspace is larger all the same.)
+    const bool modest = path == RWKV7_WKV7_SPLIT || T >= kSplitTiersTokens || wkv7_split_in_budget(B, H);
+    if ((path == RWKV7_WKV7_SPLIT || (path == RWKV7_WKV7_AUTO && T >= split_min_tokens(dtype == RWKV7_BF16))) && modest &&
         (dtype == RWKV7_BF16 || dtype == RWKV7_F32) && N == 64)
     {
         // (the size depends on whether the scan will overlap the operator kernel, i.e. on the SM count of

@@ -1445,8 +1445,8 @@ constexpr size_t kOperatorBudget = (size_t)768 << 20;
 
 // ---- host side ------------------------------------------------------------------------------
 //
-// Workspace: [flags: one int per chain][4 KB spare][carried fp32 state per chain][records of buffer 0][records of buffer 1].
-// A call is cut into segments of chunks.  With at most as many chains as SMs the scan of a segment
+// Workspace: [flags: one int per chain][carried fp32 state per chain][records of buffer 0][records of buffer 1]; a call of one
+// segment carries nothing.  A call is cut into segments of chunks.  With at most as many chains as SMs the scan of a segment
 // leaves most of the GPU idle (one latency-bound CTA per chain), so it runs on a second stream beside
 // the operator kernel of the next segment, which writes the other buffer.
 
@@ -1460,17 +1460,18 @@ struct WorkspaceLayout {
     int buffers;     // 1 or 2
 };
 
-size_t fixed_part(size_t chains) {
-    return align_up(chains * sizeof(int)) + align_up(kMaxSegments * sizeof(int)) + align_up(chains * kN * kN * sizeof(float));
+// What lies in front of the records.  (4 KB of a cut call's are not used; callers who work out the least size have counted them.)
+size_t fixed_part(size_t chains, bool cut) {
+    return align_up(chains * sizeof(int)) + (cut ? 4096 + align_up(chains * kN * kN * sizeof(float)) : 0);
 }
 
-WorkspaceLayout layout_for(size_t chains, size_t seg, int buffers) {
+WorkspaceLayout layout_for(size_t chains, size_t seg, int buffers, bool cut) {
     WorkspaceLayout l{};
     l.seg = seg;
     l.buffers = buffers;
     l.flags = 0;
-    l.carry = align_up(chains * sizeof(int)) + align_up(kMaxSegments * sizeof(int));
-    size_t off = l.carry + align_up(chains * kN * kN * sizeof(float));
+    l.carry = align_up(chains * sizeof(int)) + 4096;
+    size_t off = fixed_part(chains, cut);
     for (int b = 0; b < 2; ++b) {
         l.records[b] = off;
         if (b < buffers) off += chains * seg * kRecord;
@@ -1651,17 +1652,19 @@ int wkv7_split_overlap() { return g_split_overlap.load(); }
 void wkv7_set_split_overlap(int on) { g_split_overlap.store(on < 0 || on > 2 ? 1 : on); }
 
 size_t wkv7_split_min_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t N) {
-    (void)T;
     if (N != kN) return 0;
-    return layout_for((size_t)(B * H), 1, 1).total;
+    return layout_for((size_t)(B * H), 1, 1, T > kL).total;
 }
+
+bool wkv7_split_in_budget(int64_t B, int64_t H) { return (size_t)(B * H) * kRecord <= kOperatorBudget; }
 
 size_t wkv7_split_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int num_sms) {
     if (N != kN) return 0;
     const size_t chains = (size_t)(B * H);
     const size_t nchunks = (size_t)((T + kL - 1) / kL);
     const bool overlap = overlap_applies(chains, nchunks, num_sms);
-    return layout_for(chains, preferred_segment(chains, nchunks, overlap), overlap ? 2 : 1).total;
+    const size_t seg = preferred_segment(chains, nchunks, overlap);
+    return layout_for(chains, seg, overlap ? 2 : 1, seg < nchunks).total;
 }
 
 bool wkv7_split_supported(const Wkv7Args &p) {
@@ -1696,25 +1699,25 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
         if (part == nullptr && !shared_sm_overlap_pays(chains, (size_t)nchunks, p.num_sms)) overlap = false;
     }
     size_t seg = preferred_segment(chains, (size_t)nchunks, overlap);
-    const size_t fixed = fixed_part(chains);
-    if (workspace_bytes < fixed) return (int)cudaErrorInvalidValue;
-    const size_t per_chunk = chains * kRecord;
-    if (overlap && layout_for(chains, seg, 2).total > workspace_bytes) {
-        const size_t fit = (workspace_bytes - fixed) / (2 * per_chunk);
+    const size_t per_chunk = chains * kRecord, fixed = fixed_part(chains, true), room = workspace_bytes > fixed ? workspace_bytes - fixed : 0;
+    if (overlap && layout_for(chains, seg, 2, true).total > workspace_bytes) {
+        const size_t fit = room / (2 * per_chunk);
         if (fit >= 8) seg = fit;
         else overlap = false;
     }
     if (!overlap) {
         seg = preferred_segment(chains, (size_t)nchunks, false);
-        const size_t fit = (workspace_bytes - fixed) / per_chunk;
-        if (fit < 1) return (int)cudaErrorInvalidValue;
-        if (seg > fit) seg = fit;
+        if (seg < (size_t)nchunks || layout_for(chains, seg, 1, false).total > workspace_bytes) {
+            const size_t fit = room / per_chunk;
+            if (fit < 1) return (int)cudaErrorInvalidValue;
+            if (seg > fit) seg = fit;
+        }
     }
     if (seg > (size_t)nchunks) seg = (size_t)nchunks;
     const int nsegments = (int)(((size_t)nchunks + seg - 1) / seg);
     if (nsegments > kMaxSegments) return (int)cudaErrorInvalidValue;
     if (nsegments < 2) overlap = false;
-    const WorkspaceLayout lay = layout_for(chains, seg, overlap ? 2 : 1);
+    const WorkspaceLayout lay = layout_for(chains, seg, overlap ? 2 : 1, nsegments > 1);
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     int *flags = reinterpret_cast<int *>(ws + lay.flags);
     float *carry = reinterpret_cast<float *>(ws + lay.carry);

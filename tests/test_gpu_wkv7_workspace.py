@@ -41,3 +41,32 @@ def test_workspace_off_the_bulk_copies_boundary(pkg, oracle, workloads, cuda, T,
     close = parity.assert_close_bf16_store if dtype == torch.bfloat16 else parity.assert_close_f32
     close(out.output.float().cpu().numpy(), y_ref, 1e-3, "y")
     parity.assert_close_f32(out.next_state.cpu().numpy(), s_ref, 1e-3, "state")
+
+
+@pytest.mark.parametrize("B,T,H,chunks", [(2, 64, 3, 1), (1, 500, 5, 8), (2, 640, 3, 10)])
+def test_workspace_of_a_call_that_is_not_cut(pkg, workloads, cuda, B, T, H, chunks):
+    """Nothing is carried from segment to segment where there is one: flags and operators are all the call asks for and needs; a
+    byte less cuts it, with the same bits, or (one chunk) gives it to the tf32 kernel."""
+    inp = workloads.wkv7_inputs(B, T, H, 64, seed=103, dtype=torch.bfloat16, device=cuda, state="normal")
+    seq = pkg.Wkv7PretrainForwardInputs(*[inp[n] for n in "rwkvab"])
+    need = pkg.lib().rwkv7_wkv7_workspace_bytes(B, T, H, 64, pkg.BF16)
+    assert need == 256 + chunks * B * H * 33280
+    full = pkg.wkv7_statepass(inp["s0"], seq, reference_contract=False)
+    tail = 2 if T >= 512 else 0
+    for given, launches in ((need, 2 + tail), (need - 1, 4 + tail if chunks > 1 else 2)):
+        ws = torch.full((need + 4096,), 77, dtype=torch.uint8, device=cuda)
+        before = pkg.kernel_launch_count()
+        out = pkg.wkv7_statepass(inp["s0"], seq, reference_contract=False, workspace=ws[:given])
+        torch.cuda.synchronize()
+        assert pkg.kernel_launch_count() - before == launches and (ws[given:] == 77).all()
+        if given == need or chunks > 1:
+            assert torch.equal(out.output, full.output) and torch.equal(out.next_state, full.next_state)
+    assert pkg.read_device_status(0) == 0
+
+
+def test_workspace_of_very_many_short_chains(pkg, cuda):
+    """1024 x 64 tokens x 40 heads: the tf32 kernel's ints, not 1.4 GB of operators; 24 000 chains still get theirs."""
+    ask = lambda B, T, H: pkg.lib().rwkv7_wkv7_workspace_bytes(B, T, H, 64, pkg.BF16)  # noqa: E731
+    assert ask(1024, 64, 40) == 1024 * 40 * 4
+    assert ask(600, 64, 40) == 96000 + 600 * 40 * 33280
+    assert ask(1024, 512, 40) > 1 << 30
