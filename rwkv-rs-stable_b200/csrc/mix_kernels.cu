@@ -158,27 +158,45 @@ __device__ __forceinline__ int64_t load_id(const void *ids, int dtype, int64_t b
     return (int64_t) reinterpret_cast<const int32_t *>(ids)[b];
 }
 
-// `next` == `state`: the carried tokens are updated in place.  Otherwise the CTAs behind those of the sequences write `next`, a slot
-// each: the last token of the sequence that names it, else what `state` holds.
+// `next` == `state`: the carried tokens are updated in place.  Otherwise the CTAs behind those of the sequences write `next`, some slots
+// each: the last token of the sequence that names a slot, else what `state` holds.  Each of them reads all ids once, so there
+// are no more than four per SM, but for kMostSlots slots each, and then a warp copies a slot.
+constexpr int kMostSlots = 256;
 template <typename T, int EPV>
 __global__ void __launch_bounds__(256)
 token_shift_diff_kernel(const T *__restrict__ x, const T *state, T *next, const void *__restrict__ ids, int ids_dtype,
-                        T *__restrict__ diff, int64_t B, int64_t Tlen, int64_t C, int64_t S, int per_block, int *status) {
+                        T *__restrict__ diff, int64_t B, int64_t Tlen, int64_t C, int64_t S, int per_block, int slots_per_block, int *status) {
     const int64_t CV = C / EPV;
     const int64_t blocks_per_seq = (Tlen + per_block - 1) / per_block;
     if (blockIdx.x >= B * blocks_per_seq) {
-        const int64_t slot = blockIdx.x - B * blocks_per_seq;
-        __shared__ int named_by;
-        if (threadIdx.x == 0) named_by = -1;
+        const int64_t slot0 = (blockIdx.x - B * blocks_per_seq) * slots_per_block;
+        const int slots = (int)imin(slots_per_block, S - slot0);
+        __shared__ int named_by[kMostSlots];
+        for (int s = threadIdx.x; s < slots; s += blockDim.x) named_by[s] = -1;
         __syncthreads();
-        for (int64_t b = threadIdx.x; b < B; b += blockDim.x)
-            if (load_id(ids, ids_dtype, b) == slot) atomicMax(&named_by, (int)b);
+        for (int64_t b0 = threadIdx.x; b0 < B; b0 += 8 * blockDim.x) {
+            int64_t s[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s[u] = b0 + u * blockDim.x < B ? load_id(ids, ids_dtype, b0 + u * blockDim.x) - slot0 : -1;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (s[u] >= 0 && s[u] < slots) atomicMax(&named_by[s[u]], (int)(b0 + u * blockDim.x));
+        }
         __syncthreads();
-        const T *from = named_by < 0 ? state + slot * C : x + ((int64_t)named_by * Tlen + Tlen - 1) * C;
-        for (int64_t cv = threadIdx.x; cv < CV; cv += blockDim.x) {
-            Pack<T, EPV> v;
-            v.load(from + cv * EPV);
-            v.store(next + slot * C + cv * EPV);
+        const int threads = slots == 1 ? blockDim.x : 32;   // of a slot
+        const int first = slots == 1 ? threadIdx.x : threadIdx.x & 31;
+        for (int s = slots == 1 ? 0 : threadIdx.x >> 5; s < slots; s += blockDim.x >> 5) {
+            const T *from = named_by[s] < 0 ? state + (slot0 + s) * C : x + ((int64_t)named_by[s] * Tlen + Tlen - 1) * C;
+            T *to = next + (slot0 + s) * C;
+            for (int64_t c0 = first; c0 < CV; c0 += 4 * threads) {
+                Pack<T, EPV> v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (c0 + u * threads < CV) v[u].load(from + (c0 + u * threads) * EPV);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (c0 + u * threads < CV) v[u].store(to + (c0 + u * threads) * EPV);
+            }
         }
         return;
     }
@@ -290,9 +308,12 @@ int launch_addcmul(const AddcmulArgs &p, cudaStream_t stream) {
 template <typename T, int EPV>
 static void launch_token_shift_t(const TokenShiftArgs &p, cudaStream_t stream) {
     const int per = rows_per_block(p.B * p.T, p.num_sms);
-    const int64_t blocks = p.B * ((p.T + per - 1) / per) + (p.next != p.state ? p.S : 0);
-    token_shift_diff_kernel<T, EPV><<<(unsigned)blocks, pick_threads(p.C / EPV), 0, stream>>>(
-        (const T *)p.x, (const T *)p.state, (T *)p.next, p.ids, p.ids_dtype, (T *)p.diff, p.B, p.T, p.C, p.S, per, p.status);
+    const int64_t fair = p.S / (4 * (int64_t)(p.num_sms > 0 ? p.num_sms : 1));
+    const int slots = (int)(fair < 1 ? 1 : imin(fair, kMostSlots));
+    const int threads = slots == 1 ? pick_threads(p.C / EPV) : 256;
+    const int64_t blocks = p.B * ((p.T + per - 1) / per) + (p.next != p.state ? (p.S + slots - 1) / slots : 0);
+    token_shift_diff_kernel<T, EPV><<<(unsigned)blocks, threads, 0, stream>>>(
+        (const T *)p.x, (const T *)p.state, (T *)p.next, p.ids, p.ids_dtype, (T *)p.diff, p.B, p.T, p.C, p.S, per, slots, p.status);
 }
 
 int launch_token_shift_diff(const TokenShiftArgs &p, cudaStream_t stream) {

@@ -110,3 +110,24 @@ def test_token_shift_diff_state_of_another_layout(pkg, oracle, cuda, layout, dty
     assert torch.equal(out.next_token_shift.float().cpu(), torch.from_numpy(s_ref)) and torch.equal(table, before)
     with pytest.raises(pkg.KernelInputsError):
         pkg.token_shift_diff_custom(x.to(cuda), state, ids.to(cuda), inplace_state=True)
+
+
+@pytest.mark.parametrize("B,S,C", [(5, 592, 16), (7, 1185, 24), (2100, 3000, 264), (4096, 180000, 8), (3, 1300, 17)])
+def test_token_shift_diff_of_many_slots(pkg, cuda, B, S, C):
+    """One, two and more slots per CTA (their number follows S and the SMs), the last CTA with fewer; of sequences that name one slot
+    the last one's token stays there."""
+    g = torch.Generator().manual_seed(11)
+    x = torch.randn(B, 3, C, generator=g).to(torch.bfloat16)
+    state = torch.randn(S, C, generator=g).to(torch.bfloat16)
+    ids = torch.randint(0, S, (B,), generator=g, dtype=torch.int32)
+    ids[:3] = torch.tensor([S - 1, 0, S // 2])
+    ids[-1] = ids[1]
+    out = pkg.token_shift_diff_custom(x.to(cuda), state.to(cuda), ids.to(cuda))
+    torch.cuda.synchronize()
+    assert pkg.read_device_status(0) == 0
+    want = state.clone()
+    for b in range(B):
+        want[ids[b]] = x[b, -1]
+    assert torch.equal(out.next_token_shift.cpu(), want)
+    carried = torch.cat([state[ids.long()][:, None].float(), x[:, :-1].float()], 1) - x.float()
+    _check(out.token_shifted_diff, carried.numpy().astype(np.float64), torch.bfloat16)
