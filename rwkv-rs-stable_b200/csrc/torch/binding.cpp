@@ -131,7 +131,8 @@ at::Tensor like(const at::Tensor &t) {
 // The outputs of a call, each like its own tensor.  Small ones share one allocation (at 512-byte boundaries, as the allocator itself
 // would place them): an output costs 0.9 us to allocate and wrap, and a decode step around WKV7 has thirteen.  Up to 1 MB
 // in all, because up to there the caching allocator cuts blocks from shared 2 MB segments anyway; larger outputs stay
-// separate, so that holding one of them holds no more memory than its own.
+// separate, so that holding one of them holds no more memory than its own.  For outputs that a step uses up together: whoever keeps or saves a
+// single one keeps the memory of all of the call's, up to that 1 MB.
 template <typename... Like>
 void outputs_like(at::Tensor *out, const Like &...tensors) {
     constexpr int n = sizeof...(Like);
@@ -500,8 +501,8 @@ PyObject *token_shift_diff(PyObject *const *a) {
     const at::Tensor state = copied ? given.detach().clone() : given;
     const bool inplace = !keep || copied;
     at::Tensor out[2];   // diff, next state
-    if (inplace) out[0] = like(x);
-    else outputs_like(out, x, state);
+    out[0] = like(x);
+    if (!inplace) out[1] = like(state);   // (its own memory: a server keeps it, and must not keep the step's difference with it)
     Desc xd(x), sd(state), idd(a[2]), dd(out[0]), nd;
     if (!inplace) nd.set(out[1]);
     const rwkv7_stream st = stream_of(x);

@@ -131,3 +131,11 @@ def test_token_shift_diff_of_many_slots(pkg, cuda, B, S, C):
     assert torch.equal(out.next_token_shift.cpu(), want)
     carried = torch.cat([state[ids.long()][:, None].float(), x[:, :-1].float()], 1) - x.float()
     _check(out.token_shifted_diff, carried.numpy().astype(np.float64), torch.bfloat16)
+
+
+def test_token_shift_state_holds_no_more_than_itself(pkg, cuda):
+    """The next state outlives the step: its storage is its own, not shared with the step's difference."""
+    x, state = torch.randn(4, 1, 64, device=cuda), torch.randn(6, 64, device=cuda)
+    out = pkg.token_shift_diff_custom(x, state, torch.arange(4, dtype=torch.int32, device=cuda))
+    kept = out.next_token_shift.untyped_storage()
+    assert kept.nbytes() == state.numel() * 4 and kept.data_ptr() != out.token_shifted_diff.untyped_storage().data_ptr()
