@@ -432,7 +432,7 @@ def main():
         if not gather_ok:
             raise SystemExit("cfg4 leg: the gathered y differs from the rank-local shards")
 
-    # ---- training forward (with saved tensors) and backward at configuration 1 ------------
+    # ---- configuration 1 trained: the step autograd takes, and the two calls with the reference's saved tensors ------------
     train = None
     if not args.no_train and rank == 0:
         peak_gbs, _ = measured_peaks()
@@ -457,9 +457,20 @@ def main():
         bws = torch.empty(pkg.wkv7_backward_workspace_bytes(B, T, H, N), dtype=torch.uint8, device=dev)
         bwd_ms = timed(lambda: pkg.wkv7_backward(tin, saved, dy, None, workspace=bws))
         bwd_seq_ms = timed(lambda: pkg.wkv7_backward(tin, saved, dy, None, parallel=False), reps=2)
+        leaves = [t.detach().clone().requires_grad_(True) for t in six]
+
+        def autograd_step():
+            out, _ = pkg.wkv7_statepass_autograd(None, pkg.Wkv7PretrainForwardInputs(*leaves))
+            torch.autograd.grad(out, leaves, dy)
+
+        step_ms = timed(autograd_step, reps=10)
+        step_bytes = 14 * seq_bytes + B * H * STATE_BYTES                        # 6 in, dy, y, 6 grads, S_T
+        del leaves
         fwd_bytes = 8 * seq_bytes + snap_bytes + B * H * STATE_BYTES             # 6 in, y and sa out, snapshots, S_T
         bwd_bytes = 14 * seq_bytes + snap_bytes + B * H * STATE_BYTES            # 6 in, sa, dy, 6 grads, snapshots, dS0
         train = {"workload": f"B={B} T={T} H={H} N={N} bf16, chunk_len 16",
+                 "autograd_step_ms": step_ms, "autograd_step_gb_per_s": step_bytes / (step_ms * 1e-3) / 1e9,
+                 "autograd_step_frac_of_hbm_peak": step_bytes / (step_ms * 1e-3) / 1e9 / peak_gbs, "autograd_step_algorithmic_bytes": step_bytes,
                  "forward_saved_ms": fwd_ms, "forward_saved_gb_per_s": fwd_bytes / (fwd_ms * 1e-3) / 1e9,
                  "forward_saved_frac_of_hbm_peak": fwd_bytes / (fwd_ms * 1e-3) / 1e9 / peak_gbs,
                  "backward_ms": bwd_ms, "backward_token_by_token_ms": bwd_seq_ms, "backward_gb_per_s": bwd_bytes / (bwd_ms * 1e-3) / 1e9,
@@ -824,7 +835,7 @@ def main():
             "lm_head_ce": pick(lm_head, "ms", "tflops", "frac_of_bf16_peak", "frac_of_bf16_sustained_peak"),
             "channel_mixer": pick(channel_mixer, "ms", "tflops", "frac_of_bf16_peak", "frac_of_bf16_sustained_peak"),
             "cfg2_forward": pick(forward, "ms", "tokens_per_s"),
-            "train": pick(train, "forward_saved_ms", "forward_saved_frac_of_hbm_peak", "backward_ms",
+            "train": pick(train, "autograd_step_ms", "autograd_step_frac_of_hbm_peak", "forward_saved_ms", "forward_saved_frac_of_hbm_peak", "backward_ms",
                           "backward_frac_of_hbm_peak"),
             "streaming_frac_of_hbm_peak": None if streaming is None else
                 {k: v["frac_of_hbm_peak"] for k, v in streaming.items() if isinstance(v, dict)},

@@ -138,7 +138,8 @@ int rwkv7_set_wkv7_cluster(int cluster_size);
  * library-owned stream; events order the two streams and the caller's stream continues after the last scan, so
  * the call keeps its stream semantics.  Where the driver offers no partitions, or a profiler is injected into the
  * process (Nsight Compute cannot profile kernels in green contexts), calls of 24 to 40 chains (on 148
- * SMs) use a second stream of the primary context instead, the scan CTAs beside operator CTAs.  Partitions,
+ * SMs) and at least 256 chunks use a second stream of the primary context instead, the scans on the SMs that the operator
+ * kernel leaves free.  Partitions,
  * streams and events are created per device on the first such call and kept until the process exits; the
  * enqueueing of overlapped calls is serialised per process.  0 puts every kernel on the caller's stream (same
  * results, bitwise), 1 is the schedule described (default), 2 forces the second-stream schedule without

@@ -1,7 +1,7 @@
 // Warp-level matrix instructions (mma.sync m16n8k16, fp16 operands, fp32 accumulators), the shared-memory matrix
 // loads that feed them, and the lane layouts both use.
 //
-// The per-chunk products of the WKV7 prefill are 16 to 64 wide and depend on one another.  Through tcgen05 every link
+// The products of a chunk that depend on one another (inverses, substitution, operator rows) are 16 to 64 wide.  Through tcgen05 every link
 // of that chain costs a commit, a barrier wait, a TMEM read, a conversion, a shared-memory tile and a proxy fence, about
 // a thousand cycles; here an accumulator is repacked in registers and is the next product's operand.  The instruction
 // runs at 1024 multiply-adds per cycle and SM (measured: 8.2 cycles per instruction and warp scheduler, 21 cycles from

@@ -343,7 +343,7 @@ PyObject *wkv7_backward(PyObject *const *a) {
 }
 
 // The node of a training step (see rwkv7_fused_wkv7_training_forward).  In native code because a short step is bound by its host
-// path: with the node in Python a step of 1 x 128 tokens x 12 heads took 130 us of it, now 117 (the engine is most of that).
+// path: with the node in Python a step of 1 x 128 tokens x 12 heads took 140 us, now 123 (the engine is most of that).
 struct TrainingStep : torch::autograd::Function<TrainingStep> {
     using Tensors = torch::autograd::variable_list;
 

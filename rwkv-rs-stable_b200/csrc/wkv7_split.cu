@@ -17,9 +17,9 @@
 //     S'[i][j'] = e^{c_L} S[i][j'] + sum_j S[i][j] P[j][j'] + sum_s V[s][i] Kt[s][j']
 //     y[t][i]   = sum_j W[t][j] S[i][j] + sum_s Ark[t][s] V[s][i].
 //
-// Every tensor-core operand is fp16 (the same 11-bit significand as tf32) and every product runs on warp-level
-// matrix instructions (see sm100_mma.cuh for why not tcgen05).  fp16 has a narrow exponent range, and the factors of the
-// four A matrices, e^{c_t} and e^{-c_s}, do not.  A chunk whose decay exceeds what the references below resolve is marked
+// Every tensor-core operand is fp16 (the same 11-bit significand as tf32).  The products of a chunk that depend on one another
+// run on warp-level matrix instructions (see sm100_mma.cuh), the 128 x 128 one in front of them and all of the scan's on
+// tcgen05.  fp16 has a narrow exponent range, and the factors of the four A matrices, e^{c_t} and e^{-c_s}, do not.  A chunk whose decay exceeds what the references below resolve is marked
 // and its chain flagged; non-finite values (keys or values beyond fp16) are detected in the scan.
 // Small values do not lose bits below fp16's normal numbers: r and k rows go in times a power of two where a 16-token block of
 // them stays below 2 (the factor comes out again in the scan), and the scan scales V and the state likewise per chunk.
@@ -74,7 +74,7 @@ __host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
 // Bound by shared-memory bandwidth (2.8 k cycles per chunk at one 128-byte access a cycle) and by the latency of a chunk's
 // phases, which the CTAs of an SM cover for one another; hence few warps per chunk, each with the largest tile its
 // registers hold (eight warps per chunk read a quarter more and were slower: 153 against 121 us).  Measured, 6144 chunks (8 x
-// 4096 tokens x 12 heads): 121 us, 3.7 TB/s; the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
+// 4096 tokens x 12 heads): 118 us, 3.8 TB/s (116 without looking for small rows); the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
 //   1. decays: warp = 16-token block, lane = channel pair; prefix and suffix products within the block
 //   2. scaled fp16 operands, in place over the bf16 tiles that TMA delivered
 //   3. the A matrices: one 128 x 128 tcgen05 product [a; r] [b; k]^T, read back a row per thread, lower triangle only; with
@@ -686,7 +686,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
 // Z is written, one for the V products (tile converted, accumulator read back).  Only the completion of products and the
 // arrival of a stage go through an mbarrier.  (A version on warp-level matrix instructions, the state in their
 // accumulators, was bound by shared-memory bandwidth: each warp reads its operator columns and all of Z and V, 1.8 k
-// cycles a chunk.)  Measured: 1.35 k cycles a chunk, 53 us for 64 chunks of up to 148 chains; 512 chains 6.1 TB/s, the roof.
+// cycles a chunk.)  Measured: 60 us for 64 chunks of 96 chains (57 without scales, see ScanKind); 512 chains 6.1 TB/s, the roof.
 // ------------------------------------------------------------------------------------------
 constexpr int kConverters = 4;                    // (one per token block of a chunk; with two the prefill's scan took 60.5 us, not 58.8)
 constexpr int kScanThreads = (10 + kConverters) * 32;
@@ -939,6 +939,7 @@ __device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, con
 // before it in the scan's order and of the state as it entered the chunk three steps back, which the state warps publish.
 // Forwards values are only scaled up: a chain that overflows fp16 is recomputed in fp32.  The choice does not depend on where a call
 // is cut into segments: what the first three chunks of the next segment look back on is handed on with the chain's flag.
+// Measured, training, 96 chains x 64 chunks: 72 and 75 us.
 enum ScanKind { kPrefill, kForTraining, kGradients };
 
 template <typename TIO, int kKind>
@@ -1484,22 +1485,24 @@ WorkspaceLayout layout_for(size_t chains, size_t seg, int buffers, bool cut) {
 // overlaps) against the few microseconds a segment boundary costs, within the operator budget.
 //
 // When the scan of a segment may run beside the operator kernel of the next one.  The scan is one latency-bound
-// CTA per chain (0.75 us per chunk), the operator kernel throughput work that fills every SM (2.8 us per chunk and SM):
-// with x = chains x 2.8 / (SMs x 0.75) the two in sequence take (x + 1) scan times.  On SM partitions (the scans on `chains` SMs rounded up to eight, the operator kernel on the rest)
-// they take max(x SMs / (SMs - R), 1): a gain while x SMs / (SMs - R) < x + 1, which on 148 SMs is up to about
-// 40 chains.  Measured (B200, 148 SMs; in sequence / on partitions, us): 12 chains x 1024 chunks 945 / 799;
-// 32 x 1024 1489 / 1336; 64 x 512 1195 / 1638.  Without partitions the scan CTAs sit beside operator CTAs (the
-// operator kernel then leaves as many SMs' worth of CTAs out as there are chains) and run at half their pace: 32 x 1024 1381-1411, but 12 x 1024
-// 1204 and 64 x 512 1424, both worse than in sequence; that schedule is kept for 24 to 40 chains where the driver
-// offers no partitions.  Short sequences do not pay either way (32 chains x 128 chunks 257 against 236 us: the
-// first operator kernel and the last scan overlap nothing; on partitions 32 x 128 216 against 207 us, but 24 x 192
-// 234 against 256 and 12 x 128 133 against 138).  Hence: at most 27 % as many chains as SMs and at least 192
-// chunks, or at most 11 % and at least 128.
+// CTA per chain (0.85 us per chunk), the operator kernel throughput work that fills every SM (2.8 us per chunk and SM).  On SM partitions
+// the scans have `chains` SMs rounded up to eight and the operator kernel the rest.  Without, the operator kernel leaves as many
+// SMs' worth of CTAs out as there are chains, and the scans, on a stream of higher priority, take the SMs that have no operator
+// CTA (a scan CTA's 217 KB and an operator CTA's 57 KB do not fit one SM).  Measured (B200, 148 SMs; in sequence / on partitions /
+// beside without partitions, the last from a captured graph, where that is what runs and in sequence takes the figure in brackets; us):
+//     chains x chunks    192               256                    512                    1024
+//     12                 207 / 210         269 / 271              502 / 481              973 / 895
+//     16                 220 / 220         284 / 281              542 / 497              1045 / 919
+//     24                 249 / 240         319 / 298 / 274 (316)  614 / 522 / 490 (623)  1216 / 956 / 914 (1205)
+//     32                 274 / 256         358 / 315 / 289 (361)  685 / 551 / 516 (693)  1376 / 1000 / 957 (1356)
+// and at 128 chunks 156 / 153 for 12 chains.  With fewer than 24 chains the schedule without partitions loses (12 x 512: 537 against
+// 502).  Hence: at most 27 % as many chains as SMs and at least 192 chunks, or at most 11 % and at least 128.  (That bound is
+// from kernels of other speeds; more chains have not been measured with these.)
 bool overlap_applies(size_t chains, size_t nchunks, int num_sms) {
     return wkv7_split_overlap() != 0 && num_sms > 0 && chains * 100 <= (size_t)num_sms * 27 &&
            (nchunks >= 192 || (nchunks >= 128 && chains * 100 <= (size_t)num_sms * 11));
 }
-// (the schedule beside operator CTAs, where partitions are not to be had)
+// (the schedule without partitions, where they are not to be had: from 16 % as many chains as SMs and 256 chunks on)
 bool shared_sm_overlap_pays(size_t chains, size_t nchunks, int num_sms) {
     return chains * 100 >= (size_t)num_sms * 16 && nchunks >= 256;
 }
@@ -1545,10 +1548,9 @@ DeviceStreams *device_streams(int device) {
 
 // ---- SM partitions (green contexts) for the overlapped schedule ----------------------------------
 // The scan of a segment and the operator kernel of the next one want different things from an SM: a scan CTA is
-// one latency-bound chain that must not be slowed down, an operator CTA is throughput work.  Sharing SMs (a scan
-// CTA beside an operator CTA) costs the scan about half its pace.  Where the driver offers it, the device's SMs
-// are therefore split once into two partitions, each with a stream of its own: the scans run two to an SM on
-// the small one, the operator kernels two to an SM on the rest, and neither sees the other's CTAs.
+// one latency-bound chain that needs an SM to itself, an operator CTA is throughput work, four to an SM, and holds up a scan
+// that waits for its SM.  Where the driver offers it, the device's SMs are therefore split once into two partitions, each with
+// a stream of its own, and neither kernel sees the other's CTAs.
 struct GreenApi {
     CUresult (*deviceGet)(CUdevice *, int) = nullptr;
     CUresult (*getRes)(CUdevice, CUdevResource *, CUdevResourceType) = nullptr;
@@ -1683,7 +1685,7 @@ int launch_wkv7_split(const Wkv7Args &p, void *workspace, size_t workspace_bytes
     const int nchunks = (int)((p.T + kL - 1) / kL);
     // The plan: overlapped (two buffers) when it applies and the workspace holds two segments of a useful
     // length, else one buffer with the longest segment that fits.
-    // (fp32 tensors: one operator CTA per SM and the three-stage scan, which does not fit beside it)
+    // (fp32 tensors stay in sequence: the schedules have not been measured with their kernels)
     bool overlap = p.bf16 && overlap_applies(chains, (size_t)nchunks, p.num_sms);
     // The second stream and its events, or the two SM partitions with theirs, are shared by all calls on a device:
     // the enqueueing of an overlapped call is serialised per process from here on.
