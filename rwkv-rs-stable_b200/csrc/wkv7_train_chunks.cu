@@ -268,7 +268,7 @@ __device__ __noinline__ void chunk_by_token(const ChunkArgs &p, int unit, __nv_b
 // it (S mu, G rho, U, dU) is left in shared memory, and then warp = (block, half of the channels) sums over value rows.
 //
 // Bound by latency with two warps per scheduler (225 KB of shared memory leave room for one CTA): of 13.7 k cycles a chunk the
-// matrix instructions take 4.3 k of a scheduler and shared memory 8 k wavefronts.  Measured, 6144 chunks: 330 us; the fp32
+// matrix instructions take 4.3 k of a scheduler and shared memory 8 k wavefronts.  Measured, 6144 chunks: 340 us, and 11 more since V and k, dY and r have scales of their own; the fp32
 // replay per 16 tokens that this replaced took 880, and 90 for the reversed copies it needed.  Four more warps that prepare the next
 // chunk meanwhile gained nothing (350 us): they share the port and the issue slots.
 __global__ void __launch_bounds__(kThreads, 1)
