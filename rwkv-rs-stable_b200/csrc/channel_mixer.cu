@@ -13,8 +13,9 @@
 // hidden activation never exists unactivated: the first GEMM's epilogue squares the
 // rectified accumulator before it is rounded to bf16.
 //
-// GEMM kernel: out[M,N] = act(A[M,K] . B[N,K]^T), A and B row-major bf16 (both "K-major"),
-// fp32 accumulation in TMEM, bf16 output.  Persistent CTAs, one per SM; a tile is 128 x 256;
+// GEMM: out[M,N] = act(A[M,K] . B[N,K]^T), A and B row-major bf16 (both "K-major"), fp32 accumulation in TMEM, bf16 output.
+// From 129 rows on mostly by pairs of CTAs (gemm_tn_bf16_pair_kernel, see gemm_pair_width and sm100_pair_gemm.cuh).  Few rows, and
+// rows that fill their blocks of 256 badly, by single CTAs: persistent, one per SM; a tile is 128 x 256;
 // tiles are walked with the column block fastest, so that the CTAs running together share a
 // few row blocks of A and sweep all of B, and both stay in L2.  Warp roles as in the LM-head
 // kernel: warp 0 requests A and B tiles by TMA (128-byte swizzle, K slices of 64, 4-stage
@@ -26,10 +27,13 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "kernels.h"
+#include "launch.h"
 #include "rwkv7_b200.h"
+#include "sm100_pair_gemm.cuh"
 #include "sm100_umma.cuh"
 
 namespace rwkv7 {
@@ -49,6 +53,26 @@ struct GemmMaps {
 };
 
 enum { kEpiNone = 0, kEpiReluSquare = 1, kEpiPartial = 2 };   // partial: fp32 sums over one piece of K
+
+// 32 neighbouring accumulators of a row, from column c0 of N on (a multiple of 8), activated, rounded and stored: `nvec` pieces of eight.
+template <int EPI>
+__device__ __forceinline__ void store_row(const uint32_t (&v)[32], __nv_bfloat16 *dst, int nvec) {
+    uint4 pk[4];
+    unsigned *pw = &pk[0].x;
+#pragma unroll
+    for (int e = 0; e < 32; e += 2) {
+        float x0 = __uint_as_float(v[e]), x1 = __uint_as_float(v[e + 1]);
+        if constexpr (EPI == kEpiReluSquare) {
+            x0 = fmaxf(x0, 0.f); x0 *= x0;
+            x1 = fmaxf(x1, 0.f); x1 *= x1;
+        }
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+        pw[e >> 1] = *reinterpret_cast<const unsigned *>(&h);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (q < nvec) *reinterpret_cast<uint4 *>(dst + q * 8) = pk[q];
+}
 
 template <int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -154,21 +178,7 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, void *__restrict__ ou
                         if (q < 2 * nvec) *reinterpret_cast<uint4 *>(prow + ch * 32 + q * 4) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                     continue;
                 }
-                uint4 pk[4];
-                unsigned *pw = &pk[0].x;
-#pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    float x0 = __uint_as_float(v[e]), x1 = __uint_as_float(v[e + 1]);
-                    if constexpr (EPI == kEpiReluSquare) {
-                        x0 = fmaxf(x0, 0.f); x0 *= x0;
-                        x1 = fmaxf(x1, 0.f); x1 *= x1;
-                    }
-                    const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-                    pw[e >> 1] = *reinterpret_cast<const unsigned *>(&h);
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (q < nvec) *reinterpret_cast<uint4 *>(orow + ch * 32 + q * 8) = pk[q];
+                store_row<EPI>(v, orow + ch * 32, nvec);
             }
             tc_fence_before();
             __syncwarp();
@@ -179,6 +189,56 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, void *__restrict__ ou
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 512);
+}
+
+// The same on pairs of CTAs (see sm100_pair_gemm.cuh), tiles of 256 x width, K uncut; persistent pairs, column block fastest.
+template <int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+gemm_tn_bf16_pair_kernel(const __grid_constant__ PairMaps maps, __nv_bfloat16 *__restrict__ out, int64_t M, int N, int K, int width, int n_tiles,
+                         int tiles, int *status) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    if (smem_u32(smem) & 1023u) {
+        if (threadIdx.x == 0) atomicExch(status, (int)kDevInternal);
+        return;
+    }
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
+    const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
+    auto items = [&](int i, PairItem &w) {
+        const int tile = first + i * step;
+        w = PairItem{tile / n_tiles * kPairM, tile % n_tiles * width, 0, (K + kPairK - 1) / kPairK};
+        return tile < tiles;
+    };
+    PairGemm gemm;
+    gemm.begin(smem, maps, warp);
+    // (launched with programmatic stream serialization: set up while the kernel before it finishes)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    bool ok = true;
+    if (warp == 0) {
+        if (elect_one()) ok = gemm.produce(maps, width, items);
+    } else if (warp == 1) {
+        if (gemm.rank == 0 && elect_one()) ok = gemm.multiply(width, items);
+    } else {
+        const int quarter = warp & 3;
+        PairItem w;
+        for (int i = 0; items(i, w); ++i) {
+            if (!gemm.complete(i)) { ok = false; break; }
+            const int64_t row = (int64_t)w.m0 + gemm.rank * 128 + quarter * 32 + lane;
+            const int n1 = min(N, w.n0 + width);
+            __nv_bfloat16 *orow = out + row * N + w.n0;
+#pragma unroll 1
+            for (int c = 0; c < n1 - w.n0; c += 32) {
+                uint32_t v[32];
+                tmem_ld32(gemm.tmem + ((uint32_t)(quarter * 32) << 16) + (i & 1) * kPairN + c, v);
+                tmem_ld_wait();
+                if (row < M) store_row<EPI>(v, orow + c, min(32, n1 - w.n0 - c) / 8);
+            }
+            gemm.release(i);
+        }
+    }
+    __syncwarp();
+    if (!ok) atomicExch(status, (int)kDevTimeout);
+    gemm.end(warp);
 }
 
 // Sums the pieces of K and applies the activation; one thread per four columns.
@@ -317,21 +377,28 @@ size_t gemm_partial_bytes(int64_t M, int64_t N, int64_t K) {
     return sp > 1 ? (size_t)sp * M * N * sizeof(float) : 0;
 }
 
-template <typename... Params, typename... Args>
-cudaError_t launch_serialized(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
-    if (e == cudaSuccess) count_launch();
-    return e;
+// Width of the tiles of a product on pairs of CTAs, 0 if it goes to single CTAs (`splits`: the pieces those would cut K in).  Compared is
+// what one worker does after the other, in cycles: a K slice costs the tensor core 2 cycles a column, and its loads 240 and 0.9 a column
+// (70 bytes a cycle and SM); single CTAs are a tenth slower at the same shape, and pieces of K write and read their sums.  Narrower tiles
+// fill the waves better but read A more often, which a launch bound by power pays for, hence 4 % against them.
+// Measured (B200, whole channel mixer; single CTAs / pairs with 256 columns throughout / as chosen here, us): 4096 rows at C = 2048 242 / 215 /
+// 208, 1024 rows 90 / 99 / 71, 1500 rows 110 / 102 / 85, 2048 rows at C = 2560 249 / 223 / 176, 3000 rows at C = 768 57 / 54 / 41,
+// 8191 rows at C = 4096 1964 / 1963 / 1625, 300 rows at C = 2560 62 / 89 / 62 (three blocks of 128 rows are two of 256: single CTAs).
+int gemm_pair_width(int64_t M, int64_t N, int64_t K, int num_sms, int splits) {
+    if (M <= kBM || num_sms < 2) return 0;
+    const int64_t slices = (K + kBK - 1) / kBK, tiles = (M + kBM - 1) / kBM * ((N + kBN - 1) / kBN);
+    double best = 1.1 * 512 * (splits > 1 ? (double)((slices + splits - 1) / splits) : (double)((tiles + num_sms - 1) / num_sms * slices));
+    if (splits > 1) best += 4000 + (double)splits * M * N * 8 / 2000;
+    int width = 0;
+    for (int w = kPairN; w >= 64; w -= 16) {
+        const int64_t pair_tiles = (M + kPairM - 1) / kPairM * ((N + w - 1) / w);
+        const double cost = (double)((pair_tiles + num_sms / 2 - 1) / (num_sms / 2) * slices) * std::max(2.0 * w, 240 + 0.9 * w) * (w < kPairN ? 1.04 : 1.0);
+        if (cost < best) {
+            best = cost;
+            width = w;
+        }
+    }
+    return width;
 }
 
 // out[M,N] = act(A[M,K] . B[N,K]^T); K and N multiples of 8, all pointers 16-byte aligned.
@@ -340,11 +407,23 @@ int launch_gemm(const void *a, const void *b, void *out, float *partials, size_t
                 int *status, cudaStream_t stream) {
     EncodeTiledFn encode = gemm_encode_fn();
     if (encode == nullptr) return (int)cudaErrorNotSupported;
+    const int splits = gemm_splits(M, N, K, num_sms < kMostSms ? num_sms : kMostSms, room);
+    if (const int width = gemm_pair_width(M, N, K, num_sms, splits)) {
+        PairMaps maps;
+        if (int e = encode_rows_by_k(encode, &maps.a, a, M, K, kPairM / 2)) return e;
+        if (int e = encode_rows_by_k(encode, &maps.b, b, N, K, width / 2)) return e;
+        const int n_tiles = (int)((N + width - 1) / width), tiles = (int)((M + kPairM - 1) / kPairM) * n_tiles;
+        cudaError_t e = cudaFuncSetAttribute(gemm_tn_bf16_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem);
+        if (e == cudaSuccess)
+            e = launch_serialized(gemm_tn_bf16_pair_kernel<EPI>, 2u * (unsigned)std::min(tiles, num_sms / 2), (unsigned)kPairThreads, kPairSmem, stream, maps,
+                                  (__nv_bfloat16 *)out, M, (int)N, (int)K, width, n_tiles, tiles, status);
+        return (int)e;
+    }
     GemmMaps maps;
     if (int e = encode_rows_by_k(encode, &maps.a, a, M, K, kBM)) return e;
     if (int e = encode_rows_by_k(encode, &maps.b, b, N, K, kBN)) return e;
     const int m_tiles = (int)((M + kBM - 1) / kBM), n_tiles = (int)((N + kBN - 1) / kBN);
-    const int tiles = m_tiles * n_tiles, splits = gemm_splits(M, N, K, num_sms < kMostSms ? num_sms : kMostSms, room);
+    const int tiles = m_tiles * n_tiles;
     const int items = tiles * splits;
     const unsigned grid = (unsigned)(items < num_sms ? items : num_sms);
     auto kernel = splits > 1 ? gemm_tn_bf16_kernel<kEpiPartial> : gemm_tn_bf16_kernel<EPI>;
