@@ -95,15 +95,19 @@ constexpr uint32_t kAak = kDiag + 4 * 1024;
 constexpr uint32_t kArb = kAak + 10 * kBlk;
 constexpr uint32_t kArk = kArb + 10 * kBlk;
 constexpr uint32_t kE = kArk;                         // block decays [4][64] (dead before A_rk is written; beyond w's tile)
-constexpr uint32_t kPow = kArk + 10 * kBlk;           // exponents of powers of two (block-wise references): 19 x [64] bytes
-constexpr uint32_t kBar1 = kPow + 19 * 64;
+constexpr uint32_t kPow = kArk + 10 * kBlk;           // powers of two (block-wise references): 11 x [64] fp16,
+constexpr uint32_t kPowExp = kPow + 11 * 128;         // and exponents of further ones: 8 x [64] bytes
+constexpr uint32_t kBar1 = kPowExp + 8 * 64;
 constexpr uint32_t kSmem1 = kBar1 + 64;
 static_assert(kE >= kTiles + 5 * kPanel, "the decays must not lie under w's tile");
 static_assert(4 * (kSmem1 + 1024) <= 233472, "four CTAs per SM");
 __host__ __device__ constexpr int below(int t) { return t * (t - 1) / 2; }   // first block of row t of A_ab
-// kPow rows: the a/r side and the b/k side of a diagonal block, block pairs (2,0) (3,0) (3,1), then per block what takes
+// kPow rows: the a/r side and the b/k side of a diagonal block, block pairs (2,0) (3,0) (3,1); kPowExp rows: per block what takes
 // an a/r operand to the scale of its column of A~ (PX) and a b/k operand to Be, Ke (PE).
-enum { PA = 0, PB = 4, PF = 8, PX = 11, PE = 15 };
+// (The first go with every matrix load of phase 3, 88 pairs a warp: as bytes, widened there, they were a fifth of a chunk's
+// instructions.  The last are multiplied into b and k once, by the warps that the inverses leave idle.  Measured, 3 x 2047 tokens x 32
+// heads at a model's decays: 73.9 -> 71.8 us.  There is no room for all of them as fp16.)
+enum { PA = 0, PB = 4, PF = 8, PX = 0, PE = 4 };
 
 struct OperatorMaps {
     CUtensorMap m[5];   // a, r, b, k, w as [B*T, H*N] bf16, box 64 x 64, 128-byte swizzle (bf16 tensors only)
@@ -293,15 +297,17 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                     mB[x] = tail * exp2_of(xe - x4 + kWideShift);
                     ef[x] = 127 - x4;
                     eg[x] = 0;
-                    signed char *pw = reinterpret_cast<signed char *>(smem + kPow) + ch + x;
-                    auto power = [&](int row, int e) { pw[row * 64] = (signed char)max(e, -100); };   // (fp16 ends at 2^-24)
+                    __half *pw = reinterpret_cast<__half *>(smem + kPow) + ch + x;
+                    signed char *pe = reinterpret_cast<signed char *>(smem + kPowExp) + ch + x;
+                    auto power = [&](int row, int e) { pw[row * 64] = __float2half_rn(exp2_of(max(e, -100))); };   // (fp16 ends at 2^-24)
+                    auto exponent = [&](int row, int e) { pe[row * 64] = (signed char)max(e, -100); };
                     const int ha = (xs - xe) >> 1;
                     power(PA + tb, ha - kWideShift);
                     power(PB + tb, xs - xe - ha - kWideShift);
                     if (tb < 3)   // (2,0), (3,0), (3,1): start of the row block over the end of the column block
                         power(PF + tb, exponent_of(tb == 0 ? p2 : p3) - exponent_of(tb == 2 ? p2 : p1));
-                    power(PX + tb, xs - 127 - kWideShift);
-                    power(PE + tb, x4 - xe - kWideShift);
+                    exponent(PX + tb, xs - 127 - kWideShift);
+                    exponent(PE + tb, x4 - xe - kWideShift);
                 }
             }
             if (tb == 3 && RWKV7_IN_RANGE(unit >= 0 && unit < units, status)) {
@@ -436,17 +442,17 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                     for (int s = 0; s <= t; ++s) {
                         uint32_t As[4] = {A[0], A[1], A[2], A[3]}, Bs[4];
                         ldsm4(Bs, cols + tile_cols(lane, 16 * s, kk));
-                        const uint32_t f = sb + kPow + kk * 16 + 2 * q;
+                        const uint32_t f = sb + kPow + kk * 32 + 4 * q;
                         if (t != s + 1) {
-                            const int pa = (s == t ? PA + t : PF + (t == 2 ? 0 : 1 + s)) * 64;
-                            const uint32_t lo = power_pair(f + pa), hi = power_pair(f + pa + 8);
+                            const int pa = (s == t ? PA + t : PF + (t == 2 ? 0 : 1 + s)) * 128;
+                            const uint32_t lo = lds32(f + pa), hi = lds32(f + pa + 16);
                             As[0] = mul_half2(As[0], lo);
                             As[1] = mul_half2(As[1], lo);
                             As[2] = mul_half2(As[2], hi);
                             As[3] = mul_half2(As[3], hi);
                         }
                         if (t == s) {
-                            const uint32_t lo = power_pair(f + (PB + t) * 64), hi = power_pair(f + (PB + t) * 64 + 8);
+                            const uint32_t lo = lds32(f + (PB + t) * 128), hi = lds32(f + (PB + t) * 128 + 16);
                             Bs[0] = mul_half2(Bs[0], lo);
                             Bs[1] = mul_half2(Bs[1], hi);
                             Bs[2] = mul_half2(Bs[2], lo);
@@ -490,7 +496,8 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
             }
         }
         __syncthreads();
-        // ---------------- 4. T_bb = (I - A_bb)^-1: two warps, a half-warp per diagonal block, a column per lane
+        // ---------------- 4. T_bb = (I - A_bb)^-1: two warps, a half-warp per diagonal block, a column per lane.  The other two
+        // take b and k to Be and Ke (block-wise references).
         {
             const int pair = (warp + seq) & 3;   // (which two warps changes from chunk to chunk: each sits on its own scheduler)
             if (pair < 2) {
@@ -514,6 +521,23 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                 unsigned char *dst = smem + kDiag + b * 1024 + (cc >> 3) * 256 + (cc & 7) * 2;
 #pragma unroll
                 for (int t = 0; t < 16; ++t) *reinterpret_cast<__half *>(dst + t * 16) = __float2half_rn(x[t]);
+            } else if (wide) {
+                const uint32_t rows = sb + kTiles + (pair == 2 ? XB : XK) * kPanel + (lane >> 3) * 128, piece = lane & 7;   // eight channels of every fourth token
+#pragma unroll 1
+                for (int b = 0; b < 4; ++b) {
+                    uint32_t f[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) f[e] = power_pair(sb + kPowExp + (PE + b) * 64 + piece * 8 + 2 * e);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint32_t o = rows + (16 * b + 4 * i) * 128 + ((piece ^ ((4 * i + (lane >> 3)) & 7)) << 4);
+                        uint32_t x[4];
+                        lds128(x, o);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) x[e] = mul_half2(x[e], f[e]);
+                        sts128(o, x);
+                    }
+                }
             }
         }
         __syncthreads();
@@ -534,7 +558,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
             };
             // a/r or b/k operand block, rows = channels 16 c.., times its row's power of two (block-wise references)
             auto row_power = [&](int table, int c, uint32_t (&X)[4]) {
-                const uint32_t f0 = power_twice(sb + kPow + table * 64 + 16 * c + g), f1 = power_twice(sb + kPow + table * 64 + 16 * c + g + 8);
+                const uint32_t f0 = power_twice(sb + kPowExp + table * 64 + 16 * c + g), f1 = power_twice(sb + kPowExp + table * 64 + 16 * c + g + 8);
                 X[0] = mul_half2(X[0], f0);
                 X[1] = mul_half2(X[1], f1);
                 X[2] = mul_half2(X[2], f0);
@@ -605,13 +629,11 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                 float c[2][2][4];
                 uint32_t X[4];
                 ldsm4_t(X, sb + kTiles + XK * kPanel + tile_cols(lane, 16 * ct, n));
-                if constexpr (kWide) row_power(PE + ct, n, X);
                 unpack8(X, c[1]);
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
                     uint32_t A[4];
                     ldsm4_t(A, sb + kTiles + XB * kPanel + tile_cols(lane, 16 * b, n));
-                    if constexpr (kWide) row_power(PE + b, n, A);
                     if (b == 0) {
                         mma16816_first(c[0][0], A, U[0][b][0], U[0][b][2]);
                         mma16816_first(c[0][1], A, U[0][b][1], U[0][b][3]);
@@ -631,7 +653,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                 uint32_t X[4];
                 ldsm4(X, sb + kTiles + XR * kPanel + tile_plain(lane, 16 * n, ct));
                 if constexpr (kWide) {
-                    const uint32_t fa = sb + kPow + (PX + n) * 64 + 16 * ct + 2 * q;
+                    const uint32_t fa = sb + kPowExp + (PX + n) * 64 + 16 * ct + 2 * q;
                     const uint32_t f0 = power_pair(fa), f1 = power_pair(fa + 8);
                     X[0] = mul_half2(X[0], f0);
                     X[1] = mul_half2(X[1], f0);
