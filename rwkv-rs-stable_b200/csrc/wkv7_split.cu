@@ -74,7 +74,7 @@ __host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
 // Bound by shared-memory bandwidth (2.8 k cycles per chunk at one 128-byte access a cycle) and by the latency of a chunk's
 // phases, which the CTAs of an SM cover for one another; hence few warps per chunk, each with the largest tile its
 // registers hold (eight warps per chunk read a quarter more and were slower: 153 against 121 us).  Measured, 6144 chunks (8 x
-// 4096 tokens x 12 heads): 118 us, 3.8 TB/s (116 without looking for small rows); the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
+// 4096 tokens x 12 heads): 112.5 us, 4.0 TB/s; the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
 //   1. decays: warp = 16-token block, lane = channel pair; prefix and suffix products within the block
 //   2. scaled fp16 operands, in place over the bf16 tiles that TMA delivered
 //   3. the A matrices: one 128 x 128 tcgen05 product [a; r] [b; k]^T, read back a row per thread, lower triangle only; with
@@ -82,7 +82,8 @@ __host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
 //   4. two warps: inverses of the four diagonal blocks I - A_bb in fp32 (forward substitution, a column per lane)
 //   5. warp = 16 columns j and 16 columns s of [A~ | A~k]: block forward substitution on the transposed system, where
 //      these columns are independent of all others, then every operator row from the same registers, and out.
-// The next chunk's tiles are brought into L2 meanwhile and requested behind phase 5, w first.
+// The next chunk's tiles are requested behind phase 5, w first.  (Bringing them into L2 during phase 2, through the same TMA unit, made
+// the loads of the SM's other chunks wait: 118.5 us, 112.5 without.)
 // ------------------------------------------------------------------------------------------
 constexpr int kOpThreads = 128;
 enum { XA = 0, XR = 1, XB = 2, XK = 3, XW = 4 };
@@ -227,13 +228,6 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
         sts_f2(sb + kE + (tb * 64 + ch) * 4, e.x, e.y);
         __syncthreads();
         if (*abort_flag) break;
-        if (kTma && tid == 0 && more) {   // the next chunk's tiles: into L2 now, here when there is room
-            const long long u = unit + gridDim.x;
-            const int cn = (int)(u / seg_chunks), x0 = (cn % H) * kN, y0 = (cn / H) * Tlen + (chunk0 + (int)(u % seg_chunks)) * kL;
-#pragma unroll
-            for (int x = 0; x < 5; ++x)
-                asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(&maps.m[x]), "r"(x0), "r"(y0) : "memory");
-        }
         // Every warp sees the whole chunk's decays (its 32 lanes hold all channels): no further agreement is needed.
         float E[2][4];
 #pragma unroll
