@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.h"
+#include "launch.h"
 #include "rwkv7_b200.h"
 
 namespace rwkv7 {
@@ -84,6 +85,8 @@ struct Mix6Ptrs {
 template <typename T, int EPV>
 __global__ void __launch_bounds__(256)
 mix6_kernel(const T *__restrict__ x, Mix6Ptrs ptrs, int64_t rows, int64_t Tlen, int64_t C, int per_block) {
+    wait_for_previous();
+    let_next_in();
     const int64_t CV = C / EPV;
     const int64_t row_begin = (int64_t)blockIdx.x * per_block;
     const int64_t row_end = imin(rows, row_begin + per_block);
@@ -121,6 +124,8 @@ struct AddcmulPtrs {
 template <typename T, int EPV, int NS>
 __global__ void __launch_bounds__(256)
 addcmul_kernel(const T *base, const T *__restrict__ diff, AddcmulPtrs ptrs, int64_t rows, int64_t C, int per_block) {
+    wait_for_previous();
+    let_next_in();
     const int64_t CV = C / EPV;
     const int64_t row_begin = (int64_t)blockIdx.x * per_block;
     const int64_t row_end = imin(rows, row_begin + per_block);
@@ -166,6 +171,8 @@ template <typename T, int EPV>
 __global__ void __launch_bounds__(256)
 token_shift_diff_kernel(const T *__restrict__ x, const T *state, T *next, const void *__restrict__ ids, int ids_dtype,
                         T *__restrict__ diff, int64_t B, int64_t Tlen, int64_t C, int64_t S, int per_block, int slots_per_block, int *status) {
+    wait_for_previous();
+    let_next_in();
     const int64_t CV = C / EPV;
     const int64_t blocks_per_seq = (Tlen + per_block - 1) / per_block;
     if (blockIdx.x >= B * blocks_per_seq) {
@@ -245,6 +252,9 @@ inline int pick_threads(int64_t CV) {
     return t;
 }
 
+template <typename First, typename... Rest>
+First first_parameter(void (*)(First, Rest...));
+
 }  // namespace
 
 int launch_mix6(const MixArgs &p, cudaStream_t stream) {
@@ -259,30 +269,20 @@ int launch_mix6(const MixArgs &p, cudaStream_t stream) {
     }
     const int per = rows_per_block(rows, p.num_sms);
     const unsigned grid = (unsigned)((rows + per - 1) / per);
-    if (p.bf16) {
-        using T = __nv_bfloat16;
-        if (vec_ok && p.C % 8 == 0)
-            mix6_kernel<T, 8><<<grid, pick_threads(p.C / 8), 0, stream>>>((const T *)p.x, ptrs, rows, p.T, p.C, per);
-        else
-            mix6_kernel<T, 1><<<grid, pick_threads(p.C), 0, stream>>>((const T *)p.x, ptrs, rows, p.T, p.C, per);
-    } else {
-        if (vec_ok && p.C % 4 == 0)
-            mix6_kernel<float, 4><<<grid, pick_threads(p.C / 4), 0, stream>>>((const float *)p.x, ptrs, rows, p.T, p.C, per);
-        else
-            mix6_kernel<float, 1><<<grid, pick_threads(p.C), 0, stream>>>((const float *)p.x, ptrs, rows, p.T, p.C, per);
-    }
-    count_launch();
-    return (int)cudaGetLastError();
+    auto go = [&](auto kernel, int64_t vectors) {
+        return (int)launch_serialized(kernel, grid, (unsigned)pick_threads(vectors), 0, stream, (decltype(first_parameter(kernel)))p.x, ptrs, rows, p.T, p.C, per);
+    };
+    using bf = __nv_bfloat16;
+    if (p.bf16) return vec_ok && p.C % 8 == 0 ? go(mix6_kernel<bf, 8>, p.C / 8) : go(mix6_kernel<bf, 1>, p.C);
+    return vec_ok && p.C % 4 == 0 ? go(mix6_kernel<float, 4>, p.C / 4) : go(mix6_kernel<float, 1>, p.C);
 }
 
 template <typename T, int EPV>
-static void launch_addcmul_t(const AddcmulArgs &p, const AddcmulPtrs &ptrs, cudaStream_t stream) {
+static cudaError_t launch_addcmul_t(const AddcmulArgs &p, const AddcmulPtrs &ptrs, cudaStream_t stream) {
     const int threads = pick_threads(p.C / EPV), per = rows_per_block(p.rows, p.num_sms);
     const unsigned grid = (unsigned)((p.rows + per - 1) / per);
-    if (p.nscale == 1)
-        addcmul_kernel<T, EPV, 1><<<grid, threads, 0, stream>>>((const T *)p.base, (const T *)p.diff, ptrs, p.rows, p.C, per);
-    else
-        addcmul_kernel<T, EPV, 5><<<grid, threads, 0, stream>>>((const T *)p.base, (const T *)p.diff, ptrs, p.rows, p.C, per);
+    return launch_serialized(p.nscale == 1 ? addcmul_kernel<T, EPV, 1> : addcmul_kernel<T, EPV, 5>, grid, (unsigned)threads, 0, stream, (const T *)p.base,
+                             (const T *)p.diff, ptrs, p.rows, p.C, per);
 }
 
 int launch_addcmul(const AddcmulArgs &p, cudaStream_t stream) {
@@ -294,40 +294,28 @@ int launch_addcmul(const AddcmulArgs &p, cudaStream_t stream) {
         ptrs.out[s] = p.out[s];
         vec_ok = vec_ok && aligned16(p.scale[s]) && aligned16(p.out[s]);
     }
-    if (p.bf16) {
-        if (vec_ok && p.C % 8 == 0) launch_addcmul_t<__nv_bfloat16, 8>(p, ptrs, stream);
-        else launch_addcmul_t<__nv_bfloat16, 1>(p, ptrs, stream);
-    } else {
-        if (vec_ok && p.C % 4 == 0) launch_addcmul_t<float, 4>(p, ptrs, stream);
-        else launch_addcmul_t<float, 1>(p, ptrs, stream);
-    }
-    count_launch();
-    return (int)cudaGetLastError();
+    using bf = __nv_bfloat16;
+    if (p.bf16) return (int)(vec_ok && p.C % 8 == 0 ? launch_addcmul_t<bf, 8>(p, ptrs, stream) : launch_addcmul_t<bf, 1>(p, ptrs, stream));
+    return (int)(vec_ok && p.C % 4 == 0 ? launch_addcmul_t<float, 4>(p, ptrs, stream) : launch_addcmul_t<float, 1>(p, ptrs, stream));
 }
 
 template <typename T, int EPV>
-static void launch_token_shift_t(const TokenShiftArgs &p, cudaStream_t stream) {
+static cudaError_t launch_token_shift_t(const TokenShiftArgs &p, cudaStream_t stream) {
     const int per = rows_per_block(p.B * p.T, p.num_sms);
     const int64_t fair = p.S / (4 * (int64_t)(p.num_sms > 0 ? p.num_sms : 1));
     const int slots = (int)(fair < 1 ? 1 : imin(fair, kMostSlots));
     const int threads = slots == 1 ? pick_threads(p.C / EPV) : 256;
     const int64_t blocks = p.B * ((p.T + per - 1) / per) + (p.next != p.state ? (p.S + slots - 1) / slots : 0);
-    token_shift_diff_kernel<T, EPV><<<(unsigned)blocks, threads, 0, stream>>>(
-        (const T *)p.x, (const T *)p.state, (T *)p.next, p.ids, p.ids_dtype, (T *)p.diff, p.B, p.T, p.C, p.S, per, slots, p.status);
+    return launch_serialized(token_shift_diff_kernel<T, EPV>, (unsigned)blocks, (unsigned)threads, 0, stream, (const T *)p.x, (const T *)p.state, (T *)p.next,
+                             p.ids, p.ids_dtype, (T *)p.diff, p.B, p.T, p.C, p.S, per, slots, p.status);
 }
 
 int launch_token_shift_diff(const TokenShiftArgs &p, cudaStream_t stream) {
     if (p.B == 0 || p.T == 0 || p.C == 0) return 0;  // T == 0: diff empty, state unchanged
     const bool vec_ok = aligned16(p.x) && aligned16(p.state) && aligned16(p.next) && aligned16(p.diff);
-    if (p.bf16) {
-        if (vec_ok && p.C % 8 == 0) launch_token_shift_t<__nv_bfloat16, 8>(p, stream);
-        else launch_token_shift_t<__nv_bfloat16, 1>(p, stream);
-    } else {
-        if (vec_ok && p.C % 4 == 0) launch_token_shift_t<float, 4>(p, stream);
-        else launch_token_shift_t<float, 1>(p, stream);
-    }
-    count_launch();
-    return (int)cudaGetLastError();
+    using bf = __nv_bfloat16;
+    if (p.bf16) return (int)(vec_ok && p.C % 8 == 0 ? launch_token_shift_t<bf, 8>(p, stream) : launch_token_shift_t<bf, 1>(p, stream));
+    return (int)(vec_ok && p.C % 4 == 0 ? launch_token_shift_t<float, 4>(p, stream) : launch_token_shift_t<float, 1>(p, stream));
 }
 
 }  // namespace rwkv7

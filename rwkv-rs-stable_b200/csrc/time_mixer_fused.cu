@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.h"
+#include "launch.h"
 #include "rwkv7_b200.h"
 
 namespace rwkv7 {
@@ -110,6 +111,8 @@ __device__ __forceinline__ float group_sum(float x) {
 template <typename T, int EPV>
 __global__ void __launch_bounds__(256)
 weight_prepare_vec_kernel(WeightPrepareArgs p) {
+    wait_for_previous();
+    let_next_in();
     constexpr int kN = 64, LANES = kN / EPV, ROWS_PER_WARP = 32 / LANES;
     const int lane = threadIdx.x & 31, sub = lane % LANES;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -167,6 +170,8 @@ weight_prepare_vec_kernel(WeightPrepareArgs p) {
 template <typename T>
 __global__ void __launch_bounds__(256)
 weight_prepare_generic_kernel(WeightPrepareArgs p) {
+    wait_for_previous();
+    let_next_in();
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -202,6 +207,8 @@ weight_prepare_generic_kernel(WeightPrepareArgs p) {
 template <typename T, int EPV>
 __global__ void __launch_bounds__(256)
 gated_readout_vec_kernel(GatedReadoutArgs p) {
+    wait_for_previous();
+    let_next_in();
     constexpr int kN = 64, LANES = kN / EPV, ROWS_PER_WARP = 32 / LANES;
     const int lane = threadIdx.x & 31, sub = lane % LANES;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -250,6 +257,8 @@ gated_readout_vec_kernel(GatedReadoutArgs p) {
 template <typename T>
 __global__ void __launch_bounds__(256)
 gated_readout_generic_kernel(GatedReadoutArgs p) {
+    wait_for_previous();
+    let_next_in();
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -301,16 +310,14 @@ int launch_weight_prepare(const WeightPrepareArgs &p, cudaStream_t stream) {
                         aligned16(p.replacement_key) && aligned16(p.removal_key_normalized) &&
                         aligned16(p.replacement) && aligned16(p.value);
     constexpr int kThreads = 256;
+    auto go = [&](auto kernel, int rows_per_block) {
+        return (int)launch_serialized(kernel, pick_grid(p.rows, rows_per_block, p.num_sms), (unsigned)kThreads, 0, stream, p);
+    };
     if (p.bf16) {
         using T = __nv_bfloat16;
-        if (vec_ok) weight_prepare_vec_kernel<T, 8><<<pick_grid(p.rows, kThreads / 8, p.num_sms), kThreads, 0, stream>>>(p);
-        else weight_prepare_generic_kernel<T><<<pick_grid(p.rows, kThreads / 32, p.num_sms), kThreads, 0, stream>>>(p);
-    } else {
-        if (vec_ok) weight_prepare_vec_kernel<float, 4><<<pick_grid(p.rows, kThreads / 16, p.num_sms), kThreads, 0, stream>>>(p);
-        else weight_prepare_generic_kernel<float><<<pick_grid(p.rows, kThreads / 32, p.num_sms), kThreads, 0, stream>>>(p);
+        return vec_ok ? go(weight_prepare_vec_kernel<T, 8>, kThreads / 8) : go(weight_prepare_generic_kernel<T>, kThreads / 32);
     }
-    count_launch();
-    return (int)cudaGetLastError();
+    return vec_ok ? go(weight_prepare_vec_kernel<float, 4>, kThreads / 16) : go(weight_prepare_generic_kernel<float>, kThreads / 32);
 }
 
 int launch_gated_readout(const GatedReadoutArgs &p, cudaStream_t stream) {
@@ -319,16 +326,14 @@ int launch_gated_readout(const GatedReadoutArgs &p, cudaStream_t stream) {
                         aligned16(p.replacement_key) && aligned16(p.value) && aligned16(p.gate) &&
                         aligned16(p.gamma) && aligned16(p.beta) && aligned16(p.bonus) && aligned16(p.output);
     constexpr int kThreads = 256;
+    auto go = [&](auto kernel, int rows_per_block) {
+        return (int)launch_serialized(kernel, pick_grid(p.rows, rows_per_block, p.num_sms), (unsigned)kThreads, 0, stream, p);
+    };
     if (p.bf16) {
         using T = __nv_bfloat16;
-        if (vec_ok) gated_readout_vec_kernel<T, 8><<<pick_grid(p.rows, kThreads / 8, p.num_sms), kThreads, 0, stream>>>(p);
-        else gated_readout_generic_kernel<T><<<pick_grid(p.rows, kThreads / 32, p.num_sms), kThreads, 0, stream>>>(p);
-    } else {
-        if (vec_ok) gated_readout_vec_kernel<float, 4><<<pick_grid(p.rows, kThreads / 16, p.num_sms), kThreads, 0, stream>>>(p);
-        else gated_readout_generic_kernel<float><<<pick_grid(p.rows, kThreads / 32, p.num_sms), kThreads, 0, stream>>>(p);
+        return vec_ok ? go(gated_readout_vec_kernel<T, 8>, kThreads / 8) : go(gated_readout_generic_kernel<T>, kThreads / 32);
     }
-    count_launch();
-    return (int)cudaGetLastError();
+    return vec_ok ? go(gated_readout_vec_kernel<float, 4>, kThreads / 16) : go(gated_readout_generic_kernel<float>, kThreads / 32);
 }
 
 }  // namespace rwkv7
