@@ -7,9 +7,10 @@
 // one stated in rwkv7_b200.h: per row the triple (max_v z_v, sum_v exp(z_v - max),
 // z_target) over a vocabulary shard, then a combine over shards.
 //
-// One CTA owns a block of 128 rows and a contiguous range of 256-wide vocabulary
-// tiles.  Warp roles: warp 0 requests the x and W tiles (TMA, 128-byte swizzle, K
-// slices of 64 bf16, 4-stage ring); warp 1 issues the UMMAs (M=128, N=256, bf16 in,
+// One CTA owns a block of 128 rows, or a pair of CTAs 256 (lm_head_ce_pair_kernel, most
+// calls of more than 128 rows), and a contiguous range of vocabulary tiles of up to 256
+// columns.  Warp roles: warp 0 requests the x and W tiles (TMA, 128-byte swizzle, K
+// slices of 64 bf16, 4-stage ring); warp 1 issues the UMMAs (M=128, bf16 in,
 // fp32 accumulators, two 256-column TMEM buffers); warps 2..5 are the epilogue:
 // thread = row, it reads its accumulator row 32 columns at a time and keeps the
 // running (max, sum-exp, target logit) in registers while the next tile is being
@@ -20,10 +21,13 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "kernels.h"
+#include "launch.h"
 #include "rwkv7_b200.h"
+#include "sm100_pair_gemm.cuh"
 #include "sm100_umma.cuh"
 
 namespace rwkv7 {
@@ -48,10 +52,77 @@ __device__ __forceinline__ int64_t load_target(const void *t, int dtype, int64_t
                               : (int64_t) reinterpret_cast<const int32_t *>(t)[row];
 }
 
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// The wait for a TMEM read, with its registers: nothing that uses them moves in front of it while others are in flight.
+__device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&v)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]),
+                   "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]),
+                   "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]),
+                   "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
+                 :
+                 : "memory");
+}
+
+// What a thread keeps of its row of logits.
+struct RowSums {
+    float m = -INFINITY, ssum = 0.f, zt = 0.f;
+    // 32 neighbouring logits from column c0 on, of which those below `end` count; `tgt` is the target's column in this shard
+    __device__ __forceinline__ void take(uint32_t (&v)[32], int c0, int end, int64_t tgt) {
+        const int ncol = min(32, end - c0);
+        if (ncol < 32) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+                if (e >= ncol) v[e] = __float_as_uint(-INFINITY);
+        }
+        // (four chains each for the maximum and the sum: one warp a scheduler does this, nothing else covers its latency)
+        float most[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) most[e] = __uint_as_float(v[e]);
+#pragma unroll
+        for (int e = 4; e < 32; ++e) most[e & 3] = fmaxf(most[e & 3], __uint_as_float(v[e]));
+        const float m_new = fmaxf(m, fmaxf(fmaxf(most[0], most[1]), fmaxf(most[2], most[3])));
+        const float mb = m_new * kLog2e;
+        ssum *= ex2(m * kLog2e - mb);               // 2^-inf = 0 on the first chunk
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < 32; ++e) acc[e & 3] += ex2(fmaf(__uint_as_float(v[e]), kLog2e, -mb));   // (at most 1: subnormal terms are nothing)
+        ssum += (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        m = m_new;
+        if (tgt >= c0 && tgt < c0 + ncol) {
+            const int off = (int)(tgt - c0);
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+                if (e == off) zt = __uint_as_float(v[e]);
+        }
+    }
+    // The accumulators of columns col0 .. end - 1, from TMEM address `at` on: the next 32 are read while these are summed up.
+    __device__ __forceinline__ void take_row(uint32_t at, int col0, int end, int64_t tgt) {
+        uint32_t v0[32], v1[32];
+        auto from = [&](int c) { return at + (uint32_t)min(c - col0, kBN - 32); };   // (always a read: one under a condition would be copied in flight)
+        tmem_ld32(at, v0);
+        tmem_ld_wait_for(v0);
+#pragma unroll 1
+        for (int c = col0; c < end; c += 64) {
+            tmem_ld32(from(c + 32), v1);
+            take(v0, c, end, tgt);
+            tmem_ld_wait_for(v1);
+            tmem_ld32(from(c + 64), v0);
+            if (c + 32 < end) take(v1, c + 32, end, tgt);
+            tmem_ld_wait_for(v0);
+        }
+    }
+};
+
 __global__ void __launch_bounds__(kThreads, 1)
 lm_head_ce_kernel(const __grid_constant__ LmMaps maps, const void *__restrict__ targets, int targets_dtype,
                   int64_t vocab_offset, float *__restrict__ out /* [splits][R][3] */, int64_t R, int C, int V,
-                  int row_blocks, int tiles_per_split, int *status) {
+                  int row_blocks, int width, int tiles_per_split, int *status) {
     extern __shared__ __align__(1024) unsigned char smem[];   // swizzled TMA tiles need 1024-byte alignment
     if (smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0) atomicExch(status, (int)kDevInternal);
@@ -67,7 +138,7 @@ lm_head_ce_kernel(const __grid_constant__ LmMaps maps, const void *__restrict__ 
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (uniform, for elect_one)
     // consecutive CTAs share a vocabulary split and differ in the row block
     const int rb = blockIdx.x % row_blocks, split = blockIdx.x / row_blocks;
-    const int total_tiles = (V + kBN - 1) / kBN;
+    const int total_tiles = (V + width - 1) / width;
     const int tile0 = split * tiles_per_split;
     const int ntiles = min(tiles_per_split, total_tiles - tile0);
     const int ksteps = C / kBK;
@@ -85,6 +156,8 @@ lm_head_ce_kernel(const __grid_constant__ LmMaps maps, const void *__restrict__ 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool timed_out = false;
+    wait_for_previous();
+    let_next_in();
 
     if (warp == 0) {
         if (elect_one()) {
@@ -94,15 +167,15 @@ lm_head_ce_kernel(const __grid_constant__ LmMaps maps, const void *__restrict__ 
                     const uint32_t s = it % kStages, ph = (it / kStages) & 1;
                     if (!mbar_wait(&empty[s], ph ^ 1)) { timed_out = true; break; }
                     unsigned char *a = smem + s * kStageBytes, *b = a + kABytes;
-                    mbar_expect_tx(&full[s], kStageBytes);
+                    mbar_expect_tx(&full[s], kABytes + (uint32_t)width * kBK * 2);
                     tma_load_2d(a, &maps.x, ks * kBK, rb * kBM, &full[s]);
-                    tma_load_2d(b, &maps.w, ks * kBK, (tile0 + t) * kBN, &full[s]);
+                    tma_load_2d(b, &maps.w, ks * kBK, (tile0 + t) * width, &full[s]);
                 }
             }
         }
     } else if (warp == 1) {
         if (elect_one()) {
-            constexpr uint32_t idesc = make_idesc(kFmtBF16, kBM, kBN, false, false);
+            const uint32_t idesc = make_idesc(kFmtBF16, kBM, width, false, false);
             uint32_t it = 0;
             for (int t = 0; t < ntiles && !timed_out; ++t) {
                 const uint32_t buf = t & 1, bph = (t >> 1) & 1;
@@ -131,53 +204,22 @@ lm_head_ce_kernel(const __grid_constant__ LmMaps maps, const void *__restrict__ 
         int64_t tgt = -1;
         if (row_ok) tgt = load_target(targets, targets_dtype, row);
         const int64_t tgt_local = (tgt >= 0) ? tgt - vocab_offset : -1;   // column inside this shard
-        float m = -INFINITY, ssum = 0.f, zt = 0.f;
+        RowSums sums;
         for (int t = 0; t < ntiles && !timed_out; ++t) {
             const uint32_t buf = t & 1, bph = (t >> 1) & 1;
             if (!mbar_wait(&tmem_full[buf], bph)) { timed_out = true; break; }
             tc_fence_after();
-            const int col0 = (tile0 + t) * kBN;
-#pragma unroll 1
-            for (int ch = 0; ch < kBN / 32; ++ch) {
-                uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + buf * kBN + ch * 32, v);
-                tmem_ld_wait();
-                const int c0 = col0 + ch * 32;
-                if (c0 >= V) continue;                       // padding columns of the last tile
-                const int ncol = min(32, V - c0);
-                float cm = -INFINITY;
-#pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    if (e >= ncol) v[e] = __float_as_uint(-INFINITY);
-                    cm = fmaxf(cm, __uint_as_float(v[e]));
-                }
-                const float m_new = fmaxf(m, cm);
-                const float mb = m_new * kLog2e;
-                ssum *= exp2f(m * kLog2e - mb);               // exp2(-inf) = 0 on the first chunk
-                float acc0 = 0.f, acc1 = 0.f;
-#pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    acc0 += exp2f(fmaf(__uint_as_float(v[e]), kLog2e, -mb));
-                    acc1 += exp2f(fmaf(__uint_as_float(v[e + 1]), kLog2e, -mb));
-                }
-                ssum += acc0 + acc1;
-                m = m_new;
-                if (tgt_local >= c0 && tgt_local < c0 + ncol) {
-                    const int off = (int)(tgt_local - c0);
-#pragma unroll
-                    for (int e = 0; e < 32; ++e)
-                        if (e == off) zt = __uint_as_float(v[e]);
-                }
-            }
+            const int col0 = (tile0 + t) * width, end = min(V, col0 + width);
+            sums.take_row(tmem + ((uint32_t)(quarter * 32) << 16) + buf * kBN, col0, end, tgt_local);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tmem_empty[buf]);
         }
         if (row_ok && !timed_out) {
             float *o = out + ((size_t)split * R + row) * 3;
-            o[0] = m;
-            o[1] = ssum;
-            o[2] = zt;
+            o[0] = sums.m;
+            o[1] = sums.ssum;
+            o[2] = sums.zt;
         }
     }
     if (timed_out) atomicExch(status, (int)kDevTimeout);
@@ -186,9 +228,60 @@ lm_head_ce_kernel(const __grid_constant__ LmMaps maps, const void *__restrict__ 
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
+// The same on pairs of CTAs (see sm100_pair_gemm.cuh): a pair owns 256 rows, each CTA 128 of them.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+lm_head_ce_pair_kernel(const __grid_constant__ PairMaps maps, const void *__restrict__ targets, int targets_dtype, int64_t vocab_offset,
+                       float *__restrict__ out /* [splits][R][3] */, int64_t R, int C, int V, int row_blocks, int width, int tiles_per_split, int *status) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    if (smem_u32(smem) & 1023u) {
+        if (threadIdx.x == 0) atomicExch(status, (int)kDevInternal);
+        return;
+    }
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
+    const int pair = blockIdx.x >> 1, rb = pair % row_blocks, split = pair / row_blocks;
+    const int total_tiles = (V + width - 1) / width, tile0 = split * tiles_per_split;
+    const int ntiles = min(tiles_per_split, total_tiles - tile0);
+    auto items = [&](int i, PairItem &w) {
+        w = PairItem{rb * kPairM, (tile0 + i) * width, 0, C / kPairK};
+        return i < ntiles;
+    };
+    PairGemm gemm;
+    gemm.begin(smem, maps, warp);
+    wait_for_previous();
+    let_next_in();
+    bool ok = true;
+    if (warp == 0) {
+        if (elect_one()) ok = gemm.produce(maps, width, items);
+    } else if (warp == 1) {
+        if (gemm.rank == 0 && elect_one()) ok = gemm.multiply(width, items);
+    } else {
+        const int quarter = warp & 3;
+        const int64_t row = (int64_t)rb * kPairM + gemm.rank * 128 + quarter * 32 + lane;
+        const int64_t tgt = row < R ? load_target(targets, targets_dtype, row) : -1, tgt_local = tgt >= 0 ? tgt - vocab_offset : -1;
+        RowSums sums;
+        for (int t = 0; t < ntiles; ++t) {
+            if (!gemm.complete(t)) { ok = false; break; }
+            const int col0 = (tile0 + t) * width, end = min(V, col0 + width);
+            sums.take_row(gemm.tmem + ((uint32_t)(quarter * 32) << 16) + (t & 1) * kPairN, col0, end, tgt_local);
+            gemm.release(t);
+        }
+        if (row < R && ok) {
+            float *o = out + ((size_t)split * R + row) * 3;
+            o[0] = sums.m;
+            o[1] = sums.ssum;
+            o[2] = sums.zt;
+        }
+    }
+    __syncwarp();
+    if (!ok) atomicExch(status, (int)kDevTimeout);
+    gemm.end(warp);
+}
+
 // Combines `nparts` partial triples per row: out[row] = (M, sum_g s_g exp(m_g - M), sum_g zt_g).
 __global__ void lm_head_combine_kernel(const float *__restrict__ parts, int nparts, float *__restrict__ out,
                                        int64_t R) {
+    wait_for_previous();
+    let_next_in();
     const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= R) return;
     float M = -INFINITY;
@@ -207,6 +300,8 @@ __global__ void lm_head_combine_kernel(const float *__restrict__ parts, int npar
 __global__ void lm_head_finalize_kernel(const float *__restrict__ parts, int nparts, const void *__restrict__ targets,
                                         int targets_dtype, float *__restrict__ lse, float *__restrict__ loss,
                                         int64_t R) {
+    wait_for_previous();
+    let_next_in();
     const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= R) return;
     float M = -INFINITY;
@@ -240,10 +335,10 @@ EncodeTiledFn lm_encode_fn() {
     return fn;
 }
 
-// Vocabulary splits per row block.  A CTA takes one block of 128 rows and a run of column tiles, one CTA fits an
-// SM, so a launch runs in waves of `num_sms` CTAs and its time goes with waves x (tiles per CTA): the split count
-// that minimises that product is taken (half a tile is charged per CTA for filling its pipeline, which favours fewer
-// splits on a tie).  Example, 148 SMs, 256 row blocks x 32 column tiles: one or two splits take 2 x 32 = 4 x 16 = 64
+// Vocabulary splits per row block and the tiles' width.  A CTA takes one block of 128 rows and a run of column tiles, one CTA fits an
+// SM, so a launch runs in waves of `num_sms` CTAs (or half as many pairs) and its time goes with waves x (columns per CTA): the split
+// count and width that minimise that product are taken (half a tile is charged per CTA for filling its pipeline, which favours fewer
+// splits on a tie, and eight columns a tile, which favours wide ones).  Example, 148 SMs, 256 row blocks x 32 column tiles: one or two splits take 2 x 32 = 4 x 16 = 64
 // tile times, four splits 7 x 8 = 56 (the ideal is 55.4): 1140 -> 1195 TFLOP/s on that shape.  (Persistent CTAs that
 // walk the work items themselves measured no better: 1167.)
 // Most splits per row block: 16, and with few row blocks as many as give every SM of a large device a CTA of its own
@@ -258,28 +353,26 @@ size_t split_bytes(int64_t R, int64_t V, int most) {
     const int64_t tiles = (V + kBN - 1) / kBN, sp = tiles < most ? tiles : most;
     return sp > 1 ? (size_t)sp * (size_t)R * 3 * sizeof(float) : 0;
 }
-// `most`: splits that the workspace has room for.
-void plan(int64_t R, int64_t V, int num_sms, int64_t most, int *row_blocks, int *splits, int *tiles_per_split) {
-    const int rbs = (int)((R + kBM - 1) / kBM);
-    const int tiles = (int)((V + kBN - 1) / kBN);
-    const int sms = num_sms > 0 ? num_sms : 1;
-    int best_sp = 1, best_tps = tiles;
-    double best_cost = 0.0;
-    for (int want = 1; want <= max_splits(R) && want <= tiles && want <= most; ++want) {
-        const int tps = (tiles + want - 1) / want;
-        const int sp = (tiles + tps - 1) / tps;
-        const long long ctas = (long long)rbs * sp;
-        const long long waves = (ctas + sms - 1) / sms;
-        const double cost = (double)waves * (tps + 0.5);
-        if (want == 1 || cost < best_cost - 1e-9) {
-            best_cost = cost;
-            best_sp = sp;
-            best_tps = tps;
+// How a launch is cut.
+struct Plan {
+    int row_blocks, width, splits, tiles_per_split;
+    double cost;   // columns that a worker does one after the other
+};
+// `rows` of a block, `workers` CTAs or pairs of them; `most`: splits that the workspace has room for.
+Plan plan(int64_t R, int64_t V, int rows, int workers, int64_t most) {
+    Plan best{};
+    const int rbs = (int)((R + rows - 1) / rows);
+    for (int width = kBN; width >= 128; width -= 16) {
+        const int tiles = (int)((V + width - 1) / width);
+        for (int want = 1; want <= max_splits(R) && want <= tiles && want <= most; ++want) {
+            const int tps = (tiles + want - 1) / want;
+            const int sp = (tiles + tps - 1) / tps;
+            const long long waves = ((long long)rbs * sp + workers - 1) / workers;
+            const double cost = (double)waves * (tps * (width + 8) + 128);
+            if (best.row_blocks == 0 || cost < best.cost - 1e-9) best = Plan{rbs, width, sp, tps, cost};
         }
     }
-    *row_blocks = rbs;
-    *splits = best_sp;
-    *tiles_per_split = best_tps;
+    return best;
 }
 
 }  // namespace
@@ -300,51 +393,48 @@ int launch_lm_head_ce_partial(const LmHeadArgs &p, void *workspace, size_t works
     if (encode == nullptr) return (int)cudaErrorNotSupported;
     if ((reinterpret_cast<uintptr_t>(p.x) & 15u) || (reinterpret_cast<uintptr_t>(p.w) & 15u))
         return (int)cudaErrorMisalignedAddress;
-    LmMaps maps;
-    const cuuint32_t estr[2] = {1, 1};
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)p.C, (cuuint64_t)p.R};
-        const cuuint64_t strides[1] = {(cuuint64_t)p.C * 2};
-        const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)kBM};
-        if (encode(&maps.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(p.x), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return (int)cudaErrorInvalidValue;
-    }
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)p.C, (cuuint64_t)p.V};
-        const cuuint64_t strides[1] = {(cuuint64_t)p.C * 2};
-        const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)kBN};
-        if (encode(&maps.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(p.w), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return (int)cudaErrorInvalidValue;
-    }
-    int row_blocks, splits, tps;
-    const int64_t room = workspace == nullptr ? 1 : (int64_t)(workspace_bytes / ((size_t)p.R * 3 * sizeof(float)));
-    plan(p.R, p.V, p.num_sms, room > 1 ? room : 1, &row_blocks, &splits, &tps);
+    const int64_t room = workspace == nullptr ? 1 : std::max<int64_t>(1, (int64_t)(workspace_bytes / ((size_t)p.R * 3 * sizeof(float))));
+    const int sms = p.num_sms > 0 ? p.num_sms : 1;
+    const Plan one = plan(p.R, p.V, kBM, sms, room), two = plan(p.R, p.V, kPairM, sms / 2, room);
+    // A pair's tile costs less the longer its sums are: what two CTAs hand each other at its end weighs less.  Measured (B200, V = 65 536,
+    // single CTAs / pairs, us): 8191 rows at C = 2048 1510 / 1460, 20 000 at C = 768 1484 / 1554, 500 at C = 1024 75 / 72, 200 at
+    // C = 4096 147 / 125; 16 384 at C = 4096 and V = 8192 1065 / 997; 300 rows at C = 4096, three blocks of 128 and two of 256, 195 / 215.
+    const bool pairs = p.R > kBM && sms > 1 && two.cost * (0.92 + 80.0 / (double)p.C) < one.cost;
+    const Plan &cut = pairs ? two : one;
+    auto describe = [&](CUtensorMap *map, const void *ptr, int64_t rows, int box_rows) {
+        const cuuint32_t estr[2] = {1, 1}, box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
+        const cuuint64_t dims[2] = {(cuuint64_t)p.C, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)p.C * 2};
+        return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    const int splits = cut.splits;
     float *parts = splits == 1 ? p.partials : static_cast<float *>(workspace);
-    cudaError_t e = cudaFuncSetAttribute(lm_head_ce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
-    lm_head_ce_kernel<<<(unsigned)(row_blocks * splits), kThreads, kSmemBytes, stream>>>(
-        maps, p.targets, p.targets_dtype, p.vocab_offset, parts, p.R, (int)p.C, (int)p.V, row_blocks, tps, p.status);
-    count_launch();
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
-    if (splits > 1) {
-        lm_head_combine_kernel<<<(unsigned)((p.R + 255) / 256), 256, 0, stream>>>(parts, splits, p.partials, p.R);
-        count_launch();
-        e = cudaGetLastError();
+    cudaError_t e;
+    if (pairs) {
+        PairMaps maps;
+        if (!describe(&maps.a, p.x, p.R, kPairM / 2) || !describe(&maps.b, p.w, p.V, cut.width / 2)) return (int)cudaErrorInvalidValue;
+        e = cudaFuncSetAttribute(lm_head_ce_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem);
+        if (e != cudaSuccess) return (int)e;
+        e = launch_serialized(lm_head_ce_pair_kernel, (unsigned)(2 * cut.row_blocks * splits), (unsigned)kPairThreads, kPairSmem, stream, maps, p.targets,
+                              p.targets_dtype, p.vocab_offset, parts, p.R, (int)p.C, (int)p.V, cut.row_blocks, cut.width, cut.tiles_per_split, p.status);
+    } else {
+        LmMaps maps;
+        if (!describe(&maps.x, p.x, p.R, kBM) || !describe(&maps.w, p.w, p.V, cut.width)) return (int)cudaErrorInvalidValue;
+        e = cudaFuncSetAttribute(lm_head_ce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+        if (e != cudaSuccess) return (int)e;
+        e = launch_serialized(lm_head_ce_kernel, (unsigned)(cut.row_blocks * splits), (unsigned)kThreads, kSmemBytes, stream, maps, p.targets, p.targets_dtype,
+                              p.vocab_offset, parts, p.R, (int)p.C, (int)p.V, cut.row_blocks, cut.width, cut.tiles_per_split, p.status);
     }
+    if (e == cudaSuccess && splits > 1)
+        e = launch_serialized(lm_head_combine_kernel, (unsigned)((p.R + 255) / 256), 256u, 0, stream, (const float *)parts, splits, p.partials, p.R);
     return (int)e;
 }
 
 int launch_lm_head_ce_finalize(const float *partials_all, int num_shards, const void *targets, int targets_dtype,
                                float *lse, float *loss, int64_t R, cudaStream_t stream) {
-    lm_head_finalize_kernel<<<(unsigned)((R + 255) / 256), 256, 0, stream>>>(partials_all, num_shards, targets,
-                                                                            targets_dtype, lse, loss, R);
-    count_launch();
-    return (int)cudaGetLastError();
+    return (int)launch_serialized(lm_head_finalize_kernel, (unsigned)((R + 255) / 256), 256u, 0, stream, partials_all, num_shards, targets, targets_dtype, lse,
+                                  loss, R);
 }
 
 }  // namespace rwkv7

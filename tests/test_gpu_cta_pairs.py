@@ -25,3 +25,18 @@ def test_channel_mixer_on_pairs(pkg, workloads, cuda, shape):
     fine = (hid @ vw.double().T).reshape(B, T, C).numpy()
     tol = 2e-3 * np.abs(fine).max() + 2 * parity.BF16_ULP * np.abs(fine)
     assert (np.abs(got - fine) <= tol).all(), float((np.abs(got - fine) - tol).max())
+
+
+@pytest.mark.parametrize("R,C,V", [(129, 64, 30000), (255, 128, 777), (257, 64, 9000), (1030, 192, 8200), (3000, 64, 2064)])
+def test_lm_head_on_pairs(pkg, oracle, workloads, cuda, R, C, V):
+    """Ragged rows and vocabularies; tolerance as in the other LM-head tests (exact bf16 products, fp32 sums)."""
+    x, w, tg = workloads.lm_head_inputs(R, C, V, seed=R)
+    x = x * 4
+    tg[::5] = -1
+    tg[1] = V - 1
+    lse_ref, loss_ref = oracle.lm_head_ce(x.float().numpy(), w.float().numpy(), tg.numpy())
+    lse, loss = pkg.lm_head_ce(x.to(cuda), w.to(cuda), tg.to(cuda))
+    torch.cuda.synchronize()
+    assert pkg.read_device_status(0) == 0
+    np.testing.assert_allclose(lse.cpu().numpy(), lse_ref, rtol=0, atol=2e-4)
+    np.testing.assert_allclose(loss.cpu().numpy(), loss_ref, rtol=0, atol=2e-4)
