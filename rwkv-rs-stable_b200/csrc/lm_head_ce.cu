@@ -277,24 +277,30 @@ lm_head_ce_pair_kernel(const __grid_constant__ PairMaps maps, const void *__rest
     gemm.end(warp);
 }
 
-// Combines `nparts` partial triples per row: out[row] = (M, sum_g s_g exp(m_g - M), sum_g zt_g).
-__global__ void lm_head_combine_kernel(const float *__restrict__ parts, int nparts, float *__restrict__ out,
-                                       int64_t R) {
+// Combines `nparts` partial triples per row: out[row] = (M, sum_g s_g exp(m_g - M), sum_g zt_g).  A warp per row: a thread per row walked up
+// to 148 triples one after the other, 16 us behind the 54 of 16 rows' product; now 4.6.
+__global__ void __launch_bounds__(256) lm_head_combine_kernel(const float *__restrict__ parts, int nparts, float *__restrict__ out, int64_t R) {
     wait_for_previous();
     let_next_in();
-    const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (row >= R) return;
     float M = -INFINITY;
-    for (int g = 0; g < nparts; ++g) M = fmaxf(M, parts[((size_t)g * R + row) * 3]);
+    for (int g = lane; g < nparts; g += 32) M = fmaxf(M, parts[((size_t)g * R + row) * 3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
     float s = 0.f, zt = 0.f;
-    for (int g = 0; g < nparts; ++g) {
+    for (int g = lane; g < nparts; g += 32) {
         const float *p = parts + ((size_t)g * R + row) * 3;
         if (p[0] > -INFINITY) s += p[1] * expf(p[0] - M);
         zt += p[2];
     }
-    out[row * 3 + 0] = M;
-    out[row * 3 + 1] = s;
-    out[row * 3 + 2] = zt;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        zt += __shfl_xor_sync(0xffffffffu, zt, o);
+    }
+    if (lane < 3) out[row * 3 + lane] = lane == 0 ? M : lane == 1 ? s : zt;
 }
 
 __global__ void lm_head_finalize_kernel(const float *__restrict__ parts, int nparts, const void *__restrict__ targets,
@@ -427,7 +433,7 @@ int launch_lm_head_ce_partial(const LmHeadArgs &p, void *workspace, size_t works
                               p.vocab_offset, parts, p.R, (int)p.C, (int)p.V, cut.row_blocks, cut.width, cut.tiles_per_split, p.status);
     }
     if (e == cudaSuccess && splits > 1)
-        e = launch_serialized(lm_head_combine_kernel, (unsigned)((p.R + 255) / 256), 256u, 0, stream, (const float *)parts, splits, p.partials, p.R);
+        e = launch_serialized(lm_head_combine_kernel, (unsigned)((p.R + 7) / 8), 256u, 0, stream, (const float *)parts, splits, p.partials, p.R);
     return (int)e;
 }
 
