@@ -269,17 +269,16 @@ gemm_reduce_kernel(const float *__restrict__ parts, int splits, __nv_bfloat16 *_
 }
 
 // key_input = x + (shifted - x) * key_scale, shifted = previous token (zero at t == 0)
-// (channel_mixer/kernel.rs:4-25).  A CTA owns 16 consecutive token rows, a thread one
-// 16-byte channel vector; the previous row is carried in registers.  (Few rows: fewer per CTA, so that they are not
-// walked one after the other by one CTA.)
-constexpr int kMixRows = 16;
+// (channel_mixer/kernel.rs:4-25).  The rows are shared out evenly, a thread owns one 16-byte channel vector of its CTA's rows; the previous
+// row is carried in registers and the next one on its way while a row is written.  Bound by latency at the sizes of a prefill: 4096 rows of
+// 2048 channels took 14.3 us with two rows a CTA and a 64-bit division for each, 10.2 so.
 __global__ void __launch_bounds__(256)
 channel_mixer_mix_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ scale,
-                         __nv_bfloat16 *__restrict__ out, int64_t rows, int64_t Tlen, int64_t C, int per_block) {
+                         __nv_bfloat16 *__restrict__ out, int64_t rows, int64_t Tlen, int64_t C) {
+    wait_for_previous();
+    let_next_in();
     const int64_t CV = C / 8;
-    const int64_t row_begin = (int64_t)blockIdx.x * per_block;
-    const int64_t row_end = row_begin + per_block < rows ? row_begin + per_block : rows;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int64_t row_begin = rows * blockIdx.x / gridDim.x, row_end = rows * (blockIdx.x + 1) / gridDim.x;
     auto unpack = [](const uint4 &u, float (&f)[8]) {
         const unsigned w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -288,23 +287,28 @@ channel_mixer_mix_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat1
             f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
         }
     };
+    const int64_t t_begin = row_begin % Tlen;
     for (int64_t cv = threadIdx.x; cv < CV; cv += blockDim.x) {
         const int64_t c = cv * 8;
         float mu[8], prev[8], cur[8];
+        uint4 ahead = *reinterpret_cast<const uint4 *>(x + row_begin * C + c);
         unpack(*reinterpret_cast<const uint4 *>(scale + c), mu);
-        if (row_begin % Tlen == 0) {
+        if (t_begin == 0) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) prev[e] = 0.f;
         } else {
             unpack(*reinterpret_cast<const uint4 *>(x + (row_begin - 1) * C + c), prev);
         }
-#pragma unroll 4
+        int64_t t = t_begin;
+#pragma unroll 2
         for (int64_t row = row_begin; row < row_end; ++row) {
-            unpack(__ldcs(reinterpret_cast<const uint4 *>(x + row * C + c)), cur);
-            if (row % Tlen == 0) {
+            unpack(ahead, cur);
+            if (row + 1 < row_end) ahead = *reinterpret_cast<const uint4 *>(x + (row + 1) * C + c);
+            if (t == 0) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) prev[e] = 0.f;   // first token of a sequence
             }
+            if (++t == Tlen) t = 0;
             uint4 o;
             unsigned *ow = &o.x;
 #pragma unroll
@@ -465,11 +469,9 @@ int launch_channel_mixer(const ChannelMixerArgs &p, void *workspace, size_t work
     float *partials = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + least);
     int threads = 32;
     while (threads < 256 && threads < p.C / 8) threads <<= 1;
-    const int per_block = rows >= 2 * kMixRows * (int64_t)p.num_sms ? kMixRows : 2;
-    channel_mixer_mix_kernel<<<(unsigned)((rows + per_block - 1) / per_block), threads, 0, stream>>>(
-        (const __nv_bfloat16 *)p.x, (const __nv_bfloat16 *)p.key_scale, key_input, rows, p.T, p.C, per_block);
-    count_launch();
-    if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return (int)e;
+    const cudaError_t e = launch_serialized(channel_mixer_mix_kernel, blocks_of_rows(rows, p.num_sms, 8), (unsigned)threads, 0, stream, (const __nv_bfloat16 *)p.x,
+                                            (const __nv_bfloat16 *)p.key_scale, key_input, rows, p.T, p.C);
+    if (e != cudaSuccess) return (int)e;
     if (int e = launch_gemm<kEpiReluSquare>(key_input, p.key_weight, hidden, partials, room, rows, p.F, p.C, p.num_sms, p.status, stream))
         return e;
     return launch_gemm<kEpiNone>(hidden, p.value_weight, p.out, partials, room, rows, p.C, p.F, p.num_sms, p.status, stream);
