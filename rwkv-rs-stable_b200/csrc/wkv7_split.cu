@@ -74,7 +74,7 @@ __host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
 // Bound by shared-memory bandwidth (2.8 k cycles per chunk at one 128-byte access a cycle) and by the latency of a chunk's
 // phases, which the CTAs of an SM cover for one another; hence few warps per chunk, each with the largest tile its
 // registers hold (eight warps per chunk read a quarter more and were slower: 153 against 121 us).  Measured, 6144 chunks (8 x
-// 4096 tokens x 12 heads): 112.5 us, 4.0 TB/s; the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
+// 4096 tokens x 12 heads): 111.5 us, 4.1 TB/s; the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
 //   1. decays: warp = 16-token block, lane = channel pair; prefix and suffix products within the block
 //   2. scaled fp16 operands, in place over the bf16 tiles that TMA delivered
 //   3. the A matrices: one 128 x 128 tcgen05 product [a; r] [b; k]^T, read back a row per thread, lower triangle only; with
@@ -603,16 +603,19 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                     U[x][b][3] = pack_half2(o[x][1][2], o[x][1][3]);
                 }
             }
-            // Sixteen rows n of the operator, columns k of this warp's two blocks: four k of a row per lane (see kRecord)
-            unsigned char *dst = record + (ct >> 1) * 512 + (ct & 1) * 8 + q * 128 + g * 16;
+            // Sixteen rows n of the operator, columns k of this warp's two blocks (see kRecord).  A lane has four k of rows g and g + 8; two
+            // neighbours exchange theirs, and each stores eight k of one row: whole 32-byte sectors.
+            unsigned char *dst = record + ct * 256 + (q >> 1) * 128;
+            const int row_state = (g >> 2) * 2048 + ((g >> 1) & 1) * 64 + (q & 1) * 32 + (g & 1) * 16, row_out = (q & 1) * 2048 + g * 16;
             auto put = [&](int n16, const float (&c)[2][2][4]) {
-                if (RWKV7_IN_RANGE(unit >= 0 && unit < units && n16 < 8, status)) {
 #pragma unroll
-                    for (int r = 0; r < 2; ++r)
-#pragma unroll
-                        for (int x = 0; x < 2; ++x)
-                            *reinterpret_cast<uint2 *>(dst + (2 * n16 + r) * 2048 + x * 1024) =
-                                make_uint2(pack_half2(c[x][0][2 * r], c[x][0][2 * r + 1]), pack_half2(c[x][1][2 * r], c[x][1][2 * r + 1]));
+                for (int x = 0; x < 2; ++x) {
+                    const uint32_t lo[2] = {pack_half2(c[x][0][0], c[x][0][1]), pack_half2(c[x][1][0], c[x][1][1])};
+                    const uint32_t hi[2] = {pack_half2(c[x][0][2], c[x][0][3]), pack_half2(c[x][1][2], c[x][1][3])};
+                    const uint32_t t0 = __shfl_xor_sync(0xffffffffu, (q & 1) ? lo[0] : hi[0], 1), t1 = __shfl_xor_sync(0xffffffffu, (q & 1) ? lo[1] : hi[1], 1);
+                    if (RWKV7_IN_RANGE(unit >= 0 && unit < units && n16 < 8, status))
+                        *reinterpret_cast<uint4 *>(dst + n16 * 4096 + (n16 < 4 ? row_state : row_out) + x * 1024) =
+                            (q & 1) ? make_uint4(t0, t1, hi[0], hi[1]) : make_uint4(lo[0], lo[1], t0, t1);
                 }
             };
             // (This loop, like the one over the quarters of the product above, is kept as a loop: a chunk's straight-line code is
@@ -702,7 +705,9 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
 // Z is written, one for the V products (tile converted, accumulator read back).  Only the completion of products and the
 // arrival of a stage go through an mbarrier.  (A version on warp-level matrix instructions, the state in their
 // accumulators, was bound by shared-memory bandwidth: each warp reads its operator columns and all of Z and V, 1.8 k
-// cycles a chunk.)  Measured: 60 us for 64 chunks of 96 chains (57 without scales, see ScanKind); 512 chains 6.1 TB/s, the roof.
+// cycles a chunk.)  Rows of the accumulator are in the order of the contraction index (k_at_position), so that a warp's lanes write
+// neighbouring rows of the operand tile: with two or four of them in one bank a chunk of the chain took 40 (gradients 150) cycles more.
+// Measured: 57.8 us for 64 chunks of 96 chains (60.2 in channel order); 512 chains 6.1 TB/s, the roof.
 // ------------------------------------------------------------------------------------------
 constexpr int kConverters = 4;                    // (one per token block of a chunk; with two the prefill's scan took 60.5 us, not 58.8)
 constexpr int kScanThreads = (10 + kConverters) * 32;
@@ -729,12 +734,12 @@ struct ScanMaps {
 
 // Row of the Z tile (and position of the contraction index in the operator) of state column j, or of the V tile of token s.
 __device__ __forceinline__ int k_position(int j) {
-    return ((j >> 5) * 4 + ((j & 7) >> 1)) * 8 + ((j >> 4) & 1) * 4 + (j & 1) + (((j & 15) >> 3) << 1);
+    return (j >> 4) * 16 + ((j & 7) >> 1) * 4 + ((j & 8) >> 2) + (j & 1);
 }
 
 // ... and the state column or token of a position.
 __device__ __forceinline__ int k_at_position(int p) {
-    return (p >> 5) * 32 + ((p >> 2) & 1) * 16 + ((p >> 1) & 1) * 8 + ((p >> 3) & 3) * 2 + (p & 1);
+    return (p >> 4) * 16 + ((p >> 1) & 1) * 8 + ((p >> 2) & 3) * 2 + (p & 1);
 }
 
 // Descriptor of the operator as A operand without swizzle: 8 x 16-byte core matrices, 128 bytes apart along k, 2048
@@ -955,7 +960,7 @@ __device__ __noinline__ void scan_gradients_by_token(const OperatorPtrs &in, con
 // before it in the scan's order and of the state as it entered the chunk three steps back, which the state warps publish.
 // Forwards values are only scaled up: a chain that overflows fp16 is recomputed in fp32.  The choice does not depend on where a call
 // is cut into segments: what the first three chunks of the next segment look back on is handed on with the chain's flag.
-// Measured, training, 96 chains x 64 chunks: 72 and 75 us.
+// Measured, training, 96 chains x 64 chunks: 71 and 67 us (gradients in channel order 76).
 enum ScanKind { kPrefill, kForTraining, kGradients };
 
 template <typename TIO, int kKind>
@@ -1219,9 +1224,8 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
         const int i0 = hf * 32;                       // this thread's 32 value channels
         if (quarter < 2) {
             // ---------------- state rows j'
-            // (gradients: this accumulator row is the channel at its position of the contraction index, and operand rows are in order)
-            const int jp = kGrad ? k_at_position(quarter * 32 + lane) : quarter * 32 + lane;
-            const int zr = kGrad ? jp : k_position(jp);
+            // (accumulator rows are in the order of the contraction index, so that neighbouring lanes write neighbouring operand rows)
+            const int zr = quarter * 32 + lane, jp = k_at_position(zr);
             const uint32_t zrow = sb + SM::kZV + off16(zr, 0);
             const uint32_t sw = ((uint32_t)zr & 7u) << 4;
             float2 Z[16];

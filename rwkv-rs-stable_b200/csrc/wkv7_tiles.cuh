@@ -49,10 +49,10 @@ __device__ __forceinline__ int accumulator_place(int i, int j) {
     return (((i >> 4) * 8 + (j >> 3)) * 32 + (i & 7) * 4 + ((j & 7) >> 1)) * 4 + (j & 1) * 2 + ((i >> 3) & 1);
 }
 
-// What the builder leaves of a chunk in global memory: the 128 x 128 fp16 operator O[n][k], n = (j' | t), as the core
+// What the builder leaves of a chunk in global memory: the 128 x 128 fp16 operator O[n][k], n = (j' in the order of k | t), as the core
 // matrices (eight rows n, eight k, 128 bytes) of a K-major tcgen05 operand without swizzle, 16 of them along k and 16 along n.
 // The contraction index (64 j, then 64 s) is ordered so that a lane of the builder holds four neighbouring k of a row in its
-// accumulators: the eight of core 4 c + q are {2q, 2q+1, 2q+8, 2q+9} of the 16-block 2 c, then the same of 2 c + 1.  Behind
+// accumulators: the eight of core 2 c + m are {2q, 2q+1, 2q+8, 2q+9} of the 16-block c for q = 2 m, then for q = 2 m + 1.  Behind
 // the operator e^{c_L}[64] in fp32, two signed exponents per channel (fx = e^{c_L} 2^ef; P and Kt are stored times 2^eg), two
 // per 16-token block (its r rows were taken times 2^-er, its k rows times 2^-ek), and the mark.
 constexpr uint32_t kOperatorBytes = 4 * kPanel;
