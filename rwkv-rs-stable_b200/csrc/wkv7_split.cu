@@ -74,7 +74,7 @@ __host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
 // Bound by shared-memory bandwidth (2.8 k cycles per chunk at one 128-byte access a cycle) and by the latency of a chunk's
 // phases, which the CTAs of an SM cover for one another; hence few warps per chunk, each with the largest tile its
 // registers hold (eight warps per chunk read a quarter more and were slower: 153 against 121 us).  Measured, 6144 chunks (8 x
-// 4096 tokens x 12 heads): 111.5 us, 4.1 TB/s; the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
+// 4096 tokens x 12 heads): 111.2 us, 4.1 TB/s; the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
 //   1. decays: warp = 16-token block, lane = channel pair; prefix and suffix products within the block
 //   2. scaled fp16 operands, in place over the bf16 tiles that TMA delivered
 //   3. the A matrices: one 128 x 128 tcgen05 product [a; r] [b; k]^T, read back a row per thread, lower triangle only; with
@@ -534,6 +534,9 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                 }
             }
         }
+        // The tiles and what lies in w's place are only read from here on: handed back to TMA now, because behind the stores of phase 5 this
+        // fence would wait for them too.
+        if (kTma) fence_proxy_async();
         __syncthreads();
         // ---------------- 5. [A~ | A~k]^T for columns j = 16 ct.. and s = 16 ct.., then the operator's rows they are
         auto finish = [&](auto block_wise) {
@@ -675,7 +678,6 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
         };
         if (wide) finish(std::true_type{});   // (two copies: merging them costs the common one a move per operand register)
         else finish(std::false_type{});
-        if (kTma) fence_proxy_async();   // the tiles are handed back to TMA
         __syncthreads();
         if (kTma && tid == 0 && more) request(unit + gridDim.x);
         // (the last chunk of this CTA: the scan may be set up)

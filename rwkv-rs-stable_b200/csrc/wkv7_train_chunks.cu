@@ -748,8 +748,8 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                 }
                 bad = !(finite <= 3.0e38f);
             }
-            if (unit + (int)gridDim.x < p.units) fetch(unit + (int)gridDim.x);
             fence_proxy_async();
+            if (unit + (int)gridDim.x < p.units) fetch(unit + (int)gridDim.x);   // (behind the fence, which waits for what was issued before it)
             bad = __syncthreads_or(bad);
             if (!bad && warp == 7 && elect_one()) {
                 int x, y;
