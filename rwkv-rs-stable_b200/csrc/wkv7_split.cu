@@ -74,7 +74,7 @@ __host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
 // Bound by shared-memory bandwidth (2.8 k cycles per chunk at one 128-byte access a cycle) and by the latency of a chunk's
 // phases, which the CTAs of an SM cover for one another; hence few warps per chunk, each with the largest tile its
 // registers hold (eight warps per chunk read a quarter more and were slower: 153 against 121 us).  Measured, 6144 chunks (8 x
-// 4096 tokens x 12 heads): 111.2 us, 4.1 TB/s; the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
+// 4096 tokens x 12 heads): 107.4 us, 4.2 TB/s; the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
 //   1. decays: warp = 16-token block, lane = channel pair; prefix and suffix products within the block
 //   2. scaled fp16 operands, in place over the bf16 tiles that TMA delivered
 //   3. the A matrices: one 128 x 128 tcgen05 product [a; r] [b; k]^T, read back a row per thread, lower triangle only; with
@@ -136,6 +136,9 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                            int Tlen, int H, int chunk0, int seg_chunks, int nchains, int wide_range, int *status) {
     extern __shared__ __align__(1024) unsigned char smem[];
     constexpr bool kTma = sizeof(TIn) == 2;
+    // How rows of the diagonal blocks are moved so that the half-warps and column halves that share an access lie in different banks.  (bf16
+    // tensors: 111.2 -> 107.4 us.  The fp32 kernel has no registers for the addresses: 14.2 -> 15.0 us for 2 x 1000 tokens x 12 heads.)
+    constexpr int kSpread = kTma ? 1 : 0;
     if (smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0) atomicExch(status, (int)kDevInternal);
         return;
@@ -405,7 +408,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             const uint32_t x[4] = {d[16 * s1 + 4 * e], d[16 * s1 + 4 * e + 1], d[16 * s1 + 4 * e + 2], d[16 * s1 + 4 * e + 3]};
-                            sts128(sb + kDiag + bt * 1024 + r * 64 + ((e ^ ((r >> 1) & 3)) << 4), x);
+                            sts128(sb + kDiag + bt * 1024 + (r ^ (bt & kSpread)) * 64 + ((e ^ ((r >> 1) & 3)) << 4), x);
                         }
                     } else if (sc <= bt) {
                         const uint32_t all = sc == bt ? 0u : ~0u;
@@ -476,7 +479,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
 #pragma unroll
                             for (int r = 0; r < 2; ++r) {
                                 const int row = g + 8 * r, piece = 2 * h + (q >> 1);
-                                sts_f2(sb + kDiag + t * 1024 + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4) + (q & 1) * 8, c[s][h][2 * r], c[s][h][2 * r + 1]);
+                                sts_f2(sb + kDiag + t * 1024 + (row ^ (t & kSpread)) * 64 + ((piece ^ ((row >> 1) & 3)) << 4) + (q & 1) * 8, c[s][h][2 * r], c[s][h][2 * r + 1]);
                             }
                     } else {
                         const uint32_t o = mat + ((warp == 0 ? below(t) : tri(t)) + s) * kBlk;
@@ -496,14 +499,15 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
             const int pair = (warp + seq) & 3;   // (which two warps changes from chunk to chunk: each sits on its own scheduler)
             if (pair < 2) {
                 const int cc = lane & 15, b = 2 * pair + (lane >> 4);
-                const uint32_t src = sb + kDiag + b * 1024;
+                // (rows of blocks 1 and 3 are exchanged in pairs: the two half-warps read different banks)
+                const uint32_t src = sb + kDiag + b * 1024, even = src + (lane >> 4) * 64 * kSpread, odd = src - (lane >> 4) * 64 * kSpread;
                 float x[16];
 #pragma unroll
                 for (int t = 0; t < 16; ++t) {
                     float acc0 = 0.f, acc1 = 0.f;
 #pragma unroll
                     for (int s4 = 0; s4 < (t + 3) / 4; ++s4) {
-                        const float4 a4 = lds_f4(src + t * 64 + ((s4 ^ ((t >> 1) & 3)) << 4));
+                        const float4 a4 = lds_f4(((t & 1) ? odd : even) + t * 64 + ((s4 ^ ((t >> 1) & 3)) << 4));
                         if (4 * s4 + 0 < t) acc0 = fmaf(a4.x, x[4 * s4 + 0], acc0);
                         if (4 * s4 + 1 < t) acc1 = fmaf(a4.y, x[4 * s4 + 1], acc1);
                         if (4 * s4 + 2 < t) acc0 = fmaf(a4.z, x[4 * s4 + 2], acc0);
@@ -512,9 +516,11 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                     x[t] = (t == cc) ? 1.f : acc0 + acc1;   // (zero above: every term up to there is)
                 }
                 __syncwarp();   // (every lane has read the block that the inverse replaces)
-                unsigned char *dst = smem + kDiag + b * 1024 + (cc >> 3) * 256 + (cc & 7) * 2;
+                // (rows in an order of their own per half and parity of the block, four and two apart: a store of the warp's 32 halves is conflict-free)
+                const uint32_t dst = (kDiag + b * 1024 + (cc >> 3) * 256 + (cc & 7) * 2) ^ ((uint32_t)(cc >> 3) << 6) * kSpread ^ ((uint32_t)(lane >> 4) << 5) * kSpread;
+                static_assert(kDiag % 256 == 0, "exclusive or of the rows");
 #pragma unroll
-                for (int t = 0; t < 16; ++t) *reinterpret_cast<__half *>(dst + t * 16) = __float2half_rn(x[t]);
+                for (int t = 0; t < 16; ++t) *reinterpret_cast<__half *>(smem + (dst ^ (uint32_t)(t << 4))) = __float2half_rn(x[t]);
             } else if (wide) {
                 const uint32_t rows = sb + kTiles + (pair == 2 ? XB : XK) * kPanel + (lane >> 3) * 128, piece = lane & 7;   // eight channels of every fourth token
 #pragma unroll 1
@@ -591,7 +597,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
                     }
                 }
                 uint32_t Tb[4];
-                ldsm4(Tb, sb + kDiag + b * 1024 + blk_cols(lane));
+                ldsm4(Tb, sb + kDiag + b * 1024 + (blk_cols(lane) ^ ((uint32_t)((lane >> 3) & 1) << 6) * kSpread ^ ((uint32_t)(b & 1) << 5) * kSpread));
                 float o[2][2][4];
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
@@ -708,7 +714,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
 // arrival of a stage go through an mbarrier.  (A version on warp-level matrix instructions, the state in their
 // accumulators, was bound by shared-memory bandwidth: each warp reads its operator columns and all of Z and V, 1.8 k
 // cycles a chunk.)  Rows of the accumulator are in the order of the contraction index (k_at_position), so that a warp's lanes write
-// neighbouring rows of the operand tile: with two or four of them in one bank a chunk of the chain took 40 (gradients 150) cycles more.
+// neighbouring rows of the operand tile: with two or four of them in one bank a chunk of the chain took 70 (gradients 270) cycles more.
 // Measured: 57.8 us for 64 chunks of 96 chains (60.2 in channel order); 512 chains 6.1 TB/s, the roof.
 // ------------------------------------------------------------------------------------------
 constexpr int kConverters = 4;                    // (one per token block of a chunk; with two the prefill's scan took 60.5 us, not 58.8)
