@@ -55,8 +55,9 @@ constexpr uint32_t kT = kArb + 4 * kBlk;
 constexpr uint32_t kDiag = kT + 4 * kBlk;                        // [4] A_ab in fp32
 constexpr uint32_t kMu = kDiag + 4 * 1024;                       // [4][64] fp32 each
 constexpr uint32_t kRho = kMu + 1024;
-constexpr uint32_t kFactors = kRho + 1024;                       // [8][64] fp32: from block to block, S then G; channel order of factor_place
-constexpr uint32_t kE = kFactors + 2048;                         // [8][64] fp32: decay over half a block
+constexpr uint32_t kFactorRow = 320;                             // (16 floats for each lane of a row group and 16 bytes: their banks differ)
+constexpr uint32_t kFactors = kRho + 1024;                       // [8][80] fp32: from block to block, S then G; channel order of factor_place
+constexpr uint32_t kE = kFactors + 8 * kFactorRow;                         // [8][64] fp32: decay over half a block
 constexpr uint32_t kTop = kE + 2048;                             // [16] largest magnitudes: of S and V, of G and dY, by warp
 constexpr uint32_t kBars = kTop + 64;
 constexpr uint32_t kSmem = kBars + 64;
@@ -95,7 +96,7 @@ __device__ __forceinline__ void pack_block(uint32_t (&x)[4], const float (&c0)[4
     x[3] = pack_half2(c1[2], c1[3]);
 }
 // Channels 8 n + 2 q, + 1 of all n next to one another: what lane q of a row group multiplies its accumulators with.
-__device__ __forceinline__ int factor_place(int j) { return ((j & 7) >> 1) * 16 + (j >> 3) * 2 + (j & 1); }
+__device__ __forceinline__ int factor_place(int j) { return ((j & 7) >> 1) * 20 + (j >> 3) * 2 + (j & 1); }
 __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
     const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&b);
@@ -267,10 +268,11 @@ __device__ __noinline__ void chunk_by_token(const ChunkArgs &p, int unit, __nv_b
 // instructions' accumulators over the four blocks of the chunk, S forwards and G backwards, without a barrier.  What the gradients need of
 // it (S mu, G rho, U, dU) is left in shared memory, and then warp = (block, half of the channels) sums over value rows.
 //
-// Bound by latency with two warps per scheduler (225 KB of shared memory leave room for one CTA): of 13.7 k cycles a chunk the
-// matrix instructions take 4.3 k of a scheduler and shared memory 8 k wavefronts.  Measured, 6144 chunks: 340 us, and 11 more since V and k, dY and r have scales of their own; the fp32
-// replay per 16 tokens that this replaced took 880, and 90 for the reversed copies it needed.  Four more warps that prepare the next
-// chunk meanwhile gained nothing (350 us): they share the port and the issue slots.
+// Bound by the shared-memory port, busy two thirds of the time (9 k wavefronts of 13.5 k cycles a chunk), and by latency with two warps per
+// scheduler (225 KB of shared memory leave room for one CTA); the matrix instructions take 4.3 k of a scheduler.  Measured, 6144 chunks:
+// 335 us; the fp32 replay per 16 tokens that this replaced took 880, and 90 for the reversed copies it needed.  Not kept: four more warps
+// that prepare the next chunk meanwhile (they share the port and the issue slots), sixteen warps with half the channels or tokens each (57 us
+// more: every warp reads its first operands itself), U and V moved in registers to be second operands instead of read again (4 us more).
 __global__ void __launch_bounds__(kThreads, 1)
 wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid_constant__ ChunkArgs p) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -472,9 +474,9 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                         const uint32_t own = sb + (q * 64 + ch) * 4;
                         const float2 mu = lds_f2(own + kMu), rho = lds_f2(own + kRho);
                         const float2 fs = q == 0 ? make_float2(scale_s, scale_s) : lds_f2(own + kRho - 256), fg = q == 3 ? make_float2(scale_g, scale_g) : lds_f2(own + kMu + 256);
-                        const uint32_t o = sb + kFactors + q * 256 + factor_place(ch) * 4;
+                        const uint32_t o = sb + kFactors + q * kFactorRow + factor_place(ch) * 4;
                         sts_f2(o, mu.x * fs.x, mu.y * fs.y);
-                        sts_f2(o + 1024, rho.x * fg.x, rho.y * fg.y);
+                        sts_f2(o + 4 * kFactorRow, rho.x * fg.x, rho.y * fg.y);
                     }
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
@@ -532,7 +534,7 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
                 for (int i = 0; i < 4; ++i) {
                     const int q = g_side ? 3 - i : i;
                     {
-                        const uint32_t f0 = sb + kFactors + (g_side ? 1024 : 0) + q * 256 + (lane & 3) * 64;
+                        const uint32_t f0 = sb + kFactors + (g_side ? 4 * kFactorRow : 0) + q * kFactorRow + (lane & 3) * 80;
 #pragma unroll
                         for (int n = 0; n < 8; n += 2) {
                             const float4 f = lds_f4(f0 + n * 8);
