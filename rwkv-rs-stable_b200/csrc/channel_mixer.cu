@@ -110,16 +110,27 @@ gemm_tn_bf16_kernel(const __grid_constant__ GemmMaps maps, void *__restrict__ ou
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     bool timed_out = false;
-    // (launched with programmatic stream serialization: set up while the kernel before it finishes)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (warp != 0) {
+        wait_for_previous();
+        let_next_in();
+    }
 
     if (warp == 0) {
         if (elect_one()) {
             uint32_t it = 0;
+            // the weights' first tiles are on their way while the kernel before this one finishes (see launch_channel_mixer)
+            const int first = blockIdx.x, ahead = first < total_tiles ? min(kStages, count_ksteps(first)) : 0;
+            for (int j = 0; j < ahead; ++j) {
+                mbar_expect_tx(&full[j], kStageBytes);
+                tma_load_2d(smem + j * kStageBytes + kABytes, &maps.b, (first_kstep(first) + j) * kBK, first % mn_tiles % n_tiles * kBN, &full[j]);
+            }
+            wait_for_previous();
+            for (int j = 0; j < ahead; ++j)
+                tma_load_2d(smem + j * kStageBytes, &maps.a, (first_kstep(first) + j) * kBK, first % mn_tiles / n_tiles * kBM, &full[j]);
             for (int tile = blockIdx.x; tile < total_tiles && !timed_out; tile += gridDim.x) {
                 const int nt = tile % mn_tiles % n_tiles, mt = tile % mn_tiles / n_tiles, k0 = first_kstep(tile), ksteps = count_ksteps(tile);
                 for (int ks = k0; ks < k0 + ksteps; ++ks, ++it) {
+                    if (it < (uint32_t)ahead) continue;
                     const uint32_t s = it % kStages, ph = (it / kStages) & 1;
                     if (!mbar_wait(&empty[s], ph ^ 1)) { timed_out = true; break; }
                     unsigned char *a = smem + s * kStageBytes, *b = a + kABytes;
@@ -210,12 +221,16 @@ gemm_tn_bf16_pair_kernel(const __grid_constant__ PairMaps maps, __nv_bfloat16 *_
     };
     PairGemm gemm;
     gemm.begin(smem, maps, warp);
-    // (launched with programmatic stream serialization: set up while the kernel before it finishes)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     bool ok = true;
+    // (the weights' first tiles are on their way while the kernel before this one finishes, see launch_channel_mixer)
     if (warp == 0) {
-        if (elect_one()) ok = gemm.produce(maps, width, items);
+        if (elect_one()) ok = gemm.produce(maps, width, items, [] { wait_for_previous(); });
+        __syncwarp();
+    }
+    wait_for_previous();
+    let_next_in();
+    if (warp == 0) {
+        // (done)
     } else if (warp == 1) {
         if (gemm.rank == 0 && elect_one()) ok = gemm.multiply(width, items);
     } else {
@@ -469,6 +484,8 @@ int launch_channel_mixer(const ChannelMixerArgs &p, void *workspace, size_t work
     float *partials = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + least);
     int threads = 32;
     while (threads < 256 && threads < p.C / 8) threads <<= 1;
+    // The products request weights before the kernel in front of them is complete.  That is one of this call's, which writes no weights
+    // and lets its successor in only when everything before it is complete.
     const cudaError_t e = launch_serialized(channel_mixer_mix_kernel, blocks_of_rows(rows, p.num_sms, 8), (unsigned)threads, 0, stream, (const __nv_bfloat16 *)p.x,
                                             (const __nv_bfloat16 *)p.key_scale, key_input, rows, p.T, p.C);
     if (e != cudaSuccess) return (int)e;

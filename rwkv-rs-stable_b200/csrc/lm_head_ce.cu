@@ -251,7 +251,7 @@ lm_head_ce_pair_kernel(const __grid_constant__ PairMaps maps, const void *__rest
     let_next_in();
     bool ok = true;
     if (warp == 0) {
-        if (elect_one()) ok = gemm.produce(maps, width, items);
+        if (elect_one()) ok = gemm.produce(maps, width, items, [] {});
     } else if (warp == 1) {
         if (gemm.rank == 0 && elect_one()) ok = gemm.multiply(width, items);
     } else {

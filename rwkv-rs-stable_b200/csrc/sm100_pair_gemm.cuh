@@ -109,21 +109,32 @@ struct PairGemm {
         cluster_sync_all();
         if (warp == 1) tmem_dealloc_pair(tmem, 512);
     }
-    // One thread of either CTA.  False when a wait expired.
-    template <typename Items>
-    __device__ __forceinline__ bool produce(const PairMaps &maps, int width, const Items &items) {
+    // One thread of either CTA.  False when a wait expired.  The first stages' slices of B are requested before `a_is_there` returns,
+    // nothing of A is.
+    template <typename Items, typename F>
+    __device__ __forceinline__ bool produce(const PairMaps &maps, int width, const Items &items, const F &a_is_there) {
         uint32_t it = 0;
         bool ok = true;
         PairItem w;
+        auto bar = [&](uint32_t s) { return map_to_cta(smem_u32(&full[s]), 0); };
+        auto load_a = [&](uint32_t s, int k) {
+            tma_load_2d_pair(smem + s * 2 * kPairHalf, &maps.a, k * kPairK, w.m0 + (int)rank * 128, bar(s));
+        };
+        auto load_b = [&](uint32_t s, int k) {
+            if (rank == 0) mbar_expect_tx(&full[s], 2 * kPairHalf + (uint32_t)width * kPairK * 2);
+            tma_load_2d_pair(smem + s * 2 * kPairHalf + kPairHalf, &maps.b, k * kPairK, w.n0 + (int)rank * (width / 2), bar(s));
+        };
+        const int ahead = items(0, w) ? min(kPairStages, w.slices) : 0;
+        for (int j = 0; j < ahead; ++j) load_b(j, w.k0 + j);
+        a_is_there();
+        for (int j = 0; j < ahead; ++j) load_a(j, w.k0 + j);
         for (int i = 0; ok && items(i, w); ++i) {
             for (int k = w.k0; k < w.k0 + w.slices; ++k, ++it) {
+                if (it < (uint32_t)ahead) continue;
                 const uint32_t s = it % kPairStages, ph = (it / kPairStages) & 1;
                 if (!mbar_wait(&empty[s], ph ^ 1)) { ok = false; break; }
-                unsigned char *a = smem + s * 2 * kPairHalf, *b = a + kPairHalf;
-                const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
-                if (rank == 0) mbar_expect_tx(&full[s], 2 * kPairHalf + (uint32_t)width * kPairK * 2);
-                tma_load_2d_pair(a, &maps.a, k * kPairK, w.m0 + (int)rank * 128, bar);
-                tma_load_2d_pair(b, &maps.b, k * kPairK, w.n0 + (int)rank * (width / 2), bar);
+                load_b(s, k);
+                load_a(s, k);
             }
         }
         // What is in flight lands, and the products' arrivals come, before the CTA leaves.
