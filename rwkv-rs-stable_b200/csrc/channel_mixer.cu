@@ -284,16 +284,19 @@ gemm_reduce_kernel(const float *__restrict__ parts, int splits, __nv_bfloat16 *_
 }
 
 // key_input = x + (shifted - x) * key_scale, shifted = previous token (zero at t == 0)
-// (channel_mixer/kernel.rs:4-25).  The rows are shared out evenly, a thread owns one 16-byte channel vector of its CTA's rows; the previous
-// row is carried in registers and the next one on its way while a row is written.  Bound by latency at the sizes of a prefill: 4096 rows of
-// 2048 channels took 14.3 us with two rows a CTA and a 64-bit division for each, 10.2 so.
+// (channel_mixer/kernel.rs:4-25).  A thread owns one 16-byte channel vector of kRows consecutive rows, and all of them and the row in
+// front are on their way before the first is used.  Bound by latency at the sizes of a prefill: 4096 rows of 2048 channels took 14.3 us with
+// two rows a CTA, one after the other, and a 64-bit division for each, 10.2 with shares of three or four; the whole call 220.6 -> 216.7 us so.
+constexpr int kMixRows = 4;
+template <int kRows>
 __global__ void __launch_bounds__(256)
 channel_mixer_mix_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ scale,
                          __nv_bfloat16 *__restrict__ out, int64_t rows, int64_t Tlen, int64_t C) {
     wait_for_previous();
     let_next_in();
-    const int64_t CV = C / 8;
-    const int64_t row_begin = rows * blockIdx.x / gridDim.x, row_end = rows * (blockIdx.x + 1) / gridDim.x;
+    const int64_t row0 = (int64_t)blockIdx.x * kRows;
+    const int count = (int)min((int64_t)kRows, rows - row0);
+    const int64_t t0 = row0 % Tlen;
     auto unpack = [](const uint4 &u, float (&f)[8]) {
         const unsigned w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -302,28 +305,27 @@ channel_mixer_mix_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat1
             f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
         }
     };
-    const int64_t t_begin = row_begin % Tlen;
-    for (int64_t cv = threadIdx.x; cv < CV; cv += blockDim.x) {
-        const int64_t c = cv * 8;
-        float mu[8], prev[8], cur[8];
-        uint4 ahead = *reinterpret_cast<const uint4 *>(x + row_begin * C + c);
-        unpack(*reinterpret_cast<const uint4 *>(scale + c), mu);
-        if (t_begin == 0) {
+    for (int64_t c = (int64_t)threadIdx.x * 8; c < C; c += (int64_t)blockDim.x * 8) {
+        const __nv_bfloat16 *from = x + row0 * C + c;
+        uint4 raw[kRows + 1];   // the row in front, then this CTA's
+        raw[0] = t0 == 0 ? make_uint4(0u, 0u, 0u, 0u) : *reinterpret_cast<const uint4 *>(from - C);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) prev[e] = 0.f;
-        } else {
-            unpack(*reinterpret_cast<const uint4 *>(x + (row_begin - 1) * C + c), prev);
-        }
-        int64_t t = t_begin;
-#pragma unroll 2
-        for (int64_t row = row_begin; row < row_end; ++row) {
-            unpack(ahead, cur);
-            if (row + 1 < row_end) ahead = *reinterpret_cast<const uint4 *>(x + (row + 1) * C + c);
+        for (int i = 0; i < kRows; ++i)
+            if (i < count) raw[i + 1] = *reinterpret_cast<const uint4 *>(from + i * C);
+        float mu[8], prev[8], cur[8];
+        unpack(*reinterpret_cast<const uint4 *>(scale + c), mu);
+        unpack(raw[0], prev);
+        int64_t t = t0;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            if (i >= count) break;
+            unpack(raw[i + 1], cur);
+            if (t == Tlen) t = 0;
             if (t == 0) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) prev[e] = 0.f;   // first token of a sequence
             }
-            if (++t == Tlen) t = 0;
+            ++t;
             uint4 o;
             unsigned *ow = &o.x;
 #pragma unroll
@@ -332,7 +334,7 @@ channel_mixer_mix_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat1
                                                                fmaf(prev[e + 1] - cur[e + 1], mu[e + 1], cur[e + 1]));
                 ow[e >> 1] = *reinterpret_cast<const unsigned *>(&h);
             }
-            *reinterpret_cast<uint4 *>(out + row * C + c) = o;
+            *reinterpret_cast<uint4 *>(out + (row0 + i) * C + c) = o;
 #pragma unroll
             for (int e = 0; e < 8; ++e) prev[e] = cur[e];
         }
@@ -486,8 +488,10 @@ int launch_channel_mixer(const ChannelMixerArgs &p, void *workspace, size_t work
     while (threads < 256 && threads < p.C / 8) threads <<= 1;
     // The products request weights before the kernel in front of them is complete.  That is one of this call's, which writes no weights
     // and lets its successor in only when everything before it is complete.
-    const cudaError_t e = launch_serialized(channel_mixer_mix_kernel, blocks_of_rows(rows, p.num_sms, 8), (unsigned)threads, 0, stream, (const __nv_bfloat16 *)p.x,
-                                            (const __nv_bfloat16 *)p.key_scale, key_input, rows, p.T, p.C);
+    const bool several = rows >= 4 * kMixRows * (int64_t)p.num_sms / 2;   // (few rows: one a CTA, so that more SMs have some)
+    const cudaError_t e = launch_serialized(several ? channel_mixer_mix_kernel<kMixRows> : channel_mixer_mix_kernel<1>,
+                                            (unsigned)(several ? (rows + kMixRows - 1) / kMixRows : rows), (unsigned)threads, 0, stream,
+                                            (const __nv_bfloat16 *)p.x, (const __nv_bfloat16 *)p.key_scale, key_input, rows, p.T, p.C);
     if (e != cudaSuccess) return (int)e;
     if (int e = launch_gemm<kEpiReluSquare>(key_input, p.key_weight, hidden, partials, room, rows, p.F, p.C, p.num_sms, p.status, stream))
         return e;
