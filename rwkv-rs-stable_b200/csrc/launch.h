@@ -14,14 +14,6 @@ __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontr
 __device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 
-// CTAs for `rows` rows, which are shared out evenly: whole rounds of `per_sm` CTAs an SM, of about 16 rows each, or with few rows a row each.
-inline unsigned blocks_of_rows(int64_t rows, int num_sms, int per_sm) {
-    const int64_t round = (int64_t)per_sm * (num_sms > 0 ? num_sms : 1);
-    if (rows <= round) return (unsigned)rows;
-    const int64_t rounds = (rows + 16 * round - 1) / (16 * round);
-    return (unsigned)(rounds * round);
-}
-
 template <typename... Params, typename... Args>
 cudaError_t launch_serialized_cluster(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, unsigned cluster, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};

@@ -16,6 +16,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "kernels.h"
 #include "launch.h"
 #include "rwkv7_b200.h"
@@ -31,7 +33,7 @@ int rows_per_block(int64_t rows, int num_sms) {
     return (int)(r < 1 ? 1 : r < kMostRows ? r : kMostRows);
 }
 
-constexpr int kMixPerSm = 4;
+constexpr int kMixPerSm = 2;
 
 __host__ __device__ __forceinline__ int64_t imin(int64_t a, int64_t b) { return a < b ? a : b; }
 
@@ -107,46 +109,47 @@ struct Mix6Ptrs {
     void *out[6];
 };
 
-// Bound by HBM, six rows written for each that is read.  The rows are shared out evenly over whole rounds of CTAs; the next row is on its
-// way while six are written, and the scales stay as they lie in memory, so that four CTAs fit an SM (kept as floats they took 48
-// registers, two CTAs fitted, and 8196 rows in blocks of 16 were 1.7 rounds).  Measured: mix6 and the two epilogues on 4 x 2049 tokens
-// of 2048 channels 141.5 -> 138.4 us.
+// Bound by HBM, six rows written for each that is read.  The grid is a window of neighbouring rows that moves over the tensor, a thread always
+// at the same channels of it: with shares of consecutive rows for every CTA the writes went to thousands of places in DRAM at a time.  The row
+// in front is read again, from L2; a thread's next two vectors are on their way while it writes six, and the scales stay as they lie in
+// memory.  Measured, 4 x 2049 tokens of 2048 channels: 46.5 us (5.05 TB/s) with shares of 14 rows, 40.9 (5.75).
 template <typename T, int EPV>
-__global__ void __launch_bounds__(256, sizeof(T) == 2 ? kMixPerSm : 2)
+__global__ void __launch_bounds__(256, kMixPerSm)
 mix6_kernel(const T *__restrict__ x, Mix6Ptrs ptrs, int64_t rows, int64_t Tlen, int64_t C) {
     wait_for_previous();
     let_next_in();
-    const int64_t CV = C / EPV;
-    const int64_t row_begin = rows * blockIdx.x / gridDim.x, row_end = rows * (blockIdx.x + 1) / gridDim.x;
-    for (int64_t cv = threadIdx.x; cv < CV; cv += blockDim.x) {
-        const int64_t c = cv * EPV;
-        Raw<T, EPV> scale[6];
+    const unsigned CV = (unsigned)(C / EPV), at = blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t step = gridDim.x * blockDim.x / CV, c = (int64_t)(at % CV) * EPV;   // rows of the window (the grid has a row's threads at least)
+    int64_t row = at / CV;
+    if (row >= step || row >= rows) return;
+    Raw<T, EPV> scale[6];
 #pragma unroll
-        for (int s = 0; s < 6; ++s) scale[s].load(reinterpret_cast<const T *>(ptrs.mu[s]) + c);
-        Pack<T, EPV> prev;
-        if (row_begin % Tlen == 0) prev.zero();
-        else prev.load(x + (row_begin - 1) * C + c);
-        int64_t t = row_begin % Tlen;
-        Raw<T, EPV> ahead;   // the next row, on its way while this one is written
-        ahead.load(x + row_begin * C + c);
+    for (int s = 0; s < 6; ++s) scale[s].load(reinterpret_cast<const T *>(ptrs.mu[s]) + c);
+    const int64_t t_step = step % Tlen;
+    int64_t t = row % Tlen;
+    Raw<T, EPV> ahead, ahead_prev;   // the next row and the one in front of it
+    auto request = [&](int64_t row, int64_t t) {
+        ahead.load(x + row * C + c);
+        if (t > 0) ahead_prev.load(x + (row - 1) * C + c);
+    };
+    request(row, t);
 #pragma unroll 1
-        for (int64_t row = row_begin; row < row_end; ++row) {
-            Pack<T, EPV> cur;
-            ahead.unpack(cur);
-            if (row + 1 < row_end) ahead.load(x + (row + 1) * C + c);
-            if (t == 0) prev.zero();  // first token of a sequence: x_{-1} = 0
-            if (++t == Tlen) t = 0;
-            Pack<T, EPV> mu[1];
+    for (; row < rows; row += step) {
+        Pack<T, EPV> cur, prev;
+        ahead.unpack(cur);
+        ahead_prev.unpack(prev);
+        if (t == 0) prev.zero();  // first token of a sequence: x_{-1} = 0
+        t += t_step;
+        if (t >= Tlen) t -= Tlen;
+        if (row + step < rows) request(row + step, t);
 #pragma unroll
-            for (int s = 0; s < 6; ++s) {
-                Pack<T, EPV> o;
-                scale[s].unpack(mu[0]);
+        for (int s = 0; s < 6; ++s) {
+            Pack<T, EPV> o, mu;
+            scale[s].unpack(mu);
 #pragma unroll
-                for (int e = 0; e < EPV; ++e)
-                    o.f[e] = fmaf(prev.f[e] - cur.f[e], mu[0].f[e], cur.f[e]);
-                o.store(reinterpret_cast<T *>(ptrs.out[s]) + row * C + c);
-            }
-            prev = cur;
+            for (int e = 0; e < EPV; ++e)
+                o.f[e] = fmaf(prev.f[e] - cur.f[e], mu.f[e], cur.f[e]);
+            o.store(reinterpret_cast<T *>(ptrs.out[s]) + row * C + c);
         }
     }
 }
@@ -302,9 +305,10 @@ int launch_mix6(const MixArgs &p, cudaStream_t stream) {
         ptrs.out[s] = p.out[s];
         vec_ok = vec_ok && aligned16(p.mu[s]) && aligned16(p.out[s]);
     }
-    const unsigned grid = blocks_of_rows(rows, p.num_sms, kMixPerSm);
     auto go = [&](auto kernel, int64_t vectors) {
-        return (int)launch_serialized(kernel, grid, (unsigned)pick_threads(vectors), 0, stream, (decltype(first_parameter(kernel)))p.x, ptrs, rows, p.T, p.C);
+        // two CTAs an SM, or as many as there are vectors, and a row's at least
+        const int64_t most = (rows * vectors + 255) / 256, fill = std::max<int64_t>(2 * (int64_t)(p.num_sms > 0 ? p.num_sms : 1), (vectors + 255) / 256);
+        return (int)launch_serialized(kernel, (unsigned)imin(most, fill), 256u, 0, stream, (decltype(first_parameter(kernel)))p.x, ptrs, rows, p.T, p.C);
     };
     using bf = __nv_bfloat16;
     if (p.bf16) return vec_ok && p.C % 8 == 0 ? go(mix6_kernel<bf, 8>, p.C / 8) : go(mix6_kernel<bf, 1>, p.C);
