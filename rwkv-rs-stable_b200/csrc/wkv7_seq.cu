@@ -109,8 +109,14 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
     // Fallback mode: only the chains another kernel flagged are (re)computed.
     // (launched behind the kernel in front of it, which writes the flags, possibly before that has finished; a no-op for an ordinary launch)
     wait_for_previous();
-    let_next_in();
-    if (flags != nullptr && flags[bh] == 0) return;
+    if (flags != nullptr) {
+        // (Nobody is let in early here: behind this pass comes the next call's operator kernel, four CTAs of 57 KB to an SM.  One that
+        // starts beside CTAs of this kernel, whose SM keeps a smaller share of its memory as shared memory, finds room for one or two and keeps
+        // it at that: 3 x 2047 tokens x 32 heads 99.6 -> 113 us.)
+        if (flags[bh] == 0) return;
+    } else {
+        let_next_in();
+    }
     const int split = blockIdx.x % SPLITS;
     const int bi = bh / H, h = bh % H;
     const int row0 = split * ROWS;
@@ -369,6 +375,8 @@ int launch_seq64(const Wkv7Args &p, cudaStream_t stream, const int *flags = null
     constexpr unsigned threads = ROWS / RPT * 4;
     auto kern = wkv7_seq64_kernel<T, ROWS, RPT, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the kernel that is let in beside this one may want all of an SM's shared memory)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return (int)e;
     const unsigned grid = (unsigned)(p.B * p.H * (kN / ROWS));
     return (int)launch_serialized(kern, grid, threads, smem, stream, ptrs, p.s0, reinterpret_cast<T *>(p.y), p.s_out, (int)p.T, (int)p.H, flags, SavePtrs{});
