@@ -1519,23 +1519,28 @@ WorkspaceLayout layout_for(size_t chains, size_t seg, int buffers, bool cut) {
 // CTA per chain (0.85 us per chunk), the operator kernel throughput work that fills every SM (2.8 us per chunk and SM).  On SM partitions
 // the scans have `chains` SMs rounded up to eight and the operator kernel the rest.  Without, the operator kernel leaves as many
 // SMs' worth of CTAs out as there are chains, and the scans, on a stream of higher priority, take the SMs that have no operator
-// CTA (a scan CTA's 217 KB and an operator CTA's 57 KB do not fit one SM).  Measured (B200, 148 SMs; in sequence / on partitions /
-// beside without partitions, the last from a captured graph, where that is what runs and in sequence takes the figure in brackets; us):
-//     chains x chunks    192               256                    512                    1024
-//     12                 207 / 210         269 / 271              502 / 481              973 / 895
-//     16                 220 / 220         284 / 281              542 / 497              1045 / 919
-//     24                 249 / 240         319 / 298 / 274 (316)  614 / 522 / 490 (623)  1216 / 956 / 914 (1205)
-//     32                 274 / 256         358 / 315 / 289 (361)  685 / 551 / 516 (693)  1376 / 1000 / 957 (1356)
-// and at 128 chunks 156 / 153 for 12 chains.  With fewer than 24 chains the schedule without partitions loses (12 x 512: 537 against
-// 502).  Hence: at most 27 % as many chains as SMs and at least 192 chunks, or at most 11 % and at least 128.  (That bound is
-// from kernels of other speeds; more chains have not been measured with these.)
+// CTA (a scan CTA's 217 KB and an operator CTA's 57 KB do not fit one SM).  Measured (B200, 148 SMs; in sequence / on partitions; us):
+//     chains x chunks    128          192          256          320          384          512          1024
+//     4                               148 / 164    198 / 213    239 / 256
+//     12                 125 / 132    177 / 185    228 / 238    280 / 286    334 / 330    439 / 423    864 / 799
+//     16                 132 / 137    189 / 192    247 / 246    303 / 296    359 / 343    476 / 443    935 / 823
+//     20                              201 / 202    264 / 253    327 / 305
+//     24                              217 / 208    282 / 263    350 / 317    415 / 365    550 / 469    1098 / 867
+//     32                              241 / 225    319 / 282    392 / 338    467 / 394    618 / 502    1237 / 923
+//     40                              269 / 261    354 / 329    436 / 394
+//     44                              282 / 291    374 / 370    458 / 447
+//     48                              294 / 310    388 / 395    482 / 475
+//     56                              324 / 368    425 / 471    527 / 576
+// Without partitions (from a captured graph, where that is what runs; with kernels of other speeds): 24 x 256 274 us against 316 in
+// sequence, 24 x 512 490 (623), 32 x 256 289 (361); with fewer than 24 chains it loses (12 x 512: 537 against 502).
 bool overlap_applies(size_t chains, size_t nchunks, int num_sms) {
-    return wkv7_split_overlap() != 0 && num_sms > 0 && chains * 100 <= (size_t)num_sms * 27 &&
-           (nchunks >= 192 || (nchunks >= 128 && chains * 100 <= (size_t)num_sms * 11));
+    if (wkv7_split_overlap() == 0 || num_sms <= 0) return false;
+    const size_t share = chains * 1000 / (size_t)num_sms;   // chains in thousandths of the SMs
+    return share <= 280 && nchunks >= (share >= 160 ? 192u : share >= 130 ? 256u : share >= 105 ? 320u : 384u);
 }
-// (the schedule without partitions, where they are not to be had: from 16 % as many chains as SMs and 256 chunks on)
+// (the schedule without partitions, where they are not to be had: 16 to 27 % as many chains as SMs, from 256 chunks on)
 bool shared_sm_overlap_pays(size_t chains, size_t nchunks, int num_sms) {
-    return chains * 100 >= (size_t)num_sms * 16 && nchunks >= 256;
+    return chains * 100 >= (size_t)num_sms * 16 && chains * 100 <= (size_t)num_sms * 27 && nchunks >= 256;
 }
 
 size_t preferred_segment(size_t chains, size_t nchunks, bool overlap) {
