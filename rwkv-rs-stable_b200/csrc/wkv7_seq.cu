@@ -109,13 +109,14 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
     // Fallback mode: only the chains another kernel flagged are (re)computed.
     // (launched behind the kernel in front of it, which writes the flags, possibly before that has finished; a no-op for an ordinary launch)
     wait_for_previous();
+    // The kernel behind is not let in early: the next call's CTAs would take the places that are free beside this one's, which
+    // need not be where its load is even (short calls back to back: 12 tokens x 264 chains 7.7 us so, 10.5 let in at once, 9.4 launched in the ordinary way; 16 x 84
+    // 7.1 / 8.8 / 8.6; fp32 22 x 80 9.7 / 12.2 / 12.4; 45 x 896 64.4 / 64.4 / 66.1).
     if (flags != nullptr) {
-        // (Nobody is let in early here: behind this pass comes the next call's operator kernel, four CTAs of 57 KB to an SM.  One that
+        // (Nor behind the pass over flagged chains: there may come the next call's operator kernel, four CTAs of 57 KB to an SM.  One that
         // starts beside CTAs of this kernel, whose SM keeps a smaller share of its memory as shared memory, finds room for one or two and keeps
         // it at that: 3 x 2047 tokens x 32 heads 99.6 -> 113 us.)
         if (flags[bh] == 0) return;
-    } else {
-        let_next_in();
     }
     const int split = blockIdx.x % SPLITS;
     const int bi = bh / H, h = bh % H;
@@ -375,7 +376,7 @@ int launch_seq64(const Wkv7Args &p, cudaStream_t stream, const int *flags = null
     constexpr unsigned threads = ROWS / RPT * 4;
     auto kern = wkv7_seq64_kernel<T, ROWS, RPT, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // (the kernel that is let in beside this one may want all of an SM's shared memory)
+    // (as many CTAs on an SM as its shared memory holds: 19 tokens x 108 chains of fp32 tensors 8.3 -> 7.7 us back to back)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return (int)e;
     const unsigned grid = (unsigned)(p.B * p.H * (kN / ROWS));
