@@ -401,10 +401,11 @@ size_t gemm_partial_bytes(int64_t M, int64_t N, int64_t K) {
 // Width of the tiles of a product on pairs of CTAs, 0 if it goes to single CTAs (`splits`: the pieces those would cut K in).  Compared is
 // what one worker does after the other, in cycles: a K slice costs the tensor core 2 cycles a column, and its loads 240 and 0.9 a column
 // (70 bytes a cycle and SM); single CTAs are a tenth slower at the same shape, and pieces of K write and read their sums.  Narrower tiles
-// fill the waves better but read A more often, which a launch bound by power pays for, hence 4 % against them.
+// fill the waves better but read A more often, which a launch bound by power pays for, hence 4 % against them
+// (a charge of 35 % of the columns saved, as the LM head has it: 30000 rows at C = 1024 373.1 / 371.8 us, 20000 254.5 / 254.8).
 // Measured (B200, whole channel mixer; single CTAs / pairs with 256 columns throughout / as chosen here, us): 4096 rows at C = 2048 242 / 215 /
 // 208, 1024 rows 90 / 99 / 71, 1500 rows 110 / 102 / 85, 2048 rows at C = 2560 249 / 223 / 176, 3000 rows at C = 768 57 / 54 / 41,
-// 8191 rows at C = 4096 1964 / 1963 / 1625, 300 rows at C = 2560 62 / 89 / 62 (three blocks of 128 rows are two of 256: single CTAs).
+// 300 rows at C = 2560 62 / 89 / 62 (three blocks of 128 rows are two of 256: single CTAs).
 int gemm_pair_width(int64_t M, int64_t N, int64_t K, int num_sms, int splits) {
     if (M <= kBM || num_sms < 2) return 0;
     const int64_t slices = (K + kBK - 1) / kBK, tiles = (M + kBM - 1) / kBM * ((N + kBN - 1) / kBN);
