@@ -113,9 +113,9 @@ wkv7_seq64_kernel(SeqPtrs ptrs, const float *s0, T *__restrict__ y,
     // need not be where its load is even (short calls back to back: 12 tokens x 264 chains 7.7 us so, 10.5 let in at once, 9.4 launched in the ordinary way; 16 x 84
     // 7.1 / 8.8 / 8.6; fp32 22 x 80 9.7 / 12.2 / 12.4; 45 x 896 64.4 / 64.4 / 66.1).
     if (flags != nullptr) {
-        // (Nor behind the pass over flagged chains: there may come the next call's operator kernel, four CTAs of 57 KB to an SM.  One that
-        // starts beside CTAs of this kernel, whose SM keeps a smaller share of its memory as shared memory, finds room for one or two and keeps
-        // it at that: 3 x 2047 tokens x 32 heads 99.6 -> 113 us.)
+        // (Nor behind the pass over flagged chains: there may come the next call's operator kernel, four CTAs of 57 KB to an SM.  Those that
+        // start beside CTAs of this kernel lie unevenly for as long as they run: 3 x 2047 tokens x 32 heads 98.7 -> 105.3 us, 113 where an SM that
+        // holds CTAs of this kernel keeps a smaller share of its memory as shared memory; 8 x 4096 x 12 166 -> 181.)
         if (flags[bh] == 0) return;
     }
     const int split = blockIdx.x % SPLITS;
