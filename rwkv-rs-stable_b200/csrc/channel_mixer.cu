@@ -14,7 +14,7 @@
 // rectified accumulator before it is rounded to bf16.
 //
 // GEMM: out[M,N] = act(A[M,K] . B[N,K]^T), A and B row-major bf16 (both "K-major"), fp32 accumulation in TMEM, bf16 output.
-// From 129 rows on mostly by pairs of CTAs (gemm_tn_bf16_pair_kernel, see gemm_pair_width and sm100_pair_gemm.cuh).  Few rows, and
+// From 129 rows on mostly by pairs of CTAs (gemm_tn_bf16_pair_kernel, see gemm_plan::pair_width and sm100_pair_gemm.cuh).  Few rows, and
 // rows that fill their blocks of 256 badly, by single CTAs: persistent, one per SM; a tile is 128 x 256;
 // tiles are walked with the column block fastest, so that the CTAs running together share a
 // few row blocks of A and sweep all of B, and both stay in L2.  Warp roles as in the LM-head
@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "gemm_plan.h"
 #include "kernels.h"
 #include "launch.h"
 #include "rwkv7_b200.h"
@@ -42,6 +43,7 @@ namespace {
 using namespace sm100;
 
 constexpr int kBM = 128, kBN = 256, kBK = 64, kStages = 4;
+static_assert(kBM == gemm_plan::kRows && kBN == gemm_plan::kCols && kBK == gemm_plan::kSlice && kPairM == gemm_plan::kPairRows, "as planned");
 constexpr int kThreads = 192;  // TMA warp, MMA warp, four epilogue warps
 constexpr uint32_t kABytes = kBM * kBK * 2, kBBytes = kBN * kBK * 2;
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
@@ -371,66 +373,14 @@ int encode_rows_by_k(EncodeTiledFn encode, CUtensorMap *map, const void *base, i
                : (int)cudaErrorInvalidValue;
 }
 
-// Pieces of K per output tile.  With fewer than half as many tiles as SMs (a decode batch: 128 rows are one row of
-// tiles, 8 of them for 2048 columns) most of the device would idle while a few SMs stream the whole weight matrix, so K is
-// cut until every SM has an item, in pieces of at least four K steps, and a second kernel adds the fp32 sums up.  Measured
-// (B200, C = 2048, F = 8192): one row 91 -> 36 us, 64 rows at C = 4096 172 -> 78 us.
-// (At most 18, the 148 SMs over the 8 tiles of 2048 columns: a bound on the partial sums of narrower products, whose K is short
-// enough at the widths in use that the four K steps of a piece bind first.)
-// `room`: bytes for the sums; with less than the pieces take there are fewer of them.
-constexpr int kMaxGemmSplits = 18;
-int gemm_splits(int64_t M, int64_t N, int64_t K, int num_sms, size_t room) {
-    const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN), ksteps = (K + kBK - 1) / kBK;
-    if (2 * tiles > num_sms) return 1;
-    int64_t sp = num_sms / tiles;
-    if (sp > ksteps / 4) sp = ksteps / 4;
-    if (sp > kMaxGemmSplits) sp = kMaxGemmSplits;
-    const int64_t fit = (int64_t)(room / ((size_t)M * N * sizeof(float)));
-    if (sp > fit) sp = fit;
-    if (sp < 2) return 1;
-    const int64_t per = (ksteps + sp - 1) / sp;
-    return (int)((ksteps + per - 1) / per);   // (no piece is empty)
-}
-// fp32 partial sums of any device up to this many SMs.
-constexpr int kMostSms = 160;
-size_t gemm_partial_bytes(int64_t M, int64_t N, int64_t K) {
-    const int sp = gemm_splits(M, N, K, kMostSms, SIZE_MAX);
-    return sp > 1 ? (size_t)sp * M * N * sizeof(float) : 0;
-}
-
-// Width of the tiles of a product on pairs of CTAs, 0 if it goes to single CTAs (`splits`: the pieces those would cut K in).  Compared is
-// what one worker does after the other, in cycles: a K slice costs the tensor core 2 cycles a column, and its loads 240 and 0.9 a column
-// (70 bytes a cycle and SM); single CTAs are a tenth slower at the same shape, and pieces of K write and read their sums.  Narrower tiles
-// fill the waves better but read A more often, which a launch bound by power pays for, hence 4 % against them
-// (a charge of 35 % of the columns saved, as the LM head has it: 30000 rows at C = 1024 373.1 / 371.8 us, 20000 254.5 / 254.8).
-// Measured (B200, whole channel mixer; single CTAs / pairs with 256 columns throughout / as chosen here, us): 4096 rows at C = 2048 242 / 215 /
-// 208, 1024 rows 90 / 99 / 71, 1500 rows 110 / 102 / 85, 2048 rows at C = 2560 249 / 223 / 176, 3000 rows at C = 768 57 / 54 / 41,
-// 300 rows at C = 2560 62 / 89 / 62 (three blocks of 128 rows are two of 256: single CTAs).
-int gemm_pair_width(int64_t M, int64_t N, int64_t K, int num_sms, int splits) {
-    if (M <= kBM || num_sms < 2) return 0;
-    const int64_t slices = (K + kBK - 1) / kBK, tiles = (M + kBM - 1) / kBM * ((N + kBN - 1) / kBN);
-    double best = 1.1 * 512 * (splits > 1 ? (double)((slices + splits - 1) / splits) : (double)((tiles + num_sms - 1) / num_sms * slices));
-    if (splits > 1) best += 4000 + (double)splits * M * N * 8 / 2000;
-    int width = 0;
-    for (int w = kPairN; w >= 64; w -= 16) {
-        const int64_t pair_tiles = (M + kPairM - 1) / kPairM * ((N + w - 1) / w);
-        const double cost = (double)((pair_tiles + num_sms / 2 - 1) / (num_sms / 2) * slices) * std::max(2.0 * w, 240 + 0.9 * w) * (w < kPairN ? 1.04 : 1.0);
-        if (cost < best) {
-            best = cost;
-            width = w;
-        }
-    }
-    return width;
-}
-
 // out[M,N] = act(A[M,K] . B[N,K]^T); K and N multiples of 8, all pointers 16-byte aligned.
 template <int EPI>
 int launch_gemm(const void *a, const void *b, void *out, float *partials, size_t room, int64_t M, int64_t N, int64_t K, int num_sms,
                 int *status, cudaStream_t stream) {
     EncodeTiledFn encode = gemm_encode_fn();
     if (encode == nullptr) return (int)cudaErrorNotSupported;
-    const int splits = gemm_splits(M, N, K, num_sms < kMostSms ? num_sms : kMostSms, room);
-    if (const int width = gemm_pair_width(M, N, K, num_sms, splits)) {
+    const int splits = gemm_plan::k_pieces(M, N, K, std::min(num_sms, gemm_plan::kMostSms), room);
+    if (const int width = gemm_plan::pair_width(M, N, K, num_sms, splits)) {
         PairMaps maps;
         if (int e = encode_rows_by_k(encode, &maps.a, a, M, K, kPairM / 2)) return e;
         if (int e = encode_rows_by_k(encode, &maps.b, b, N, K, width / 2)) return e;
@@ -472,7 +422,7 @@ size_t channel_mixer_min_workspace_bytes(int64_t rows, int64_t C, int64_t F) {
 
 size_t channel_mixer_workspace_bytes(int64_t rows, int64_t C, int64_t F) {
     if (rows <= 0 || C <= 0 || F <= 0) return 0;
-    const size_t p1 = gemm_partial_bytes(rows, F, C), p2 = gemm_partial_bytes(rows, C, F);
+    const size_t p1 = gemm_plan::partial_bytes(rows, F, C), p2 = gemm_plan::partial_bytes(rows, C, F);
     return channel_mixer_min_workspace_bytes(rows, C, F) + align256(p1 > p2 ? p1 : p2);
 }
 

@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "gemm_plan.h"
 #include "kernels.h"
 #include "launch.h"
 #include "rwkv7_b200.h"
@@ -36,6 +37,7 @@ namespace {
 using namespace sm100;
 
 constexpr int kBM = 128, kBN = 256, kBK = 64, kStages = 4;
+static_assert(kBM == gemm_plan::kRows && kBN == gemm_plan::kCols && kBK == gemm_plan::kSlice && kPairM == gemm_plan::kPairRows, "as planned");
 constexpr int kThreads = 192;  // TMA warp, MMA warp, four epilogue warps
 constexpr uint32_t kABytes = kBM * kBK * 2, kBBytes = kBN * kBK * 2;
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
@@ -341,59 +343,17 @@ EncodeTiledFn lm_encode_fn() {
     return fn;
 }
 
-// Vocabulary splits per row block and the tiles' width.  A CTA takes one block of 128 rows and a run of column tiles, one CTA fits an
-// SM, so a launch runs in waves of `num_sms` CTAs (or half as many pairs) and its time goes with waves x (columns per CTA): the split
-// count and width that minimise that product are taken (half a tile is charged per CTA for filling its pipeline, which favours fewer
-// splits on a tie, and eight columns a tile, which favours wide ones).  Example, 148 SMs, 256 row blocks x 32 column tiles: one or two splits take 2 x 32 = 4 x 16 = 64
-// tile times, four splits 7 x 8 = 56 (the ideal is 55.4): 1140 -> 1195 TFLOP/s on that shape.  (Persistent CTAs that
-// walk the work items themselves measured no better: 1167.)
-// Most splits per row block: 16, and with few row blocks as many as give every SM of a large device a CTA of its own
-// (a call of up to 128 rows is one row block: with 16 splits, 16 SMs read the whole weight matrix: 188 us for 16 rows
-// at C = 2048, V = 65 536, against 73).
-constexpr int kFewSplits = 16;
-int max_splits(int64_t R) {
-    const int64_t rbs = (R + kBM - 1) / kBM, fill = rbs > 0 ? 160 / rbs : 160;
-    return (int)(fill > kFewSplits ? fill : kFewSplits);
-}
-size_t split_bytes(int64_t R, int64_t V, int most) {
-    const int64_t tiles = (V + kBN - 1) / kBN, sp = tiles < most ? tiles : most;
-    return sp > 1 ? (size_t)sp * (size_t)R * 3 * sizeof(float) : 0;
-}
-// How a launch is cut.
-struct Plan {
-    int row_blocks, width, splits, tiles_per_split;
-    double cost;   // columns that a worker does one after the other
-};
-// `rows` of a block, `workers` CTAs or pairs of them; `most`: splits that the workspace has room for.
-Plan plan(int64_t R, int64_t V, int rows, int workers, int64_t most) {
-    Plan best{};
-    const int rbs = (int)((R + rows - 1) / rows);
-    for (int width = kBN; width >= 128; width -= 16) {
-        const int tiles = (int)((V + width - 1) / width);
-        for (int want = 1; want <= max_splits(R) && want <= tiles && want <= most; ++want) {
-            const int tps = (tiles + want - 1) / want;
-            const int sp = (tiles + tps - 1) / tps;
-            const long long waves = ((long long)rbs * sp + workers - 1) / workers;
-            // (narrow tiles read x more often, which costs power where the tensor cores are the bound: 8831 rows at C = 1024 851 us with 256
-            // columns, 945 with 192, which fit their waves 2 % better; a single row block is bound by reading W)
-            const double cost = (double)waves * (tps * (width + 8) + 128) * (R > kBM ? 1.0 + 0.35 * (kBN - width) / kBN : 1.0);
-            if (best.row_blocks == 0 || cost < best.cost - 1e-9) best = Plan{rbs, width, sp, tps, cost};
-        }
-    }
-    return best;
-}
-
 }  // namespace
 
 // Upper bound for any device: one triple per row per vocabulary split, at most max_splits of them.  (Fewer rows may have more
 // splits: a workspace laid out for the largest batch serves a smaller one with as many as it has room for.)
 size_t lm_head_ce_workspace_bytes(int64_t R, int64_t C, int64_t V) {
     (void)C;
-    return split_bytes(R, V, max_splits(R));
+    return gemm_plan::split_bytes(R, V, gemm_plan::max_splits(R));
 }
 size_t lm_head_ce_min_workspace_bytes(int64_t R, int64_t C, int64_t V) {
     (void)C;
-    return split_bytes(R, V, kFewSplits);
+    return gemm_plan::split_bytes(R, V, gemm_plan::kFewSplits);
 }
 
 int launch_lm_head_ce_partial(const LmHeadArgs &p, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
@@ -402,13 +362,7 @@ int launch_lm_head_ce_partial(const LmHeadArgs &p, void *workspace, size_t works
     if ((reinterpret_cast<uintptr_t>(p.x) & 15u) || (reinterpret_cast<uintptr_t>(p.w) & 15u))
         return (int)cudaErrorMisalignedAddress;
     const int64_t room = workspace == nullptr ? 1 : std::max<int64_t>(1, (int64_t)(workspace_bytes / ((size_t)p.R * 3 * sizeof(float))));
-    const int sms = p.num_sms > 0 ? p.num_sms : 1;
-    const Plan one = plan(p.R, p.V, kBM, sms, room), two = plan(p.R, p.V, kPairM, sms / 2, room);
-    // A pair's tile costs less the longer its sums are: what two CTAs hand each other at its end weighs less.  Measured (B200, V = 65 536,
-    // single CTAs / pairs, us): 8191 rows at C = 2048 1510 / 1460, 20 000 at C = 768 1484 / 1554, 500 at C = 1024 75 / 72, 200 at
-    // C = 4096 147 / 125; 16 384 at C = 4096 and V = 8192 1065 / 997; 300 rows at C = 4096, three blocks of 128 and two of 256, 195 / 215.
-    const bool pairs = p.R > kBM && sms > 1 && two.cost * (0.92 + 80.0 / (double)p.C) < one.cost;
-    const Plan &cut = pairs ? two : one;
+    const gemm_plan::LmHeadCut cut = gemm_plan::lm_head_cut(p.R, p.C, p.V, p.num_sms, room);
     auto describe = [&](CUtensorMap *map, const void *ptr, int64_t rows, int box_rows) {
         const cuuint32_t estr[2] = {1, 1}, box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
         const cuuint64_t dims[2] = {(cuuint64_t)p.C, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)p.C * 2};
@@ -419,7 +373,7 @@ int launch_lm_head_ce_partial(const LmHeadArgs &p, void *workspace, size_t works
     const int splits = cut.splits;
     float *parts = splits == 1 ? p.partials : static_cast<float *>(workspace);
     cudaError_t e;
-    if (pairs) {
+    if (cut.pairs) {
         PairMaps maps;
         if (!describe(&maps.a, p.x, p.R, kPairM / 2) || !describe(&maps.b, p.w, p.V, cut.width / 2)) return (int)cudaErrorInvalidValue;
         e = cudaFuncSetAttribute(lm_head_ce_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem);
