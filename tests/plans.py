@@ -17,6 +17,8 @@ def library():
     lib = ctypes.CDLL(out)
     lib.plan_lm_head.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int] + [ctypes.c_int64, ctypes.POINTER(ctypes.c_int64)]
     lib.plan_product.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int] + [ctypes.c_size_t, ctypes.POINTER(ctypes.c_int64)]
+    lib.plan_lm_head_ns.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int] + [ctypes.c_int64]
+    lib.plan_lm_head_ns.restype = ctypes.c_int64
     return lib
 
 
@@ -24,6 +26,10 @@ def lm_head(R, C, V, num_sms=148, most=ALL):
     out = (ctypes.c_int64 * 5)()
     library().plan_lm_head(R, C, V, num_sms, most, out)
     return dict(zip(("row_blocks", "width", "splits", "tiles_per_split", "pairs"), out))
+
+
+def lm_head_ns(R, C, V, num_sms=148, most=ALL):
+    return library().plan_lm_head_ns(R, C, V, num_sms, most)
 
 
 def product(M, N, K, num_sms=148, room=ALL):
