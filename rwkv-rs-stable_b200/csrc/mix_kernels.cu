@@ -33,7 +33,10 @@ int rows_per_block(int64_t rows, int num_sms) {
     return (int)(r < 1 ? 1 : r < kMostRows ? r : kMostRows);
 }
 
-constexpr int kMixPerSm = 2;
+// CTAs of mix6 on an SM.  With one element a thread (odd channel counts, tensors off 16 bytes) two of them have too little in flight:
+// 4 x 2049 tokens of 2049 channels, bf16 / fp32 tensors, 140 / 168 us with two, 92 / 124 with four, 68 / 121 with six, 75 / 147 with eight.
+template <int EPV>
+constexpr int kMixPerSm = EPV == 1 ? 6 : 2;
 
 __host__ __device__ __forceinline__ int64_t imin(int64_t a, int64_t b) { return a < b ? a : b; }
 
@@ -114,7 +117,7 @@ struct Mix6Ptrs {
 // in front is read again, from L2; a thread's next two vectors are on their way while it writes six, and the scales stay as they lie in
 // memory.  Measured, 4 x 2049 tokens of 2048 channels: 46.5 us (5.05 TB/s) with shares of 14 rows, 40.9 (5.75).
 template <typename T, int EPV>
-__global__ void __launch_bounds__(256, kMixPerSm)
+__global__ void __launch_bounds__(256, kMixPerSm<EPV>)
 mix6_kernel(const T *__restrict__ x, Mix6Ptrs ptrs, int64_t rows, int64_t Tlen, int64_t C) {
     wait_for_previous();
     let_next_in();
@@ -305,14 +308,14 @@ int launch_mix6(const MixArgs &p, cudaStream_t stream) {
         ptrs.out[s] = p.out[s];
         vec_ok = vec_ok && aligned16(p.mu[s]) && aligned16(p.out[s]);
     }
-    auto go = [&](auto kernel, int64_t vectors) {
-        // two CTAs an SM, or as many as there are vectors, and a row's at least
-        const int64_t most = (rows * vectors + 255) / 256, fill = std::max<int64_t>(2 * (int64_t)(p.num_sms > 0 ? p.num_sms : 1), (vectors + 255) / 256);
+    auto go = [&](auto kernel, int per_sm, int64_t vectors) {
+        // so many CTAs an SM, or as many as there are vectors, and a row's at least
+        const int64_t most = (rows * vectors + 255) / 256, fill = std::max<int64_t>(per_sm * (int64_t)(p.num_sms > 0 ? p.num_sms : 1), (vectors + 255) / 256);
         return (int)launch_serialized(kernel, (unsigned)imin(most, fill), 256u, 0, stream, (decltype(first_parameter(kernel)))p.x, ptrs, rows, p.T, p.C);
     };
     using bf = __nv_bfloat16;
-    if (p.bf16) return vec_ok && p.C % 8 == 0 ? go(mix6_kernel<bf, 8>, p.C / 8) : go(mix6_kernel<bf, 1>, p.C);
-    return vec_ok && p.C % 4 == 0 ? go(mix6_kernel<float, 4>, p.C / 4) : go(mix6_kernel<float, 1>, p.C);
+    if (p.bf16) return vec_ok && p.C % 8 == 0 ? go(mix6_kernel<bf, 8>, kMixPerSm<8>, p.C / 8) : go(mix6_kernel<bf, 1>, kMixPerSm<1>, p.C);
+    return vec_ok && p.C % 4 == 0 ? go(mix6_kernel<float, 4>, kMixPerSm<4>, p.C / 4) : go(mix6_kernel<float, 1>, kMixPerSm<1>, p.C);
 }
 
 template <typename T, int EPV>
