@@ -52,6 +52,7 @@
 #include "sm100_mma.cuh"
 #include "sm100_umma.cuh"
 #include "trace.h"
+#include "wkv7_overlap.h"
 #include "wkv7_tiles.cuh"
 
 namespace rwkv7 {
@@ -1515,32 +1516,9 @@ WorkspaceLayout layout_for(size_t chains, size_t seg, int buffers, bool cut) {
 // How a call is cut: the number of segments that balances the scan of the last segment (which nothing
 // overlaps) against the few microseconds a segment boundary costs, within the operator budget.
 //
-// When the scan of a segment may run beside the operator kernel of the next one.  The scan is one latency-bound
-// CTA per chain (0.85 us per chunk), the operator kernel throughput work that fills every SM (2.8 us per chunk and SM).  On SM partitions
-// the scans have `chains` SMs rounded up to eight and the operator kernel the rest.  Without, the operator kernel leaves as many
-// SMs' worth of CTAs out as there are chains, and the scans, on a stream of higher priority, take the SMs that have no operator
-// CTA (a scan CTA's 217 KB and an operator CTA's 57 KB do not fit one SM).  Measured (B200, 148 SMs; in sequence / on partitions; us):
-//     chains x chunks    128          192          256          320          384          512          1024
-//     4                               148 / 164    198 / 213    239 / 256
-//     12                 125 / 132    177 / 185    228 / 238    280 / 286    334 / 330    439 / 423    864 / 799
-//     16                 132 / 137    189 / 192    247 / 246    303 / 296    359 / 343    476 / 443    935 / 823
-//     20                              201 / 202    264 / 253    327 / 305
-//     24                              217 / 208    282 / 263    350 / 317    415 / 365    550 / 469    1098 / 867
-//     32                              241 / 225    319 / 282    392 / 338    467 / 394    618 / 502    1237 / 923
-//     40                              269 / 261    354 / 329    436 / 394
-//     44                              282 / 291    374 / 370    458 / 447
-//     48                              294 / 310    388 / 395    482 / 475
-//     56                              324 / 368    425 / 471    527 / 576
-// Without partitions (from a captured graph, where that is what runs; with kernels of other speeds): 24 x 256 274 us against 316 in
-// sequence, 24 x 512 490 (623), 32 x 256 289 (361); with fewer than 24 chains it loses (12 x 512: 537 against 502).
+// When the scan of a segment may run beside the operator kernel of the next one: see wkv7_overlap.h.
 bool overlap_applies(size_t chains, size_t nchunks, int num_sms) {
-    if (wkv7_split_overlap() == 0 || num_sms <= 0) return false;
-    const size_t share = chains * 1000 / (size_t)num_sms;   // chains in thousandths of the SMs
-    return share <= 280 && nchunks >= (share >= 160 ? 192u : share >= 130 ? 256u : share >= 105 ? 320u : 384u);
-}
-// (the schedule without partitions, where they are not to be had: 16 to 27 % as many chains as SMs, from 256 chunks on)
-bool shared_sm_overlap_pays(size_t chains, size_t nchunks, int num_sms) {
-    return chains * 100 >= (size_t)num_sms * 16 && chains * 100 <= (size_t)num_sms * 27 && nchunks >= 256;
+    return wkv7_split_overlap() != 0 && partition_overlap_pays(chains, nchunks, num_sms);
 }
 
 size_t preferred_segment(size_t chains, size_t nchunks, bool overlap) {

@@ -1,5 +1,6 @@
-// The cuts of the matrix products (csrc/gemm_plan.h) as plain functions, for the tests.
+// The host arithmetic that cuts and schedules launches (csrc/gemm_plan.h, csrc/wkv7_overlap.h) as plain functions, for the tests.
 #include "gemm_plan.h"
+#include "wkv7_overlap.h"
 
 #include <chrono>
 
@@ -29,3 +30,5 @@ extern "C" int64_t plan_lm_head_ns(int64_t R, int64_t C, int64_t V, int num_sms,
     }
     return best;
 }
+
+extern "C" int plan_overlap(size_t chains, size_t nchunks, int num_sms) { return rwkv7::partition_overlap_pays(chains, nchunks, num_sms); }

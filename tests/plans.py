@@ -1,4 +1,4 @@
-"""The host-side cuts of the matrix products, compiled from the product's header and called through ctypes."""
+"""The host arithmetic that cuts and schedules launches, compiled from the product's headers and called through ctypes."""
 import ctypes
 import functools
 import os
@@ -11,13 +11,14 @@ ALL = 2**62   # a workspace with room for every split
 
 @functools.lru_cache(maxsize=None)
 def library():
-    out = os.path.join(tempfile.mkdtemp(), "gemm_plan.so")
+    out = os.path.join(tempfile.mkdtemp(), "plans.so")
     subprocess.check_call(["/usr/bin/g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-I", os.path.join(ROOT, "rwkv-rs-stable_b200", "csrc"),
-                           os.path.join(ROOT, "tests", "cpp", "gemm_plan.cpp"), "-o", out])
+                           os.path.join(ROOT, "tests", "cpp", "plans.cpp"), "-o", out])
     lib = ctypes.CDLL(out)
     lib.plan_lm_head.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int] + [ctypes.c_int64, ctypes.POINTER(ctypes.c_int64)]
     lib.plan_product.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int] + [ctypes.c_size_t, ctypes.POINTER(ctypes.c_int64)]
     lib.plan_lm_head_ns.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int] + [ctypes.c_int64]
+    lib.plan_overlap.argtypes = [ctypes.c_size_t, ctypes.c_size_t, ctypes.c_int]
     lib.plan_lm_head_ns.restype = ctypes.c_int64
     return lib
 
@@ -36,3 +37,7 @@ def product(M, N, K, num_sms=148, room=ALL):
     out = (ctypes.c_int64 * 2)()
     library().plan_product(M, N, K, num_sms, room, out)
     return dict(zip(("pieces", "pair_width"), out))
+
+
+def overlap(chains, nchunks, num_sms=148):
+    return bool(library().plan_overlap(chains, nchunks, num_sms))
