@@ -39,5 +39,14 @@ def product(M, N, K, num_sms=148, room=ALL):
     return dict(zip(("pieces", "pair_width"), out))
 
 
+def channel_mixer(M, C, F, num_sms=148):
+    """The two products of a call whose workspace is as large as the query says."""
+    room = 0
+    for N, K in ((F, C), (C, F)):
+        pieces = product(M, N, K, 160)["pieces"]
+        room = max(room, pieces * M * N * 4 if pieces > 1 else 0)
+    return product(M, F, C, num_sms, room), product(M, C, F, num_sms, room)
+
+
 def overlap(chains, nchunks, num_sms=148):
     return bool(library().plan_overlap(chains, nchunks, num_sms))
