@@ -11,6 +11,7 @@ import pytest
 import torch
 
 import parity
+import plans
 
 pytestmark = pytest.mark.gpu
 
@@ -205,7 +206,8 @@ def test_split_overlapped_scan_is_bitwise_the_serial_one(pkg, oracle, workloads,
     """Few chains and a long sequence: the call is cut into segments, and the scan of a segment runs beside the
     operator kernel of the next one, each on its own partition of the SMs.  Same kernels on the same data: the
     result must be bitwise that of the single-stream schedule, and both must match the oracle."""
-    B, T, H = 1, 16384, 3
+    B, T, H = 1, 16384, 20
+    assert plans.overlap(B * H, T // 64, torch.cuda.get_device_properties(cuda).multi_processor_count)
     inp = workloads.wkv7_inputs(B, T, H, 64, seed=81, dtype=torch.bfloat16, state="normal")
     y_ref, s_ref = _oracle(oracle, inp)
     before = pkg.kernel_launch_count()
