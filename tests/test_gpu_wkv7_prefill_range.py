@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("T,decay", [(64, "model"), (65, "edge"), (127, "model"), (333, "edge"), (511, "beyond"), (512, "edge"),
-                                     (577, "mixed")])
+                                     (577, "mixed"), (2047, "model"), (6000, "model")])
 def test_prefill_decay_range(pkg, oracle, workloads, cuda, T, decay):
     inp = workloads.wkv7_inputs(2, T, 3, 64, seed=61, dtype=torch.bfloat16, state="normal")
     g = torch.Generator().manual_seed(17)
