@@ -262,8 +262,8 @@ gemm_tn_bf16_pair_kernel(const __grid_constant__ PairMaps maps, __nv_bfloat16 *_
 template <int EPI>
 __global__ void __launch_bounds__(256)
 gemm_reduce_kernel(const float *__restrict__ parts, int splits, __nv_bfloat16 *__restrict__ out, int64_t quads) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    wait_for_previous();
+    let_next_in();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= quads) return;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);

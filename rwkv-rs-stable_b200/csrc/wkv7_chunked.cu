@@ -41,6 +41,7 @@
 #include <mutex>
 
 #include "kernels.h"
+#include "launch.h"
 #include "sm100_umma.cuh"
 
 namespace rwkv7 {
@@ -209,10 +210,10 @@ wkv7_chunked_kernel(const __grid_constant__ TmaMaps maps, const float *s0,
     if constexpr (K == 1 && !SAVE) {
         // Second in line after the two-kernel prefill: only the chains that one left flagged are computed.
         if (only_flagged) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");   // (may have been launched before the flags' writer finished)
+            wait_for_previous();   // (may have been launched before the flags' writer finished)
             // (All CTAs of this pass have their places by then, so the sequential pass behind it can take what is left and wait there:
             // 99.5 -> 98.3 us at 3 x 2047 tokens x 32 heads.)
-            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+            let_next_in();
             if (flags[chain0 + blockIdx.x] == 0) return;
         }
     }

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.h"
+#include "launch.h"
 
 namespace rwkv7 {
 namespace {
@@ -62,7 +63,7 @@ wkv7_decode_kernel(DecPtrs ptrs, const float *s0, T *__restrict__ y, float *s_ou
     // Launched with programmatic stream serialization: this grid's CTAs may take their places while the kernel
     // before it on the stream (typically the previous layer's sweep) is still draining; nothing is read before
     // that kernel has completed.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    wait_for_previous();
     float4 S[R][Q];
     if (s0 != nullptr) {
 #pragma unroll
@@ -79,7 +80,7 @@ wkv7_decode_kernel(DecPtrs ptrs, const float *s0, T *__restrict__ y, float *s_ou
     }
 
     // (this CTA's state loads are under way: the next kernel on the stream may start taking places)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    let_next_in();
     for (int t = 0; t < Tlen; ++t) {
         const size_t o = (((size_t)bi * Tlen + t) * H + h) * kN;
         if (t > 0) __syncthreads();  // previous token's vectors fully consumed
@@ -152,24 +153,11 @@ wkv7_decode_kernel(DecPtrs ptrs, const float *s0, T *__restrict__ y, float *s_ou
 
 int launch_wkv7_decode(const Wkv7Args &p, cudaStream_t stream) {
     DecPtrs ptrs{{p.r, p.w, p.k, p.v, p.a, p.b}};
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(p.B * p.H));
-    cfg.blockDim = dim3(128);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaError_t e;
-    if (p.bf16)
-        e = cudaLaunchKernelEx(&cfg, wkv7_decode_kernel<__nv_bfloat16, RWKV7_DECODE_ROWS>, ptrs, p.s0,
-                               reinterpret_cast<__nv_bfloat16 *>(p.y), p.s_out, (int)p.T, (int)p.H);
-    else
-        e = cudaLaunchKernelEx(&cfg, wkv7_decode_kernel<float, RWKV7_DECODE_ROWS>, ptrs, p.s0, reinterpret_cast<float *>(p.y),
-                               p.s_out, (int)p.T, (int)p.H);
-    if (e == cudaSuccess) count_launch();
-    return (int)e;
+    auto go = [&](auto kernel, auto *y) {
+        return (int)launch_serialized(kernel, (unsigned)(p.B * p.H), 128u, 0, stream, ptrs, p.s0, y, p.s_out, (int)p.T, (int)p.H);
+    };
+    if (p.bf16) return go(wkv7_decode_kernel<__nv_bfloat16, RWKV7_DECODE_ROWS>, reinterpret_cast<__nv_bfloat16 *>(p.y));
+    return go(wkv7_decode_kernel<float, RWKV7_DECODE_ROWS>, reinterpret_cast<float *>(p.y));
 }
 
 }  // namespace rwkv7

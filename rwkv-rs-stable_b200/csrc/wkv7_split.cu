@@ -691,7 +691,7 @@ wkv7_chunk_operator_kernel(const __grid_constant__ OperatorMaps maps, OperatorPt
         __syncthreads();
         if (kTma && tid == 0 && more) request(unit + gridDim.x);
         // (the last chunk of this CTA: the scan may be set up)
-        if (!more) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (!more) let_next_in();
     }
     if (tid == 0 && *abort_flag) {
         if (kTma) {   // what is in flight lands before the CTA leaves
@@ -1034,8 +1034,8 @@ wkv7_state_scan_kernel(const __grid_constant__ ScanMaps maps, OperatorPtrs ptrs,
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     // (launched behind the operator kernel with programmatic stream serialization: everything below reads what it wrote)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    wait_for_previous();
+    let_next_in();
     const float *s_in = state_in ? state_in + (size_t)chain * kN * kN : nullptr;
     float *s_out = state_out ? state_out + (size_t)chain * kN * kN : nullptr;
     const unsigned char *rec = records + (size_t)chain * n * kRecord;
@@ -1865,21 +1865,9 @@ int launch_training_scan(const ScanMaps &maps, const OperatorPtrs &ptrs, const v
     auto kern = wkv7_state_scan_kernel<bf, kKind>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Scan<bf>::kBytes);
     if (e != cudaSuccess) return (int)e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)l.chains);
-    cfg.blockDim = dim3((unsigned)kScanThreads);
-    cfg.dynamicSmemBytes = Scan<bf>::kBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kern, maps, ptrs, static_cast<const bf *>(in), records, s_in, s_out, static_cast<bf *>(out), states,
-                           reinterpret_cast<uint32_t *>(states + l.chains * l.nchunks * kN * kN), flags,
-                           (int)T, (int)H, 0, (int)l.nchunks, 1, status);
-    if (e == cudaSuccess) count_launch();
-    return (int)e;
+    return (int)launch_serialized(kern, (unsigned)l.chains, (unsigned)kScanThreads, Scan<bf>::kBytes, stream, maps, ptrs, static_cast<const bf *>(in), records, s_in,
+                                  s_out, static_cast<bf *>(out), states, reinterpret_cast<uint32_t *>(states + l.chains * l.nchunks * kN * kN), flags, (int)T,
+                                  (int)H, 0, (int)l.nchunks, 1, status);
 }
 
 }  // namespace

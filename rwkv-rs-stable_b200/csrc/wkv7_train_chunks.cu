@@ -30,6 +30,7 @@
 #include <cstdint>
 
 #include "kernels.h"
+#include "launch.h"
 #include "sm100_mma.cuh"
 #include "sm100_umma.cuh"
 #include "trace.h"
@@ -305,10 +306,10 @@ wkv7_chunk_gradients_kernel(const __grid_constant__ ChunkMaps maps, const __grid
         for (int i = 0; i < kTensors; ++i) tma_load_2d(smem + buf * kTilesBytes + i * kPanel, &maps.in[i], x, y, bar + buf);
     };
     __syncthreads();
+    // (the call's inputs are requested while the gradient scan in front, which writes none of them, finishes: see launch.h)
     if (warp == 7 && elect_one() && (int)blockIdx.x < p.units) request(blockIdx.x, 0);
     __syncwarp();
-    // (launched behind the gradient scan with programmatic stream serialization)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    wait_for_previous();
     // this warp's 16 rows of S or G, in accumulator order: c[n] = rows g, g + 8, columns 8 n + c2, + 1
     const int wr = warp & 3;
     const bool g_side = warp >= 4;
@@ -831,19 +832,8 @@ int launch_wkv7_chunk_gradients(const Wkv7TrainingBackwardArgs &p, const unsigne
     if (int e = device_status_ptr(p.device, &args.status)) return e;
     cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_gradients_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return (int)e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(args.units < p.num_sms ? args.units : p.num_sms));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, wkv7_chunk_gradients_kernel, maps, args);
-    if (e == cudaSuccess) count_launch();
-    return (int)e;
+    return (int)launch_serialized(wkv7_chunk_gradients_kernel, (unsigned)(args.units < p.num_sms ? args.units : p.num_sms), (unsigned)kThreads, kSmem, stream,
+                                  maps, args);
 }
 
 }  // namespace rwkv7
