@@ -1,11 +1,12 @@
 // Token-shift mixing kernels: mix6, addcmul / addcmul5, token_shift_diff.
 //
-// All three are pure streaming kernels bound by HBM bandwidth.  A CTA owns a
-// block of consecutive token rows; a thread owns one 16-byte channel vector of
-// every row in the block, keeps the per-channel scales in registers for the
-// whole block and carries the previous row in registers, so each input element
-// is read from memory once (plus one halo row per block) and every access is a
-// coalesced 128-bit load or store.  Arithmetic is fp32, rounded once on store.
+// All three are pure streaming kernels bound by HBM bandwidth.  A thread owns one
+// 16-byte channel vector of every row it takes and keeps the per-channel scales in
+// registers; every access is a coalesced 128-bit load or store.  A CTA of addcmul and
+// token_shift_diff owns consecutive token rows, and the latter carries the previous
+// row in registers (one halo row per CTA is read again).  mix6 moves the whole grid
+// over the tensor as a window of neighbouring rows and reads the row in front from
+// L2.  Arithmetic is fp32, rounded once on store.
 //
 // Reference semantics (paths inside the rwkv-rs repository):
 //   mix6              crates/rwkv-nn/src/kernels/train/time_mixer/mix6/kernel.rs:25-57
@@ -84,7 +85,7 @@ struct Pack {
     }
 };
 
-// A vector as it lies in memory: bf16 scales take half the registers so, and twice the CTAs fit.
+// A vector as it lies in memory: bf16 scales take half the registers so, which leaves room for the rows on their way (124 registers, two CTAs an SM).
 template <typename T, int EPV>
 struct Raw {
     Pack<T, EPV> v;

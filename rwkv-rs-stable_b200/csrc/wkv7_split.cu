@@ -73,9 +73,9 @@ __host__ __device__ constexpr int tri(int t) { return t * (t + 1) / 2; }
 // ------------------------------------------------------------------------------------------
 // Kernel 1: the operator of every chunk.  One CTA of four warps per chunk at a time, four CTAs per SM.
 //
-// Bound by shared-memory bandwidth (2.8 k cycles per chunk at one 128-byte access a cycle) and by the latency of a chunk's
-// phases, which the CTAs of an SM cover for one another; hence few warps per chunk, each with the largest tile its
-// registers hold (eight warps per chunk read a quarter more and were slower: 153 against 121 us).  Measured, 6144 chunks (8 x
+// Bound by the latency of a chunk's phases, which the four CTAs of an SM cover for one another in part: no unit is saturated (shared-memory
+// port 63 %, issue slots 50 %, DRAM 65 %).  What a phase reads from shared memory is its length; hence few warps per chunk, each with
+// the largest tile its registers hold (eight warps per chunk read a quarter more and were slower: 153 against 121 us).  Measured, 6144 chunks (8 x
 // 4096 tokens x 12 heads): 107.4 us, 4.2 TB/s; the form on six tcgen05 products per chunk that this replaced took 170.  Per chunk:
 //   1. decays: warp = 16-token block, lane = channel pair; prefix and suffix products within the block
 //   2. scaled fp16 operands, in place over the bf16 tiles that TMA delivered
