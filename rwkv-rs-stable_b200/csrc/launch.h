@@ -1,6 +1,7 @@
 // Launches with programmatic stream serialization: a kernel's CTAs take their places while the one before it on the stream drains.
 // Every kernel launched so waits (`wait_for_previous`) before it reads or writes anything that others may have written or
-// may still read; its own successor is let in from `let_next_in` on, and waits in turn until this kernel is complete.
+// may still read; its own successor is let in from `let_next_in` on, and waits in turn until this kernel is complete.  A kernel without
+// `let_next_in` has it in as its CTAs leave.
 //
 // Two kernels read before they wait: the products of the channel mixer request tiles of the weights, the chunk gradients of the training step
 // tiles of the sequence and the output's gradient.  That is sound only behind a kernel of the same call that writes none of it and itself

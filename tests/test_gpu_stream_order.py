@@ -131,16 +131,15 @@ def test_inputs_written_right_in_front_in_a_graph(pkg, workloads, cuda, name):
 
 @pytest.mark.parametrize("rows", [16, 300, 3000])
 def test_weights_from_a_kernel_that_lets_the_next_one_in_early(pkg, workloads, cuda, rows):
-    """addcmul lets its successor start when it has begun to write the weights itself."""
+    """mix6 lets its successor start before it has written the weights."""
     x, scale, kw, vw = workloads.channel_mixer_inputs(1, rows, 768, 3072, seed=3, device="cuda")
     h, w, targets = workloads.lm_head_inputs(rows, 768, 4100, seed=4, device="cuda")
     g = torch.Generator(device="cuda")
     g.manual_seed(5)
-    step = {n: (0.1 * torch.randn((1, *t.shape), generator=g, device="cuda")).to(bf16) for n, t in (("kw", kw), ("vw", vw), ("w", w))}
-    rates = {n: torch.rand((1, 1, t.shape[-1]), generator=g, device="cuda").to(bf16) for n, t in step.items()}
+    rates = {n: [torch.rand((1, 1, t.shape[-1]), generator=g, device="cuda").to(bf16) for _ in range(6)] for n, t in (("kw", kw), ("vw", vw), ("w", w))}
 
     def updated(name, weight):
-        return pkg.addcmul(weight[None], step[name], rates[name])[0]
+        return pkg.mix6(weight[None], *rates[name])["learning_rate_input"][0]
 
     def calls(pause):
         out = []
